@@ -374,7 +374,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc(p.NT);
       uint32_t tcount = 0, sa = 0, pa = 0, sb = 0, pb = 0, itm = 0;
       // The commit of a stage is issued after the FIRST MMA of the next one: its 65 cycles then pass
@@ -481,7 +481,9 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
       const unsigned short* sc = reinterpret_cast<const unsigned short*>(p.scales) + (size_t)row * row_groups;
       const unsigned short* bi = reinterpret_cast<const unsigned short*>(p.biases) + (size_t)row * row_groups;
       cur_chunk = -1;
-      for (int ks = dset; ks < kstages; ks += 2) {
+      // The sets alternate over the stage counter, not over ks: with an odd number of stages per tile a
+      // set would otherwise take two stages in a row and could pass the other set in the packed ring.
+      for (int ks = (int)((dset ^ (tcount * (uint32_t)kstages)) & 1u); ks < kstages; ks += 2) {
         const uint32_t it = tcount * (uint32_t)kstages + (uint32_t)ks;
         const uint32_t sa = it % kStagesA;
         const uint32_t sp = it % kStagesP, pp = (it / kStagesP) & 1u;

@@ -15,6 +15,14 @@ constexpr uint32_t kSpinLimit = 1u << 21;
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
+// True in exactly one lane of a converged warp.  Code under this predicate, unlike code under
+// "lane == 0", is compiled for the uniform data path: a tcgen05.mma then costs its issuing thread a few
+// cycles instead of about 85 for moving its descriptors into uniform registers one by one.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
+}
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
