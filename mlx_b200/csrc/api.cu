@@ -4,7 +4,8 @@
 // mlx/backend/cuda/quantized/quantized.cpp:106-136):
 //   bf16, transpose, M <= 16, bits 2/4/8, K % (16 * group) == 0 -> qmv_rows    (HBM-bound decode)
 //   bf16, transpose, M <= 16, K % 128 == 0 (any width)           -> qmv_mma     (register-path decode)
-//   bf16, transpose, M  > 16, K % 128 == 0, N % 8 == 0           -> qmm_tcgen05 (TMA + tcgen05 + TMEM)
+//   bf16, f16, transpose, K % 128 == 0                           -> qmm_tcgen05 (TMA + tcgen05 + TMEM)
+//   bf16, f16, transpose == 0, M > 16, N % 128 == 0              -> qmm_tcgen05 (fewer rows waste half of the 32-token tile)
 //   transpose == 0, M <= 4, bits 2/4/8                           -> qvm
 //   everything else                                              -> qmm_generic
 #include <cstdlib>
@@ -79,7 +80,7 @@ Path choose(const QmmArgs& a) {
   if (force_tc() && qmm_tc_supported(a)) return Path::Tc;  // tuning aid: tensor-memory path for any M
   if (ov == 0 && qmv_rows_supported(a)) return Path::QmvRows;
   if (qmv_mma_supported(a)) return Path::Qmv;
-  if (qmm_tc_supported(a)) return Path::Tc;
+  if (qmm_tc_supported(a) && (a.transpose || a.M > 16)) return Path::Tc;
   if (qvm_supported(a)) return Path::Qvm;
   return Path::Generic;
 }

@@ -99,8 +99,8 @@ size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 int pick_nt(int64_t n_rows, int64_t E) {
   const double avg = (double)n_rows / (double)(E > 0 ? E : 1);
   int64_t nt = (int64_t)(avg + 3.0 * sqrt(avg) + 8.0);
-  nt = (nt + 15) / 16 * 16;
-  return (int)(nt < 16 ? 16 : (nt > 256 ? 256 : nt));
+  nt = (nt + 31) / 32 * 32;
+  return (int)(nt > 256 ? 256 : nt);
 }
 
 struct FastLayout {

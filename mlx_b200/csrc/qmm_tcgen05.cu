@@ -1,46 +1,58 @@
-// Prefill path: y[M, N] = x[M, K] * dequant(W[N, K])^T on the 5th-generation tensor cores.
+// Products with many token rows on the 5th-generation tensor cores:
+//   y[M, N] = x[M, K] * dequant(W[N, K])^T      (transpose)
+//   y[M, N] = x[M, K] * dequant(W[K, N])        (no transpose: the gradient of the first with respect to x)
 //
 // Replaces cu::qmm_sm80_kernel / qmm_naive_kernel of the reference
 // (mlx/backend/cuda/device/qmm_sm80.cuh:70-356, quantized/qmm/qmm.cu:20-185), which run
 // Ampere-style mma.sync code on this GPU.
 //
-// Formulation (swap-AB): the MMA computes D[128 weight rows, NT tokens] so that the
-// operand that has to be dequantised (W) is the 128-row A operand and is re-used by up
-// to 256 tokens per instruction, and the operand that streams unchanged (x) is B.
+// Formulation (swap-AB): D[256 output columns, NT tokens], so that the operand that has to be
+// dequantised (W) is the A operand and is re-used by up to 256 tokens per instruction, and the operand
+// that streams unchanged (x) is B.  A tile belongs to a PAIR of thread blocks (a cluster of two,
+// tcgen05 cta_group::2): each block unpacks and accumulates 128 of the 256 output columns and holds half
+// of the tokens.  At 256 tokens a stage of 128 k takes 1024 cycles on the tensor pipe; one block alone
+// would have to fetch 64 KB of x in that time, the SM's whole L2 bandwidth (64 bytes per clock), and was
+// bound by it.  A pair fetches every x tile once: 32 bytes per clock and SM.
 //
-//   thread A: TMA  --packed W tile [128 rows x 128 k, 16*bits bytes per row]-->  smem ring P
-//   16 dequant warps (4 TMEM lane quadrants x 4 quarters of the 128-k stage): one thread per
-//        weight row (= one TMEM lane) unpacks 32 k, applies s*q+b in bf16x2 (4- and 8-bit:
-//        mask + one fma on the field read as a subnormal bf16; other widths shift/lop3/prmt),
-//        tcgen05.st into the A ring in TMEM; scales and biases come as 16-byte chunks per row
-//   thread B: TMA  --two x sub-tiles [NT tokens x 64 k], 128B-swizzled K-major-->  smem ring B
-//   1 thread: tcgen05.mma.kind::f16 (A from TMEM, B from smem descriptors), fp32
-//        accumulator [128 lanes x NT columns] in TMEM, tcgen05.commit on mbarriers
-//   8 epilogue warps (two per TMEM lane quadrant, half of the token columns each):
-//        tcgen05.ld the accumulator, round to bf16, store y (transposed; scattered through
-//        a row table in grouped mode)
+//   warp 0: TMA  --two x sub-tiles [NT/2 tokens x 64 k], 128B-swizzled K-major-->  smem ring B
+//   warp 1: tcgen05.mma.cta_group::2.kind::f16 (leader block only; one elected thread: under
+//        elect.sync an MMA issues at its own rate, N/2 cycles, under "lane == 0" it cost 85)
+//   warp 2: TMA  --packed W tile [128 rows x 16*bits bytes]-->  smem ring P (swizzled where the row is
+//        32, 64 or 128 bytes: the unpack threads' 16-byte reads are then free of bank conflicts)
+//   warp 3: cp.async --scales and biases of the same tile--> smem ring S.  A value of each is needed per row
+//        and group, from as many cache lines as rows: one warp fetches every value once per block
+//        where sixteen unpack warps fetched it four times.
+//   warps 4-19: unpack W into the A operand, in sets that take A slots in turn: a warp's trip through a
+//        slot is a chain of dependent latencies, and four sets (two for SplitT) give each trip as many
+//        slot times
+//   warps 20-27: tcgen05.ld the accumulator, round, store y (scattered through a row table in grouped
+//        mode); with at most 128 tokens per tile there are two accumulators and the store of one tile
+//        runs under the next
 //
-// The two TMA streams have a thread each: behind the x-tile waits the packed tiles would
-// arrive late and starve the dequant warps.
+// How W becomes the A operand (Form):
+//   Round   bf16, transpose: s*q+b rounded once to bf16 (one fma.rn.bf16x2 per pair), in tensor memory
+//   Split   f16, transpose: s*q+b in fp32, split into two f16 numbers hi + lo, two MMAs per k step: the
+//           product keeps the weights' fp32 value (to 2^-22), as the CUDA-core kernel did
+//   SplitT  no transpose, bf16 and f16: W is packed along the output columns, so A is written to shared
+//           memory M-major (hi and lo)
+//
+// Few tiles (a short batch through a narrow matrix): K is split over pairs so that all SMs have
+// work; every pair leaves fp32 partial sums in the workspace and the last one to arrive adds them in
+// order.  No block ever waits for another pair.
 //
 // Grouped mode (gather_qmm): a device-side table lists (expert, first row, valid rows) for
-// every NT-row slice of the expert-sorted activations; the weight tensor map spans the
+// every slice of up to NT rows of the expert-sorted activations; the weight tensor map spans the
 // stacked experts [E*N, K*bits/8].
 //
-// TMEM columns (512 allocated): [0, 256) accumulator, [256, 512) A ring of 4 stages
-// (128 k of bf16 = 64 columns each).  One CTA per SM (persistent), tiles are taken
-// round-robin; no CTA ever waits on another CTA.
+// The token width of a tile is rounded up to 32, not to NT: ragged token counts and experts with few rows
+// pay for what they have.
 //
-// A pipeline stage is 128 k: the MMA-issuing thread is blocked while the tensor pipe is busy
-// (the queue behind tcgen05.mma is about one instruction deep; an M=128, K=16 instruction
-// takes 128 cycles at N=256 and no less than about 100 at any smaller N) and pays about 65
-// cycles for every tcgen05.commit, so every wait and commit per stage is time the tensor pipe
-// idles: eight MMAs per pair of commits instead of four.
-//
-// Every mbarrier wait is bounded.  When a wait expires the role sets the CTA abort
+// Every mbarrier wait is bounded.  When a wait expires the role sets the block's abort
 // flag and the device status word, all roles leave their loops, TMEM is released and
 // the kernel ends normally (its results are then invalid and the host reports it).
 #include <cuda.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -49,63 +61,65 @@
 namespace b200q {
 namespace {
 
-constexpr int kTileN = 128;       // weight rows per tile (MMA M)
-constexpr int kBlockK = 64;       // k per x sub-tile (one 128-byte swizzle row of bf16)
-constexpr int kStageK = 128;      // k per pipeline stage: two x sub-tiles, one packed tile, 8 MMAs
-constexpr int kStagesA = 4;       // A ring in TMEM (64 columns each)
-constexpr int kMaxStagesB = 6;    // x stages in shared memory: as many as fit (3 at 256 tokens)
-constexpr int kMaxStagesP = 4;    // packed W tiles in shared memory
-// Packed stages: 16 * bits bytes per row and stage; next to three 64 KB x stages 35 KB remain.
-__host__ __device__ constexpr int stages_p(int bits) { return bits <= 4 ? 4 : (bits == 5 ? 3 : 2); }
-constexpr size_t kSmemMax = 227 * 1024;
-constexpr int kDoneRing = 12;
-constexpr int kAccCols = 256;
-constexpr int kTmemCols = 512;
-constexpr int kDequantWarps = 16;   // two sets of 8: 4 TMEM lane quadrants x 2 halves (64 k) of a stage
-constexpr int kDequantSet = 8;      // set 0 unpacks the even stages of a tile, set 1 the odd ones
-constexpr int kEpilogueWarps = 8;   // two per TMEM lane quadrant, each drains half of the columns
-constexpr int kProducerPWarp = 2 + kDequantWarps + kEpilogueWarps;  // last warp
-constexpr int kThreads = 32 * (3 + kDequantWarps + kEpilogueWarps);  // 864
-
 using namespace tc;
 
-// Waits of the three single-thread roles.
-#ifndef B200Q_TC_PARK
-#define TC_WAIT1 mbar_wait_spin
-#else
-#define TC_WAIT1 mbar_wait
-#endif
-// Waits of the dequant warps.
-#ifdef B200Q_TC_DQ_SPIN
-#define TC_WAIT16 mbar_wait_spin
-#else
-#define TC_WAIT16 mbar_wait
-#endif
+enum class Form { Round, Split, SplitT };
 
-// Shared-memory matrix descriptor of a K-major, 128-byte-swizzled operand tile whose
-// rows are 128 bytes (64 bf16): 8-row groups are 1024 bytes apart (SBO), descriptor
-// version 1 (sm_100), layout type 2 = SWIZZLE_128B.  `addr` may point 32*j bytes into
-// the first row to select the j-th 16-element K slice.
-__device__ __forceinline__ uint64_t make_sw128_desc(uint32_t addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFF) >> 4);        // start address  [0,14)
-  d |= (uint64_t)1 << 16;                        // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;              // stride byte offset [32,46)
-  d |= (uint64_t)1 << 46;                        // descriptor version
-  d |= (uint64_t)2 << 61;                        // SWIZZLE_128B
-  return d;
+constexpr int kTileRows = 128;    // output columns per block and tile (MMA M = 256 over the pair)
+constexpr int kStageK = 128;      // k per pipeline stage of x, W, scales
+constexpr int kMaxStagesB = 6;
+constexpr int kMaxStagesP = 4;
+constexpr int kMaxSlotsA = 4;
+constexpr int kSlotsS = 4;        // chunks of scales and biases
+constexpr int kDoneRing = 16;     // one commit per A slot; longer than any distance a waiter can be behind
+constexpr int kTmemCols = 512;    // [0, 256) accumulators, [256, 512) A ring (4 slots of 64 columns)
+constexpr int kAccCols = 256;
+constexpr int kUnpackWarps = 16;
+constexpr int kEpilogueWarps = 8;
+constexpr int kFirstUnpack = 4, kFirstEpilogue = kFirstUnpack + kUnpackWarps;
+constexpr int kThreads = 32 * (kFirstEpilogue + kEpilogueWarps);   // 896
+constexpr size_t kSmemMax = 227 * 1024;
+
+template <int BITS, Form F>
+struct Shape {
+  static constexpr bool kT = F == Form::SplitT;
+  static constexpr int kSub = F == Form::Round ? 1 : 2;        // A slots per stage (64 k each when split)
+  static constexpr int kSlotsA = kT ? 3 : 4;
+  static constexpr int kSets = kT ? 2 : 4;                     // sets of unpack warps, on A slots in turn
+  static constexpr int kStagesP = !kT ? 4 : (BITS <= 4 ? 3 : 2);
+  static constexpr int kPRowBytes = 16 * BITS;                 // 128 fields
+  static constexpr int kPStageBytes = kTileRows * kPRowBytes;
+  static constexpr int kSmemA = kT ? kSlotsA * 32768 : 0;      // 64 k x 128 columns, hi and lo
+  static constexpr int kPArrivals = kSub * kUnpackWarps / kSets;   // of a packed stage: every set that takes one of its slots
+};
+
+// Shared-memory matrix descriptor of a 128-byte-swizzled operand tile, descriptor version 1 (sm_100).
+// K-major (x): rows of 64 k, 8-row groups 1024 bytes apart (sbo); `addr` may point 32*j bytes into the
+// first row to select the j-th 16-element K slice.  M-major (A of SplitT): rows of 64 columns, one per k,
+// 8-k groups `sbo` apart, 64-column blocks `lbo` apart.
+__device__ __forceinline__ uint64_t sw128_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+  return (uint64_t)((addr & 0x3FFFF) >> 4) | (uint64_t)(lbo >> 4) << 16 | (uint64_t)(sbo >> 4) << 32 | (uint64_t)1 << 46 |
+         (uint64_t)2 << 61;
 }
-// Instruction descriptor: D f32, A/B bf16, both K-major, M = 128, N = n.
+// Instruction descriptor: D f32, A and B of the same 16-bit type, B K-major, M = 256, N = n.
+template <typename T, Form F>
 __device__ __forceinline__ uint32_t make_idesc(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTileN >> 4) << 24);
+  constexpr uint32_t fmt = sizeof(T) == 2 && std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+  return (1u << 4) | (fmt << 7) | (fmt << 10) | (F == Form::SplitT ? 1u << 15 : 0u) | ((uint32_t)(n >> 3) << 17) |
+         ((uint32_t)(2 * kTileRows >> 4) << 24);
 }
 
-// One entry per group of NT consecutive rows of the (expert-sorted) activation matrix.
+// One entry per group of up to NT consecutive rows of the (expert-sorted) activation matrix.
 struct MTile {
   int expert;     // weight matrix the rows multiply
   int row0;       // first row in the activation matrix
-  int rows;       // valid rows (<= NT): the rest of the TMA box belongs to another expert
+  int rows;       // valid rows: what follows in the TMA box belongs to another expert
   int pad;
+};
+
+struct TcMaps {
+  CUtensorMap x[4];   // boxes of 128, 64, 32 and 16 tokens x 64 k
+  CUtensorMap w;
 };
 
 struct TcParams {
@@ -113,35 +127,121 @@ struct TcParams {
   const MTile* mtiles;
   const int* n_mtiles;      // device scalar: entries of `mtiles`
   const int* dst_row;       // output row of every activation row
-  const __nv_bfloat16* scales;
-  const __nv_bfloat16* biases;
-  __nv_bfloat16* y;
-  // plain mode: output buffers (one, or one per GPU of an N-sharded layer), row pitch and first column
-  __nv_bfloat16* y_out[kMaxPeers];
+  const unsigned short* scales;
+  const unsigned short* biases;
+  // output buffers (one, or one per GPU of an N-sharded layer), row pitch and first column
+  void* y_out[kMaxPeers];
   int n_out;
   long long ld, col0;
   PeerSignal sig;    // completion signal towards the ranks that receive y (n == 0: none)
   uint32_t* status;
   int M, N, K;
-  int NT;            // tokens per tile (multiple of 16, <= 256)
+  int NT;            // most tokens per tile (multiple of 32, <= 256)
   int nsb;           // x stages in shared memory (2 .. kMaxStagesB)
   int n_tiles, m_tiles;
-  int group_shift;   // log2(group / 32)
+  int splits;        // parts of K (1 unless a tile is shared by several pairs)
+  float* partial;    // [tile][split][block of the pair][NT tokens][128 columns], splits > 1 only
+  uint32_t* counters;   // [tile][block of the pair]
+  int g4;            // groups per 128 fields of a row: 4, 2, 1
+  int row_groups;    // groups per packed row
+  int spc, cb;       // stages per chunk of scales, bytes per row of a chunk (4, 8 or 16)
+  long long n_scales;   // elements of `scales`
 };
 
 struct __align__(8) Barriers {
   uint64_t full_p[kMaxStagesP], empty_p[kMaxStagesP];
+  uint64_t full_s[kSlotsS], empty_s[kSlotsS];
+  // Of the pair's leader: x tiles of both blocks have landed; both blocks' unpack warps have filled an A slot
   uint64_t full_b[kMaxStagesB];
-  uint64_t full_a[kStagesA];
-  // One commit per stage: stage `it` (counted across tiles) arrives on done[it % kDoneRing] when its
-  // MMAs have completed.  The A slot it % 4 and the x slot it % nsb are free again from then on: the
-  // unpack warps and the x producer look at the entry of the stage that used their slot last.  The
-  // ring length is a common multiple of both slot counts (nsb is 2, 3, 4 or 6).
+  uint64_t full_a[kMaxSlotsA];
+  // One commit per A slot, to both blocks: slot use `ia` (counted across tiles) arrives on
+  // done[ia % kDoneRing] when its MMAs have completed.  Whatever it read (A slot, with the last slot
+  // of a stage the x stage too) is free again from then on.
   uint64_t done[kDoneRing];
-  uint64_t acc_full, acc_empty;
+  uint64_t acc_full[2], acc_empty[2];
   uint32_t tmem_base;
-  int abort_flag;
+  int abort_flag, last;
 };
+
+// ------------------------------------------------------------------------------------ unpacking
+__device__ __forceinline__ uint32_t lds_u16(uint32_t at) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(at));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds_u32(uint32_t at) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(at));
+  return v;
+}
+__device__ __forceinline__ void lds_v2(uint32_t at, uint32_t& a, uint32_t& b) {
+  asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(a), "=r"(b) : "r"(at));
+}
+__device__ __forceinline__ void lds_v4(uint32_t at, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+  asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(at));
+}
+// The 32 fields of unit u (0..3) of row r of a packed tile: BITS words.
+template <int BITS>
+__device__ __forceinline__ void load_fields(uint32_t tile, int r, int u, uint32_t (&w)[BITS]) {
+  if constexpr (BITS == 2) {          // 32-byte swizzle
+    lds_v2(tile + r * 32 + ((((u >> 1) ^ (r >> 2)) & 1) << 4) + (u & 1) * 8, w[0], w[1]);
+  } else if constexpr (BITS == 4) {   // 64-byte swizzle
+    lds_v4(tile + r * 64 + (((u ^ (r >> 1)) & 3) << 4), w[0], w[1], w[2], w[3]);
+  } else if constexpr (BITS == 8) {   // 128-byte swizzle
+    lds_v4(tile + r * 128 + (((2 * u) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+    lds_v4(tile + r * 128 + (((2 * u + 1) ^ (r & 7)) << 4), w[4], w[5], w[6], w[7]);
+  } else if constexpr (BITS == 6) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) lds_v2(tile + r * 96 + u * 24 + 8 * i, w[2 * i], w[2 * i + 1]);
+  } else {                            // 3 and 5 words: an odd unit starts on an odd word
+    const uint32_t at = tile + r * (16 * BITS) + u * (4 * BITS);
+    if (u & 1) {
+      w[0] = lds_u32(at);
+#pragma unroll
+      for (int i = 1; i < BITS; i += 2) lds_v2(at + 4 * i, w[i], w[i + 1]);
+    } else {
+#pragma unroll
+      for (int i = 0; i + 1 < BITS; i += 2) lds_v2(at + 4 * i, w[i], w[i + 1]);
+      w[BITS - 1] = lds_u32(at + 4 * (BITS - 1));
+    }
+  }
+}
+
+// Field e of a BITS-word chunk, not yet masked.
+template <int BITS>
+__device__ __forceinline__ uint32_t field_raw(const uint32_t (&w)[BITS], int e) {
+  const int wi = (e * BITS) >> 5, sh = (e * BITS) & 31;
+  return sh + BITS > 32 ? __funnelshift_r(w[wi], w[(wi + 1) % BITS], sh) : (w[wi] >> sh);
+}
+
+// s*q+b of 32 consecutive fields in fp32, split into hi + lo numbers of T (16 registers of pairs each, in
+// order).  bf16: hi is the value cut off after 8 bits, lo the rounded rest; f16: both rounded.
+template <int BITS, typename T>
+__device__ __forceinline__ void split32(const uint32_t (&w)[BITS], float s, float b, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
+  constexpr uint32_t mask = (1u << BITS) - 1u;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    float v[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int e = 2 * j + h;
+      uint32_t f;   // 0x4B0000qq is 2^23 + q exactly
+      if constexpr (BITS == 8) f = __byte_perm(w[e >> 2], 0x4B000000u, 0x7540 | (e & 3));
+      else f = lop3_and_or(field_raw<BITS>(w, e), mask, 0x4B000000u);
+      v[h] = fmaf(__uint_as_float(f) - 8388608.0f, s, b);
+    }
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      hi[j] = __byte_perm(__float_as_uint(v[0]), __float_as_uint(v[1]), 0x7632);
+      const float l0 = v[0] - __uint_as_float(__float_as_uint(v[0]) & 0xFFFF0000u);
+      const float l1 = v[1] - __uint_as_float(__float_as_uint(v[1]) & 0xFFFF0000u);
+      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo[j]) : "f"(l1), "f"(l0));
+    } else {
+      asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(hi[j]) : "f"(v[1]), "f"(v[0]));
+      const float2 h2 = __half22float2(*reinterpret_cast<const __half2*>(&hi[j]));
+      asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(lo[j]) : "f"(v[1] - h2.y), "f"(v[0] - h2.x));
+    }
+  }
+}
 
 // Unpacks 32 consecutive BITS-wide fields (BITS words, LSB-first bit stream) of one row into
 // 16 bf16x2 registers in natural k order, applying w = s*q + b (one rounding).  s and b are
@@ -159,7 +259,7 @@ __device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_
   // to stay finite and normal: biased exponent of s in [1, 121]; other scales (zero, subnormal,
   // |s| >= 2^-6 * 2, inf, nan) take the general form below.
   const uint32_t s_exp = (s_bits >> 7) & 0xFFu;
-  const bool fast = s_exp >= 1u && s_exp <= 121u;
+  const bool fast = __all_sync(0xFFFFFFFFu, s_exp >= 1u && s_exp <= 121u);   // one branch per warp: a predicated mixture would run both forms
   if constexpr (BITS == 4) {
     if (fast) {
       const uint32_t sl = (s_bits + (133u << 7)) * 0x00010001u, sh = (s_bits + (129u << 7)) * 0x00010001u;
@@ -233,83 +333,116 @@ __device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_
   }
 }
 
-struct TileCoord {
-  int w_row0;   // first row of the tile in the stacked weight tensor [E*N, ...]
-  int w_rows_end;  // one past the last valid stacked row of this expert
-  int n0;       // first output column
-  int x_row0;   // first activation row
-  int rows;     // valid activation rows
+
+template <typename T>
+__device__ __forceinline__ float bits_to_float(uint32_t v) {
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) return __uint_as_float(v << 16);
+  else return __half2float(__ushort_as_half((unsigned short)v));
+}
+// N bytes, of which the first `n` are read and the rest are zeros.
+template <int N>
+__device__ __forceinline__ void cp_async(uint32_t dst, const void* src, int n) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(N), "r"(n) : "memory");
+}
+__device__ __forceinline__ void st_shared_v4(uint32_t at, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// One unit of work of a pair: a tile, or one of the parts of K of a tile.
+struct Unit {
+  int w_row0;      // transpose: first packed row of this block's half of the tile; else first output column
+  int w_row_end;   // transpose: one past the last packed row of this matrix
+  int n0;          // first output column of this block's half
+  int x_row0;      // first activation row
+  int rows, neff;  // valid activation rows, and the same rounded up to what the MMA takes
+  int ks0, ks1;    // stages of K
+  int slot;        // index of the unit's partial sums
 };
-__device__ __forceinline__ TileCoord tile_coord(const TcParams& p, int tile) {
-  TileCoord t;
+__device__ __forceinline__ Unit unit_at(const TcParams& p, int u, int rank) {
+  Unit t;
+  const int kst = p.K / kStageK + (p.K % kStageK != 0);
   if (p.mtiles == nullptr) {
-    const int tm = tile % p.m_tiles, tn = tile / p.m_tiles;
-    t.w_row0 = tn * kTileN;
-    t.w_rows_end = p.N;
-    t.n0 = tn * kTileN;
+    const int tile = u / p.splits, sp = u - tile * p.splits;
+    const int tn = tile / p.m_tiles, tm = tile - tn * p.m_tiles;
+    t.n0 = tn * (2 * kTileRows) + rank * kTileRows;
+    t.w_row0 = t.n0;
+    t.w_row_end = p.N;
     t.x_row0 = tm * p.NT;
-    t.rows = p.M - t.x_row0 < p.NT ? p.M - t.x_row0 : p.NT;
+    t.rows = min(p.M - t.x_row0, p.NT);
+    t.ks0 = sp * (kst / p.spc) / p.splits * p.spc;   // whole chunks of scales
+    t.ks1 = (sp + 1) * (kst / p.spc) / p.splits * p.spc;
   } else {
-    const int g = tile / p.n_tiles, tn = tile - g * p.n_tiles;
+    const int g = u / p.n_tiles, tn = u - g * p.n_tiles;
     const MTile mt = p.mtiles[g];
-    t.w_row0 = mt.expert * p.N + tn * kTileN;
-    t.w_rows_end = mt.expert * p.N + p.N;
-    t.n0 = tn * kTileN;
+    t.n0 = tn * (2 * kTileRows) + rank * kTileRows;
+    t.w_row0 = mt.expert * p.N + t.n0;
+    t.w_row_end = mt.expert * p.N + p.N;
     t.x_row0 = mt.row0;
     t.rows = mt.rows;
+    t.ks0 = 0;
+    t.ks1 = kst;
   }
+  t.neff = (t.rows + 31) & ~31;
+  t.slot = u;
   return t;
 }
 
-#ifdef B200Q_PROFILE
-__device__ uint32_t g_tc_prof[64];
-#endif
+// Columns c .. c+lim of the tile's tokens for output column n, one value per lane.
+template <typename T>
+__device__ __forceinline__ void store_chunk(const TcParams& p, const Unit& t, int n, int c, int lim, const uint32_t (&v)[32]) {
+  if (p.dst_row == nullptr) {
+    for (int q = 0; q < p.n_out; ++q) {
+      T* yp = static_cast<T*>(p.y_out[q]) + (size_t)(t.x_row0 + c) * p.ld + p.col0 + n;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        if (j < lim) *yp = Elem<T>::from_float(__uint_as_float(v[j]));
+        yp += p.ld;
+      }
+    }
+  } else {
+    const int* dr = p.dst_row + t.x_row0 + c;
+    for (int q = 0; q < p.n_out; ++q) {
+      T* yq = static_cast<T*>(p.y_out[q]) + n;
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < lim) yq[(size_t)dr[j] * p.ld] = Elem<T>::from_float(__uint_as_float(v[j]));
+    }
+  }
+}
 
-template <int BITS>
-__global__ void __launch_bounds__(kThreads, 1)
-qmm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
-              const TcParams p) {
-  // A packed stage holds 128 k of every row (16*BITS bytes, a multiple of 16 for every width).
-  constexpr int kPRowBytes = 16 * BITS;
-  constexpr int kStagesP = stages_p(BITS);
-  constexpr int kPStageBytes = kTileN * kPRowBytes;
-  const int kStagesB = p.nsb;
+template <typename T, int BITS, Form F>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
+  using S = Shape<BITS, F>;
+  constexpr bool kT = S::kT;
+  constexpr int kSub = S::kSub, kSlotsA = S::kSlotsA, kStagesP = S::kStagesP;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  // carve-up: [B ring: nsb stages of two NT*128-byte sub-tiles (1024-aligned)] [P ring] [barriers]
+  // carve-up: [A ring of SplitT] [B ring: nsb stages of two NT/2 * 128-byte sub-tiles] [P ring] [S ring] [barriers]
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const uint32_t b_sub_bytes = (uint32_t)p.NT * 128u;     // NT is a multiple of 16: a multiple of 2048
-  const uint32_t b_stage_bytes = 2u * b_sub_bytes;
-  const uint32_t b_stage_pitch = b_stage_bytes;
-  unsigned char* ring_b = smem;
-  unsigned char* ring_p = ring_b + (size_t)kStagesB * b_stage_pitch;
-  Barriers* bars = reinterpret_cast<Barriers*>(ring_p + (size_t)kStagesP * kPStageBytes);
+  const uint32_t b_sub = (uint32_t)p.NT * 64u;       // NT / 2 rows of 128 bytes (NT is a multiple of 32)
+  const uint32_t b_stage = 2u * b_sub;
+  unsigned char* ring_b = smem + S::kSmemA;
+  unsigned char* ring_p = ring_b + (size_t)p.nsb * b_stage;
+  unsigned char* ring_s = ring_p + (size_t)kStagesP * S::kPStageBytes;   // per chunk: 128 rows of scales, 128 of biases
+  Barriers* bars = reinterpret_cast<Barriers*>(ring_s + kSlotsS * 2 * kTileRows * p.cb);
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#ifdef B200Q_PROFILE
-  // Tuning builds (plain mode only): thread block 0 leaves per-role wait cycles / 16 in a buffer of
-  // its own (g_tc_prof), which a test harness reads back with cudaMemcpyFromSymbol.
-  uint32_t* dbg = g_tc_prof;
-  long long pw0 = 0, pw1 = 0, pw2 = 0, pw3 = 0, pw4 = 0, pt = 0;
-  const long long prof_entry = clock64();
-#define TC_T0() pt = clock64()
-#define TC_ACC(v) v += clock64() - pt
-#define TC_OUT(slot, v) if (blockIdx.x == 0 && lane == 0 && p.mtiles == nullptr) dbg[slot] = (uint32_t)((v) >> 4)
-#else
-#define TC_T0()
-#define TC_ACC(v)
-#define TC_OUT(slot, v)
-#endif
-  const int kstages = p.K / kStageK;
-  const int total_tiles = p.mtiles ? *p.n_mtiles * p.n_tiles : p.n_tiles * p.m_tiles;
+  const int rank = (int)cluster_rank();
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int total = p.mtiles ? *p.n_mtiles * p.n_tiles : p.n_tiles * p.m_tiles * p.splits;
+  const int nacc = p.NT <= kAccCols / 2 ? 2 : 1;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kStagesP; ++i) { mbar_init(smem_u32(&bars->full_p[i]), 1); mbar_init(smem_u32(&bars->empty_p[i]), kDequantSet); }
-    for (int i = 0; i < kStagesB; ++i) mbar_init(smem_u32(&bars->full_b[i]), 1);
-    for (int i = 0; i < kStagesA; ++i) mbar_init(smem_u32(&bars->full_a[i]), kDequantSet);
+    for (int i = 0; i < kStagesP; ++i) { mbar_init(smem_u32(&bars->full_p[i]), 1); mbar_init(smem_u32(&bars->empty_p[i]), S::kPArrivals); }
+    for (int i = 0; i < kSlotsS; ++i) {
+      mbar_init(smem_u32(&bars->full_s[i]), 32);
+      mbar_init(smem_u32(&bars->empty_s[i]), p.spc * S::kPArrivals);
+    }
+    for (int i = 0; i < p.nsb; ++i) mbar_init(smem_u32(&bars->full_b[i]), 1);
+    for (int i = 0; i < kSlotsA; ++i) mbar_init(smem_u32(&bars->full_a[i]), 2 * kUnpackWarps / S::kSets);
     for (int i = 0; i < kDoneRing; ++i) mbar_init(smem_u32(&bars->done[i]), 1);
-    mbar_init(smem_u32(&bars->acc_full), 1);
-    mbar_init(smem_u32(&bars->acc_empty), kEpilogueWarps);
+    for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&bars->acc_full[i]), 1); mbar_init(smem_u32(&bars->acc_empty[i]), 2 * kEpilogueWarps); }
     bars->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -319,318 +452,359 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   }
   tcgen05_fence_before();
   __syncthreads();
+  cluster_sync();
   tcgen05_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-  const uint32_t tmem_acc = tmem_base;
   const uint32_t tmem_a = tmem_base + kAccCols;
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer: x tiles (B ring)
-    if (lane == 0) {
-      uint32_t sb = 0, it = 0;  // slot and stage counter, running across tiles
-      for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x) {
-        const TileCoord tc_ = tile_coord(p, tile);
-        bool ok = true;
-        for (int ks = 0; ks < kstages; ++ks) {
-          TC_T0();
-          if (it >= (uint32_t)kStagesB) {   // the stage that used this slot last has been multiplied
-            const uint32_t prev = it - (uint32_t)kStagesB;
-            if (!TC_WAIT1(smem_u32(&bars->done[prev % kDoneRing]), (prev / kDoneRing) & 1u, abort_flag)) { ok = false; break; }
+    // ------------------------------------------------------------ x tiles: this block's half of the tokens
+    // (The three one-thread roles run at one instruction in ten to twenty cycles beside the unpack warps: their
+    // loops hold addresses and ring positions and nothing else.)
+    if (elect_one()) {
+      const uint32_t full = smem_u32(&bars->full_b[0]), lfull = leader_addr(full), done = smem_u32(&bars->done[0]);
+      const uint32_t ring = smem_u32(ring_b), nsb = p.nsb;
+      uint32_t sb = 0, it = 0, dst = ring;
+      bool ok = true;
+      for (int u = pair; ok && u < total; u += pairs) {
+        const Unit t = unit_at(p, u, rank);
+        const int half = t.neff >> 1, row = t.x_row0 + rank * half;
+        const uint32_t bytes = (uint32_t)t.neff * 256u;   // both blocks' halves
+        for (int k = t.ks0 * kStageK, k1 = t.ks1 * kStageK; k < k1; k += kStageK, ++it) {
+          if (it >= nsb) {   // the stage that used this slot last has been multiplied
+            const uint32_t ia = (it - nsb) * kSub + kSub - 1;
+            if (!mbar_nap<40>(done + (ia % kDoneRing) * 8, (ia / kDoneRing) & 1u, abort_flag)) { ok = false; break; }
           }
-          TC_ACC(pw1);
-          const uint32_t bar = smem_u32(&bars->full_b[sb]);
-          const uint32_t dst = smem_u32(ring_b + sb * b_stage_pitch);
-          mbar_expect_tx(bar, b_stage_bytes);
-          tma_load_2d(dst, &map_x, ks * kStageK, tc_.x_row0, bar);
-          tma_load_2d(dst + b_sub_bytes, &map_x, ks * kStageK + kBlockK, tc_.x_row0, bar);
-          ++it;
-          if (++sb == (uint32_t)kStagesB) sb = 0;
+          if (rank == 0) mbar_expect_tx(full + sb * 8, bytes);
+          const uint32_t lbar = lfull + sb * 8;
+          int r = 0;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int box = 128 >> i;
+            if (half & box) {
+              tma_load_2d_pair(dst + r * 128, &maps.x[i], k, row + r, lbar);
+              tma_load_2d_pair(dst + b_sub + r * 128, &maps.x[i], k + 64, row + r, lbar);
+              r += box;
+            }
+          }
+          dst += b_stage;
+          if (++sb == nsb) { sb = 0; dst = ring; }
         }
-        if (!ok) break;
       }
-      TC_OUT(1, pw1); TC_OUT(2, clock64() - prof_entry);
-    }
-  } else if (warp == kProducerPWarp) {
-    // ------------------------------------------------------------ TMA producer: packed W tiles (P ring).
-    // A separate thread: behind the x-tile waits of the other producer the packed tiles would
-    // arrive late and starve the dequant warps.
-    if (lane == 0) {
-      uint32_t sp = 0, pp = 0;
-      for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x) {
-        const TileCoord tc_ = tile_coord(p, tile);
-        bool ok = true;
-        for (int ks = 0; ks < kstages; ++ks) {
-          TC_T0();
-          if (!TC_WAIT1(smem_u32(&bars->empty_p[sp]), pp ^ 1, abort_flag)) { ok = false; break; }
-          TC_ACC(pw0);
-          mbar_expect_tx(smem_u32(&bars->full_p[sp]), kPStageBytes);
-          tma_load_2d(smem_u32(ring_p + sp * kPStageBytes), &map_w, ks * kPRowBytes, tc_.w_row0,
-                      smem_u32(&bars->full_p[sp]));
-          if (++sp == (uint32_t)kStagesP) { sp = 0; pp ^= 1; }
-        }
-        if (!ok) break;
-      }
-      TC_OUT(0, pw0);
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (elect_one()) {
-      const uint32_t idesc = make_idesc(p.NT);
-      uint32_t tcount = 0, sa = 0, pa = 0, sb = 0, pb = 0, itm = 0;
-      // The commit of a stage is issued after the FIRST MMA of the next one: its 65 cycles then pass
-      // while the tensor pipe works, not between two stages.  (The barrier then also covers that one
-      // MMA: the stage is released 128 cycles later.)
-      bool commit_due = false;
-      for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x, ++tcount) {
-        TC_T0();
-        if (!TC_WAIT1(smem_u32(&bars->acc_empty), (tcount & 1) ^ 1, abort_flag)) break;
-        TC_ACC(pw2);
-        tcgen05_fence_after();
-        bool ok = true;
-        for (int ks = 0; ks < kstages; ++ks) {
-          TC_T0();
-          if (!TC_WAIT1(smem_u32(&bars->full_a[sa]), pa, abort_flag)) { ok = false; break; }
-          TC_ACC(pw0);
-          TC_T0();
-          if (!TC_WAIT1(smem_u32(&bars->full_b[sb]), pb, abort_flag)) { ok = false; break; }
-          TC_ACC(pw1);
-          tcgen05_fence_after();
-          const uint32_t b_addr = smem_u32(ring_b + sb * b_stage_pitch);
-          TC_T0();
+    // ------------------------------------------------------------ MMA issuer (leader block)
+    if (rank == 0 && elect_one()) {
+      const uint32_t full_b = smem_u32(&bars->full_b[0]), full_a = smem_u32(&bars->full_a[0]), done = smem_u32(&bars->done[0]);
+      const uint64_t desc0 = sw128_desc(smem_u32(ring_b), 16, 1024);
+      const uint32_t d_stage = b_stage >> 4, d_sub = b_sub >> 4, nsb = p.nsb;
+      const uint64_t desc_a0 = sw128_desc(smem_u32(smem), 8192, 1024);
+      uint32_t tcount = 0, ia = 0, sa = 0, pa = 0, sb = 0, pb = 0;
+      uint64_t bd0 = desc0;
+      bool ok = true;
+      for (int u = pair; ok && u < total; u += pairs, ++tcount) {
+        const Unit t = unit_at(p, u, 0);
+        const uint32_t idesc = make_idesc<T, F>(t.neff);
+        const uint32_t ab = nacc == 2 ? (tcount & 1) : 0, an = nacc == 2 ? (tcount >> 1) : tcount;
+        const uint32_t acc = tmem_base + ab * (kAccCols / 2);
+        if (!mbar_wait_spin(smem_u32(&bars->acc_empty[ab]), (an & 1) ^ 1, abort_flag)) break;
+        uint32_t first = 0;
+        for (int ks = t.ks0; ok && ks < t.ks1; ++ks) {
+          const uint64_t bd1 = bd0 + d_sub;
 #pragma unroll
-          for (int kk = 0; kk < kStageK / 16; ++kk) {
-            tcgen05_mma_ts(tmem_acc, tmem_a + sa * 64 + kk * 8,
-                           make_sw128_desc(b_addr + (kk >> 2) * b_sub_bytes + (kk & 3) * 32), idesc,
-                           (ks | kk) != 0 ? 1u : 0u);
-            if (kk == 0 && commit_due) {
-              // one commit per stage: a stage is 128 k (eight MMAs) deep and both rings are released
-              // through the same barrier
-              tcgen05_commit(smem_u32(&bars->done[(itm - 1) % kDoneRing]));
-              commit_due = false;
+          for (int sub = 0; sub < kSub; ++sub) {
+            // both looks are under way before either is needed
+            const bool ra = mbar_test(full_a + sa * 8, pa), rb = sub > 0 || mbar_test(full_b + sb * 8, pb);
+            if (!(ra && rb)) {
+              if (!mbar_wait_spin(full_a + sa * 8, pa, abort_flag) || !mbar_wait_spin(full_b + sb * 8, pb, abort_flag)) { ok = false; break; }
             }
-          }
-          TC_ACC(pw3);
-          commit_due = true;
-          ++itm;
-          if (++sa == (uint32_t)kStagesA) { sa = 0; pa ^= 1; }
-          if (++sb == (uint32_t)kStagesB) { sb = 0; pb ^= 1; }
-        }
-        if (!ok) break;
-        if (commit_due) {
-          tcgen05_commit(smem_u32(&bars->done[(itm - 1) % kDoneRing]));
-          commit_due = false;
-        }
-        tcgen05_commit(smem_u32(&bars->acc_full));
-      }
-      TC_OUT(4, pw0); TC_OUT(5, pw1); TC_OUT(6, pw2); TC_OUT(7, clock64() - prof_entry); TC_OUT(14, pw3); TC_OUT(15, pw4);
-    }
-  } else if (warp < 2 + kDequantWarps) {
-    // ------------------------------------------------------------ dequant: one thread per weight row
-    // A warp's trip through one stage (wait for the packed tile, unpack, publish, wait for a free
-    // A stage, store) is a chain of dependent latencies of about the length of a stage's MMAs; with
-    // every warp on every stage that chain bounded the kernel.  So the warps form two sets that
-    // take alternate stages, 64 k per thread and stage: each set has two stage times per trip.
-    const int dq = warp - 2;
-    const int dset = dq >> 3;            // stages ks = dset (mod 2) of every tile are this warp's
-    const int quad = warp & 3;           // TMEM lane quadrant this warp may access
-    const int half = (dq >> 2) & 1;      // which 64-k half of the 128-k stage
-    const int row_in_tile = quad * 32 + lane;
-    const uint32_t lane_field = (uint32_t)(quad * 32) << 16;
-    const int row_groups = p.K >> (5 + p.group_shift);
-    uint32_t tcount = 0;                 // tiles done: the stage counter of (tile, ks) is tcount * kstages + ks
-    // An A stage is published as soon as its stores have completed: each set has a stage time of
-    // slack, and the issuing thread gets the stage earlier than when the arrival waited for the
-    // next unpack (388 -> 382 us on M=4096).
-    auto publish = [&](uint32_t stage) {
-      tcgen05_wait_st();
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&bars->full_a[stage]));
-    };
-    // Scales and biases: a thread needs one 2-byte value of each per stage, from a row of its own,
-    // so a warp's load touches 32 cache lines whatever its width.  Fetched per stage they kept the
-    // load/store pipe busier than anything else in the kernel; fetched as 16-byte chunks (eight
-    // groups of the row) there are up to eight times fewer loads.  `cur` holds the chunk in use,
-    // `nxt` the next one of the sequence (tile by tile, chunk by chunk), requested one chunk early.
-    const int gs5 = 5 + p.group_shift;
-    const bool vec = (row_groups & 7) == 0 && ((reinterpret_cast<uintptr_t>(p.scales) | reinterpret_cast<uintptr_t>(p.biases)) & 15) == 0;
-    const int nchunks = row_groups >> 3;
-    uint4 s_cur4 = make_uint4(0, 0, 0, 0), b_cur4 = s_cur4, s_nxt4 = s_cur4, b_nxt4 = s_cur4;
-    int pf_tile = blockIdx.x, pf_chunk = 0;   // next chunk to request
-    auto row_of = [&](int tile_) {
-      const TileCoord t_ = tile_coord(p, tile_);
-      const int r_ = t_.w_row0 + row_in_tile;
-      return r_ < t_.w_rows_end ? r_ : t_.w_rows_end - 1;   // rows past N: results are never stored
-    };
-    auto prefetch = [&]() {
-      if (pf_tile >= total_tiles) return;
-      const size_t off = (size_t)row_of(pf_tile) * row_groups + (size_t)pf_chunk * 8;
-      s_nxt4 = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p.scales) + off));
-      b_nxt4 = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p.biases) + off));
-      if (++pf_chunk == nchunks) { pf_chunk = 0; pf_tile += gridDim.x; }
-    };
-    auto pick = [](const uint4& c, int idx) {
-      const uint32_t wsel = idx < 4 ? (idx < 2 ? c.x : c.y) : (idx < 6 ? c.z : c.w);
-      return (idx & 1) ? (wsel >> 16) : (wsel & 0xFFFFu);
-    };
-    if (vec) prefetch();
-    int cur_chunk = -1;
-    bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < total_tiles && !*abort_flag; tile += gridDim.x) {
-      const int row = row_of(tile);
-      const unsigned short* sc = reinterpret_cast<const unsigned short*>(p.scales) + (size_t)row * row_groups;
-      const unsigned short* bi = reinterpret_cast<const unsigned short*>(p.biases) + (size_t)row * row_groups;
-      cur_chunk = -1;
-      // The sets alternate over the stage counter, not over ks: with an odd number of stages per tile a
-      // set would otherwise take two stages in a row and could pass the other set in the packed ring.
-      for (int ks = (int)((dset ^ (tcount * (uint32_t)kstages)) & 1u); ks < kstages; ks += 2) {
-        const uint32_t it = tcount * (uint32_t)kstages + (uint32_t)ks;
-        const uint32_t sa = it % kStagesA;
-        const uint32_t sp = it % kStagesP, pp = (it / kStagesP) & 1u;
-        // scale and bias of the two 32-k quarters of this thread's half (one group or two)
-        uint32_t s_q[2], b_q[2];
-        if (vec) {
-          const int g0 = (ks * kStageK + half * 64) >> gs5, g1 = (ks * kStageK + half * 64 + 32) >> gs5;
-          if ((g0 >> 3) != cur_chunk) {
-            s_cur4 = s_nxt4; b_cur4 = b_nxt4;
-            cur_chunk = g0 >> 3;
-            prefetch();
-          }
-          s_q[0] = pick(s_cur4, g0 & 7); b_q[0] = pick(b_cur4, g0 & 7);
-          s_q[1] = g1 == g0 ? s_q[0] : pick(s_cur4, g1 & 7);
-          b_q[1] = g1 == g0 ? b_q[0] : pick(b_cur4, g1 & 7);
-        } else {
-          const int g0 = (ks * kStageK + half * 64) >> gs5, g1 = (ks * kStageK + half * 64 + 32) >> gs5;
-          s_q[0] = __ldg(sc + g0); b_q[0] = __ldg(bi + g0);
-          s_q[1] = __ldg(sc + g1); b_q[1] = __ldg(bi + g1);
-        }
-        TC_T0();
-        if (!TC_WAIT16(smem_u32(&bars->full_p[sp]), pp, abort_flag)) { ok = false; break; }
-        TC_ACC(pw0);
-        const unsigned char* src0 = ring_p + sp * kPStageBytes + row_in_tile * kPRowBytes + half * (8 * BITS);
-        bool freed = false;
+            tcgen05_fence_after();
+            if constexpr (F == Form::Round) {
+              const uint32_t ta = tmem_a + sa * 64;
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          // this thread's 32 fields of quarter 2 * half + q: BITS words of its row
-          uint32_t w[BITS];
-          {
-            const unsigned char* src = src0 + q * (4 * BITS);
-            if constexpr (BITS == 4) {
-              const uint4 v = *reinterpret_cast<const uint4*>(src);
-              w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-            } else if constexpr (BITS == 8) {
-              const uint4 v = *reinterpret_cast<const uint4*>(src), u = *reinterpret_cast<const uint4*>(src + 16);
-              w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w; w[4] = u.x; w[5] = u.y; w[6] = u.z; w[7] = u.w;
-            } else if constexpr (BITS == 2 || BITS == 6) {
+              for (int kk = 0; kk < 8; ++kk) tcgen05_mma_ts(acc, ta + kk * 8, (kk < 4 ? bd0 : bd1) + (kk & 3) * 2, idesc, kk ? 1u : first);
+            } else if constexpr (F == Form::Split) {
+              const uint32_t ta = tmem_a + sa * 64;
 #pragma unroll
-              for (int i = 0; i < BITS / 2; ++i) {
-                const uint2 v = *reinterpret_cast<const uint2*>(src + 8 * i);
-                w[2 * i] = v.x; w[2 * i + 1] = v.y;
+              for (int kk = 0; kk < 4; ++kk) {
+                tcgen05_mma_ts(acc, ta + kk * 8, (sub ? bd1 : bd0) + kk * 2, idesc, kk ? 1u : first);
+                tcgen05_mma_ts(acc, ta + 32 + kk * 8, (sub ? bd1 : bd0) + kk * 2, idesc, 1u);
               }
             } else {
+              const uint64_t ad = desc_a0 + sa * 2048;
 #pragma unroll
-              for (int i = 0; i < BITS; ++i) w[i] = *reinterpret_cast<const uint32_t*>(src + 4 * i);
+              for (int kk = 0; kk < 4; ++kk) {
+                tcgen05_mma_ss(acc, ad + kk * 128, (sub ? bd1 : bd0) + kk * 2, idesc, kk ? 1u : first);
+                tcgen05_mma_ss(acc, ad + 1024 + kk * 128, (sub ? bd1 : bd0) + kk * 2, idesc, 1u);
+              }
             }
+            first = 1;
+            tcgen05_commit_pair(done + (ia % kDoneRing) * 8);
+            ++ia;
+            if (++sa == (uint32_t)kSlotsA) { sa = 0; pa ^= 1; }
           }
-          uint32_t vals[16];
-          TC_T0();
-          dequant32<BITS>(w, s_q[q], b_q[q], vals);
-#ifdef B200Q_PROFILE
-          asm volatile("" ::"r"(vals[0]), "r"(vals[5]), "r"(vals[10]), "r"(vals[15]));
-#endif
-          TC_ACC(pw3);
-          if (q == 0) {
-            TC_T0();
-            if (it >= (uint32_t)kStagesA) {   // the stage that used this A slot last has been multiplied
-              const uint32_t prev = it - (uint32_t)kStagesA;
-              if (!TC_WAIT16(smem_u32(&bars->done[prev % kDoneRing]), (prev / kDoneRing) & 1u, abort_flag)) { ok = false; break; }
-            }
-            TC_ACC(pw2);
-            tcgen05_fence_after();
-            freed = true;
-          }
-          TC_T0();
-          tcgen05_st_x16(tmem_a + lane_field + sa * 64 + (2 * half + q) * 16, vals);
-          TC_ACC(pw4);
+          bd0 += d_stage;
+          if (++sb == nsb) { sb = 0; pb ^= 1; bd0 = desc0; }
         }
-        if (!freed) break;
-        TC_T0();
-        publish(sa);
-        TC_ACC(pw1);
-        // The packed stage is released only here, after the stores that consume the unpacked
-        // registers have been issued: the shared-memory reads above have then returned for every
-        // lane, so the refill of the stage cannot overtake them.
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bars->empty_p[sp]));
+        if (!ok) break;
+        tcgen05_commit_pair(smem_u32(&bars->acc_full[ab]));
       }
-      ++tcount;
     }
-    if (warp == 2) { TC_OUT(8, pw0); TC_OUT(9, pw1); TC_OUT(10, pw2); TC_OUT(11, clock64() - prof_entry); }
-    TC_OUT(16 + dq, pw2); TC_OUT(32 + dq, pw0);
-    if (warp == 2) { TC_OUT(48, pw3); TC_OUT(49, pw4); }
-  } else if (warp < kProducerPWarp) {
+  } else if (warp == 2) {
+    // ------------------------------------------------------------ packed W tiles
+    if (elect_one()) {
+      const uint32_t full = smem_u32(&bars->full_p[0]), empty = smem_u32(&bars->empty_p[0]), ring = smem_u32(ring_p);
+      uint32_t sp = 0, pp = 1, dst = ring;
+      bool ok = true;
+      for (int u = pair; ok && u < total; u += pairs) {
+        const Unit t = unit_at(p, u, rank);
+        // transpose: 128 k of 128 rows; else 128 columns of 128 rows (= k)
+        int c0 = kT ? (t.n0 / kTileRows) * S::kPRowBytes : t.ks0 * S::kPRowBytes;
+        int c1 = kT ? t.ks0 * kStageK : t.w_row0;
+        for (int n = t.ks1 - t.ks0; n > 0; --n) {
+          if (!mbar_nap<40>(empty + sp * 8, pp, abort_flag)) { ok = false; break; }
+          mbar_expect_tx(full + sp * 8, S::kPStageBytes);
+          tma_load_2d(dst, &maps.w, c0, c1, full + sp * 8);
+          if constexpr (kT) c1 += kStageK; else c0 += S::kPRowBytes;
+          dst += S::kPStageBytes;
+          if (++sp == (uint32_t)kStagesP) { sp = 0; pp ^= 1; dst = ring; }
+        }
+      }
+    }
+  } else if (warp == 3) {
+    // ------------------------------------------------------------ scales and biases
+    // Asynchronous copies straight into the ring, counted on the chunk's barrier; a lane serves four rows.
+    // A copy instruction touches as many cache lines as it has lanes and costs a thousand cycles per eight:
+    // a chunk is as many stages as a copy's 16 bytes and the rows' alignment allow.  cp.async moves no
+    // less than 4 bytes: where a stage needs one value, the aligned word that holds it is copied.
+    uint32_t ss = 0, ps = 0;
+    bool ok = true;
+    const uint32_t half_chunk = (uint32_t)kTileRows * p.cb;   // bytes of a chunk's scales; the biases follow
+    for (int u = pair; ok && u < total; u += pairs) {
+      const Unit t = unit_at(p, u, rank);
+      for (int ks = t.ks0; ks < t.ks1; ks += p.spc) {
+        if (!mbar_nap<100>(smem_u32(&bars->empty_s[ss]), ps ^ 1, abort_flag)) { ok = false; break; }
+        const uint32_t dst = smem_u32(ring_s) + ss * 2 * half_chunk + lane * p.cb;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          long long o;   // rows past the end: results are never stored (transpose), x is zero (no transpose)
+          if constexpr (kT) o = (long long)min(ks * kStageK + lane + 32 * i, p.K - 1) * p.row_groups + min(t.n0 / kTileRows * p.g4, p.row_groups - p.g4);
+          else o = (long long)min(t.w_row0 + lane + 32 * i, t.w_row_end - 1) * p.row_groups + ks * p.g4;
+          const uint32_t d = dst + 32 * i * p.cb;
+          if (p.cb == 16) {
+            cp_async<16>(d, p.scales + o, 16);
+            cp_async<16>(d + half_chunk, p.biases + o, 16);
+          } else if (p.cb == 8) {
+            cp_async<8>(d, p.scales + o, 8);
+            cp_async<8>(d + half_chunk, p.biases + o, 8);
+          } else {
+            const long long w = o & ~1ll;   // (even already unless the chunk is one value)
+            const int n = w + 1 < p.n_scales ? 4 : 2;
+            cp_async<4>(d, p.scales + w, n);
+            cp_async<4>(d + half_chunk, p.biases + w, n);
+          }
+        }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->full_s[ss])) : "memory");
+        if (++ss == (uint32_t)kSlotsS) { ss = 0; ps ^= 1; }
+      }
+    }
+  } else if (warp < kFirstEpilogue) {
+    // ------------------------------------------------------------ unpack
+    // Everything here is counted in instructions: the warps of a scheduler make one instruction about
+    // every ten cycles each, and a trip of 450 instructions for 64 fields per thread (150 of them the
+    // unpacking) bounded the kernel at 2000 cycles per stage.  So a warp takes a whole slot row per trip
+    // (128 or 64 k), ring positions are masks, and addresses are kept as shared-memory words.
+    constexpr int kSets = S::kSets, kSetWarps = kUnpackWarps / kSets;
+    const int wu = warp - kFirstUnpack;
+    const uint32_t set = wu / kSetWarps;   // A slot uses ia = set (mod kSets) are this warp's
+    const int quad = warp & 3;             // TMEM lane quadrant this warp may access
+    const int half = kT ? (wu >> 2) & 1 : 0;   // kT: which half of the slot's k
+    const uint32_t sub = set % kSub;       // which slot of a stage
+    const int row = kT ? (int)sub * 64 + half * 32 + lane : quad * 32 + lane;   // packed row of the tile (transpose: TMEM lane)
+    const uint32_t t_slot = tmem_a + ((uint32_t)(quad * 32) << 16) + set * 64;   // (transpose) as many slots as sets
+    // offset of unit un's value in a chunk row's stage: one value per 1, 2 or 4 units
+    const int gsh = p.g4 == 4 ? 0 : (p.g4 == 2 ? 1 : 2);
+    const uint32_t spc_sh = p.spc == 4 ? 2 : (p.spc == 2 ? 1 : 0), half_chunk = (uint32_t)kTileRows * p.cb;
+    const bool single = p.spc * p.g4 == 1;   // a chunk is one value: the odd or the even half of the copied word
+    const uint32_t s_row = smem_u32(ring_s) + row * p.cb;
+    const uint32_t p_base = smem_u32(ring_p);
+    const uint32_t bar_a = leader_addr(smem_u32(&bars->full_a[0])), bar_done = smem_u32(&bars->done[0]);
+    const uint32_t bar_fp = smem_u32(&bars->full_p[0]), bar_ep = smem_u32(&bars->empty_p[0]);
+    const uint32_t bar_fs = smem_u32(&bars->full_s[0]), bar_es = smem_u32(&bars->empty_s[0]);
+    uint32_t it0 = 0, c0 = 0;              // stages and chunks of the units before this one
+    uint32_t ia = set;
+    bool ok = true;
+    for (int u = pair; ok && u < total; u += pairs) {
+      const Unit t = unit_at(p, u, rank);
+      const uint32_t n_st = t.ks1 - t.ks0;
+      const uint32_t o_row = kT ? min(t.n0 / kTileRows, p.row_groups - 1) : (uint32_t)min(t.w_row0 + row, t.w_row_end - 1) * p.row_groups + t.ks0;
+      for (; ia < (it0 + n_st) * kSub; ia += kSets) {
+        const uint32_t it = ia / kSub, ks = it - it0;      // ks counts from the unit's first stage
+        const uint32_t c = c0 + (ks >> spc_sh), sp = it % kStagesP;
+        if (!mbar_wait_hot(bar_fs + (c % kSlotsS) * 8, (c / kSlotsS) & 1u, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_hot(bar_fp + sp * 8, (it / kStagesP) & 1u, abort_flag)) { ok = false; break; }
+        const uint32_t tile = p_base + sp * S::kPStageBytes;
+        uint32_t at = s_row + (c % kSlotsS) * 2 * half_chunk + (ks & (p.spc - 1)) * 2 * p.g4;
+        if (single) {
+          const uint32_t o = kT ? (uint32_t)min((int)((t.ks0 + ks) * kStageK + row), p.K - 1) * p.row_groups + o_row : o_row + ks;
+          at += (o & 1) * 2;
+        }
+        const uint32_t sa = kT ? ia % kSlotsA : set;
+        auto slot_free = [&]() {   // the slot's last use has been multiplied
+          const uint32_t prev = ia - kSlotsA;
+          return ia < (uint32_t)kSlotsA || mbar_wait_hot(bar_done + (prev % kDoneRing) * 8, (prev / kDoneRing) & 1u, abort_flag);
+        };
+        if constexpr (F == Form::Round) {
+#pragma unroll
+          for (int un = 0; un < 4; ++un) {
+            uint32_t w[BITS], vals[16];
+            load_fields<BITS>(tile, row, un, w);
+            const uint32_t v = at + 2 * (un >> gsh);
+            dequant32<BITS>(w, lds_u16(v), lds_u16(v + half_chunk), vals);
+            if (un == 0) {
+              if (!slot_free()) { ok = false; break; }
+              tcgen05_fence_after();
+            }
+            tcgen05_st_x16(t_slot + un * 16, vals);
+          }
+        } else if constexpr (F == Form::Split) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t w[BITS], hi[16], lo[16];
+            const int un = 2 * (int)sub + h;
+            load_fields<BITS>(tile, row, un, w);
+            const uint32_t v = at + 2 * (un >> gsh);
+            split32<BITS, T>(w, bits_to_float<T>(lds_u16(v)), bits_to_float<T>(lds_u16(v + half_chunk)), hi, lo);
+            if (h == 0) {
+              if (!slot_free()) { ok = false; break; }
+              tcgen05_fence_after();
+            }
+            tcgen05_st_x16(t_slot + h * 16, hi);
+            tcgen05_st_x16(t_slot + 32 + h * 16, lo);
+          }
+        } else {
+          uint32_t w[BITS], hi[16], lo[16];
+          load_fields<BITS>(tile, row, quad, w);
+          const uint32_t v = at + 2 * (quad >> gsh);
+          split32<BITS, T>(w, bits_to_float<T>(lds_u16(v)), bits_to_float<T>(lds_u16(v + half_chunk)), hi, lo);
+          if (!slot_free()) { ok = false; break; }
+          // M-major tile: 128 bytes (64 columns) per k, 16-byte chunks xor-ed with k mod 8
+          const int k = half * 32 + lane;
+          const uint32_t a0 = smem_u32(smem) + sa * 32768 + (quad >> 1) * 8192 + k * 128;
+#pragma unroll
+          for (int c4 = 0; c4 < 4; ++c4) {
+            const uint32_t d = a0 + (((((quad & 1) << 2) + c4) ^ (k & 7)) << 4);
+            st_shared_v4(d, hi[4 * c4], hi[4 * c4 + 1], hi[4 * c4 + 2], hi[4 * c4 + 3]);
+            st_shared_v4(d + 16384, lo[4 * c4], lo[4 * c4 + 1], lo[4 * c4 + 2], lo[4 * c4 + 3]);
+          }
+        }
+        if (!ok) break;
+        // Publish the slot; the packed stage and the scales are released only here, after the stores that
+        // consume the unpacked registers: the shared-memory reads above have then returned for every lane.
+        if constexpr (kT) {
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        } else {
+          tcgen05_wait_st();
+          tcgen05_fence_before();
+        }
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive_cluster(bar_a + sa * 8);
+          mbar_arrive(bar_ep + sp * 8);
+          mbar_arrive(bar_es + (c % kSlotsS) * 8);
+        }
+      }
+      it0 += n_st;
+      c0 += n_st >> spc_sh;
+    }
+  } else {
     // ------------------------------------------------------------ epilogue
     const int quad = warp & 3;
-    const int chalf = (warp - (2 + kDequantWarps)) >> 2;  // which half of the token columns
+    const int chalf = (warp - kFirstEpilogue) >> 2;  // which half of the token columns
     const uint32_t lane_field = (uint32_t)(quad * 32) << 16;
     uint32_t tcount = 0;
-    for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x, ++tcount) {
-      const TileCoord tc_ = tile_coord(p, tile);
-      TC_T0();
-      if (!mbar_wait(smem_u32(&bars->acc_full), tcount & 1, abort_flag)) break;
-      TC_ACC(pw0);
+    for (int u = pair; u < total; u += pairs, ++tcount) {
+      const Unit t = unit_at(p, u, rank);
+      const uint32_t ab = nacc == 2 ? (tcount & 1) : 0, an = nacc == 2 ? (tcount >> 1) : tcount;
+      // one warp looks, the others are held by a hardware barrier
+      if (warp == kFirstEpilogue) mbar_nap<100>(smem_u32(&bars->acc_full[ab]), an & 1, abort_flag);
+      asm volatile("bar.sync 3, %0;" ::"n"(kEpilogueWarps * 32) : "memory");
+      if (*abort_flag) break;
       tcgen05_fence_after();
-      const int n = tc_.n0 + quad * 32 + lane;
-      const int m0 = tc_.x_row0;
-      const int c_begin = chalf * (p.NT / 2 / 16 * 16);            // NT is a multiple of 16
-      const int c_end = chalf == 0 ? c_begin + (p.NT / 2 / 16 * 16) : p.NT;
+      const int n = t.n0 + quad * 32 + lane;
+      const int c_begin = chalf * (t.neff >> 1), c_end = c_begin + (t.neff >> 1);
+      float* part = nullptr;
+      if (p.splits > 1) part = p.partial + ((size_t)t.slot * 2 + rank) * ((size_t)p.NT * kTileRows) + quad * 32 + lane;
       for (int c = c_begin; c < c_end; c += 32) {
         uint32_t v[32];
-        tcgen05_ld_x32(tmem_acc + lane_field + c, v);
+        tcgen05_ld_x32(tmem_base + ab * (kAccCols / 2) + lane_field + c, v);
         tcgen05_wait_ld();
         if (c + 32 >= c_end) {
-          // the last chunk is in registers: the accumulator is free for the next tile's MMAs while
+          // the last chunk is in registers: the accumulator is free for another tile's MMAs while
           // this chunk is converted and stored
           tcgen05_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&bars->acc_empty));
+          if (lane == 0) mbar_arrive_cluster(leader_addr(smem_u32(&bars->acc_empty[ab])));
         }
-        const int lim = (tc_.rows < c_end ? tc_.rows : c_end) - c;  // valid columns of this chunk
-        if (n < p.N && lim > 0) {
-          if (p.dst_row == nullptr) {
-            for (int q = 0; q < p.n_out; ++q) {
-              __nv_bfloat16* yp = p.y_out[q] + (size_t)(m0 + c) * p.ld + p.col0 + n;
+        const int lim = min(t.rows, c_end) - c;  // valid columns of this chunk
+        if (part != nullptr) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                if (j < lim) *yp = __float2bfloat16_rn(__uint_as_float(v[j]));
-                yp += p.ld;
+          for (int j = 0; j < 32; ++j)
+            if (j < lim) __stcg(part + (size_t)(c + j) * kTileRows, __uint_as_float(v[j]));
+        } else if (n < p.N && lim > 0) {
+          store_chunk<T>(p, t, n, c, lim, v);
+        }
+      }
+      if (p.splits > 1) {
+        // The last of the tile's pairs to arrive (per block of the pair: each has its own 128 columns) adds
+        // the parts in order and leaves them zeroed.
+        __threadfence();
+        asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueWarps * 32) : "memory");
+        const int tile = t.slot / p.splits;
+        if (warp == kFirstEpilogue && lane == 0) {
+          uint32_t* ctr = p.counters + tile * 2 + rank;
+          const bool last = atomicAdd(ctr, 1u) == (uint32_t)p.splits - 1;
+          if (last) *ctr = 0;
+          bars->last = last;
+        }
+        asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueWarps * 32) : "memory");
+        if (bars->last) {
+          __threadfence();
+          const size_t pitch = 2 * (size_t)p.NT * kTileRows;   // from one part to the next
+          float* p0 = p.partial + ((size_t)tile * p.splits * 2 + rank) * ((size_t)p.NT * kTileRows) + quad * 32 + lane;
+          for (int c = c_begin; c < c_end; c += 8) {
+            float sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            for (int s = 0; s < p.splits; ++s) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if (c + j < t.rows) {
+                  float* q = p0 + s * pitch + (size_t)(c + j) * kTileRows;
+                  sum[j] += __ldcg(q);
+                  __stcg(q, 0.0f);
+                }
+            }
+            if (n < p.N)
+              for (int q = 0; q < p.n_out; ++q) {
+                T* yp = static_cast<T*>(p.y_out[q]) + (size_t)(t.x_row0 + c) * p.ld + p.col0 + n;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                  if (c + j < t.rows) yp[(size_t)j * p.ld] = Elem<T>::from_float(sum[j]);
               }
-            }
-          } else {
-            const int* dr = p.dst_row + m0 + c;
-            for (int q = 0; q < p.n_out; ++q) {
-              __nv_bfloat16* yq = p.y_out[q] + n;
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (j < lim) yq[(size_t)dr[j] * p.N] = __float2bfloat16_rn(__uint_as_float(v[j]));
-            }
           }
         }
-      }
-      if (c_begin >= c_end) {   // no column of this tile for this warp: release at once
-        tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bars->acc_empty));
+        asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueWarps * 32) : "memory");   // `last` may be written again
       }
     }
-    if (warp == 2 + kDequantWarps) { TC_OUT(12, pw0); TC_OUT(13, clock64() - prof_entry); }
   }
 
-  // ---- teardown: everyone meets, then the allocating warp returns the tensor memory
+  // ---- teardown: both blocks meet, then the tensor memory is returned
+  __syncwarp();
   tcgen05_fence_before();
   __syncthreads();
   if (threadIdx.x == 0 && *abort_flag) atomicMax(&p.status[0], 3u);
   if (threadIdx.x == 0) peer_signal_tail(p.sig);   // every store of the block precedes the barrier above
+  __syncwarp();
+  cluster_sync();
   if (warp == 1) {
     tcgen05_fence_after();
     tcgen05_dealloc(tmem_base, kTmemCols);
@@ -643,178 +817,228 @@ using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, voi
                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeFn encode_fn() {
-  static EncodeFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
+  static EncodeFn fn = [] {
     void* sym = nullptr;
     cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeFn>(sym);
-  }
+    const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) == cudaSuccess &&
+                    qres == cudaDriverEntryPointSuccess;
+    return ok ? reinterpret_cast<EncodeFn>(sym) : nullptr;
+  }();
   return fn;
 }
 
-int pick_nt(int64_t M) {
-  int64_t nt = (M + 15) / 16 * 16;
-  return (int)(nt > 256 ? 256 : nt);
+// cuTensorMapEncodeTiled is a driver call and needs a current context, which a thread that has not yet
+// made a runtime call that touches the device (an autograd worker) does not have.
+int bind_context() {
+  static thread_local bool bound = false;
+  if (!bound) B200Q_CUDA_OK(cudaFree(nullptr));
+  bound = true;
+  return B200Q_OK;
 }
 
-// x stages that fit next to the packed ring (each holds 128 k of nt tokens).
-int x_stages(int nt, int bits) {
-  const size_t fixed = 1024 + (size_t)stages_p(bits) * kTileN * 16 * bits + sizeof(Barriers) + 64;
-  const size_t n = (kSmemMax - fixed) / ((size_t)nt * 256);
-  return n >= 6 ? 6 : (n >= 4 ? 4 : (n >= 3 ? 3 : 2));   // a divisor of the length of the `done` ring
+int sm_pairs() {
+  static int cached[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 74;
+  if (!cached[dev]) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 2) n = 148;
+    cached[dev] = n / 2;
+  }
+  return cached[dev];
 }
 
-size_t smem_bytes(int nt, int bits) {
-  const size_t need = 1024 + (size_t)x_stages(nt, bits) * nt * 256 + (size_t)stages_p(bits) * kTileN * 16 * bits +
-                      sizeof(Barriers) + 64;
-  // More than half of an SM's shared memory: guarantees one CTA per SM, so the 512-column
-  // tensor-memory allocation never has to wait for a co-resident CTA of this kernel.
-  const size_t one_per_sm = 120 * 1024;
-  return need > one_per_sm ? need : one_per_sm;
+Form form_of(int dtype, bool transpose) {
+  return !transpose ? Form::SplitT : (dtype == B200Q_BF16 ? Form::Round : Form::Split);
 }
 
-// Launches the kernel instantiated for `bits`.
-int launch_tc(int bits, int grid, size_t smem, cudaStream_t st, const CUtensorMap& map_x, const CUtensorMap& map_w,
-              const TcParams& p) {
-  int rc = B200Q_ERR_UNSUPPORTED;
+template <int BITS, Form F>
+size_t fixed_smem(int cb) {
+  using S = Shape<BITS, F>;
+  return 1024 + S::kSmemA + (size_t)S::kStagesP * S::kPStageBytes + (size_t)kSlotsS * 2 * kTileRows * cb + sizeof(Barriers) + 64;
+}
+size_t fixed_smem(int bits, Form f, int cb) {
+  size_t n = 0;
   B200Q_DISPATCH_BITS(bits, BITS, {
-    cudaError_t e = cudaFuncSetAttribute(qmm_tc_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return fail(B200Q_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
-    qmm_tc_kernel<BITS><<<grid, kThreads, smem, st>>>(map_x, map_w, p);
-    rc = B200Q_OK;
+    n = f == Form::Round ? fixed_smem<BITS, Form::Round>(cb)
+                         : (f == Form::Split ? fixed_smem<BITS, Form::Split>(cb) : fixed_smem<BITS, Form::SplitT>(cb));
   });
-  if (rc != B200Q_OK) return fail(rc, "[quantized_matmul] unsupported bits %d", bits);
+  return n;
+}
+
+// Token width of a tile and number of parts of K: the pair with the least estimated time.  A stage takes
+// the longer of its MMAs (4 cycles per token, 8 when split) and of its unpacking; a tile adds the
+// exposed part of its epilogue, and a shared tile the trip of its partial sums through L2.
+struct TcPlan {
+  int nt, m_tiles, n_tiles, splits;
+};
+TcPlan tc_plan(int64_t M, int64_t N, int64_t K, Form f) {
+  TcPlan best{};
+  double best_t = 1e300;
+  const int pairs = sm_pairs();
+  const int kst = (int)((K + kStageK - 1) / kStageK);
+  const int n_tiles = (int)((N + 2 * kTileRows - 1) / (2 * kTileRows));
+  const int cap = (int)(M >= 256 ? 256 : (M + 31) / 32 * 32);
+  for (int nt = cap; nt >= 32; nt -= 32) {
+    const int64_t m_tiles = (M + nt - 1) / nt;
+    const int64_t tiles = m_tiles * n_tiles;
+    const double stage = f == Form::Round ? (4.0 * nt > 800 ? 4.0 * nt : 800.0) : (8.0 * nt > 1000 ? 8.0 * nt : 1000.0);
+    for (int s = 1; s == 1 || (s <= 16 && s * 4 <= kst); ++s) {
+      if (s > 1 && tiles * s > pairs) break;
+      const double waves = (double)((tiles * s + pairs - 1) / pairs);
+      const double tile = (kst + s - 1) / s * stage + (nt <= kAccCols / 2 ? 1000.0 : 1000.0 + 6.0 * nt) + (s > 1 ? 3000.0 + 8.0 * nt * s : 0.0);
+      if (waves * tile < best_t) {
+        best_t = waves * tile;
+        best = TcPlan{nt, (int)m_tiles, n_tiles, s};
+      }
+    }
+  }
+  return best;
+}
+
+size_t split_bytes(const TcPlan& pl) {
+  if (pl.splits == 1) return 0;
+  const size_t tiles = (size_t)pl.m_tiles * pl.n_tiles;
+  return (tiles * 2 * 4 + 255) / 256 * 256 + tiles * pl.splits * 2 * pl.nt * kTileRows * 4;
+}
+
+// x maps (boxes of 128, 64, 32 and 16 rows of 64 k) and the map of the packed matrix.
+int encode_maps(TcMaps& m, const char* tag, const void* x, int64_t x_rows, int64_t K, int dtype, const void* wq,
+                int64_t w_rows, int64_t w_row_bytes, int bits) {
+  EncodeFn enc = encode_fn();
+  if (!enc) return fail(B200Q_ERR_CUDA, "[%s] cuTensorMapEncodeTiled is not available", tag);
+  if (int rc = bind_context()) return rc;
+  const cuuint32_t estr[2] = {1, 1};
+  for (int i = 0; i < 4; ++i) {
+    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)x_rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+    const cuuint32_t box[2] = {64, (cuuint32_t)(128 >> i)};
+    CUresult r = enc(&m.x[i], dtype == B200Q_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
+                     const_cast<void*>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[%s] tensor map for x failed (%d)", tag, (int)r);
+  }
+  const cuuint64_t dims[2] = {(cuuint64_t)w_row_bytes, (cuuint64_t)w_rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)w_row_bytes};
+  const cuuint32_t box[2] = {(cuuint32_t)(16 * bits), (cuuint32_t)kTileRows};
+  const CUtensorMapSwizzle sw = bits == 2 ? CU_TENSOR_MAP_SWIZZLE_32B : (bits == 4 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                : (bits == 8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE));
+  CUresult r = enc(&m.w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(wq), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[%s] tensor map for w failed (%d)", tag, (int)r);
+  return B200Q_OK;
+}
+
+template <typename T, int BITS, Form F>
+int launch_one(unsigned grid, size_t smem, cudaStream_t st, const TcMaps& maps, const TcParams& p) {
+  B200Q_CUDA_OK(cudaFuncSetAttribute(qmm_tc_kernel<T, BITS, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
+  qmm_tc_kernel<T, BITS, F><<<grid, kThreads, smem, st>>>(maps, p);
   B200Q_LAUNCH_OK("qmm_tc_kernel");
   return B200Q_OK;
 }
 
-}  // namespace
-
-bool qmm_tc_supported(const QmmArgs& a) {
-  if (a.dtype != B200Q_BF16 || !a.transpose || a.w_batched || a.batch != 1) return false;
-  if (a.M < 1 || a.N < 1 || a.K < 128 || a.K % 128 != 0) return false;  // packed stages hold 128 k
-  if (a.K % a.group != 0) return false;
-  // TMA: 16-byte aligned bases and row pitches (x rows: 2K bytes, packed rows: K/2 bytes)
-  if ((reinterpret_cast<uintptr_t>(a.x) & 15) || (reinterpret_cast<uintptr_t>(a.wq) & 15)) return false;
-  if ((a.K * 2) % 16 != 0 || (a.K * a.bits / 8) % 16 != 0) return false;
-  return true;
+// Completes the parameters that depend on the shape of the kernel and launches it for `units` units of work.
+int launch_tc(int dtype, int bits, int group, Form f, long long units, cudaStream_t st, const TcMaps& maps, TcParams& p) {
+  p.g4 = kTileRows / group;
+  p.spc = 1;
+  if (f != Form::SplitT)
+    while (p.spc < 4 && p.spc * p.g4 < 8 && p.row_groups % (2 * p.spc * p.g4) == 0 &&
+           ((reinterpret_cast<uintptr_t>(p.scales) | reinterpret_cast<uintptr_t>(p.biases)) % (4 * p.spc * p.g4)) == 0)
+      p.spc *= 2;
+  p.cb = p.spc * p.g4 * 2 < 4 ? 4 : p.spc * p.g4 * 2;
+  const size_t fixed = fixed_smem(bits, f, p.cb);
+  const size_t stage = (size_t)p.NT * 128;
+  long long nsb = (long long)((kSmemMax - fixed) / stage);
+  p.nsb = (int)(nsb > kMaxStagesB ? kMaxStagesB : nsb);
+  size_t smem = fixed + p.nsb * stage;
+  // More than half of an SM's shared memory: guarantees one block per SM, so the 512-column
+  // tensor-memory allocation never has to wait for a co-resident block of this kernel.
+  if (smem < 120 * 1024) smem = 120 * 1024;
+  const long long pairs = sm_pairs();
+  const unsigned grid = 2u * (unsigned)(units < pairs ? units : pairs);
+  int rc = fail(B200Q_ERR_UNSUPPORTED, "[quantized_matmul] unsupported bits %d", bits);
+  B200Q_DISPATCH_BITS(bits, BITS, {
+    if (f == Form::Round) rc = launch_one<__nv_bfloat16, BITS, Form::Round>(grid, smem, st, maps, p);
+    else if (f == Form::Split) rc = launch_one<__half, BITS, Form::Split>(grid, smem, st, maps, p);
+    else if (dtype == B200Q_BF16) rc = launch_one<__nv_bfloat16, BITS, Form::SplitT>(grid, smem, st, maps, p);
+    else rc = launch_one<__half, BITS, Form::SplitT>(grid, smem, st, maps, p);
+  });
+  return rc;
 }
 
-size_t qmm_tc_workspace_bytes(const QmmArgs&) { return kStatusBytes; }
+void set_outputs(TcParams& p, const PeerOut& peers, void* y, int64_t ld) {
+  if (peers.n > 0) {
+    p.n_out = peers.n; p.ld = peers.ld; p.col0 = peers.col0;
+    for (int q = 0; q < peers.n; ++q) p.y_out[q] = peers.y[q];
+    p.sig = peers.sig;
+  } else {
+    p.n_out = 1; p.ld = ld; p.col0 = 0; p.y_out[0] = y;
+  }
+}
+
+}  // namespace
+
+// bf16 or f16, one matrix.  Transposed: whole stages of 128 k.  Not transposed: whole blocks of 128
+// columns (a tile row of the packed matrix) and a row pitch of x that TMA takes.
+bool qmm_tc_supported(const QmmArgs& a) {
+  if ((a.dtype != B200Q_BF16 && a.dtype != B200Q_F16) || a.w_batched || a.batch != 1) return false;
+  if (a.M < 1 || a.N < 1 || a.K < 1 || a.M > (1 << 30) || a.N > (1 << 30)) return false;
+  if ((a.transpose ? a.K : a.N) % kStageK != 0 || a.K % 8 != 0) return false;
+  // TMA: 16-byte aligned bases and row pitches
+  if ((reinterpret_cast<uintptr_t>(a.x) & 15) || (reinterpret_cast<uintptr_t>(a.wq) & 15)) return false;
+  return !((reinterpret_cast<uintptr_t>(a.scales) | reinterpret_cast<uintptr_t>(a.biases)) & 7);
+}
+
+size_t qmm_tc_workspace_bytes(const QmmArgs& a) {
+  return split_bytes(tc_plan(a.M, a.N, a.K, form_of(a.dtype, a.transpose))) + kStatusBytes;
+}
 
 int qmm_tc(const QmmArgs& a, cudaStream_t st) {
-  EncodeFn enc = encode_fn();
-  if (!enc) return fail(B200Q_ERR_CUDA, "[quantized_matmul] cuTensorMapEncodeTiled is not available");
   if (!a.ws || a.ws_bytes < kStatusBytes)
     return fail(B200Q_ERR_WORKSPACE, "[quantized_matmul] workspace of %zu bytes required, %zu given",
                 (size_t)kStatusBytes, a.ws_bytes);
-  const int nt = pick_nt(a.M);
-  CUtensorMap map_x, map_w;
-  {
-    const cuuint64_t dims[2] = {(cuuint64_t)a.K, (cuuint64_t)a.M};
-    const cuuint64_t strides[1] = {(cuuint64_t)a.K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)kBlockK, (cuuint32_t)nt};
-    const cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(&map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(a.x), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[quantized_matmul] tensor map for x failed (%d)", (int)r);
-  }
-  {
-    const cuuint64_t dims[2] = {(cuuint64_t)a.K * a.bits / 8, (cuuint64_t)a.N};
-    const cuuint64_t strides[1] = {(cuuint64_t)a.K * a.bits / 8};
-    const cuuint32_t box[2] = {(cuuint32_t)(16 * a.bits), (cuuint32_t)kTileN};
-    const cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint32_t*>(a.wq), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[quantized_matmul] tensor map for w failed (%d)", (int)r);
-  }
+  const Form f = form_of(a.dtype, a.transpose);
+  TcPlan pl = tc_plan(a.M, a.N, a.K, f);
+  if (a.ws_bytes < split_bytes(pl) + kStatusBytes) pl.splits = 1;   // a caller's smaller workspace: no shared tiles
+  const int64_t qaxis = a.transpose ? a.K : a.N;
+  TcMaps maps;
+  if (int rc = encode_maps(maps, "quantized_matmul", a.x, a.M, a.K, a.dtype, a.wq, a.transpose ? a.N : a.K,
+                           qaxis * a.bits / 8, a.bits))
+    return rc;
   TcParams p{};
-  p.scales = (const __nv_bfloat16*)a.scales;
-  p.biases = (const __nv_bfloat16*)a.biases;
-  p.y = (__nv_bfloat16*)a.y;
-  if (a.peers.n > 0) {
-    p.n_out = a.peers.n; p.ld = a.peers.ld; p.col0 = a.peers.col0;
-    for (int q = 0; q < a.peers.n; ++q) p.y_out[q] = (__nv_bfloat16*)a.peers.y[q];
-    p.sig = a.peers.sig;
-  } else {
-    p.n_out = 1; p.ld = a.N; p.col0 = 0; p.y_out[0] = (__nv_bfloat16*)a.y;
-  }
+  p.scales = (const unsigned short*)a.scales;
+  p.biases = (const unsigned short*)a.biases;
+  set_outputs(p, a.peers, a.y, a.N);
   p.status = reinterpret_cast<uint32_t*>(static_cast<char*>(a.ws) + a.ws_bytes - kStatusBytes);
   p.M = (int)a.M; p.N = (int)a.N; p.K = (int)a.K;
-  p.NT = nt;
-  p.nsb = x_stages(nt, (int)a.bits);
-  p.n_tiles = (int)((a.N + kTileN - 1) / kTileN);
-  p.m_tiles = (int)((a.M + nt - 1) / nt);
-  p.group_shift = a.group == 32 ? 0 : (a.group == 64 ? 1 : 2);
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long tiles = (long long)p.n_tiles * p.m_tiles;
-  const int grid = (int)(tiles < sms ? tiles : sms);
-  return launch_tc(a.bits, grid, smem_bytes(nt, a.bits), st, map_x, map_w, p);
+  p.NT = pl.nt; p.m_tiles = pl.m_tiles; p.n_tiles = pl.n_tiles; p.splits = pl.splits;
+  p.counters = static_cast<uint32_t*>(a.ws);
+  p.partial = reinterpret_cast<float*>(static_cast<char*>(a.ws) + ((size_t)pl.m_tiles * pl.n_tiles * 8 + 255) / 256 * 256);
+  p.row_groups = (int)(qaxis / a.group);
+  p.n_scales = (a.transpose ? a.N : a.K) * p.row_groups;
+  return launch_tc(a.dtype, a.bits, a.group, f, (long long)pl.m_tiles * pl.n_tiles * pl.splits, st, maps, p);
 }
 
 int qmm_tc_grouped(const GroupedArgs& a, cudaStream_t st) {
-  EncodeFn enc = encode_fn();
-  if (!enc) return fail(B200Q_ERR_CUDA, "[gather_qmm] cuTensorMapEncodeTiled is not available");
-  const int nt = a.nt;
-  CUtensorMap map_x, map_w;
-  {
-    const cuuint64_t dims[2] = {(cuuint64_t)a.K, (cuuint64_t)a.n_rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)a.K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)kBlockK, (cuuint32_t)nt};
-    const cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(&map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(a.x_sorted), dims, strides, box,
-                     estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[gather_qmm] tensor map for x failed (%d)", (int)r);
-  }
-  {
-    const cuuint64_t dims[2] = {(cuuint64_t)a.K * a.bits / 8, (cuuint64_t)(a.E * a.N)};
-    const cuuint64_t strides[1] = {(cuuint64_t)a.K * a.bits / 8};
-    const cuuint32_t box[2] = {(cuuint32_t)(16 * a.bits), (cuuint32_t)kTileN};
-    const cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint32_t*>(a.wq), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[gather_qmm] tensor map for w failed (%d)", (int)r);
-  }
+  TcMaps maps;
+  if (int rc = encode_maps(maps, "gather_qmm", a.x_sorted, a.n_rows, a.K, B200Q_BF16, a.wq, a.E * a.N, a.K * a.bits / 8, a.bits))
+    return rc;
   TcParams p{};
   p.mtiles = static_cast<const MTile*>(a.mtiles);
   p.n_mtiles = a.n_mtiles;
   p.dst_row = a.dst_row;
-  p.scales = (const __nv_bfloat16*)a.scales;
-  p.biases = (const __nv_bfloat16*)a.biases;
-  p.y = (__nv_bfloat16*)a.y;
-  if (a.peers.n > 0) {
-    p.n_out = a.peers.n;
-    for (int q = 0; q < a.peers.n; ++q) p.y_out[q] = (__nv_bfloat16*)a.peers.y[q];
-    p.sig = a.peers.sig;
-  } else {
-    p.n_out = 1; p.y_out[0] = (__nv_bfloat16*)a.y;
-  }
+  p.scales = (const unsigned short*)a.scales;
+  p.biases = (const unsigned short*)a.biases;
+  set_outputs(p, a.peers, a.y, a.N);
   p.ld = a.N; p.col0 = 0;
   p.status = a.status;
   p.M = (int)a.n_rows; p.N = (int)a.N; p.K = (int)a.K;
-  p.NT = nt;
-  p.nsb = x_stages(nt, (int)a.bits);
-  p.n_tiles = (int)((a.N + kTileN - 1) / kTileN);
-  p.m_tiles = 0;
-  p.group_shift = a.group == 32 ? 0 : (a.group == 64 ? 1 : 2);
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long tiles = (long long)p.n_tiles * a.max_mtiles;  // upper bound; the kernel reads the exact count
-  const int grid = (int)(tiles < sms ? tiles : sms);
-  return launch_tc(a.bits, grid, smem_bytes(nt, a.bits), st, map_x, map_w, p);
+  p.NT = a.nt; p.m_tiles = 0; p.splits = 1;
+  p.n_tiles = (int)((a.N + 2 * kTileRows - 1) / (2 * kTileRows));
+  p.row_groups = (int)(a.K / a.group);
+  p.n_scales = a.E * a.N * p.row_groups;
+  // an upper bound of the units; the kernel reads the exact count
+  return launch_tc(B200Q_BF16, a.bits, a.group, Form::Round, (long long)p.n_tiles * a.max_mtiles, st, maps, p);
 }
-
-size_t qmm_tc_mtile_bytes() { return sizeof(MTile); }
 
 }  // namespace b200q

@@ -1,0 +1,79 @@
+"""The tensor-core kernel at the edges of its tiles: every way it forms the weight operand (bf16 rounded, f16
+split in two, packed along the output columns), against the oracle's fp32 accumulation.
+
+Sizes: one stage of 128 k and odd numbers of stages, token counts around 32, 128 and 256, output columns that
+end inside a block's or a pair's half of a tile, one scale per stage at an odd position of its 4-byte
+word, and few tiles with a long K (K shared by several pairs of thread blocks)."""
+import pytest
+import torch
+
+import mlx_b200 as mb
+import oracle as O
+from util import from_torch, make_w, make_x, qmm_close, to_torch, u32_to_torch
+
+pytestmark = pytest.mark.gpu
+DT = {"bf16": torch.bfloat16, "f16": torch.float16}
+
+
+def check(dtype, M, N, K, g, bits, transpose, rel):
+    w = make_w(M + N, (N, K) if transpose else (K, N), dtype)
+    wq, s, b = O.quantize(w, g, bits, dtype)
+    x = make_x(M + K, (M, K), dtype)
+    assert mb.qmm_kernel_name(DT[dtype], M, N, K, g, bits, transpose) == "qmm_tcgen05"
+    ref = O.qmm_f32_from(x, wq, s, b, dtype, transpose=transpose, group_size=g, bits=bits)
+    args = (to_torch(x, dtype), u32_to_torch(wq), to_torch(s, dtype), to_torch(b, dtype))
+    for _ in range(2):   # the second call finds the counters and partial sums the first has left
+        y = mb.quantized_matmul(*args, transpose=transpose, group_size=g, bits=bits)
+    ok, err = qmm_close(O.to_f32(from_torch(y), dtype), ref, rel)
+    assert ok, err
+
+
+@pytest.mark.parametrize("bits", (2, 3, 4, 5, 6, 8))
+@pytest.mark.parametrize("M,N,K,g", [(33, 130, 128, 128), (96, 257, 384, 128), (257, 385, 640, 64), (129, 128, 1152, 32)])
+def test_transposed(bits, M, N, K, g):
+    check("bf16", M, N, K, g, bits, True, 1e-2)
+    check("f16", M, N, K, g, bits, True, 2e-3)   # the weights keep their fp32 value: only the result is rounded
+
+
+@pytest.mark.parametrize("dtype,rel", [("bf16", 6e-3), ("f16", 2e-3)])
+@pytest.mark.parametrize("bits", (2, 3, 4, 5, 6, 8))
+@pytest.mark.parametrize("M,N,K,g", [(17, 128, 8, 128), (33, 384, 200, 64), (257, 256, 136, 32), (128, 640, 1000, 128)])
+def test_not_transposed(dtype, rel, bits, M, N, K, g):
+    check(dtype, M, N, K, g, bits, False, rel)
+
+
+@pytest.mark.parametrize("dtype", ("bf16", "f16"))
+@pytest.mark.parametrize("M,N,K,g,bits", [(57, 512, 8192, 64, 4), (40, 300, 5504, 128, 3), (200, 256, 4224, 32, 8)])
+def test_k_shared_by_pairs_of_blocks(dtype, M, N, K, g, bits):
+    check(dtype, M, N, K, g, bits, True, 1e-2)
+
+
+@pytest.mark.parametrize("bits", (5, 6, 8))
+def test_experts_with_an_odd_number_of_stages(bits):
+    """Nine stages per tile and several tiles per pair of blocks: the unpack warps' turns cross tile borders."""
+    E, tokens, N, K, g = 16, 96, 640, 1152, 64
+    wq, s, b = O.quantize(make_w(5, (E, N, K), "bf16"), g, bits, "bf16")
+    x = to_torch(make_x(6, (tokens, 1, K), "bf16"), "bf16")
+    wt, st, bt = u32_to_torch(wq), to_torch(s, "bf16"), to_torch(b, "bf16")
+    rhs = torch.arange(tokens, device="cuda") * 7 % E
+    y = mb.gather_qmm(x, wt, st, bt, rhs_indices=rhs, group_size=g, bits=bits)
+    for e in range(E):
+        rows = torch.nonzero(rhs == e).flatten()
+        ref = O.qmm_f32_from(from_torch(x[rows, 0]), wq[e], s[e], b[e], "bf16", transpose=True, group_size=g, bits=bits)
+        ok, err = qmm_close(O.to_f32(from_torch(y[rows, 0]), "bf16"), ref)
+        assert ok, (e, err)
+
+
+def test_autograd_worker_thread():
+    """The backward pass runs in a thread of its own, which has made no CUDA call yet."""
+    from mlx_b200 import grad
+
+    M, N, K = 64, 256, 384
+    wq, s, b = O.quantize(make_w(8, (N, K), "bf16"), 64, 4, "bf16")
+    x = to_torch(make_x(9, (M, K), "bf16"), "bf16").requires_grad_(True)
+    dy = make_x(10, (M, N), "bf16")
+    y = grad.quantized_matmul(x, u32_to_torch(wq), to_torch(s, "bf16"), to_torch(b, "bf16"))
+    dx, = torch.autograd.grad(y, x, to_torch(dy, "bf16"))
+    ref = O.qmm_f32_from(dy, wq, s, b, "bf16", transpose=False, group_size=64, bits=4)
+    ok, err = qmm_close(O.to_f32(from_torch(dx), "bf16"), ref)
+    assert ok, err
