@@ -13,5 +13,6 @@ def __getattr__(name):
     if name in __all__:
         from . import ops
 
-        return getattr(ops, name)
+        globals()[name] = value = getattr(ops, name)   # the next look-up finds it without coming here
+        return value
     raise AttributeError(name)

@@ -3,6 +3,7 @@
 Each .cu file is compiled to an object in mlx_b200/_obj/ (in parallel, rebuilt only
 when the source or a header is newer) and linked into mlx_b200/libb200q.so.  nvcc
 cross-compiles without a GPU, so this runs anywhere the CUDA toolkit is installed.
+csrc/front.cpp becomes the Python extension mlx_b200/_front.so (g++ against torch's headers).
 
     python -m mlx_b200.build [--force] [--verbose]
 """
@@ -19,6 +20,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_obj")
 LIB = os.path.join(HERE, "libb200q.so")
+FRONT = os.path.join(HERE, "_front.so")   # Python extension over LIB (csrc/front.cpp)
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 NVCC_FLAGS = [*os.environ.get("B200Q_EXTRA_NVCC", "").split(),
@@ -82,7 +84,24 @@ def build(force: bool = False, verbose: bool = False) -> str:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError("link failed:\n" + res.stdout + res.stderr)
+    front_src = os.path.join(CSRC, "front.cpp")
+    if force or not os.path.exists(FRONT) or os.path.getmtime(FRONT) < max(os.path.getmtime(front_src), hdr):
+        _build_front(front_src)
     return LIB
+
+
+def _build_front(src: str) -> None:
+    import sysconfig
+
+    from torch.utils import cpp_extension as ce
+
+    inc = [f"-I{p}" for p in (*ce.include_paths(), sysconfig.get_paths()["include"], "/usr/local/cuda/include", INCLUDE)]
+    libs = [f"-L{p}" for p in ce.library_paths()] + ["-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", *inc, src, "-o", FRONT, *libs,
+           f"-L{HERE}", "-l:libb200q.so", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("building the native front-end failed:\n" + (res.stdout + res.stderr)[-4000:])
 
 
 if __name__ == "__main__":

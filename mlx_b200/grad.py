@@ -50,6 +50,9 @@ def quantized_matmul(x: torch.Tensor, w: torch.Tensor, scales: torch.Tensor, bia
                      transpose: bool = True, group_size: Optional[int] = None, bits: Optional[int] = None,
                      mode: str = "affine") -> torch.Tensor:
     """ops.quantized_matmul with autograd support for x, scales and biases."""
+    y = ops._front.qmm_grad(x, w, scales, biases, transpose, group_size, bits, mode)   # frozen scales and biases
+    if y is not None:
+        return y
     group_size, bits = ops._mode_params(mode, group_size, bits, "quantized_matmul")
     return _QuantizedMatmulFn.apply(x, w, scales, biases, transpose, group_size, bits)
 

@@ -17,6 +17,10 @@ import torch
 
 from . import _lib
 
+_lib.load()   # with its symbols present, and its message if it is not built
+from . import _front  # noqa: E402  (the native form of the ordinary calls: csrc/front.cpp)
+
+_SCRATCH_OPS = {"qmm": 0, "gather": 1}
 _DT = {torch.float32: _lib.F32, torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}
 _MODES = ("affine", "mxfp4", "mxfp8", "nvfp4")
 
@@ -62,6 +66,7 @@ class _Workspaces:
             with torch.cuda.device(dev):
                 buf = torch.zeros(max(nbytes, 256), dtype=torch.uint8, device=dev)
             self._bufs[key] = buf
+            _front.scratch(dev.index, key[1], _SCRATCH_OPS[op], buf.data_ptr(), buf.numel())
         return buf
 
 
@@ -184,6 +189,9 @@ def _extract_dims(tag, x, w, scales, biases, transpose, group_size, bits):
 def quantize(w: torch.Tensor, group_size: Optional[int] = None, bits: Optional[int] = None,
              mode: str = "affine"):
     """-> (w_q uint32 [..., K*bits/32], scales [..., K/g], biases [..., K/g]); mlx/ops.cpp:5208."""
+    q = _front.quantize(w, group_size, bits, mode)
+    if q is not None:
+        return q
     group_size, bits = _mode_params(mode, group_size, bits, "quantize")
     if not w.dtype.is_floating_point or w.dtype not in _DT:
         raise ValueError(f"[quantize] Only real floating types can be quantized but w has type {w.dtype}.")
@@ -225,6 +233,10 @@ def dequantize(w: torch.Tensor, scales: torch.Tensor, biases: Optional[torch.Ten
                group_size: Optional[int] = None, bits: Optional[int] = None, mode: str = "affine",
                dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """mlx/ops.cpp:5465-5517 (+ affine_dequantize :5258-5340)."""
+    if dtype is None or dtype == scales.dtype:
+        out = _front.dequantize(w, scales, biases, group_size, bits, mode)
+        if out is not None:
+            return out
     group_size, bits = _mode_params(mode, group_size, bits, "dequantize")
     out_type = _validate_mode_with_type("dequantize", scales, biases, dtype)
     if bits <= 0:
@@ -318,6 +330,9 @@ def quantized_matmul(x: torch.Tensor, w: torch.Tensor, scales: torch.Tensor,
                      group_size: Optional[int] = None, bits: Optional[int] = None,
                      mode: str = "affine") -> torch.Tensor:
     """mlx/ops.cpp:4784-4834.  x [..., M, K] (or [K]); w [..., N, K*bits/32] when transposed."""
+    y = _front.qmm(x, w, scales, biases, transpose, group_size, bits, mode)
+    if y is not None:
+        return y
     group_size, bits = _mode_params(mode, group_size, bits, "quantized_matmul")
     dtype = _validate_mode_with_type("quantized_matmul", scales, biases, None)
     _, w_outer = _extract_dims("quantized_matmul", x, w, scales, biases, transpose, group_size, bits)
