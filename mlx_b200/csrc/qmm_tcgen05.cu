@@ -68,9 +68,9 @@ enum class Form { Round, Split, SplitT };
 constexpr int kTileRows = 128;    // output columns per block and tile (MMA M = 256 over the pair)
 constexpr int kStageK = 128;      // k per pipeline stage of x, W, scales
 constexpr int kMaxStagesB = 6;
-constexpr int kMaxStagesP = 4;
+constexpr int kMaxStagesP = 8;
 constexpr int kMaxSlotsA = 4;
-constexpr int kSlotsS = 4;        // chunks of scales and biases
+constexpr int kMaxSlotsS = 4;     // chunks of scales and biases: 2 of four stages, else 4
 constexpr int kDoneRing = 16;     // one commit per A slot; longer than any distance a waiter can be behind
 constexpr int kTmemCols = 512;    // [0, 256) accumulators, [256, 512) A ring (4 slots of 64 columns)
 constexpr int kAccCols = 256;
@@ -78,6 +78,7 @@ constexpr int kUnpackWarps = 16;
 constexpr int kEpilogueWarps = 8;
 constexpr int kFirstUnpack = 4, kFirstEpilogue = kFirstUnpack + kUnpackWarps;
 constexpr int kThreads = 32 * (kFirstEpilogue + kEpilogueWarps);   // 896
+constexpr int kStageOut = 4096;    // bytes of the epilogue's staging tile per warp: 64 tokens x 32 columns
 constexpr size_t kSmemMax = 227 * 1024;
 
 template <int BITS, Form F>
@@ -86,7 +87,9 @@ struct Shape {
   static constexpr int kSub = F == Form::Round ? 1 : 2;        // A slots per stage (64 k each when split)
   static constexpr int kSlotsA = kT ? 3 : 4;
   static constexpr int kSets = kT ? 2 : 4;                     // sets of unpack warps, on A slots in turn
-  static constexpr int kStagesP = !kT ? 4 : (BITS <= 4 ? 3 : 2);
+  // Packed stages: four sets hold one each while they unpack; with no more than that every set would wait for a
+  // whole TMA latency after each slot.
+  static constexpr int kStagesP = kT ? (BITS == 8 ? 2 : 3) : (BITS <= 4 ? 8 : (BITS == 8 ? 5 : 6));
   static constexpr int kPRowBytes = 16 * BITS;                 // 128 fields
   static constexpr int kPStageBytes = kTileRows * kPRowBytes;
   static constexpr int kSmemA = kT ? kSlotsA * 32768 : 0;      // 64 k x 128 columns, hi and lo
@@ -144,13 +147,14 @@ struct TcParams {
   uint32_t* counters;   // [tile][block of the pair]
   int g4;            // groups per 128 fields of a row: 4, 2, 1
   int row_groups;    // groups per packed row
+  int s_slots;       // chunks of scales in their ring
   int spc, cb;       // stages per chunk of scales, bytes per row of a chunk (4, 8 or 16)
   long long n_scales;   // elements of `scales`
 };
 
 struct __align__(8) Barriers {
   uint64_t full_p[kMaxStagesP], empty_p[kMaxStagesP];
-  uint64_t full_s[kSlotsS], empty_s[kSlotsS];
+  uint64_t full_s[kMaxSlotsS], empty_s[kMaxSlotsS];
   // Of the pair's leader: x tiles of both blocks have landed; both blocks' unpack warps have filled an A slot
   uint64_t full_b[kMaxStagesB];
   uint64_t full_a[kMaxSlotsA];
@@ -362,15 +366,19 @@ __device__ __forceinline__ Unit unit_at(const TcParams& p, int u, int rank) {
   Unit t;
   const int kst = p.K / kStageK + (p.K % kStageK != 0);
   if (p.mtiles == nullptr) {
-    const int tile = u / p.splits, sp = u - tile * p.splits;
-    const int tn = tile / p.m_tiles, tm = tile - tn * p.m_tiles;
+    const int tile = p.splits == 1 ? u : u / p.splits, sp = u - tile * p.splits;
+    const int tn = p.m_tiles == 1 ? tile : tile / p.m_tiles, tm = tile - tn * p.m_tiles;
     t.n0 = tn * (2 * kTileRows) + rank * kTileRows;
     t.w_row0 = t.n0;
     t.w_row_end = p.N;
     t.x_row0 = tm * p.NT;
     t.rows = min(p.M - t.x_row0, p.NT);
-    t.ks0 = sp * (kst / p.spc) / p.splits * p.spc;   // whole chunks of scales
-    t.ks1 = (sp + 1) * (kst / p.spc) / p.splits * p.spc;
+    t.ks0 = 0;
+    t.ks1 = kst;
+    if (p.splits > 1) {                              // whole chunks of scales
+      t.ks0 = sp * (kst / p.spc) / p.splits * p.spc;
+      t.ks1 = (sp + 1) * (kst / p.spc) / p.splits * p.spc;
+    }
   } else {
     const int g = u / p.n_tiles, tn = u - g * p.n_tiles;
     const MTile mt = p.mtiles[g];
@@ -387,25 +395,47 @@ __device__ __forceinline__ Unit unit_at(const TcParams& p, int u, int rank) {
   return t;
 }
 
-// Columns c .. c+lim of the tile's tokens for output column n, one value per lane.
+// Epilogue of 32 output columns (one warp): the accumulator comes as mma fragments, is rounded in pairs, transposed
+// through shared memory (stmatrix; 64 bytes per token, 16-byte chunks xor-ed with token / 2) and leaves as
+// 16-byte stores, 64 contiguous bytes per token.  While an accumulator that has no twin is being read, the tensor
+// pipe waits: 64 tokens are staged with one load in flight ahead of the one being rounded, and stored after.
 template <typename T>
-__device__ __forceinline__ void store_chunk(const TcParams& p, const Unit& t, int n, int c, int lim, const uint32_t (&v)[32]) {
-  if (p.dst_row == nullptr) {
-    for (int q = 0; q < p.n_out; ++q) {
-      T* yp = static_cast<T*>(p.y_out[q]) + (size_t)(t.x_row0 + c) * p.ld + p.col0 + n;
+__device__ __forceinline__ uint32_t pack_pair(uint32_t a, uint32_t b) {
+  uint32_t d;
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(__uint_as_float(b)), "f"(__uint_as_float(a)));
+  else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(__uint_as_float(b)), "f"(__uint_as_float(a)));
+  return d;
+}
+__device__ __forceinline__ void load_piece(uint32_t tmem, uint32_t (&r)[16]) {   // 32 lanes x 16 columns
+  tcgen05_ld_16x16(tmem, r);
+  tcgen05_ld_16x16(tmem + (16u << 16), r + 8);
+}
+template <typename T>
+__device__ __forceinline__ void stage_piece(uint32_t stg, int lane, const uint32_t (&r)[16]) {
+  const uint32_t row = lane & 7, at = stg + row * 64 + ((((uint32_t)lane >> 3) ^ (row >> 1)) << 4);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        if (j < lim) *yp = Elem<T>::from_float(__uint_as_float(v[j]));
-        yp += p.ld;
+  for (int i = 0; i < 2; ++i)
+    stmatrix_x4_trans(at + i * 512, pack_pair<T>(r[4 * i], r[4 * i + 1]), pack_pair<T>(r[4 * i + 2], r[4 * i + 3]),
+                      pack_pair<T>(r[8 + 4 * i], r[8 + 4 * i + 1]), pack_pair<T>(r[8 + 4 * i + 2], r[8 + 4 * i + 3]));
+}
+template <typename T>
+__device__ __forceinline__ void store_chunk(const TcParams& p, const Unit& t, uint32_t stg, int lane, int n0, int c, int lim) {
+  const int n = n0 + (lane & 3) * 8;
+  const bool whole = n + 8 <= p.N;
+  if (n >= p.N) return;
+  for (int tok = lane >> 2; tok < lim; tok += 8) {
+    uint4 v;
+    lds_v4(stg + tok * 64 + (((lane & 3) ^ ((tok >> 1) & 3)) << 4), v.x, v.y, v.z, v.w);
+    const int m = t.x_row0 + c + tok;
+    const long long at = (long long)(p.dst_row ? p.dst_row[m] : m) * p.ld + p.col0 + n;
+    for (int q = 0; q < p.n_out; ++q) {
+      T* dst = static_cast<T*>(p.y_out[q]) + at;
+      if (whole && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+        *reinterpret_cast<uint4*>(dst) = v;
+      } else {
+        const T* e = reinterpret_cast<const T*>(&v);
+        for (int j = 0; j < 8 && n + j < p.N; ++j) dst[j] = e[j];
       }
-    }
-  } else {
-    const int* dr = p.dst_row + t.x_row0 + c;
-    for (int q = 0; q < p.n_out; ++q) {
-      T* yq = static_cast<T*>(p.y_out[q]) + n;
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (j < lim) yq[(size_t)dr[j] * p.ld] = Elem<T>::from_float(__uint_as_float(v[j]));
     }
   }
 }
@@ -424,18 +454,24 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   unsigned char* ring_b = smem + S::kSmemA;
   unsigned char* ring_p = ring_b + (size_t)p.nsb * b_stage;
   unsigned char* ring_s = ring_p + (size_t)kStagesP * S::kPStageBytes;   // per chunk: 128 rows of scales, 128 of biases
-  Barriers* bars = reinterpret_cast<Barriers*>(ring_s + kSlotsS * 2 * kTileRows * p.cb);
+  unsigned char* staging = ring_s + p.s_slots * 2 * kTileRows * p.cb;    // a tile per epilogue warp
+  Barriers* bars = reinterpret_cast<Barriers*>(staging + kEpilogueWarps * kStageOut);
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_rank();
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-  const int total = p.mtiles ? *p.n_mtiles * p.n_tiles : p.n_tiles * p.m_tiles * p.splits;
   const int nacc = p.NT <= kAccCols / 2 ? 2 : 1;
 
+  asm volatile("griddepcontrol.launch_dependents;");
+  if (threadIdx.x == 32 * 3) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.w) : "memory");
+#pragma unroll
+    for (int i = 0; i < 4; ++i) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.x[i]) : "memory");
+  }
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStagesP; ++i) { mbar_init(smem_u32(&bars->full_p[i]), 1); mbar_init(smem_u32(&bars->empty_p[i]), S::kPArrivals); }
-    for (int i = 0; i < kSlotsS; ++i) {
+    for (int i = 0; i < p.s_slots; ++i) {
       mbar_init(smem_u32(&bars->full_s[i]), 32);
       mbar_init(smem_u32(&bars->empty_s[i]), p.spc * S::kPArrivals);
     }
@@ -454,6 +490,9 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   __syncthreads();
   cluster_sync();
   tcgen05_fence_after();
+  // The set-up above runs while the previous kernel of the stream drains; nothing of memory is touched before this.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int total = p.mtiles ? *p.n_mtiles * p.n_tiles : p.n_tiles * p.m_tiles * p.splits;
   const uint32_t tmem_base = bars->tmem_base;
   const uint32_t tmem_a = tmem_base + kAccCols;
 
@@ -605,7 +644,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           }
         }
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->full_s[ss])) : "memory");
-        if (++ss == (uint32_t)kSlotsS) { ss = 0; ps ^= 1; }
+        if (++ss == (uint32_t)p.s_slots) { ss = 0; ps ^= 1; }
       }
     }
   } else if (warp < kFirstEpilogue) {
@@ -624,6 +663,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     const uint32_t t_slot = tmem_a + ((uint32_t)(quad * 32) << 16) + set * 64;   // (transpose) as many slots as sets
     // offset of unit un's value in a chunk row's stage: one value per 1, 2 or 4 units
     const int gsh = p.g4 == 4 ? 0 : (p.g4 == 2 ? 1 : 2);
+    const uint32_t s_mask = p.s_slots - 1, s_sh = p.s_slots == 2 ? 1 : 2;
     const uint32_t spc_sh = p.spc == 4 ? 2 : (p.spc == 2 ? 1 : 0), half_chunk = (uint32_t)kTileRows * p.cb;
     const bool single = p.spc * p.g4 == 1;   // a chunk is one value: the odd or the even half of the copied word
     const uint32_t s_row = smem_u32(ring_s) + row * p.cb;
@@ -641,10 +681,10 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
       for (; ia < (it0 + n_st) * kSub; ia += kSets) {
         const uint32_t it = ia / kSub, ks = it - it0;      // ks counts from the unit's first stage
         const uint32_t c = c0 + (ks >> spc_sh), sp = it % kStagesP;
-        if (!mbar_wait_hot(bar_fs + (c % kSlotsS) * 8, (c / kSlotsS) & 1u, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_hot(bar_fs + (c & s_mask) * 8, (c >> s_sh) & 1u, abort_flag)) { ok = false; break; }
         if (!mbar_wait_hot(bar_fp + sp * 8, (it / kStagesP) & 1u, abort_flag)) { ok = false; break; }
         const uint32_t tile = p_base + sp * S::kPStageBytes;
-        uint32_t at = s_row + (c % kSlotsS) * 2 * half_chunk + (ks & (p.spc - 1)) * 2 * p.g4;
+        uint32_t at = s_row + (c & s_mask) * 2 * half_chunk + (ks & (p.spc - 1)) * 2 * p.g4;
         if (single) {
           const uint32_t o = kT ? (uint32_t)min((int)((t.ks0 + ks) * kStageK + row), p.K - 1) * p.row_groups + o_row : o_row + ks;
           at += (o & 1) * 2;
@@ -711,7 +751,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         if (lane == 0) {
           mbar_arrive_cluster(bar_a + sa * 8);
           mbar_arrive(bar_ep + sp * 8);
-          mbar_arrive(bar_es + (c % kSlotsS) * 8);
+          mbar_arrive(bar_es + (c & s_mask) * 8);
         }
       }
       it0 += n_st;
@@ -721,6 +761,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     // ------------------------------------------------------------ epilogue
     const int quad = warp & 3;
     const int chalf = (warp - kFirstEpilogue) >> 2;  // which half of the token columns
+    const uint32_t stg = smem_u32(staging) + (warp - kFirstEpilogue) * kStageOut;
     const uint32_t lane_field = (uint32_t)(quad * 32) << 16;
     uint32_t tcount = 0;
     for (int u = pair; u < total; u += pairs, ++tcount) {
@@ -733,26 +774,42 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
       tcgen05_fence_after();
       const int n = t.n0 + quad * 32 + lane;
       const int c_begin = chalf * (t.neff >> 1), c_end = c_begin + (t.neff >> 1);
-      float* part = nullptr;
-      if (p.splits > 1) part = p.partial + ((size_t)t.slot * 2 + rank) * ((size_t)p.NT * kTileRows) + quad * 32 + lane;
-      for (int c = c_begin; c < c_end; c += 32) {
-        uint32_t v[32];
-        tcgen05_ld_x32(tmem_base + ab * (kAccCols / 2) + lane_field + c, v);
-        tcgen05_wait_ld();
-        if (c + 32 >= c_end) {
-          // the last chunk is in registers: the accumulator is free for another tile's MMAs while
-          // this chunk is converted and stored
-          tcgen05_fence_before();
+      const uint32_t acc = tmem_base + ab * (kAccCols / 2) + lane_field;
+      // after the last load the accumulator is free for another tile's MMAs
+      auto release = [&]() {
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(leader_addr(smem_u32(&bars->acc_empty[ab])));
+      };
+      if (p.splits == 1) {
+        uint32_t r[2][16];
+        load_piece(acc + c_begin, r[0]);
+        for (int c0 = c_begin; c0 < c_end; c0 += 64) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int c = c0 + 16 * i;
+            if (c < c_end) {                             // (halves are whole 16-column pieces)
+              tcgen05_wait_ld16(r[i & 1]);
+              if (c + 16 < c_end) load_piece(acc + c + 16, r[(i + 1) & 1]);
+              else release();
+              stage_piece<T>(stg + i * 1024, lane, r[i & 1]);
+            }
+          }
           __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(leader_addr(smem_u32(&bars->acc_empty[ab])));
+          store_chunk<T>(p, t, stg, lane, t.n0 + quad * 32, c0, min(min(t.rows, c_end) - c0, 64));
+          __syncwarp();   // the staging tile may be written again
         }
-        const int lim = min(t.rows, c_end) - c;  // valid columns of this chunk
-        if (part != nullptr) {
+      } else {
+        float* part = p.partial + ((size_t)t.slot * 2 + rank) * ((size_t)p.NT * kTileRows) + quad * 32 + lane;
+        for (int c = c_begin; c < c_end; c += 32) {
+          uint32_t v[32];
+          tcgen05_ld_x32(acc + c, v);
+          tcgen05_wait_ld();
+          if (c + 32 >= c_end) release();
+          const int lim = min(t.rows, c_end) - c;  // valid columns of this chunk
 #pragma unroll
           for (int j = 0; j < 32; ++j)
             if (j < lim) __stcg(part + (size_t)(c + j) * kTileRows, __uint_as_float(v[j]));
-        } else if (n < p.N && lim > 0) {
-          store_chunk<T>(p, t, n, c, lim, v);
         }
       }
       if (p.splits > 1) {
@@ -772,17 +829,22 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           __threadfence();
           const size_t pitch = 2 * (size_t)p.NT * kTileRows;   // from one part to the next
           float* p0 = p.partial + ((size_t)tile * p.splits * 2 + rank) * ((size_t)p.NT * kTileRows) + quad * 32 + lane;
-          for (int c = c_begin; c < c_end; c += 8) {
+          for (int c = c_begin; c < min(c_end, t.rows); c += 8) {
             float sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            for (int s = 0; s < p.splits; ++s) {
+            for (int s = 0; s < p.splits; s += 2) {   // 16 loads in flight
+              float a[8], b[8];
 #pragma unroll
-              for (int j = 0; j < 8; ++j)
-                if (c + j < t.rows) {
-                  float* q = p0 + s * pitch + (size_t)(c + j) * kTileRows;
-                  sum[j] += __ldcg(q);
-                  __stcg(q, 0.0f);
-                }
+              for (int j = 0; j < 8; ++j) {           // (rows past t.rows: zeros, inside the part)
+                const float* q = p0 + s * pitch + (size_t)(c + j) * kTileRows;
+                a[j] = __ldcg(q);
+                b[j] = s + 1 < p.splits ? __ldcg(q + pitch) : 0.0f;
+              }
+#pragma unroll
+              for (int j = 0; j < 8; ++j) sum[j] = (sum[j] + a[j]) + b[j];
             }
+            for (int s = 0; s < p.splits; ++s)
+#pragma unroll
+              for (int j = 0; j < 8; ++j) __stcg(p0 + s * pitch + (size_t)(c + j) * kTileRows, 0.0f);
             if (n < p.N)
               for (int q = 0; q < p.n_out; ++q) {
                 T* yp = static_cast<T*>(p.y_out[q]) + (size_t)(t.x_row0 + c) * p.ld + p.col0 + n;
@@ -853,15 +915,16 @@ Form form_of(int dtype, bool transpose) {
 }
 
 template <int BITS, Form F>
-size_t fixed_smem(int cb) {
+size_t fixed_smem(int cb, int slots) {
   using S = Shape<BITS, F>;
-  return 1024 + S::kSmemA + (size_t)S::kStagesP * S::kPStageBytes + (size_t)kSlotsS * 2 * kTileRows * cb + sizeof(Barriers) + 64;
+  return 1024 + S::kSmemA + (size_t)S::kStagesP * S::kPStageBytes + (size_t)slots * 2 * kTileRows * cb + kEpilogueWarps * kStageOut +
+         sizeof(Barriers) + 64;
 }
-size_t fixed_smem(int bits, Form f, int cb) {
+size_t fixed_smem(int bits, Form f, int cb, int slots) {
   size_t n = 0;
   B200Q_DISPATCH_BITS(bits, BITS, {
-    n = f == Form::Round ? fixed_smem<BITS, Form::Round>(cb)
-                         : (f == Form::Split ? fixed_smem<BITS, Form::Split>(cb) : fixed_smem<BITS, Form::SplitT>(cb));
+    n = f == Form::Round ? fixed_smem<BITS, Form::Round>(cb, slots)
+                         : (f == Form::Split ? fixed_smem<BITS, Form::Split>(cb, slots) : fixed_smem<BITS, Form::SplitT>(cb, slots));
   });
   return n;
 }
@@ -882,11 +945,11 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, Form f) {
   for (int nt = cap; nt >= 32; nt -= 32) {
     const int64_t m_tiles = (M + nt - 1) / nt;
     const int64_t tiles = m_tiles * n_tiles;
-    const double stage = f == Form::Round ? (4.0 * nt > 800 ? 4.0 * nt : 800.0) : (8.0 * nt > 1000 ? 8.0 * nt : 1000.0);
+    const double stage = f == Form::Round ? (4.0 * nt > 700 ? 4.0 * nt : 700.0) : (8.0 * nt > 1300 ? 8.0 * nt : 1300.0);
     for (int s = 1; s == 1 || (s <= 16 && s * 4 <= kst); ++s) {
       if (s > 1 && tiles * s > pairs) break;
       const double waves = (double)((tiles * s + pairs - 1) / pairs);
-      const double tile = (kst + s - 1) / s * stage + (nt <= kAccCols / 2 ? 1000.0 : 1000.0 + 6.0 * nt) + (s > 1 ? 3000.0 + 8.0 * nt * s : 0.0);
+      const double tile = (kst + s - 1) / s * stage + (nt <= kAccCols / 2 ? 1000.0 : 1000.0 + 10.0 * nt) + (s > 1 ? 3000.0 + 8.0 * nt * s : 0.0);
       if (waves * tile < best_t) {
         best_t = waves * tile;
         best = TcPlan{nt, (int)m_tiles, n_tiles, s};
@@ -929,10 +992,35 @@ int encode_maps(TcMaps& m, const char* tag, const void* x, int64_t x_rows, int64
   return B200Q_OK;
 }
 
+// Once per kernel, device and thread.
+int allow_smem(const void* kernel) {
+  constexpr int kMost = 32;   // instantiations: 24
+  static thread_local const void* done[64][kMost];
+  static thread_local int count[64];
+  int dev = 0;
+  B200Q_CUDA_OK(cudaGetDevice(&dev));
+  const bool known = dev >= 0 && dev < 64;
+  for (int i = 0; known && i < count[dev]; ++i)
+    if (done[dev][i] == kernel) return B200Q_OK;
+  B200Q_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
+  if (known && count[dev] < kMost) done[dev][count[dev]++] = kernel;
+  return B200Q_OK;
+}
+
 template <typename T, int BITS, Form F>
 int launch_one(unsigned grid, size_t smem, cudaStream_t st, const TcMaps& maps, const TcParams& p) {
-  B200Q_CUDA_OK(cudaFuncSetAttribute(qmm_tc_kernel<T, BITS, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
-  qmm_tc_kernel<T, BITS, F><<<grid, kThreads, smem, st>>>(maps, p);
+  if (int rc = allow_smem((const void*)qmm_tc_kernel<T, BITS, F>)) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  B200Q_CUDA_OK(cudaLaunchKernelEx(&cfg, qmm_tc_kernel<T, BITS, F>, maps, (const TcParams)p));
   B200Q_LAUNCH_OK("qmm_tc_kernel");
   return B200Q_OK;
 }
@@ -946,7 +1034,8 @@ int launch_tc(int dtype, int bits, int group, Form f, long long units, cudaStrea
            ((reinterpret_cast<uintptr_t>(p.scales) | reinterpret_cast<uintptr_t>(p.biases)) % (4 * p.spc * p.g4)) == 0)
       p.spc *= 2;
   p.cb = p.spc * p.g4 * 2 < 4 ? 4 : p.spc * p.g4 * 2;
-  const size_t fixed = fixed_smem(bits, f, p.cb);
+  p.s_slots = p.spc == 4 ? 2 : 4;
+  const size_t fixed = fixed_smem(bits, f, p.cb, p.s_slots);
   const size_t stage = (size_t)p.NT * 128;
   long long nsb = (long long)((kSmemMax - fixed) / stage);
   p.nsb = (int)(nsb > kMaxStagesB ? kMaxStagesB : nsb);
