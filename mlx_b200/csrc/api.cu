@@ -34,7 +34,7 @@ void count_launch(int n) { g_launches += (uint64_t)n; }
 
 namespace {
 
-enum class Path { QmvRows, Qmv, Stream, Tc, Qvm, Generic };
+enum class Path { QmvRows, Qmv, Tc, Qvm, Generic };
 
 int check_qmm_args(const char* tag, const QmmArgs& a) {
   if (a.dtype != B200Q_F32 && a.dtype != B200Q_F16 && a.dtype != B200Q_BF16)
@@ -80,9 +80,6 @@ Path choose(const QmmArgs& a) {
   if (force_tc() && qmm_tc_supported(a)) return Path::Tc;  // tuning aid: tensor-memory path for any M
   if (ov == 0 && qmv_rows_supported(a)) return Path::QmvRows;
   if (qmv_mma_supported(a)) return Path::Qmv;
-  // f16: up to 32 rows (two trips over W) at 2 and 4 bits: 30 us against 34 for a tensor-core tile with its weights split
-  // in two (14336 x 4096); at 8 bits the second trip costs more than that.
-  if (a.dtype == B200Q_F16 && a.M <= (a.bits <= 4 ? 32 : 16) && qmv_stream_supported(a)) return Path::Stream;
   if (qmm_tc_supported(a) && (a.transpose || a.M > 16)) return Path::Tc;
   if (qvm_supported(a)) return Path::Qvm;
   return Path::Generic;
@@ -113,13 +110,8 @@ int run_qmm(const QmmArgs& a, cudaStream_t st) {
   if (!a.x || !a.wq || !a.scales || !a.biases || !a.y)
     return fail(B200Q_ERR_INVALID_ARGUMENT, "[quantized_matmul] null pointer");
   switch (choose(a)) {
-    // 17 to 32 rows: the row-owning kernel would read W twice; one tensor-core tile does it in 18 us against 27
-    // (14336 x 4096, 4 bits) and in 25 against 50 (4096 x 14336, 8 bits).
-    case Path::QmvRows: return a.M > 16 && qmm_tc_supported(a) ? qmm_tc(a, st) : qmv_rows(a, st);
-    // The streaming kernel takes what the row-owning one leaves; the register-path kernel keeps the peer-store
-    // epilogue, odd numbers of scales per row and the allocation-free entry point.
-    case Path::Qmv: return qmv_override() == 0 && qmv_stream_supported(a) ? qmv_stream(a, st) : qmv_mma(a, st);
-    case Path::Stream: return qmv_stream(a, st);
+    case Path::QmvRows: return qmv_rows(a, st);
+    case Path::Qmv: return qmv_mma(a, st);
     case Path::Tc: return qmm_tc(a, st);
     case Path::Qvm: return qvm(a, st);
     default: return qmm_generic(a, st);
@@ -172,7 +164,6 @@ extern "C" const char* b200q_qmm_kernel_name(int dtype, int64_t batch, int64_t M
   switch (choose(a)) {
     case Path::QmvRows: return "qmv_rows";
     case Path::Qmv: return "qmv_mma";
-    case Path::Stream: return "qmv_stream";
     case Path::Tc: return "qmm_tcgen05";
     case Path::Qvm: return "qvm";
     default: return "qmm_generic";

@@ -130,14 +130,6 @@ int qmv_rows(const QmmArgs& a, cudaStream_t st);
 bool weights_constant();
 void set_weights_constant(int on);
 
-// qmv_stream.cu : decode path of a plain (not sharded) call, every bit width, bf16 and f16; grouped over experts
-struct QmvEntry {      // up to 16 activation rows that multiply one matrix
-  int expert, n;
-  int x_row[16], y_row[16];
-};
-bool qmv_stream_supported(const QmmArgs& a);
-int qmv_stream(const QmmArgs& a, cudaStream_t st);
-
 // qvm.cu : non-transposed decode (M <= 4, bits 2/4/8): y = x * dequant(W[K, N])
 bool qvm_supported(const QmmArgs& a);
 size_t qvm_workspace_bytes(const QmmArgs& a);
