@@ -6,30 +6,13 @@
 // T with round-to-nearest-even.  dequantize reproduces the op-composed reference
 // (mlx/ops.cpp:5320-5323): multiply then add, each rounded to T.
 //
-// Data layout: every thread owns 8 consecutive values of the flattened [rows*K]
-// tensor (one 128-bit load for 16-bit types).  A group of g values is owned by g/8
-// adjacent lanes, which combine min/max with xor-shuffles.  The 8*bits packed bits of
-// a thread are merged across each 4-lane quad so that global stores are whole 32-bit
-// words for every bit width (3-, 5- and 6-bit fields straddle word boundaries).
+// Both are bound by HBM only if a value costs about ten instructions; how they get there stands at the kernels.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace b200q {
 namespace {
-
-template <typename T>
-__device__ __forceinline__ void load8(const T* __restrict__ p, float (&v)[8]) {
-  if constexpr (sizeof(T) == 4) {
-    float4 a = __ldg(reinterpret_cast<const float4*>(p));
-    float4 b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  } else {
-    uint4 raw = __ldg(reinterpret_cast<const uint4*>(p));
-    const T* e = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = Elem<T>::to_float(e[i]);
-  }
-}
 
 template <typename T>
 __device__ __forceinline__ void store8(T* __restrict__ p, const float (&v)[8]) {
@@ -45,33 +28,133 @@ __device__ __forceinline__ void store8(T* __restrict__ p, const float (&v)[8]) {
   }
 }
 
+// ---------------------------------------------------------------------------- quantize
+// A warp takes kIter * 512 consecutive values: a lane loads 16 of every 512 (two 128-bit loads of a 16-bit type,
+// coalesced), so a group of g values lies in g/16 neighbouring lanes.  Minima and maxima are found by
+// shuffles; then every lane computes scale and bias of ONE group (the three IEEE divisions, which in a thread per
+// eight values cost more than everything else) and hands them back by shuffles.
+//
+// q = rint((w - bias) / scale) without a division per value: fma(w - bias, r, 1.5 * 2^23) rounds the product to
+// an integer (half to even) in the low mantissa bits.  It is done twice, with r a few units in the last
+// place below and above 1 / scale: where both agree, the correctly rounded quotient rounds to the same
+// integer; the others are divided as the reference does.  That is no rare case: for 16-bit weights w - bias is a
+// multiple of a coarse unit, and about one value in 250 lies exactly half way between two fields.
+// No lower clamp is needed: w - bias has the sign of scale, and where bias is 0 every |w / scale| is at most 1/2.
+// The fields are packed by multiply-adds on the bit patterns: sum_i u_i 2^(i bits) mod 2^32 is the packed word plus a
+// constant.  About 12 instructions per value, none on the quarter-rate conversion unit (which rint and
+// the float-to-int conversion used).
+template <int GROUP>
+struct QuantShape {
+  static constexpr int kIter = GROUP == 32 ? 2 : 4;         // 512-value rows per warp: at most one group per lane
+  static constexpr int kLanes = GROUP / 16;                 // lanes per group
+  static constexpr int kPerIter = 512 / GROUP;              // groups per row
+};
+
+constexpr float kMagic = 12582912.0f;                       // 1.5 * 2^23
+constexpr uint32_t kMagicBits = 0x4B400000u;
+
+// sum of u[i] * 2^(i * BITS) over N values, without the magic numbers' share
+template <int BITS, int N>
+__device__ __forceinline__ uint32_t pack_fields(const float* u) {
+  uint32_t acc = __float_as_uint(u[N - 1]), c = kMagicBits;
+#pragma unroll
+  for (int i = N - 2; i >= 0; --i) {
+    acc = acc * (1u << BITS) + __float_as_uint(u[i]);
+    c = c * (1u << BITS) + kMagicBits;
+  }
+  acc -= c;
+  return acc;
+}
+
+// Fields whose bit is set in `which` (field 0: bit 15), computed with the division of the reference and put into
+// the packed words o.  Out of line: inlined divisions push the loop out of the instruction cache.
+template <typename T, int BITS>
+__device__ __noinline__ uint4 exact_fields(const T* __restrict__ w, float s, float b, uint32_t which, uint4 o) {
+  constexpr float n_bins = (float)((1 << BITS) - 1);
+  constexpr unsigned long long kMask = (1ull << BITS) - 1ull;
+  unsigned long long lo = (unsigned long long)o.y << 32 | o.x, hi = (unsigned long long)o.w << 32 | o.z;
+  while (which) {
+    const int i = __clz((int)which) - 16;
+    which &= ~(0x8000u >> i);
+    float q = rintf(__fdiv_rn(__fsub_rn(Elem<T>::to_float(w[i]), b), s));
+    q = (q < 0.0f) ? 0.0f : q;
+    q = (n_bins < q) ? n_bins : q;
+    const unsigned long long f = (uint32_t)q;
+    const int at = i * BITS;
+    if (at < 64) lo = (lo & ~(kMask << at)) | f << at;
+    if (at >= 64) hi = (hi & ~(kMask << (at - 64))) | f << (at - 64);
+    else if (at + BITS > 64) hi = (hi & ~(kMask >> (64 - at))) | f >> (64 - at);
+  }
+  return make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
+}
+
+template <typename T>
+struct Pack16 {   // 16 values in the form they are loaded in
+  T v[16];
+};
+template <typename T>
+__device__ __forceinline__ void load16(const T* p, Pack16<T>& d) {
+  const uint4* s = reinterpret_cast<const uint4*>(p);
+  uint4* o = reinterpret_cast<uint4*>(d.v);
+#pragma unroll
+  for (int i = 0; i < (int)sizeof(T); ++i) o[i] = __ldg(s + i);
+}
+template <typename T>
+__device__ __forceinline__ void minmax16(const Pack16<T>& d, float& lo, float& hi) {
+  if constexpr (sizeof(T) == 4) {
+    lo = hi = d.v[0];
+#pragma unroll
+    for (int i = 1; i < 16; ++i) { lo = fminf(lo, d.v[i]); hi = fmaxf(hi, d.v[i]); }
+  } else {
+    using T2 = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
+    const T2* p = reinterpret_cast<const T2*>(d.v);
+    T2 l = p[0], h = p[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) { l = __hmin2(l, p[i]); h = __hmax2(h, p[i]); }
+    lo = fminf(Elem<T>::to_float(l.x), Elem<T>::to_float(l.y));
+    hi = fmaxf(Elem<T>::to_float(h.x), Elem<T>::to_float(h.y));
+  }
+}
+
 template <typename T, int BITS, int GROUP>
 __global__ void __launch_bounds__(256)
 quantize_kernel(const T* __restrict__ w, uint32_t* __restrict__ wq, T* __restrict__ scales,
-                T* __restrict__ biases, int64_t n_chunks) {
-  constexpr int LPG = GROUP / 8;  // lanes per group
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = c < n_chunks;
+                T* __restrict__ biases, int64_t n) {
+  using Q = QuantShape<GROUP>;
+  constexpr int IT = Q::kIter;
   const int lane = threadIdx.x & 31;
+  const int64_t base = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * (IT * 512);
+  if (base >= n) return;
 
-  float v[8];
-  float w_min = INFINITY, w_max = -INFINITY;
-  if (active) {
-    load8(w + c * 8, v);
+  Pack16<T> v[IT];
+  float lo[IT], hi[IT];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      w_max = (w_max < v[i]) ? v[i] : w_max;
-      w_min = (v[i] < w_min) ? v[i] : w_min;
+  for (int k = 0; k < IT; ++k) {
+    const int64_t at = base + k * 512 + lane * 16;
+    if (at < n) {
+      load16(w + at, v[k]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[k].v[i] = Elem<T>::from_float(0.0f);
     }
   }
 #pragma unroll
-  for (int off = 1; off < LPG; off <<= 1) {
-    float omax = __shfl_xor_sync(0xffffffffu, w_max, off);
-    float omin = __shfl_xor_sync(0xffffffffu, w_min, off);
-    w_max = (w_max < omax) ? omax : w_max;
-    w_min = (omin < w_min) ? omin : w_min;
+  for (int k = 0; k < IT; ++k) {
+    minmax16(v[k], lo[k], hi[k]);
+#pragma unroll
+    for (int off = 1; off < Q::kLanes; off <<= 1) {
+      lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], off));
+      hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], off));
+    }
   }
-
+  // lane j takes group j of the warp's values: group j % kPerIter of row j / kPerIter
+  float w_min = 0.0f, w_max = 0.0f;
+#pragma unroll
+  for (int k = 0; k < IT; ++k) {
+    const int src = (lane % Q::kPerIter) * Q::kLanes;
+    const float l = __shfl_sync(0xffffffffu, lo[k], src), h = __shfl_sync(0xffffffffu, hi[k], src);
+    if (lane / Q::kPerIter == k) { w_min = l; w_max = h; }
+  }
   constexpr float n_bins = (float)((1 << BITS) - 1);
   const float eps = 1e-7f;
   const bool mask = fabsf(w_min) > fabsf(w_max);
@@ -85,114 +168,209 @@ quantize_kernel(const T* __restrict__ w, uint32_t* __restrict__ wq, T* __restric
     scale = __fdiv_rn(edge, q0);
     bias = edge;
   }
-
-  uint64_t packed = 0;
-  if (active) {
-    // q = rint((w - bias) / scale) with the IEEE division of the reference, but the division is
-    // only carried out where it can matter: t = (w - bias) * (1 / scale) is within 1.2e-7 * |t|
-    // of the true quotient, so rint(t) equals rint of the rounded quotient unless t lies within
-    // that distance of a rounding tie k + 1/2.  Below |t| = 512 that is less than 1e-4; above, both
-    // roundings clamp to the same bin.  Threads that see a t closer than 1e-4 to a tie (or a NaN)
-    // redo their eight values with the exact division.
-    const float inv = __frcp_rn(scale);
-    float q[8];
-    bool redo = !(fabsf(scale) < 1e30f);   // 1/scale would lose bits as a subnormal
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float t = __fmul_rn(__fsub_rn(v[i], bias), inv);
-      q[i] = rintf(t);
-      redo |= !(fabsf(fabsf(__fsub_rn(t, q[i])) - 0.5f) >= 1e-4f);   // also true for NaN
-    }
-    if (redo) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) q[i] = rintf(__fdiv_rn(__fsub_rn(v[i], bias), scale));
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float qi = (q[i] < 0.0f) ? 0.0f : q[i];
-      qi = (n_bins < qi) ? n_bins : qi;
-      packed |= (uint64_t)(uint32_t)qi << (i * BITS);
-    }
-    if ((c % LPG) == 0) {
-      scales[c / LPG] = Elem<T>::from_float(scale);
-      biases[c / LPG] = Elem<T>::from_float(bias);
+  const float inv = __frcp_rn(scale);
+  {
+    const int64_t g = base / GROUP + lane;
+    if (lane < IT * Q::kPerIter && g * GROUP < n) {
+      scales[g] = Elem<T>::from_float(scale);
+      biases[g] = Elem<T>::from_float(bias);
     }
   }
 
-  // 4 and 8 bits: a thread's eight fields are exactly one or two words.
-  if constexpr (BITS == 4) {
-    if (active) wq[c] = (uint32_t)packed;
-    return;
-  } else if constexpr (BITS == 8) {
-    if (active) reinterpret_cast<uint2*>(wq)[c] = make_uint2((uint32_t)packed, (uint32_t)(packed >> 32));
-    return;
-  }
-  // Merge the four 8*BITS-bit fragments of a quad into BITS whole words.
-  constexpr int SEG = 8 * BITS;
-  const int qbase = lane & ~3;
-  uint64_t seg[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    uint32_t lo = __shfl_sync(0xffffffffu, (uint32_t)packed, qbase + j);
-    uint32_t hi = __shfl_sync(0xffffffffu, (uint32_t)(packed >> 32), qbase + j);
-    seg[j] = ((uint64_t)hi << 32) | lo;
-  }
-  if (active) {
-    uint32_t* out = wq + (c >> 2) * BITS;
-    const int l = lane & 3;
+  for (int k = 0; k < IT; ++k) {
+    const int src = k * Q::kPerIter + lane / Q::kLanes;
+    const float s = __shfl_sync(0xffffffffu, scale, src), b = __shfl_sync(0xffffffffu, bias, src);
+    const float r = __shfl_sync(0xffffffffu, inv, src);
+    const float r0 = r * (1.0f - 0x1p-21f), r1 = r * (1.0f + 0x1p-21f);
+    float u[16];
+    float differ = 0.0f;   // 16 bits, value 0 in the highest: both results are integers k or k + 1
 #pragma unroll
-    for (int i = 0; i < BITS; ++i) {
-      const int p = 32 * i;
-      const int j = p / SEG;
-      const int o = p % SEG;
-      uint64_t word = seg[j] >> o;
-      if (SEG - o < 32 && j + 1 < 4) word |= seg[j + 1] << (SEG - o);
-      if ((i & 3) == l) out[i] = (uint32_t)word;
+    for (int i = 0; i < 16; ++i) {
+      const float d = __fsub_rn(Elem<T>::to_float(v[k].v[i]), b);
+      const float t = __fmaf_rn(d, r0, kMagic);
+      differ = __fmaf_rn(differ, 2.0f, __fsub_rn(__fmaf_rn(d, r1, kMagic), t));
+      u[i] = fminf(t, kMagic + n_bins);
+    }
+    const int64_t at = base + k * 512 + lane * 16;
+    uint32_t o[4] = {0, 0, 0, 0};   // 16 * BITS bits per lane: whole words, or with 3 and 5 bits half a word more
+    if constexpr (BITS == 2) {
+      o[0] = pack_fields<2, 16>(u);
+    } else if constexpr (BITS == 4) {
+      o[0] = pack_fields<4, 8>(u); o[1] = pack_fields<4, 8>(u + 8);
+    } else if constexpr (BITS == 8) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) o[i] = pack_fields<8, 4>(u + 4 * i);
+    } else if constexpr (BITS == 3) {
+      const uint32_t a = pack_fields<3, 8>(u), c = pack_fields<3, 8>(u + 8);   // 24 bits each
+      o[0] = a | c << 24; o[1] = c >> 8;
+    } else if constexpr (BITS == 6) {
+      const uint32_t a = pack_fields<6, 4>(u), c = pack_fields<6, 4>(u + 4), d = pack_fields<6, 4>(u + 8), e = pack_fields<6, 4>(u + 12);
+      o[0] = a | c << 24; o[1] = c >> 8 | d << 16; o[2] = d >> 16 | e << 8;
+    } else {
+      const uint32_t a = pack_fields<5, 4>(u), c = pack_fields<5, 4>(u + 4), d = pack_fields<5, 4>(u + 8), e = pack_fields<5, 4>(u + 12);   // 20 bits each
+      o[0] = a | c << 20; o[1] = c >> 12 | d << 8 | e << 28; o[2] = e >> 4;
+    }
+    // (The comparison means nothing where 1 / scale or a product is not an ordinary number: all sixteen then.)
+    const bool plain = fabsf(s) < 1e30f && fabsf(r) < 1e30f;
+    if ((differ != 0.0f || !plain) && at < n) {
+      const uint32_t which = plain && differ > 0.0f && differ < 65536.0f ? (uint32_t)differ : 0xFFFFu;
+      const uint4 e = exact_fields<T, BITS>(w + at, s, b, which, make_uint4(o[0], o[1], o[2], o[3]));
+      o[0] = e.x; o[1] = e.y; o[2] = e.z; o[3] = e.w;
+    }
+    if constexpr (BITS == 3 || BITS == 5) {
+      // two lanes share a word: the even lane stores it and the words before it, the odd lane the words after it
+      constexpr int F = BITS / 2;                            // whole words of a lane
+      uint32_t* out = wq + (at / 32) * BITS;
+      const uint32_t next = __shfl_down_sync(0xffffffffu, o[0], 1);
+      if (at < n) {
+        if ((lane & 1) == 0) {
+#pragma unroll
+          for (int i = 0; i < F; ++i) out[i] = o[i];
+          out[F] = (o[F] & 0xFFFFu) | next << 16;
+        } else {
+#pragma unroll
+          for (int i = 0; i < F; ++i) out[F + 1 + i] = o[i] >> 16 | o[i + 1] << 16;
+        }
+      }
+    } else if (at < n) {
+      uint32_t* out = wq + at * BITS / 32;
+      if constexpr (BITS == 2) {
+        out[0] = o[0];
+      } else if constexpr (BITS == 4) {   // wq may be only 4-byte aligned
+        if ((reinterpret_cast<uintptr_t>(wq) & 7) == 0) *reinterpret_cast<uint2*>(out) = make_uint2(o[0], o[1]);
+        else { out[0] = o[0]; out[1] = o[1]; }
+      } else if constexpr (BITS == 8) {
+        if ((reinterpret_cast<uintptr_t>(wq) & 15) == 0) *reinterpret_cast<uint4*>(out) = make_uint4(o[0], o[1], o[2], o[3]);
+        else { out[0] = o[0]; out[1] = o[1]; out[2] = o[2]; out[3] = o[3]; }
+      } else {
+        out[0] = o[0]; out[1] = o[1]; out[2] = o[2];
+      }
     }
   }
 }
+
+// ---------------------------------------------------------------------------- dequantize
+// The 8 fields of chunk c: they start at byte c*BITS, at byte offset 0..3 of a word, and for every supported
+// width end within 64 bits from there.
+template <int BITS>
+__device__ __forceinline__ uint2 chunk_bits(const uint32_t* __restrict__ wq, int64_t c, int64_t n_words) {
+  if constexpr (BITS == 4) return make_uint2(__ldg(wq + c), 0u);
+  const int64_t byte = c * BITS, w0 = byte >> 2;
+  const int sh = (int)(byte & 3) * 8;
+  const uint32_t a = __ldg(wq + w0);
+  const uint32_t b = (w0 + 1 < n_words) ? __ldg(wq + w0 + 1) : 0u;
+  if constexpr (BITS == 8) return make_uint2(a, b);
+  return make_uint2(__funnelshift_r(a, b, sh), b >> sh);
+}
+
+// Values of a chunk: round_T(round_T(q * s) + b), multiply and add being separate operations of type T in the
+// reference.  16-bit types in packed pairs: q comes out of the bit pattern 128 + q (bf16) or 1024 + q (f16) exactly;
+// mul.rn and add.rn on pairs round as the fp32 operation followed by the conversion does (the fp32 product is
+// exact, and so is every fp32 sum that could land between two values of T).
+template <typename T, int BITS>
+__device__ __forceinline__ void store_chunk(T* __restrict__ dst, uint2 bits, T s_t, T b_t) {
+  if constexpr (sizeof(T) == 4) {
+    const uint64_t v64 = (uint64_t)bits.y << 32 | bits.x;
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __fadd_rn(__fmul_rn((float)(uint32_t)((v64 >> (i * BITS)) & ((1u << BITS) - 1u)), s_t), b_t);
+    store8(dst, v);
+  } else {
+    constexpr bool kBf = std::is_same<T, __nv_bfloat16>::value;
+    using T2 = typename std::conditional<kBf, __nv_bfloat162, __half2>::type;
+    constexpr uint32_t kMask = (1u << BITS) - 1u;
+    constexpr uint32_t kOff = kBf ? 0x43004300u : 0x64006400u;   // (128, 128) or (1024, 1024)
+    T2 s2, b2;
+    s2.x = s2.y = s_t;
+    b2.x = b2.y = b_t;
+    uint32_t q[4];   // fields (2i, 2i+1)
+    if constexpr (kBf && BITS == 8) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t w = i < 2 ? bits.x : bits.y;
+        const float f0 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540 | (2 * i & 3))) - 8388608.0f;
+        const float f1 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540 | ((2 * i + 1) & 3))) - 8388608.0f;
+        const __nv_bfloat162 t = __floats2bfloat162_rn(f0, f1);
+        q[i] = *reinterpret_cast<const uint32_t*>(&t);
+      }
+    } else {
+      uint32_t m[4];
+      if constexpr (BITS == 4 || BITS == 2) {   // masks over both halves: fields (i, i + 4)
+        const uint32_t w = BITS == 4 ? bits.x : __byte_perm(bits.x, 0u, 0x4140);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) m[i] = ((w >> (BITS * i)) & (kMask * 0x00010001u)) | kOff;
+        q[0] = __byte_perm(m[0], m[1], 0x5410); q[1] = __byte_perm(m[2], m[3], 0x5410);
+        q[2] = __byte_perm(m[0], m[1], 0x7632); q[3] = __byte_perm(m[2], m[3], 0x7632);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t f[2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int at = (2 * i + h) * BITS;
+            f[h] = ((at >= 32 ? bits.y >> (at - 32) : (at + BITS > 32 ? __funnelshift_r(bits.x, bits.y, at) : bits.x >> at)) & kMask);
+          }
+          q[i] = (f[0] | f[1] << 16) | kOff;
+        }
+      }
+      T2 off;
+      *reinterpret_cast<uint32_t*>(&off) = kOff;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const T2 t = __hsub2(*reinterpret_cast<const T2*>(&q[i]), off);
+        q[i] = *reinterpret_cast<const uint32_t*>(&t);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const T2 t = __hadd2_rn(__hmul2_rn(*reinterpret_cast<const T2*>(&q[i]), s2), b2);   // (_rn: never contracted to one fma)
+      q[i] = *reinterpret_cast<const uint32_t*>(&t);
+    }
+    *reinterpret_cast<uint4*>(dst) = make_uint4(q[0], q[1], q[2], q[3]);
+  }
+}
+
+constexpr int kDequantChunks = 4;   // chunks of 8 values per thread, a block apart: enough loads in flight for HBM
 
 template <typename T, int BITS>
 __global__ void __launch_bounds__(256)
 dequantize_kernel(const uint32_t* __restrict__ wq, const T* __restrict__ scales,
                   const T* __restrict__ biases, T* __restrict__ out, int64_t n_chunks,
                   int group_shift /* log2(group/8) */, int64_t n_words) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n_chunks) return;
-  // The 8 fields of chunk c start at byte c*BITS; fetch the covering aligned words.
-  const int64_t byte = c * BITS;
-  const int64_t w0 = byte >> 2;
-  const int sh = (int)(byte & 3) * 8;
-  uint32_t a = __ldg(wq + w0);
-  uint32_t b = (w0 + 1 < n_words) ? __ldg(wq + w0 + 1) : 0u;
-  // 8*BITS <= 64 bits starting at a byte offset of 0..3 inside `a`: for every supported
-  // width the fields end within the first 64 bits, so two words suffice.
-  uint64_t bitsv = ((uint64_t)(b >> sh) << 32) | __funnelshift_r(a, b, sh);
-  const int64_t g = c >> group_shift;
-  const float s = Elem<T>::to_float(scales[g]);
-  const float bs = Elem<T>::to_float(biases[g]);
-  float v[8];
+  const int64_t c0 = (int64_t)blockIdx.x * (256 * kDequantChunks) + threadIdx.x;
+  uint2 bits[kDequantChunks];
+  T s[kDequantChunks], b[kDequantChunks];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float q = (float)(uint32_t)((bitsv >> (i * BITS)) & ((1u << BITS) - 1u));
-    // multiply and add are separate operations of type T in the reference.
-    float t = Elem<T>::to_float(Elem<T>::from_float(__fmul_rn(q, s)));
-    v[i] = __fadd_rn(t, bs);
+  for (int i = 0; i < kDequantChunks; ++i) {
+    const int64_t c = c0 + 256 * i;
+    if (c < n_chunks) {
+      bits[i] = chunk_bits<BITS>(wq, c, n_words);
+      s[i] = scales[c >> group_shift];
+      b[i] = biases[c >> group_shift];
+    }
   }
-  store8(out + c * 8, v);
+#pragma unroll
+  for (int i = 0; i < kDequantChunks; ++i) {
+    const int64_t c = c0 + 256 * i;
+    if (c < n_chunks) store_chunk<T, BITS>(out + c * 8, bits[i], s[i], b[i]);
+  }
 }
 
 template <typename T>
 int launch_quantize(const T* w, int64_t n_elems, int group, int bits, uint32_t* wq, T* s, T* b,
                     cudaStream_t st) {
-  const int64_t n_chunks = n_elems / 8;
-  if (n_chunks == 0) return B200Q_OK;
-  const unsigned grid = (unsigned)((n_chunks + 255) / 256);
+  if (n_elems == 0) return B200Q_OK;
   bool done = false;
   B200Q_DISPATCH_BITS(bits, BITS, {
-    if (group == 32) quantize_kernel<T, BITS, 32><<<grid, 256, 0, st>>>(w, wq, s, b, n_chunks);
-    else if (group == 64) quantize_kernel<T, BITS, 64><<<grid, 256, 0, st>>>(w, wq, s, b, n_chunks);
-    else quantize_kernel<T, BITS, 128><<<grid, 256, 0, st>>>(w, wq, s, b, n_chunks);
+    auto go = [&](auto gtag) {
+      constexpr int G = decltype(gtag)::value;
+      constexpr int64_t per_block = 8 * QuantShape<G>::kIter * 512;
+      quantize_kernel<T, BITS, G><<<(unsigned)((n_elems + per_block - 1) / per_block), 256, 0, st>>>(w, wq, s, b, n_elems);
+    };
+    if (group == 32) go(std::integral_constant<int, 32>{});
+    else if (group == 64) go(std::integral_constant<int, 64>{});
+    else go(std::integral_constant<int, 128>{});
     done = true;
   });
   if (!done) return fail(B200Q_ERR_INVALID_ARGUMENT, "[quantize] unsupported bits %d", bits);
@@ -205,7 +383,7 @@ int launch_dequantize(const uint32_t* wq, const T* s, const T* b, int64_t n_elem
                       int bits, T* out, cudaStream_t st) {
   const int64_t n_chunks = n_elems / 8;
   if (n_chunks == 0) return B200Q_OK;
-  const unsigned grid = (unsigned)((n_chunks + 255) / 256);
+  const unsigned grid = (unsigned)((n_chunks + 256 * kDequantChunks - 1) / (256 * kDequantChunks));
   const int gshift = group == 32 ? 2 : (group == 64 ? 3 : 4);
   const int64_t n_words = n_elems * bits / 32;
   bool done = false;
@@ -230,30 +408,16 @@ dequantize_rows_kernel(const uint32_t* __restrict__ wq, const T* __restrict__ sc
   const int64_t i = blockIdx.y;
   const uint32_t id = __ldg(ids + i);
   T* dst = out + (i * chunks_per_row + c) * 8;
-  float v[8];
   if ((int64_t)id >= rows) {
+    float v[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) v[k] = 0.f;
     store8(dst, v);
     return;
   }
   const int64_t cg = (int64_t)id * chunks_per_row + c;  // chunk index in the whole matrix
-  const int64_t byte = cg * BITS;
-  const int64_t w0 = byte >> 2;
-  const int sh = (int)(byte & 3) * 8;
-  uint32_t a = __ldg(wq + w0);
-  uint32_t b = (w0 + 1 < n_words) ? __ldg(wq + w0 + 1) : 0u;
-  uint64_t bitsv = ((uint64_t)(b >> sh) << 32) | __funnelshift_r(a, b, sh);
   const int64_t g = cg >> group_shift;
-  const float s = Elem<T>::to_float(scales[g]);
-  const float bs = Elem<T>::to_float(biases[g]);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    float q = (float)(uint32_t)((bitsv >> (k * BITS)) & ((1u << BITS) - 1u));
-    float t = Elem<T>::to_float(Elem<T>::from_float(__fmul_rn(q, s)));
-    v[k] = __fadd_rn(t, bs);
-  }
-  store8(dst, v);
+  store_chunk<T, BITS>(dst, chunk_bits<BITS>(wq, cg, n_words), scales[g], biases[g]);
 }
 
 template <typename T>
