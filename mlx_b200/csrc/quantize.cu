@@ -43,6 +43,7 @@ __device__ __forceinline__ void store8(T* __restrict__ p, const float (&v)[8]) {
 // The fields are packed by multiply-adds on the bit patterns: sum_i u_i 2^(i bits) mod 2^32 is the packed word plus a
 // constant.  About 12 instructions per value, none on the quarter-rate conversion unit (which rint and
 // the float-to-int conversion used).
+// 28672 x 8192 bf16, groups of 64 (device time): to 4 bits 321 -> 136 us (4.4 TB/s), to 8 bits 401 -> 152; f32 99.
 template <int GROUP>
 struct QuantShape {
   static constexpr int kIter = GROUP == 32 ? 2 : 4;         // 512-value rows per warp: at most one group per lane
@@ -331,7 +332,9 @@ __device__ __forceinline__ void store_chunk(T* __restrict__ dst, uint2 bits, T s
   }
 }
 
-constexpr int kDequantChunks = 4;   // chunks of 8 values per thread, a block apart: enough loads in flight for HBM
+// Chunks of 8 values per thread, a block apart: enough loads in flight for HBM.  28672 x 8192 bf16, groups of 64: from
+// 4 bits 134 -> 99 us (6.1 TB/s), from 3 bits 138 -> 111.
+constexpr int kDequantChunks = 4;
 
 template <typename T, int BITS>
 __global__ void __launch_bounds__(256)
