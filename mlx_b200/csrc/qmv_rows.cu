@@ -1,4 +1,4 @@
-// Decode path, row-owning form: y[M<=16, N] = x[M, K] * dequant(W[N, K])^T, bf16, HBM-bound.
+// Decode path, row-owning form: y[M<=16, N] = x[M, K] * dequant(W[N, K])^T, bf16 and f16, HBM-bound.
 //
 // Replaces cu::qmv_kernel / the small-M use of cu::qmm_sm80_kernel of the reference
 // (mlx/backend/cuda/quantized/qmm/qmv.cu:84-209, quantized.cpp:106-136).
@@ -36,6 +36,7 @@
 #include <cuda.h>
 
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -77,22 +78,35 @@ __device__ unsigned int g_rows_launch_in, g_rows_launch_out;
 #define RP_MARK(i)
 #endif
 
-__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+template <typename T>
+constexpr bool is_bf16 = std::is_same<T, __nv_bfloat16>::value;
+template <typename T>
+__device__ __forceinline__ uint32_t mul_x2(uint32_t a, uint32_t b) {
   uint32_t d;
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  if constexpr (is_bf16<T>) asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  else asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
+template <typename T>
+__device__ __forceinline__ uint32_t pack_x2(float lo, float hi) {
   uint32_t d;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  if constexpr (is_bf16<T>) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
   return d;
 }
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+template <typename T>
+__device__ __forceinline__ void mma16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                      uint32_t b0, uint32_t b1) {
+  if constexpr (is_bf16<T>)
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  else
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 // Four 8x8 matrices of 16-bit elements; lane l supplies the address of row l%8 of matrix l/8 and
 // receives, from matrix m, the 32-bit word (l%4) of row l/4.
@@ -118,10 +132,20 @@ __device__ __forceinline__ uint2 ldg_nc_u64(const void* p) {
   asm volatile("ld.global.nc.v2.b32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
   return v;
 }
-__device__ __forceinline__ float bf16lo(uint32_t v) { return __uint_as_float(v << 16); }
-__device__ __forceinline__ float bf16hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
-__device__ __forceinline__ float sum_bf16x2(uint32_t v) { return bf16lo(v) + bf16hi(v); }
-__device__ __forceinline__ float asum_bf16x2(uint32_t v) { return fabsf(bf16lo(v)) + fabsf(bf16hi(v)); }
+template <typename T>
+__device__ __forceinline__ float lo_f(uint32_t v) {
+  if constexpr (is_bf16<T>) return __uint_as_float(v << 16);
+  else return __half2float(__ushort_as_half((unsigned short)(v & 0xFFFFu)));
+}
+template <typename T>
+__device__ __forceinline__ float hi_f(uint32_t v) {
+  if constexpr (is_bf16<T>) return __uint_as_float(v & 0xFFFF0000u);
+  else return __half2float(__ushort_as_half((unsigned short)(v >> 16)));
+}
+template <typename T>
+__device__ __forceinline__ float sum_x2(uint32_t v) { return lo_f<T>(v) + hi_f<T>(v); }
+template <typename T>
+__device__ __forceinline__ float asum_x2(uint32_t v) { return fabsf(lo_f<T>(v)) + fabsf(hi_f<T>(v)); }
 
 __host__ __device__ constexpr int cmin(int a, int b) { return a < b ? a : b; }
 __host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
@@ -144,8 +168,8 @@ struct Cfg {
 };
 
 struct RowsParams {
-  const __nv_bfloat16* x;
-  __nv_bfloat16* y[kMaxPeers];
+  const uint16_t* x;   // 16-bit elements of either type
+  uint16_t* y[kMaxPeers];
   int n_out;
   long long ld, col0;
   PeerSignal sig;       // completion signal towards the ranks that receive y (n == 0: none)
@@ -194,7 +218,7 @@ __device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
   return v;
 }
 
-template <int BITS, int G, int MT>
+template <typename T, int BITS, int G, int MT>
 __global__ void __launch_bounds__(kThreads, 1)
 qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s,
                 const __grid_constant__ CUtensorMap map_b, const RowsParams p) {
@@ -369,12 +393,12 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
           // transpose the 16 rows x 8*MT tokens through shared memory so that every lane stores 16
           // contiguous bytes of one token's row of y
           const int row0 = (b0 + 2 * rrg) * 8;
-          __nv_bfloat16* yt = reinterpret_cast<__nv_bfloat16*>(smem + 512);   // [16 tokens][16 rows]
+          T* yt = reinterpret_cast<T*>(smem + 512);   // [16 tokens][16 rows]
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-              yt[(mt * 8 + 2 * t + (c & 1)) * 16 + g + (c >> 1) * 8] = __float2bfloat16_rn(sum[mt][c]);
+              yt[(mt * 8 + 2 * t + (c & 1)) * 16 + g + (c >> 1) * 8] = Elem<T>::from_float(sum[mt][c]);
           __syncwarp();
           const int tok = lane >> 1, r8 = row0 + (lane & 1) * 8;
           if (tok < p.M && r8 < row_end) {
@@ -382,11 +406,11 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             const long long at = (long long)tok * p.ld + p.col0 + r8;
             const bool vec = r8 + 8 <= row_end && ((at | p.ld) & 7) == 0;
             for (int q = 0; q < p.n_out; ++q) {
-              __nv_bfloat16* dst = p.y[q] + at;
+              uint16_t* dst = p.y[q] + at;
               if (vec && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
                 *reinterpret_cast<uint4*>(dst) = v;
               } else {
-                const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
+                const uint16_t* e = reinterpret_cast<const uint16_t*>(&v);
                 for (int i = 0; i < 8 && r8 + i < row_end; ++i) dst[i] = e[i];
               }
             }
@@ -462,28 +486,28 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       for (int mt = 0; mt < MT; ++mt) {
         const int tok = mt * 8 + g;
         const bool live = i < cnt * UG && tok < p.M;
-        const __nv_bfloat16* xp = p.x + (long long)tok * p.K + k0 + i * (4 * KW);
+        const uint16_t* xp = p.x + (long long)tok * p.K + k0 + i * (4 * KW);
         // pair q = (x_q, x_{q + NP}), the order the unpack delivers the fields in
         if constexpr (BITS == 8) {
           uint2 v = make_uint2(0, 0);
           if (live) v = ldg_nc_u64(xp);
-          sx[i / UG][mt] += sum_bf16x2(v.x) + sum_bf16x2(v.y);
-          asum[mt] += asum_bf16x2(v.x) + asum_bf16x2(v.y);
+          sx[i / UG][mt] += sum_x2<T>(v.x) + sum_x2<T>(v.y);
+          asum[mt] += asum_x2<T>(v.x) + asum_x2<T>(v.y);
           X[i][mt][0] = __byte_perm(v.x, v.y, 0x5410); X[i][mt][1] = __byte_perm(v.x, v.y, 0x7632);
         } else if constexpr (BITS == 4) {
           uint4 v = make_uint4(0, 0, 0, 0);
           if (live) v = ldg_nc_u128(xp);
-          sx[i / UG][mt] += (sum_bf16x2(v.x) + sum_bf16x2(v.y)) + (sum_bf16x2(v.z) + sum_bf16x2(v.w));
-          asum[mt] += (asum_bf16x2(v.x) + asum_bf16x2(v.y)) + (asum_bf16x2(v.z) + asum_bf16x2(v.w));
+          sx[i / UG][mt] += (sum_x2<T>(v.x) + sum_x2<T>(v.y)) + (sum_x2<T>(v.z) + sum_x2<T>(v.w));
+          asum[mt] += (asum_x2<T>(v.x) + asum_x2<T>(v.y)) + (asum_x2<T>(v.z) + asum_x2<T>(v.w));
           X[i][mt][0] = __byte_perm(v.x, v.z, 0x5410); X[i][mt][1] = __byte_perm(v.x, v.z, 0x7632);
           X[i][mt][2] = __byte_perm(v.y, v.w, 0x5410); X[i][mt][3] = __byte_perm(v.y, v.w, 0x7632);
         } else {
           uint4 a = make_uint4(0, 0, 0, 0), b = make_uint4(0, 0, 0, 0);
           if (live) { a = ldg_nc_u128(xp); b = ldg_nc_u128(xp + 8); }
-          sx[i / UG][mt] += (sum_bf16x2(a.x) + sum_bf16x2(a.y)) + (sum_bf16x2(a.z) + sum_bf16x2(a.w)) +
-                            (sum_bf16x2(b.x) + sum_bf16x2(b.y)) + (sum_bf16x2(b.z) + sum_bf16x2(b.w));
-          asum[mt] += (asum_bf16x2(a.x) + asum_bf16x2(a.y)) + (asum_bf16x2(a.z) + asum_bf16x2(a.w)) +
-                      (asum_bf16x2(b.x) + asum_bf16x2(b.y)) + (asum_bf16x2(b.z) + asum_bf16x2(b.w));
+          sx[i / UG][mt] += (sum_x2<T>(a.x) + sum_x2<T>(a.y)) + (sum_x2<T>(a.z) + sum_x2<T>(a.w)) +
+                            (sum_x2<T>(b.x) + sum_x2<T>(b.y)) + (sum_x2<T>(b.z) + sum_x2<T>(b.w));
+          asum[mt] += (asum_x2<T>(a.x) + asum_x2<T>(a.y)) + (asum_x2<T>(a.z) + asum_x2<T>(a.w)) +
+                      (asum_x2<T>(b.x) + asum_x2<T>(b.y)) + (asum_x2<T>(b.z) + asum_x2<T>(b.w));
           X[i][mt][0] = __byte_perm(a.x, b.x, 0x5410); X[i][mt][1] = __byte_perm(a.x, b.x, 0x7632);
           X[i][mt][2] = __byte_perm(a.y, b.y, 0x5410); X[i][mt][3] = __byte_perm(a.y, b.y, 0x7632);
           X[i][mt][4] = __byte_perm(a.z, b.z, 0x5410); X[i][mt][5] = __byte_perm(a.z, b.z, 0x7632);
@@ -499,23 +523,25 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       am += __shfl_xor_sync(0xFFFFFFFFu, am, 1);
       am += __shfl_xor_sync(0xFFFFFFFFu, am, 2);
       const uint32_t m = __float_as_uint(am);
-      // E: x is multiplied by 2^E so that its largest element lands at or below 2^65
-      int E = 191 - (int)((m >> 23) & 0xFF);
-      E = E < -62 ? -62 : (E > 120 ? 120 : E);
-      const uint32_t sc = (uint32_t)(127 + E) << 7;   // bf16 bits of 2^E
-      const uint32_t sc2 = sc | (sc << 16);
+      // E: x is multiplied by 2^E so that its largest element lands at or below 2^65 (f16: 2^15; the powers of two
+      // below that the fields ask for stay normal numbers)
+      int E = (is_bf16<T> ? 191 : 141) - (int)((m >> 23) & 0xFF);
+      if constexpr (is_bf16<T>) E = E < -62 ? -62 : (E > 120 ? 120 : E);
+      else E = E < -8 ? -8 : (E > 15 ? 15 : E);
+      constexpr uint32_t kOne = is_bf16<T> ? 0x00800080u : 0x04000400u;   // one binary place of both halves
+      const uint32_t sc2 = (uint32_t)((is_bf16<T> ? 127 : 15) + E) * kOne;   // 2^E twice
 #pragma unroll
       for (int i = 0; i < UW; ++i)
 #pragma unroll
         for (int q = 0; q < NP; ++q)
-          X[i][mt][q] = mul_bf16x2(X[i][mt][q], sc2 - (uint32_t)field_shift<BITS>(q) * 0x00800080u);
-      // the weights come out as field * 2^-133: the sums of this token are true value * 2^(E - 133);
-      // 2^(64 - E) is applied when the sums leave the warp, 2^69 with it
-      const float un = __uint_as_float((uint32_t)(127 + 64 - E) << 23);
+          X[i][mt][q] = mul_x2<T>(X[i][mt][q], sc2 - (uint32_t)field_shift<BITS>(q) * kOne);
+      // the weights come out as field * 2^-133 (f16: 2^-24): the sums of this token are true value * 2^(E - 133);
+      // 2^(64 - E) is applied when the sums leave the warp, 2^69 with it (f16: 2^(24 - E))
+      const float un = __uint_as_float((uint32_t)(127 + (is_bf16<T> ? 64 : 24) - E) << 23);
       unscale[mt][0] = __shfl_sync(0xFFFFFFFFu, un, (2 * t) * 4);
       unscale[mt][1] = __shfl_sync(0xFFFFFFFFu, un, (2 * t + 1) * 4);
-      // group sums over the quad, in the same units; lane t keeps groups 2t and 2t+1 (the k slots it feeds)
-      const float down = __uint_as_float((uint32_t)(127 + E - 64) << 23) * 0x1p-69f;
+      // group sums over the quad, in the same units (f16: times 2^(E - 2), which keeps both parts normal); lane t keeps groups 2t and 2t+1 (the k slots it feeds)
+      const float down = is_bf16<T> ? __uint_as_float((uint32_t)(127 + E - 64) << 23) * 0x1p-69f : __uint_as_float((uint32_t)(125 + E) << 23);
       float e0 = 0.0f, e1 = 0.0f;
 #pragma unroll
       for (int j = 0; j < NGW; ++j) {
@@ -527,9 +553,9 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
       }
       e0 *= down; e1 *= down;
-      const uint32_t hi = pack_bf16x2(e0, e1);
+      const uint32_t hi = pack_x2<T>(e0, e1);
       sx_hi[mt] = hi;
-      sx_lo[mt] = pack_bf16x2(e0 - bf16lo(hi), e1 - bf16hi(hi));
+      sx_lo[mt] = pack_x2<T>(e0 - lo_f<T>(hi), e1 - hi_f<T>(hi));
     }
   };
   setup_phase();
@@ -591,15 +617,15 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             for (int st = 0; st < NP / 2; ++st)
 #pragma unroll
               for (int mt = 0; mt < MT; ++mt)
-                mma_bf16(acc[u][mt][(iu * (NP / 2) + st) % SPLIT], Pl[2 * st], Ph[2 * st], Pl[2 * st + 1], Ph[2 * st + 1],
+                mma16<T>(acc[u][mt][(iu * (NP / 2) + st) % SPLIT], Pl[2 * st], Ph[2 * st], Pl[2 * st + 1], Ph[2 * st + 1],
                          X[(gq + u) * UG + iu][mt][2 * st], X[(gq + u) * UG + iu][mt][2 * st + 1]);
           }
         }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           // a group beyond cnt (cnt == 1) contributes acc == 0 times a finite neighbour's scale
-          const float s_l = __uint_as_float(lds_u16(sa + 2 * (gq + u)) << 16);
-          const float s_h = __uint_as_float(lds_u16(sa + 1024 + 2 * (gq + u)) << 16);
+          const float s_l = lo_f<T>(lds_u16(sa + 2 * (gq + u)));
+          const float s_h = lo_f<T>(lds_u16(sa + 1024 + 2 * (gq + u)));
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
@@ -624,19 +650,29 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         bl = lds_u16(ba); bh = lds_u16(ba + 1024);
       }
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) mma_bf16(out[mt], bl, bh, bl, bh, sx_hi[mt], sx_lo[mt]);
+      for (int mt = 0; mt < MT; ++mt) {
+        if constexpr (is_bf16<T>) {
+          mma16<T>(out[mt], bl, bh, bl, bh, sx_hi[mt], sx_lo[mt]);
+        } else {
+          float ob[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // in units of 2^(E - 2); out: 2^(E - 24)
+          mma16<T>(ob, bl, bh, bl, bh, sx_hi[mt], sx_lo[mt]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) out[mt][c] = fmaf(ob[c], 0x1p-22f, out[mt][c]);
+        }
+      }
     }
     }
     RP_MARK(6 + 3 * s);
     // the partial buffer of this stage was read by the reducer kPartialBufs stages ago
     if (pbe > 0 && !mbar_wait(pfree0 + 8 * pbi, (pbe - 1) & 1, abort_flag)) break;
     {
+      constexpr float kOut = is_bf16<T> ? 0x1p69f : 1.0f;
       const uint32_t pa = pb_mine + (uint32_t)pbi * (kConsumers * MT * 512);
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt)   // back to true units on the way out (two exact multiplications)
+      for (int mt = 0; mt < MT; ++mt)   // back to true units on the way out (exact multiplications)
         asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(pa + mt * 512),
-                     "f"(out[mt][0] * 0x1p69f * unscale[mt][0]), "f"(out[mt][1] * 0x1p69f * unscale[mt][1]),
-                     "f"(out[mt][2] * 0x1p69f * unscale[mt][0]), "f"(out[mt][3] * 0x1p69f * unscale[mt][1]) : "memory");
+                     "f"(out[mt][0] * kOut * unscale[mt][0]), "f"(out[mt][1] * kOut * unscale[mt][1]),
+                     "f"(out[mt][2] * kOut * unscale[mt][0]), "f"(out[mt][3] * kOut * unscale[mt][1]) : "memory");
     }
     __syncwarp();
     if (lane == 0) tc::mbar_arrive(done0 + 8 * slot);   // release: the partial tile is visible to the reducer
@@ -740,7 +776,7 @@ bool fill_plan(const QmmArgs& a, RowsPlan& pl) {
 RowsPlan make_plan(const QmmArgs& a) {
   RowsPlan pl{};
   pl.ok = false;
-  if (a.dtype != B200Q_BF16 || !a.transpose || a.w_batched || a.batch != 1) return pl;
+  if ((a.dtype != B200Q_BF16 && !(a.dtype == B200Q_F16 && a.peers.n == 0)) || !a.transpose || a.w_batched || a.batch != 1) return pl;
   if (a.M < 1 || a.M > 16 || a.N < 1 || a.K < 1) return pl;
   if (a.bits != 2 && a.bits != 4 && a.bits != 8) return pl;
   if (a.bits == 2 && a.group == 32) return pl;   // a group would be half a 16-byte unit
@@ -757,13 +793,13 @@ RowsPlan make_plan(const QmmArgs& a) {
 #undef B200Q_ROWS_CASE
   if (!ok) return pl;
   RowsParams& p = pl.prm;
-  p.x = (const __nv_bfloat16*)a.x;
+  p.x = (const uint16_t*)a.x;
   if (a.peers.n > 0) {
     p.n_out = a.peers.n; p.ld = a.peers.ld; p.col0 = a.peers.col0;
-    for (int q = 0; q < a.peers.n; ++q) p.y[q] = (__nv_bfloat16*)a.peers.y[q];
+    for (int q = 0; q < a.peers.n; ++q) p.y[q] = (uint16_t*)a.peers.y[q];
     p.sig = a.peers.sig;
   } else {
-    p.n_out = 1; p.ld = a.N; p.col0 = 0; p.y[0] = (__nv_bfloat16*)a.y;
+    p.n_out = 1; p.ld = a.N; p.col0 = 0; p.y[0] = (uint16_t*)a.y;
   }
   p.M = (int)a.M; p.N = (int)a.N; p.K = (int)a.K;
   p.status = nullptr;
@@ -799,7 +835,7 @@ int rows_inflight(int mt, int bits, int nph) {
   return bits >= 8 ? 2 : 1;
 }
 
-template <int BITS, int G, int MT>
+template <typename T, int BITS, int G, int MT>
 int launch_rows(const QmmArgs& a, const RowsPlan& pl, cudaStream_t st) {
   EncodeFn enc = rows_encode_fn();
   if (!enc) return fail(B200Q_ERR_CUDA, "[quantized_matmul] cuTensorMapEncodeTiled is not available");
@@ -828,7 +864,7 @@ int launch_rows(const QmmArgs& a, const RowsPlan& pl, cudaStream_t st) {
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[quantized_matmul] tensor map for scales / biases failed (%d)", (int)r);
   }
-  auto kern = qmv_rows_kernel<BITS, G, MT>;
+  auto kern = qmv_rows_kernel<T, BITS, G, MT>;
   if (pl.smem > 48 * 1024)
     B200Q_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
   cudaLaunchConfig_t cfg = {};
@@ -900,7 +936,9 @@ int qmv_rows(const QmmArgs& a, cudaStream_t st) {
   int rc = B200Q_ERR_UNSUPPORTED;
 #define B200Q_ROWS_CASE(BITS_, G_)                                                                  \
   if (a.bits == BITS_ && a.group == G_)                                                             \
-    rc = pl.mt == 2 ? launch_rows<BITS_, G_, 2>(a, pl, st) : launch_rows<BITS_, G_, 1>(a, pl, st);
+    rc = a.dtype == B200Q_BF16                                                                      \
+             ? (pl.mt == 2 ? launch_rows<__nv_bfloat16, BITS_, G_, 2>(a, pl, st) : launch_rows<__nv_bfloat16, BITS_, G_, 1>(a, pl, st)) \
+             : (pl.mt == 2 ? launch_rows<__half, BITS_, G_, 2>(a, pl, st) : launch_rows<__half, BITS_, G_, 1>(a, pl, st));
   B200Q_ROWS_CASE(2, 64) B200Q_ROWS_CASE(2, 128)
   B200Q_ROWS_CASE(4, 32) B200Q_ROWS_CASE(4, 64) B200Q_ROWS_CASE(4, 128)
   B200Q_ROWS_CASE(8, 32) B200Q_ROWS_CASE(8, 64) B200Q_ROWS_CASE(8, 128)
