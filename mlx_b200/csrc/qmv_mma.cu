@@ -113,7 +113,7 @@ __device__ __forceinline__ void load_chunk(const uint32_t* __restrict__ p, uint3
 // first byte is masked in place and read as the bf16 subnormal q * 2^(off - 133); the others are shifted down
 // first; one fma with s * 2^(133 - off) gives s*q+b, rounded once.  Between 3 and 4 instructions per pair
 // instead of 6 (extracting both fields, joining them, subtracting an offset).
-constexpr bool straddles(int bits) { return bits == 3 || bits == 5 || bits == 6; }
+__host__ __device__ constexpr bool straddles(int bits) { return bits == 3 || bits == 5 || bits == 6; }
 template <int BITS>
 __device__ __forceinline__ uint32_t window(const uint32_t (&w)[BITS], int by, bool one_byte) {
   const int b2 = by + 2 * BITS, i0 = by >> 2, i1 = b2 >> 2, r0 = by & 3, r1 = b2 & 3;
