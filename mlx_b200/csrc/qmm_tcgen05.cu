@@ -463,7 +463,6 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int nacc = p.NT <= kAccCols / 2 ? 2 : 1;
 
-  asm volatile("griddepcontrol.launch_dependents;");
   if (threadIdx.x == 32 * 3) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.w) : "memory");
 #pragma unroll
@@ -490,8 +489,6 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   __syncthreads();
   cluster_sync();
   tcgen05_fence_after();
-  // The set-up above runs while the previous kernel of the stream drains; nothing of memory is touched before this.
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int total = p.mtiles ? *p.n_mtiles * p.n_tiles : p.n_tiles * p.m_tiles * p.splits;
   const uint32_t tmem_base = bars->tmem_base;
   const uint32_t tmem_a = tmem_base + kAccCols;
@@ -1010,17 +1007,9 @@ int allow_smem(const void* kernel) {
 template <typename T, int BITS, Form F>
 int launch_one(unsigned grid, size_t smem, cudaStream_t st, const TcMaps& maps, const TcParams& p) {
   if (int rc = allow_smem((const void*)qmm_tc_kernel<T, BITS, F>)) return rc;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  B200Q_CUDA_OK(cudaLaunchKernelEx(&cfg, qmm_tc_kernel<T, BITS, F>, maps, (const TcParams)p));
+  // A plain launch: programmatic stream serialization would hide about 2 us of set-up, but clusters launched that way
+  // faulted (once in some hundred thousand launches here) for a reason that was not found.
+  qmm_tc_kernel<T, BITS, F><<<grid, kThreads, smem, st>>>(maps, p);
   B200Q_LAUNCH_OK("qmm_tc_kernel");
   return B200Q_OK;
 }
