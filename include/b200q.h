@@ -213,6 +213,29 @@ int b200q_gather_qmm_swiglu(const void* x, const uint32_t* wq_gate, const void* 
                             int group_size, int bits, void* ws, size_t ws_bytes, void* stream);
 
 /*
+ * b200q_gather_qmm (transposed, the sort-by-expert path only) and b200q_gather_qmm_swiglu over index pairs as a caller
+ * has them: `shape` is the broadcast shape of the pairs (four dimensions, leading ones 1), each view gives the element
+ * strides (0 where it is broadcast) of 4- or 8-byte integers, of which the low 32 bits count; data == NULL: the
+ * element's offset itself is the index (the default of an index that was not given).  Workspaces as for the
+ * array forms, with n_idx the product of `shape`.  B200Q_ERR_UNSUPPORTED where the sort-by-expert path does not
+ * take the problem.
+ */
+typedef struct {
+  const void* data;
+  int elem_bytes;
+  int64_t stride[4];
+} b200q_index;
+int b200q_gather_qmm_indexed(const void* x, const uint32_t* wq, const void* scales, const void* biases, const b200q_index* lhs,
+                             const b200q_index* rhs, const int64_t shape[4], void* y, int dtype, int64_t x_batch, int64_t E,
+                             int64_t M, int64_t N, int64_t K, int group_size, int bits, void* ws, size_t ws_bytes, void* stream);
+int b200q_gather_qmm_swiglu_indexed(const void* x, const uint32_t* wq_gate, const void* scales_gate, const void* biases_gate,
+                                    const uint32_t* wq_up, const void* scales_up, const void* biases_up,
+                                    const uint32_t* wq_down, const void* scales_down, const void* biases_down,
+                                    const b200q_index* lhs, const b200q_index* rhs, const int64_t shape[4], void* y, int dtype,
+                                    int64_t x_batch, int64_t E, int64_t M, int64_t H, int64_t K1, int64_t N2, int group_size,
+                                    int bits, void* ws, size_t ws_bytes, void* stream);
+
+/*
  * N-sharded linear with the all_gather fused into the matmul epilogue.  Replaces the pair
  * QuantizedAllToShardedLinear.__call__ + all_gather of the reference
  * (python/mlx/nn/layers/distributed.py:357-455, mlx/distributed/ops.cpp:62-84,

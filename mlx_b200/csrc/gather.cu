@@ -26,19 +26,61 @@ struct Header { int n_mtiles; int n_rows_valid; int pad[62]; };
 
 constexpr int kMaxExpertsFast = 1024;
 
+// Index pair i as the caller has it: up to four dimensions of strided 32- or 64-bit integers (their low 32 bits
+// count), or none, where an element's index is its offset.  Read in place: converting, broadcasting and copying the
+// indices first took six launches, more than the sort itself.
+struct IndexView {
+  const void* data;
+  int bytes;            // 4 or 8
+  int stride[4];
+};
+struct Pairs {
+  IndexView lhs, rhs;
+  int shape[4];         // [0] is not needed to decompose an offset
+  int simple;           // two plain arrays of 32-bit indices
+};
+__device__ __forceinline__ uint32_t index_at(const IndexView& v, const int (&c)[4]) {
+  const long long off = (long long)c[0] * v.stride[0] + (long long)c[1] * v.stride[1] + (long long)c[2] * v.stride[2] + (long long)c[3] * v.stride[3];
+  if (v.data == nullptr) return (uint32_t)off;
+  return v.bytes == 8 ? (uint32_t) static_cast<const unsigned long long*>(v.data)[off] : static_cast<const uint32_t*>(v.data)[off];
+}
+__device__ __forceinline__ void pair_at(const Pairs& p, int i, uint32_t& l, uint32_t& e) {
+  if (p.simple) {
+    l = static_cast<const uint32_t*>(p.lhs.data)[i];
+    e = static_cast<const uint32_t*>(p.rhs.data)[i];
+    return;
+  }
+  int c[4];
+  c[3] = i % p.shape[3]; i /= p.shape[3];
+  c[2] = i % p.shape[2]; i /= p.shape[2];
+  c[1] = i % p.shape[1]; c[0] = i / p.shape[1];
+  l = index_at(p.lhs, c);
+  e = index_at(p.rhs, c);
+}
+Pairs plain_pairs(const uint32_t* lhs, const uint32_t* rhs) {
+  Pairs p{};
+  p.lhs.data = lhs; p.rhs.data = rhs;
+  p.simple = 1;
+  return p;
+}
+
+// One block: counting sort of the pairs by expert, and the tile table.  Latency-bound (a few microseconds): the offsets
+// of slots and tiles come from one scan over the experts instead of one thread's walk.
 __global__ void __launch_bounds__(1024)
-gather_sort_kernel(const uint32_t* __restrict__ lhs, const uint32_t* __restrict__ rhs, int n_idx, uint32_t x_batch,
-                   uint32_t E_total, uint32_t e_lo, uint32_t E, int M, int NT, Header* hdr, int* __restrict__ sorted_slot, MTileRec* __restrict__ mtiles,
+gather_sort_kernel(const Pairs pairs, int n_idx, uint32_t x_batch, uint32_t E_total, uint32_t e_lo, uint32_t E, int M, int NT,
+                   Header* hdr, int* __restrict__ sorted_slot, int* __restrict__ sorted_lhs, MTileRec* __restrict__ mtiles,
                    void* y, size_t y_slot_bytes, uint32_t* status) {
   __shared__ int counts[kMaxExpertsFast];
   __shared__ int cursor[kMaxExpertsFast];
-  const int tid = threadIdx.x;
-  for (int e = tid; e < (int)E; e += blockDim.x) counts[e] = 0;
+  __shared__ int warp_sum[2][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  counts[tid] = 0;   // (as many threads as experts at most)
   __syncthreads();
   // Experts [e_lo, e_lo + E) are the ones whose weights this call holds (all of them unless the
   // experts are spread over several GPUs); pairs for other valid experts are somebody else's.
   for (int i = tid; i < n_idx; i += blockDim.x) {
-    const uint32_t e = rhs[i], l = lhs[i];
+    uint32_t l, e;
+    pair_at(pairs, i, l, e);
     if (e < E_total && l < x_batch) {
       if (e - e_lo < E) atomicAdd(&counts[e - e_lo], 1);
     } else {
@@ -48,28 +90,46 @@ gather_sort_kernel(const uint32_t* __restrict__ lhs, const uint32_t* __restrict_
     }
   }
   __syncthreads();
-  if (tid == 0) {
-    int slot0 = 0, g = 0;
-    for (int e = 0; e < (int)E; ++e) {
-      cursor[e] = slot0;
-      const int rows = counts[e] * M, row0 = slot0 * M;
-      for (int r = 0; r < rows; r += NT) {
-        mtiles[g].expert = e;
-        mtiles[g].row0 = row0 + r;
-        mtiles[g].rows = rows - r < NT ? rows - r : NT;
-        mtiles[g].pad = 0;
-        ++g;
-      }
-      slot0 += counts[e];
+  // exclusive sums of (slots, tiles) over the experts
+  const int n = counts[tid], rows = n * M, nt = (rows + NT - 1) / NT;
+  int sn = n, st = nt;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, sn, d), b = __shfl_up_sync(0xffffffffu, st, d);
+    if (lane >= d) { sn += a; st += b; }
+  }
+  if (lane == 31) { warp_sum[0][warp] = sn; warp_sum[1][warp] = st; }
+  __syncthreads();
+  if (warp < 2) {
+    int v = warp_sum[warp][lane];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, v, d);
+      if (lane >= d) v += a;
     }
-    hdr->n_mtiles = g;
-    hdr->n_rows_valid = slot0 * M;
+    warp_sum[warp][lane] = v;
+  }
+  __syncthreads();
+  const int slot0 = sn - n + (warp ? warp_sum[0][warp - 1] : 0), g0 = st - nt + (warp ? warp_sum[1][warp - 1] : 0);
+  cursor[tid] = slot0;
+  for (int k = 0; k < nt; ++k) {
+    const int r = k * NT;
+    mtiles[g0 + k] = MTileRec{tid, slot0 * M + r, rows - r < NT ? rows - r : NT, 0};
+  }
+  if (tid == 0) {
+    hdr->n_mtiles = warp_sum[1][31];
+    hdr->n_rows_valid = warp_sum[0][31] * M;
   }
   __syncthreads();
   for (int i = tid; i < n_idx; i += blockDim.x) {
-    const uint32_t e = rhs[i], l = lhs[i];
+    uint32_t l, e;
+    pair_at(pairs, i, l, e);
     if (e < E_total && l < x_batch) {
-      if (e - e_lo < E) sorted_slot[atomicAdd(&cursor[e - e_lo], 1)] = i;
+      if (e - e_lo < E) {
+        const int at = atomicAdd(&cursor[e - e_lo], 1);
+        sorted_slot[at] = i;
+        sorted_lhs[at] = (int)l;
+      }
     } else {
       unsigned short* dst = reinterpret_cast<unsigned short*>(static_cast<char*>(y) + (size_t)i * y_slot_bytes);
       for (size_t b = 0; b < y_slot_bytes / 2; ++b) dst[b] = 0;
@@ -80,13 +140,13 @@ gather_sort_kernel(const uint32_t* __restrict__ lhs, const uint32_t* __restrict_
 // One CTA per activation row of the sorted order: copies x[lhs[slot]] row m and records where
 // the result row goes.
 __global__ void __launch_bounds__(256)
-gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __restrict__ lhs, const Header* hdr,
+gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ sorted_lhs, const Header* hdr,
                    const int* __restrict__ sorted_slot, int M, int K, __nv_bfloat16* __restrict__ x_sorted,
                    int* __restrict__ dst_row) {
   const int r = blockIdx.x;
   if (r >= hdr->n_rows_valid) return;
   const int slot = sorted_slot[r / M], m = r % M;
-  const uint4* src = reinterpret_cast<const uint4*>(x + ((size_t)lhs[slot] * M + m) * K);
+  const uint4* src = reinterpret_cast<const uint4*>(x + ((size_t)sorted_lhs[r / M] * M + m) * K);
   uint4* dst = reinterpret_cast<uint4*>(x_sorted + (size_t)r * K);
   for (int i = threadIdx.x; i < K / 8; i += blockDim.x) dst[i] = __ldg(src + i);
   if (threadIdx.x == 0) dst_row[r] = slot * M + m;
@@ -104,7 +164,7 @@ int pick_nt(int64_t n_rows, int64_t E) {
 }
 
 struct FastLayout {
-  size_t hdr, sorted, dst, mtiles, xs, total;
+  size_t hdr, sorted, lhs, dst, mtiles, xs, total;
   int64_t n_rows, max_mtiles;
   int nt;
 };
@@ -117,6 +177,7 @@ FastLayout fast_layout(int64_t n_idx, int64_t E, int64_t M, int64_t K) {
   size_t off = 0;
   L.hdr = off; off += align256(sizeof(Header));
   L.sorted = off; off += align256((size_t)n_idx * 4);
+  L.lhs = off; off += align256((size_t)n_idx * 4);
   L.dst = off; off += align256((size_t)L.n_rows * 4);
   L.mtiles = off; off += align256((size_t)L.max_mtiles * sizeof(MTileRec));
   L.xs = off; off += align256((size_t)L.n_rows * K * 2);
@@ -138,8 +199,7 @@ bool fast_supported(int dtype, int64_t n_idx, int64_t x_batch, int64_t E, int64_
 // Sort by expert, gather the activation rows, one grouped tensor-core launch.  Experts
 // [e_lo, e_lo + E_local) of E_total are the ones whose weights `wq` holds; with `peers` every
 // result row is stored into all of the given [n_idx * M, N] buffers.
-int run_grouped(const void* x, const uint32_t* wq, const void* scales, const void* biases, const uint32_t* lhs_idx,
-                const uint32_t* rhs_idx, int64_t n_idx, void* y, const PeerOut* peers, int64_t x_batch, int64_t E_total,
+int run_grouped(const void* x, const uint32_t* wq, const void* scales, const void* biases, const Pairs& pairs, int64_t n_idx, void* y, const PeerOut* peers, int64_t x_batch, int64_t E_total,
                 int64_t e_lo, int64_t E_local, int64_t M, int64_t N, int64_t K, int group_size, int bits, void* ws,
                 size_t ws_bytes, cudaStream_t st) {
   uint32_t* status = reinterpret_cast<uint32_t*>(static_cast<char*>(ws) + ws_bytes - kStatusBytes);
@@ -147,13 +207,14 @@ int run_grouped(const void* x, const uint32_t* wq, const void* scales, const voi
   char* base = static_cast<char*>(ws);
   Header* hdr = reinterpret_cast<Header*>(base + L.hdr);
   int* sorted = reinterpret_cast<int*>(base + L.sorted);
+  int* slhs = reinterpret_cast<int*>(base + L.lhs);
   int* dst = reinterpret_cast<int*>(base + L.dst);
   MTileRec* mt = reinterpret_cast<MTileRec*>(base + L.mtiles);
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(base + L.xs);
-  gather_sort_kernel<<<1, 1024, 0, st>>>(lhs_idx, rhs_idx, (int)n_idx, (uint32_t)x_batch, (uint32_t)E_total, (uint32_t)e_lo,
-                                         (uint32_t)E_local, (int)M, L.nt, hdr, sorted, mt, y, (size_t)M * N * 2, status);
+  gather_sort_kernel<<<1, 1024, 0, st>>>(pairs, (int)n_idx, (uint32_t)x_batch, (uint32_t)E_total, (uint32_t)e_lo,
+                                         (uint32_t)E_local, (int)M, L.nt, hdr, sorted, slhs, mt, y, (size_t)M * N * 2, status);
   B200Q_LAUNCH_OK("gather_sort_kernel");
-  gather_rows_kernel<<<(unsigned)L.n_rows, 256, 0, st>>>((const __nv_bfloat16*)x, lhs_idx, hdr, sorted, (int)M, (int)K,
+  gather_rows_kernel<<<(unsigned)L.n_rows, 256, 0, st>>>((const __nv_bfloat16*)x, slhs, hdr, sorted, (int)M, (int)K,
                                                          xs, dst);
   B200Q_LAUNCH_OK("gather_rows_kernel");
   GroupedArgs g{};
@@ -215,7 +276,7 @@ extern "C" int b200q_gather_qmm(const void* x, const uint32_t* wq, const void* s
   const bool aligned = !((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wq) |
                           reinterpret_cast<uintptr_t>(ws) | reinterpret_cast<uintptr_t>(y)) & 15);
   if (aligned && fast_supported(dtype, n_idx, x_batch, E, M, N, K, group_size, bits, transpose))
-    return run_grouped(x, wq, scales, biases, lhs_idx, rhs_idx, n_idx, y, nullptr, x_batch, E, 0, E, M, N, K, group_size,
+    return run_grouped(x, wq, scales, biases, plain_pairs(lhs_idx, rhs_idx), n_idx, y, nullptr, x_batch, E, 0, E, M, N, K, group_size,
                        bits, ws, ws_bytes, st);
 
   QmmArgs a{};
@@ -270,7 +331,7 @@ int gather_sharded_impl(const void* x, const uint32_t* wq_local, const void* sca
                           reinterpret_cast<uintptr_t>(ws)) & 15);
   if (!aligned || E_local < 1 || !fast_supported(dtype, n_idx, x_batch, E_total, M, N, K, group_size, bits, 1))
     return fail(B200Q_ERR_UNSUPPORTED, "[gather_qmm_sharded] only bfloat16 with K a multiple of 128 has a peer-store epilogue");
-  return run_grouped(x, wq_local, scales_local, biases_local, lhs_idx, rhs_idx, n_idx, y_peers[self], &peers, x_batch, E_total,
+  return run_grouped(x, wq_local, scales_local, biases_local, plain_pairs(lhs_idx, rhs_idx), n_idx, y_peers[self], &peers, x_batch, E_total,
                      e_lo, E_local, M, N, K, group_size, bits, ws, ws_bytes, static_cast<cudaStream_t>(stream));
 }
 }  // namespace
@@ -335,14 +396,15 @@ extern "C" int b200q_gather_qmm_chain(const void* x, const uint32_t* wq1, const 
   char* base = static_cast<char*>(ws);
   Header* hdr = reinterpret_cast<Header*>(base + L.hdr);
   int* sorted = reinterpret_cast<int*>(base + L.sorted);
+  int* slhs = reinterpret_cast<int*>(base + L.lhs);
   int* dst = reinterpret_cast<int*>(base + L.dst);
   MTileRec* mt = reinterpret_cast<MTileRec*>(base + L.mtiles);
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(base + L.xs);
   __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(base + L.total - 256);   // after the gathered rows
-  gather_sort_kernel<<<1, 1024, 0, st>>>(lhs_idx, rhs_idx, (int)n_idx, (uint32_t)x_batch, (uint32_t)E, 0u, (uint32_t)E, (int)M,
-                                         L.nt, hdr, sorted, mt, y, (size_t)M * N2 * 2, status);
+  gather_sort_kernel<<<1, 1024, 0, st>>>(plain_pairs(lhs_idx, rhs_idx), (int)n_idx, (uint32_t)x_batch, (uint32_t)E, 0u, (uint32_t)E, (int)M,
+                                         L.nt, hdr, sorted, slhs, mt, y, (size_t)M * N2 * 2, status);
   B200Q_LAUNCH_OK("gather_sort_kernel");
-  gather_rows_kernel<<<(unsigned)L.n_rows, 256, 0, st>>>((const __nv_bfloat16*)x, lhs_idx, hdr, sorted, (int)M, (int)K1, xs, dst);
+  gather_rows_kernel<<<(unsigned)L.n_rows, 256, 0, st>>>((const __nv_bfloat16*)x, slhs, hdr, sorted, (int)M, (int)K1, xs, dst);
   B200Q_LAUNCH_OK("gather_rows_kernel");
   GroupedArgs g{};
   g.mtiles = mt; g.n_mtiles = &hdr->n_mtiles;
@@ -389,12 +451,11 @@ extern "C" size_t b200q_gather_qmm_swiglu_workspace_bytes(int64_t n_idx, int64_t
   return L.total + 2 * align256((size_t)L.n_rows * H * 2);
 }
 
-extern "C" int b200q_gather_qmm_swiglu(const void* x, const uint32_t* wq_gate, const void* scales_gate, const void* biases_gate,
-                                       const uint32_t* wq_up, const void* scales_up, const void* biases_up,
-                                       const uint32_t* wq_down, const void* scales_down, const void* biases_down,
-                                       const uint32_t* lhs_idx, const uint32_t* rhs_idx, int64_t n_idx, void* y, int dtype,
-                                       int64_t x_batch, int64_t E, int64_t M, int64_t H, int64_t K1, int64_t N2,
-                                       int group_size, int bits, void* ws, size_t ws_bytes, void* stream) {
+namespace {
+int swiglu_impl(const void* x, const uint32_t* wq_gate, const void* scales_gate, const void* biases_gate, const uint32_t* wq_up,
+                const void* scales_up, const void* biases_up, const uint32_t* wq_down, const void* scales_down,
+                const void* biases_down, const Pairs& pairs, int64_t n_idx, void* y, int dtype, int64_t x_batch, int64_t E,
+                int64_t M, int64_t H, int64_t K1, int64_t N2, int group_size, int bits, void* ws, size_t ws_bytes, void* stream) {
   if (!valid_group(group_size) || !valid_bits(bits))
     return fail(B200Q_ERR_INVALID_ARGUMENT, "[gather_qmm_swiglu] group size must be 32, 64 or 128 and bits 2, 3, 4, 5, 6 or 8");
   if (n_idx < 0 || x_batch < 0 || E < 1 || M < 0 || H < 0 || K1 < 0 || N2 < 0)
@@ -403,7 +464,7 @@ extern "C" int b200q_gather_qmm_swiglu(const void* x, const uint32_t* wq_gate, c
     return fail(B200Q_ERR_INVALID_ARGUMENT, "[gather_qmm_swiglu] The shapes of the weight and scales are incompatible based on bits and group_size");
   if (n_idx == 0 || M == 0 || N2 == 0) return B200Q_OK;
   if (!x || !wq_gate || !scales_gate || !biases_gate || !wq_up || !scales_up || !biases_up || !wq_down || !scales_down ||
-      !biases_down || !lhs_idx || !rhs_idx || !y)
+      !biases_down || !y || (pairs.simple && (!pairs.lhs.data || !pairs.rhs.data)))
     return fail(B200Q_ERR_INVALID_ARGUMENT, "[gather_qmm_swiglu] null pointer");
   const bool aligned = !((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wq_gate) | reinterpret_cast<uintptr_t>(wq_up) |
                           reinterpret_cast<uintptr_t>(wq_down) | reinterpret_cast<uintptr_t>(ws) | reinterpret_cast<uintptr_t>(y)) & 15);
@@ -419,16 +480,17 @@ extern "C" int b200q_gather_qmm_swiglu(const void* x, const uint32_t* wq_gate, c
   char* base = static_cast<char*>(ws);
   Header* hdr = reinterpret_cast<Header*>(base + L.hdr);
   int* sorted = reinterpret_cast<int*>(base + L.sorted);
+  int* slhs = reinterpret_cast<int*>(base + L.lhs);
   int* dst = reinterpret_cast<int*>(base + L.dst);
   MTileRec* mt = reinterpret_cast<MTileRec*>(base + L.mtiles);
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(base + L.xs);
   const size_t h_bytes = align256((size_t)L.n_rows * H * 2);
   __nv_bfloat16* hg = reinterpret_cast<__nv_bfloat16*>(base + L.total - 256);
   __nv_bfloat16* hu = reinterpret_cast<__nv_bfloat16*>(base + L.total - 256 + h_bytes);
-  gather_sort_kernel<<<1, 1024, 0, st>>>(lhs_idx, rhs_idx, (int)n_idx, (uint32_t)x_batch, (uint32_t)E, 0u, (uint32_t)E, (int)M,
-                                         L.nt, hdr, sorted, mt, y, (size_t)M * N2 * 2, status);
+  gather_sort_kernel<<<1, 1024, 0, st>>>(pairs, (int)n_idx, (uint32_t)x_batch, (uint32_t)E, 0u, (uint32_t)E, (int)M,
+                                         L.nt, hdr, sorted, slhs, mt, y, (size_t)M * N2 * 2, status);
   B200Q_LAUNCH_OK("gather_sort_kernel");
-  gather_rows_kernel<<<(unsigned)L.n_rows, 256, 0, st>>>((const __nv_bfloat16*)x, lhs_idx, hdr, sorted, (int)M, (int)K1, xs, dst);
+  gather_rows_kernel<<<(unsigned)L.n_rows, 256, 0, st>>>((const __nv_bfloat16*)x, slhs, hdr, sorted, (int)M, (int)K1, xs, dst);
   B200Q_LAUNCH_OK("gather_rows_kernel");
   GroupedArgs g{};
   g.mtiles = mt; g.n_mtiles = &hdr->n_mtiles;
@@ -444,4 +506,76 @@ extern "C" int b200q_gather_qmm_swiglu(const void* x, const uint32_t* wq_gate, c
   B200Q_LAUNCH_OK("swiglu_kernel");
   g.x_sorted = hg; g.wq = wq_down; g.scales = scales_down; g.biases = biases_down; g.y = y; g.dst_row = dst; g.N = N2; g.K = H;
   return qmm_tc_grouped(g, st);
+}
+}  // namespace
+
+extern "C" int b200q_gather_qmm_swiglu(const void* x, const uint32_t* wq_gate, const void* scales_gate, const void* biases_gate,
+                                       const uint32_t* wq_up, const void* scales_up, const void* biases_up,
+                                       const uint32_t* wq_down, const void* scales_down, const void* biases_down,
+                                       const uint32_t* lhs_idx, const uint32_t* rhs_idx, int64_t n_idx, void* y, int dtype,
+                                       int64_t x_batch, int64_t E, int64_t M, int64_t H, int64_t K1, int64_t N2,
+                                       int group_size, int bits, void* ws, size_t ws_bytes, void* stream) {
+  return swiglu_impl(x, wq_gate, scales_gate, biases_gate, wq_up, scales_up, biases_up, wq_down, scales_down, biases_down,
+                     plain_pairs(lhs_idx, rhs_idx), n_idx, y, dtype, x_batch, E, M, H, K1, N2, group_size, bits, ws, ws_bytes, stream);
+}
+
+// ---------------------------------------------------------------- the same two operators over strided index views
+namespace {
+bool view_pairs(const b200q_index* lhs, const b200q_index* rhs, const int64_t shape[4], Pairs& p, int64_t& n_idx) {
+  n_idx = 1;
+  p = Pairs{};
+  for (int d = 0; d < 4; ++d) {
+    if (shape[d] < 0 || shape[d] > INT32_MAX) return false;
+    n_idx *= shape[d];
+    if (n_idx > INT32_MAX) return false;
+    p.shape[d] = (int)shape[d];
+  }
+  const b200q_index* in[2] = {lhs, rhs};
+  IndexView* out[2] = {&p.lhs, &p.rhs};
+  for (int k = 0; k < 2; ++k) {
+    if (in[k]->data != nullptr && in[k]->elem_bytes != 4 && in[k]->elem_bytes != 8) return false;
+    out[k]->data = in[k]->data;
+    out[k]->bytes = in[k]->elem_bytes;
+    for (int d = 0; d < 4; ++d) {
+      if (in[k]->stride[d] > INT32_MAX || in[k]->stride[d] < INT32_MIN) return false;
+      out[k]->stride[d] = (int)in[k]->stride[d];
+    }
+  }
+  return true;
+}
+}  // namespace
+
+extern "C" int b200q_gather_qmm_indexed(const void* x, const uint32_t* wq, const void* scales, const void* biases,
+                                        const b200q_index* lhs, const b200q_index* rhs, const int64_t shape[4], void* y,
+                                        int dtype, int64_t x_batch, int64_t E, int64_t M, int64_t N, int64_t K, int group_size,
+                                        int bits, void* ws, size_t ws_bytes, void* stream) {
+  Pairs p;
+  int64_t n_idx = 0;
+  if (!lhs || !rhs || !shape || !view_pairs(lhs, rhs, shape, p, n_idx))
+    return fail(B200Q_ERR_INVALID_ARGUMENT, "[gather_qmm] bad index view");
+  if (!valid_group(group_size) || !valid_bits(bits) || K % group_size != 0)
+    return fail(B200Q_ERR_INVALID_ARGUMENT, "[gather_qmm] unsupported group size %d, bits %d or K", group_size, bits);
+  if (n_idx == 0 || M == 0 || N == 0) return B200Q_OK;
+  const bool aligned = !((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wq) |
+                          reinterpret_cast<uintptr_t>(ws) | reinterpret_cast<uintptr_t>(y)) & 15);
+  if (!x || !wq || !scales || !biases || !y || !aligned || !fast_supported(dtype, n_idx, x_batch, E, M, N, K, group_size, bits, 1))
+    return fail(B200Q_ERR_UNSUPPORTED, "[gather_qmm] index views need bfloat16 with K a multiple of 128");
+  if (!ws || ws_bytes < fast_layout(n_idx, E, M, K).total)
+    return fail(B200Q_ERR_WORKSPACE, "[gather_qmm] workspace of %zu bytes required, %zu given", fast_layout(n_idx, E, M, K).total, ws_bytes);
+  return run_grouped(x, wq, scales, biases, p, n_idx, y, nullptr, x_batch, E, 0, E, M, N, K, group_size, bits, ws, ws_bytes,
+                     static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int b200q_gather_qmm_swiglu_indexed(const void* x, const uint32_t* wq_gate, const void* scales_gate, const void* biases_gate,
+                                               const uint32_t* wq_up, const void* scales_up, const void* biases_up,
+                                               const uint32_t* wq_down, const void* scales_down, const void* biases_down,
+                                               const b200q_index* lhs, const b200q_index* rhs, const int64_t shape[4], void* y,
+                                               int dtype, int64_t x_batch, int64_t E, int64_t M, int64_t H, int64_t K1, int64_t N2,
+                                               int group_size, int bits, void* ws, size_t ws_bytes, void* stream) {
+  Pairs p;
+  int64_t n_idx = 0;
+  if (!lhs || !rhs || !shape || !view_pairs(lhs, rhs, shape, p, n_idx))
+    return fail(B200Q_ERR_INVALID_ARGUMENT, "[gather_qmm_swiglu] bad index view");
+  return swiglu_impl(x, wq_gate, scales_gate, biases_gate, wq_up, scales_up, biases_up, wq_down, scales_down, biases_down, p,
+                     n_idx, y, dtype, x_batch, E, M, H, K1, N2, group_size, bits, ws, ws_bytes, stream);
 }
