@@ -11,6 +11,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <vector>
@@ -223,6 +224,148 @@ PyObject* py_qmm_grad(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// ---- gather_qmm and the gated expert layer
+// An index operand as a view over the pairs: right-aligned to four dimensions.  `t` null: the default index, which is
+// the offset into `lead` (the batch dimensions of the operand it selects from).
+struct View {
+  b200q_index v;
+  int64_t shape[4];
+};
+bool make_view(const Tensor* t, at::IntArrayRef lead, at::Device dev, View* out) {
+  for (int d = 0; d < 4; ++d) { out->shape[d] = 1; out->v.stride[d] = 0; }
+  out->v.data = nullptr;
+  out->v.elem_bytes = 4;
+  const int64_t nd = t ? t->dim() : (int64_t)lead.size();
+  if (nd > 4) return false;
+  if (t) {
+    const at::ScalarType k = t->scalar_type();
+    if (t->device() != dev || (k != at::kLong && k != at::kInt && k != at::kUInt32)) return false;
+    if (t->numel() == 0) return false;
+    out->v.data = t->data_ptr();
+    out->v.elem_bytes = k == at::kLong ? 8 : 4;
+    for (int64_t d = 0; d < nd; ++d) {
+      out->shape[4 - nd + d] = t->size(d);
+      out->v.stride[4 - nd + d] = t->size(d) == 1 ? 0 : t->stride(d);
+    }
+  } else {
+    int64_t st = 1;
+    for (int64_t d = nd - 1; d >= 0; --d) {
+      out->shape[4 - nd + d] = lead[d];
+      out->v.stride[4 - nd + d] = lead[d] == 1 ? 0 : st;
+      st *= lead[d];
+    }
+  }
+  return true;
+}
+// The pairs' shape (and the output's leading dimensions); false where the views do not broadcast.
+bool broadcast(View* a, View* b, int64_t nd_a, int64_t nd_b, int64_t shape[4], int64_t* n, c10::SmallVector<int64_t, 6>* lead) {
+  *n = 1;
+  for (int d = 0; d < 4; ++d) {
+    if (a->shape[d] != b->shape[d] && a->shape[d] != 1 && b->shape[d] != 1) return false;
+    shape[d] = a->shape[d] == 1 ? b->shape[d] : a->shape[d];
+    *n *= shape[d];
+  }
+  lead->clear();
+  for (int d = 4 - (int)std::max(nd_a, nd_b); d < 4; ++d) lead->push_back(shape[d]);
+  return true;
+}
+int64_t product(at::IntArrayRef v) {
+  int64_t n = 1;
+  for (int64_t x : v) n *= x;
+  return n;
+}
+// Index argument: None, or a plain tensor.
+bool index_arg(PyObject* o, const Tensor** t) {
+  if (o == Py_None) { *t = nullptr; return true; }
+  return (*t = tensor(o)) != nullptr;
+}
+
+// (x, w, scales, biases, lhs_indices, rhs_indices, transpose, group_size, bits, mode)
+PyObject* py_gather(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const Tensor *x, *w, *s, *b, *li, *ri;
+  int group, bits;
+  if (n != 10 || !(x = tensor(a[0])) || !(w = tensor(a[1])) || !(s = tensor(a[2])) || !(b = tensor(a[3])) || !index_arg(a[4], &li) ||
+      !index_arg(a[5], &ri) || (!li && !ri) || a[6] != Py_True || !integer(a[7], 64, &group) || !integer(a[8], 4, &bits) ||
+      !affine(a[9]))
+    return none();
+  const at::Device dev = x->device();
+  if (x->scalar_type() != at::kBFloat16 || !params_ok(group, bits) || !current(dev) || x->dim() < 2 || w->dim() < 3 ||
+      !x->is_contiguous() || !plain_weights(*w, *s, *b, at::kBFloat16, dev, group, bits) || checked())
+    return none();
+  const int64_t M = x->size(-2), K = x->size(-1), N = w->size(-2), x_batch = product(x->sizes().slice(0, x->dim() - 2)),
+                E = product(w->sizes().slice(0, w->dim() - 2));
+  if (w->size(-1) * 32 / bits != K || M == 0 || N == 0 || K == 0 || x_batch == 0 || E == 0) return none();
+  View l, r;
+  int64_t shape[4], n_idx;
+  c10::SmallVector<int64_t, 6> size;
+  const auto xl = x->sizes().slice(0, x->dim() - 2), wl = w->sizes().slice(0, w->dim() - 2);
+  if (!make_view(li, xl, dev, &l) || !make_view(ri, wl, dev, &r) ||
+      !broadcast(&l, &r, li ? li->dim() : (int64_t)xl.size(), ri ? ri->dim() : (int64_t)wl.size(), shape, &n_idx, &size))
+    return none();
+  void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  const Scratch* ws = find_scratch(dev.index(), stream, 1, b200q_gather_qmm_workspace_bytes(B200Q_BF16, n_idx, x_batch, E, M, N, K, group, bits, 1));
+  if (!ws) return none();
+  size.push_back(M);
+  size.push_back(N);
+  Tensor y = at::detail::empty_cuda(size, at::kBFloat16, dev, std::nullopt);
+  if (b200q_gather_qmm_indexed(x->data_ptr(), static_cast<const uint32_t*>(w->data_ptr()), s->data_ptr(), b->data_ptr(), &l.v, &r.v,
+                               shape, y.data_ptr(), B200Q_BF16, x_batch, E, M, N, K, group, bits, ws->ptr, ws->bytes, stream) != B200Q_OK)
+    return none();
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// A (w, scales, biases) triple of plain tensors.
+bool triple(PyObject* o, const Tensor* (&t)[3]) {
+  if (!(PyTuple_CheckExact(o) || PyList_CheckExact(o)) || PySequence_Fast_GET_SIZE(o) != 3) return false;
+  for (int i = 0; i < 3; ++i)
+    if (!(t[i] = tensor(PySequence_Fast_GET_ITEM(o, i)))) return false;
+  return true;
+}
+
+// (x, gate, up, down, rhs_indices, lhs_indices, group_size, bits)
+PyObject* py_swiglu(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const Tensor *x, *g[3], *u[3], *d[3], *li, *ri;
+  int group, bits;
+  if (n != 8 || !(x = tensor(a[0])) || !triple(a[1], g) || !triple(a[2], u) || !triple(a[3], d) || !index_arg(a[4], &ri) || !ri ||
+      !index_arg(a[5], &li) || !integer(a[6], 64, &group) || !integer(a[7], 4, &bits))
+    return none();
+  const at::Device dev = x->device();
+  if (x->scalar_type() != at::kBFloat16 || !params_ok(group, bits) || !current(dev) || x->dim() < 2 || g[0]->dim() < 3 ||
+      !x->is_contiguous() || checked())
+    return none();
+  for (const auto& t : {g, u, d})
+    if (!plain_weights(*t[0], *t[1], *t[2], at::kBFloat16, dev, group, bits)) return none();
+  const int64_t M = x->size(-2), K1 = x->size(-1), H = g[0]->size(-2), N2 = d[0]->size(-2),
+                x_batch = product(x->sizes().slice(0, x->dim() - 2)), E = product(g[0]->sizes().slice(0, g[0]->dim() - 2));
+  if (g[0]->sizes() != u[0]->sizes() || g[0]->size(-1) * 32 / bits != K1 || d[0]->size(-1) * 32 / bits != H ||
+      g[0]->dim() != d[0]->dim() || g[0]->sizes().slice(0, g[0]->dim() - 2) != d[0]->sizes().slice(0, d[0]->dim() - 2) || M == 0 ||
+      K1 == 0 || H == 0 || N2 == 0 || x_batch == 0 || E == 0)
+    return none();
+  View l, r;
+  int64_t shape[4], n_idx;
+  c10::SmallVector<int64_t, 6> size;
+  const auto xl = x->sizes().slice(0, x->dim() - 2);
+  if (!make_view(li, xl, dev, &l) || !make_view(ri, xl, dev, &r) ||
+      !broadcast(&l, &r, li ? li->dim() : (int64_t)xl.size(), ri->dim(), shape, &n_idx, &size))
+    return none();
+  void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  const Scratch* ws = find_scratch(dev.index(), stream, 1, b200q_gather_qmm_swiglu_workspace_bytes(n_idx, E, M, H, K1));
+  if (!ws) return none();
+  size.push_back(M);
+  size.push_back(N2);
+  Tensor y = at::detail::empty_cuda(size, at::kBFloat16, dev, std::nullopt);
+  auto w = [](const Tensor* t) { return static_cast<const uint32_t*>(t->data_ptr()); };
+  if (b200q_gather_qmm_swiglu_indexed(x->data_ptr(), w(g[0]), g[1]->data_ptr(), g[2]->data_ptr(), w(u[0]), u[1]->data_ptr(),
+                                      u[2]->data_ptr(), w(d[0]), d[1]->data_ptr(), d[2]->data_ptr(), &l.v, &r.v, shape, y.data_ptr(),
+                                      B200Q_BF16, x_batch, E, M, H, K1, N2, group, bits, ws->ptr, ws->bytes, stream) != B200Q_OK)
+    return none();
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
 // (device index, stream, operator, address, bytes): ops._workspaces has a new buffer
 PyObject* py_scratch(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 5) { PyErr_SetString(PyExc_TypeError, "scratch takes five arguments"); return nullptr; }
@@ -239,6 +382,8 @@ PyMethodDef methods[] = {
     {"qmm_grad", (PyCFunction)(void (*)(void))py_qmm_grad, METH_FASTCALL, nullptr},
     {"quantize", (PyCFunction)(void (*)(void))py_quantize, METH_FASTCALL, nullptr},
     {"dequantize", (PyCFunction)(void (*)(void))py_dequantize, METH_FASTCALL, nullptr},
+    {"gather", (PyCFunction)(void (*)(void))py_gather, METH_FASTCALL, nullptr},
+    {"swiglu", (PyCFunction)(void (*)(void))py_swiglu, METH_FASTCALL, nullptr},
     {"scratch", (PyCFunction)(void (*)(void))py_scratch, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_front", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -401,6 +401,9 @@ def gather_qmm(x: torch.Tensor, w: torch.Tensor, scales: torch.Tensor, biases: O
     """mlx/ops.cpp:5553-5629.  out shape = broadcast(lhs, rhs).shape + [M, N]."""
     if lhs_indices is None and rhs_indices is None:
         return quantized_matmul(x, w, scales, biases, transpose, group_size, bits, mode)
+    y = _front.gather(x, w, scales, biases, lhs_indices, rhs_indices, transpose, group_size, bits, mode)
+    if y is not None:
+        return y
     group_size, bits = _mode_params(mode, group_size, bits, "gather_qmm")
     out_type = _validate_mode_with_type("gather_qmm", scales, biases, None)
     _, w_outer = _extract_dims("gather_qmm", x, w, scales, biases, transpose, group_size, bits)
@@ -506,6 +509,9 @@ def gather_qmm_swiglu(x: torch.Tensor, gate, up, down, rhs_indices: torch.Tensor
     index pairs with one sort (three mlx/ops.cpp:5553-5629 calls and the activation in the reference).
     gate, up, down: (w, scales, biases) triples; gate/up [E, H, K1*bits/32], down [E, N2, H*bits/32];
     x [B, M, K1] bf16; out: idx_shape + [M, N2]."""
+    y = _front.swiglu(x, gate, up, down, rhs_indices, lhs_indices, group_size, bits)
+    if y is not None:
+        return y
     group_size, bits = _mode_params("affine", group_size, bits, "gather_qmm_swiglu")
     for t in (gate, up, down):
         _validate_quantized_input("gather_qmm_swiglu", t[0], t[1], group_size, bits, t[2])
