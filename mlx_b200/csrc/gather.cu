@@ -165,7 +165,7 @@ int pick_nt(int64_t n_rows, int64_t E) {
 
 struct FastLayout {
   size_t hdr, sorted, lhs, dst, mtiles, xs, total;
-  int64_t n_rows, max_mtiles;
+  int64_t n_rows, max_mtiles, max_few;   // max_few: tiles of kRowsTile rows
   int nt;
 };
 
@@ -174,12 +174,13 @@ FastLayout fast_layout(int64_t n_idx, int64_t E, int64_t M, int64_t K) {
   L.n_rows = n_idx * M;
   L.nt = pick_nt(L.n_rows, E);
   L.max_mtiles = L.n_rows / L.nt + E + 1;
+  L.max_few = L.n_rows / kRowsTile + (E < L.n_rows ? E : L.n_rows);
   size_t off = 0;
   L.hdr = off; off += align256(sizeof(Header));
   L.sorted = off; off += align256((size_t)n_idx * 4);
   L.lhs = off; off += align256((size_t)n_idx * 4);
   L.dst = off; off += align256((size_t)L.n_rows * 4);
-  L.mtiles = off; off += align256((size_t)L.max_mtiles * sizeof(MTileRec));
+  L.mtiles = off; off += align256((size_t)(L.max_mtiles > L.max_few ? L.max_mtiles : L.max_few) * sizeof(MTileRec));
   L.xs = off; off += align256((size_t)L.n_rows * K * 2);
   L.total = off + 256;  // status word lives in the last 16 bytes
   return L;
@@ -196,6 +197,26 @@ bool fast_supported(int dtype, int64_t n_idx, int64_t x_batch, int64_t E, int64_
 }
 
 
+// Experts with few rows go through the row-owning decode kernel: it reads a matrix at 1.6 times the rate at which the
+// tensor-core kernel unpacks one (8 experts [14336, 4096] at 4 bits), takes the rows of x where they lie and needs no
+// second launch for a gated pair.  At more than about four rows per expert on average the tiles of 8 rows begin to
+// split experts, and every part reads the matrix again.
+bool few_rows(int64_t n_rows, int64_t E) { return n_rows <= 4 * E; }
+
+RowsGroup rows_group(const FastLayout& L, char* base, int64_t E, int64_t M, int64_t N, int64_t K, int group, int bits, uint32_t* status) {
+  RowsGroup r{};
+  r.tiles = base + L.mtiles;
+  r.n_tiles = &reinterpret_cast<Header*>(base + L.hdr)->n_mtiles;
+  r.max_tiles = L.max_few;
+  r.per_slot = M; r.E = E; r.N = N; r.K = K;
+  r.group = group; r.bits = bits;
+  r.status = status;
+  return r;
+}
+void set_matrix(RowsGroup& r, int i, const uint32_t* wq, const void* scales, const void* biases) {
+  r.wq[i] = wq; r.scales[i] = scales; r.biases[i] = biases;
+}
+
 // Sort by expert, gather the activation rows, one grouped tensor-core launch.  Experts
 // [e_lo, e_lo + E_local) of E_total are the ones whose weights `wq` holds; with `peers` every
 // result row is stored into all of the given [n_idx * M, N] buffers.
@@ -211,6 +232,15 @@ int run_grouped(const void* x, const uint32_t* wq, const void* scales, const voi
   int* dst = reinterpret_cast<int*>(base + L.dst);
   MTileRec* mt = reinterpret_cast<MTileRec*>(base + L.mtiles);
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(base + L.xs);
+  RowsGroup r = rows_group(L, base, E_local, M, N, K, group_size, bits, status);
+  set_matrix(r, 0, wq, scales, biases);
+  if (!peers && few_rows(L.n_rows, E_total) && qmv_rows_grouped_supported(r)) {
+    gather_sort_kernel<<<1, 1024, 0, st>>>(pairs, (int)n_idx, (uint32_t)x_batch, (uint32_t)E_total, (uint32_t)e_lo, (uint32_t)E_local,
+                                           (int)M, kRowsTile, hdr, sorted, slhs, mt, y, (size_t)M * N * 2, status);
+    B200Q_LAUNCH_OK("gather_sort_kernel");
+    r.x = x; r.src_slot = slhs; r.y = y; r.dst_slot = sorted;
+    return qmv_rows_grouped(r, st);
+  }
   gather_sort_kernel<<<1, 1024, 0, st>>>(pairs, (int)n_idx, (uint32_t)x_batch, (uint32_t)E_total, (uint32_t)e_lo,
                                          (uint32_t)E_local, (int)M, L.nt, hdr, sorted, slhs, mt, y, (size_t)M * N * 2, status);
   B200Q_LAUNCH_OK("gather_sort_kernel");
@@ -401,6 +431,18 @@ extern "C" int b200q_gather_qmm_chain(const void* x, const uint32_t* wq1, const 
   MTileRec* mt = reinterpret_cast<MTileRec*>(base + L.mtiles);
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(base + L.xs);
   __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(base + L.total - 256);   // after the gathered rows
+  RowsGroup r1 = rows_group(L, base, E, M, N1, K1, group_size, bits, status), r2 = rows_group(L, base, E, M, N2, N1, group_size, bits, status);
+  set_matrix(r1, 0, wq1, scales1, biases1);
+  set_matrix(r2, 0, wq2, scales2, biases2);
+  if (few_rows(L.n_rows, E) && qmv_rows_grouped_supported(r1) && qmv_rows_grouped_supported(r2)) {
+    gather_sort_kernel<<<1, 1024, 0, st>>>(plain_pairs(lhs_idx, rhs_idx), (int)n_idx, (uint32_t)x_batch, (uint32_t)E, 0u, (uint32_t)E,
+                                           (int)M, kRowsTile, hdr, sorted, slhs, mt, y, (size_t)M * N2 * 2, status);
+    B200Q_LAUNCH_OK("gather_sort_kernel");
+    r1.x = x; r1.src_slot = slhs; r1.y = h;
+    if (int rc = qmv_rows_grouped(r1, st)) return rc;
+    r2.x = h; r2.y = y; r2.dst_slot = sorted;
+    return qmv_rows_grouped(r2, st);
+  }
   gather_sort_kernel<<<1, 1024, 0, st>>>(plain_pairs(lhs_idx, rhs_idx), (int)n_idx, (uint32_t)x_batch, (uint32_t)E, 0u, (uint32_t)E, (int)M,
                                          L.nt, hdr, sorted, slhs, mt, y, (size_t)M * N2 * 2, status);
   B200Q_LAUNCH_OK("gather_sort_kernel");
@@ -487,6 +529,19 @@ int swiglu_impl(const void* x, const uint32_t* wq_gate, const void* scales_gate,
   const size_t h_bytes = align256((size_t)L.n_rows * H * 2);
   __nv_bfloat16* hg = reinterpret_cast<__nv_bfloat16*>(base + L.total - 256);
   __nv_bfloat16* hu = reinterpret_cast<__nv_bfloat16*>(base + L.total - 256 + h_bytes);
+  RowsGroup r1 = rows_group(L, base, E, M, H, K1, group_size, bits, status), r2 = rows_group(L, base, E, M, N2, H, group_size, bits, status);
+  set_matrix(r1, 0, wq_gate, scales_gate, biases_gate);
+  set_matrix(r1, 1, wq_up, scales_up, biases_up);
+  set_matrix(r2, 0, wq_down, scales_down, biases_down);
+  if (few_rows(L.n_rows, E) && qmv_rows_grouped_supported(r1) && qmv_rows_grouped_supported(r2)) {
+    gather_sort_kernel<<<1, 1024, 0, st>>>(pairs, (int)n_idx, (uint32_t)x_batch, (uint32_t)E, 0u, (uint32_t)E, (int)M, kRowsTile, hdr,
+                                           sorted, slhs, mt, y, (size_t)M * N2 * 2, status);
+    B200Q_LAUNCH_OK("gather_sort_kernel");
+    r1.x = x; r1.src_slot = slhs; r1.y = hg;
+    if (int rc = qmv_rows_grouped(r1, st)) return rc;
+    r2.x = hg; r2.y = y; r2.dst_slot = sorted;
+    return qmv_rows_grouped(r2, st);
+  }
   gather_sort_kernel<<<1, 1024, 0, st>>>(pairs, (int)n_idx, (uint32_t)x_batch, (uint32_t)E, 0u, (uint32_t)E, (int)M,
                                          L.nt, hdr, sorted, slhs, mt, y, (size_t)M * N2 * 2, status);
   B200Q_LAUNCH_OK("gather_sort_kernel");

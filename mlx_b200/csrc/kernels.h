@@ -105,6 +105,26 @@ struct GroupedArgs {
   PeerOut peers;            // n > 0: every result row is stored into all of these [n_rows, N] buffers
 };
 
+// The row-owning decode kernel over the experts that have rows, for tiles of up to 8 expert-sorted rows.  With a
+// second matrix the result is silu(x W0^T) * (x W1^T).
+constexpr int kRowsTile = 8;
+struct RowsGroup {
+  const void* x;            // bf16 rows of K
+  const uint32_t* wq[2];    // [E, N, K*bits/32]; the second may be null
+  const void* scales[2];
+  const void* biases[2];
+  void* y;                  // rows of N
+  const void* tiles;        // device: (expert, first row, rows, -)[max_tiles]
+  const int* n_tiles;       // device scalar
+  const int* src_slot;      // device: pair -> the x it multiplies, or null: x is in sorted order
+  const int* dst_slot;      // device: pair -> the y it writes, or null: y is in sorted order
+  int64_t max_tiles, per_slot, E, N, K;
+  int group, bits;
+  uint32_t* status;
+};
+bool qmv_rows_grouped_supported(const RowsGroup& a);
+int qmv_rows_grouped(const RowsGroup& a, cudaStream_t st);
+
 // Per-problem operand selection of the gather form: problem i of `batch` multiplies
 // x[lhs[i]] with w[rhs[i]].  Indices are range-checked on the device against
 // x_batch / n_mats; a bad index zeroes its output and sets status[0].

@@ -185,7 +185,43 @@ struct RowsParams {
   int inflight;         // stages requested but not yet landed, at most
   uint32_t* status;     // may be null
   int early;            // weights, scales and biases may be read before the previous kernel ended
+  // grouped (gather_qmm) launches only: device-side table of tiles of up to 8 expert-sorted rows
+  const int4* tiles;       // expert, first row, rows
+  const int* n_tiles;
+  const int* src_slot;     // per sorted pair: which x it multiplies (null: x is in sorted order)
+  const int* dst_slot;     // per sorted pair: which y it writes (null: y is in sorted order)
+  int per_slot;            // rows per pair
+  int rgs;                 // 16-row groups per matrix
 };
+
+// What a launch works on.  Plain: one matrix.  Grouped: the matrices of the experts that have rows.  Gated: the same
+// with two matrices per expert, y = silu(gate) * up; their stages alternate, so both results of a row group meet in
+// the reducer warp and neither product goes through memory.
+enum class Work { Plain, Grouped, Gated };
+template <Work W>
+struct RowsMaps {
+  static constexpr int kN = W == Work::Gated ? 2 : 1;
+  CUtensorMap w[kN], s[kN], b[kN];
+};
+// A run of consecutive 16-row groups of one tile.  Units of grouped work are (tile, row group) pairs in that order; a
+// block takes a contiguous range of them, which spans two tiles at most while there are fewer tiles than blocks.
+struct Segment {
+  int row0;        // first row of the run inside the matrix
+  int base;        // rows of the tensor map before the matrix
+  int n;           // row groups
+  int x0, rows;    // first sorted row and number of rows of the tile
+};
+__device__ __forceinline__ Segment segment_at(const RowsParams& p, int u, int u_end) {
+  const int tile = u / p.rgs, rg = u - tile * p.rgs;
+  const int4 t = p.tiles[tile];
+  return Segment{rg * 16, t.x * p.N, min(p.rgs - rg, u_end - u), t.y, t.z};
+}
+// Row of x or y that sorted row r stands for.
+__device__ __forceinline__ long long slot_row(const int* table, int r, int per) {
+  if (table == nullptr) return r;
+  const int q = r / per;
+  return (long long)table[q] * per + (r - q * per);
+}
 
 // One packed word -> NP registers of two bf16 subnormals each; register i holds fields (i, i + NP)
 // of the word, scaled by 2^-133 and by the power of two in xscale<BITS>(i).
@@ -218,10 +254,12 @@ __device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
   return v;
 }
 
-template <typename T, int BITS, int G, int MT>
+template <typename T, int BITS, int G, int MT, Work W>
 __global__ void __launch_bounds__(kThreads, 1)
-qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s,
-                const __grid_constant__ CUtensorMap map_b, const RowsParams p) {
+qmv_rows_kernel(const __grid_constant__ RowsMaps<W> maps, const RowsParams p) {
+  constexpr bool kGrouped = W != Work::Plain;
+  constexpr int NW = RowsMaps<W>::kN;
+  static_assert(!kGrouped || MT == 1, "grouped tiles have up to 8 rows");
   using C = Cfg<BITS, G, MT>;
   constexpr int NGW = C::NGW, NP = C::NP, UG = C::UG, UW = C::UW, KW = C::KW;
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -253,18 +291,42 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 #endif
   asm volatile("griddepcontrol.launch_dependents;");
   if (tid == kConsumers * 32) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_s) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.w[i]) : "memory");
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.s[i]) : "memory");
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.b[i]) : "memory");
+    }
   }
 
   const int G_ = gridDim.x;
-  const int b0 = (int)((long long)blockIdx.x * p.nblk8 / G_);
-  const int b1 = (int)((long long)(blockIdx.x + 1) * p.nblk8 / G_);
-  const int nrg = (b1 - b0 + 1) >> 1;           // 16-row groups of this CTA
-  const int total = nrg * p.nph;                // stages
-  const int row_end = min(b1 * 8, p.N);
   const int nst = p.nst;
+  // The range of this CTA: plain, 8-row blocks [b0, b1) as one segment; grouped, units [b0, b1), which are known only
+  // once the table has been written.
+  int b0 = 0, b1 = 0;
+  Segment seg{};
+  auto find_range = [&]() {
+    const long long n = kGrouped ? (long long)*p.n_tiles * p.rgs : (long long)p.nblk8;
+    b0 = (int)(blockIdx.x * n / G_);
+    b1 = (int)((blockIdx.x + 1) * n / G_);
+  };
+  if constexpr (!kGrouped) {
+    find_range();
+    seg = Segment{b0 * 8, 0, (b1 - b0 + 1) >> 1, 0, p.M};
+  }
+  const int row_end = kGrouped ? p.N : min(b1 * 8, p.N);
+  // Walks the segments: `at` is the next unit; false when there is none.
+  auto next_segment = [&](int& at) -> bool {
+    if constexpr (kGrouped) {
+      if (at >= b1) return false;
+      seg = segment_at(p, at, b1);
+      at += seg.n;
+    } else {
+      if (at > b0) return false;
+      ++at;
+    }
+    return true;
+  };
 
   // Barriers are set up by the loader thread, which then starts requesting weights at once; the
   // other warps meet it at a named barrier (id 1) only when they first need the barriers - the
@@ -286,61 +348,51 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       RP_MARK(1);
       // ================================= loader warp ==========================================
       // Without the caller's promise the weights may have been written by the previous kernel.
-      if (!p.early) asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (kGrouped || !p.early) asm volatile("griddepcontrol.wait;" ::: "memory");
       RP_MARK(2);
       if (lane == 0) {
         // This one thread shares its scheduler with four busy consumer warps: everything it needs
         // per stage is kept incremental (no divisions, no parameter reloads).
+        if constexpr (kGrouped) find_range();
         const uint32_t stage_bytes = p.slot_bytes, sb_off = (uint32_t)p.nch * 2048, bb_off = (uint32_t)(p.nch + p.nsb) * 2048;
-#ifdef B200Q_ROWS_PROFILE
-        const int dbg = p.inflight >> 8;
-        const int nsb = (dbg & 1) ? 0 : p.nsb, inflight = p.inflight & 255;
-        const uint32_t stage_bytes_dbg = (dbg & 1) ? (uint32_t)p.nch * 2048 : stage_bytes;
-#define STAGE_TX stage_bytes_dbg
-#else
         const int nsb = p.nsb, inflight = p.inflight;
-#define STAGE_TX stage_bytes
-#endif
         int slot = 0, use = 0;        // ring position of stage s
         int lslot = 0, luse = 0;      // ring position of the oldest stage not yet known to have landed
-        int landed = 0, iph = 0, irg = 0;
-        int grp0 = p.ph_g0[0];
+        int landed = 0, s = 0;
         uint32_t dst = smem_base + p.off_slots;
-        for (int s = 0; s < total; ++s) {
-          // slot free: all consumer warps arrived for the stage that used it last
-          if (use > 0 && !mbar_wait(done0 + 8 * slot, (use - 1) & 1, abort_flag)) break;
-          // at most `inflight` stages outstanding
-          while (landed < s && mbar_test(full0 + 8 * lslot, luse & 1)) {
-            ++landed;
-            if (++lslot == nst) { lslot = 0; ++luse; }
+        bool ok = true;
+        for (int at = b0; ok && next_segment(at);) {
+          for (int ph = 0; ok && ph < p.nph; ++ph) {
+            const int grp0 = p.ph_g0[ph];
+            for (int i = 0; i < seg.n * NW; ++i, ++s) {
+              // slot free: all consumer warps arrived for the stage that used it last
+              if (use > 0 && !mbar_wait(done0 + 8 * slot, (use - 1) & 1, abort_flag)) { ok = false; break; }
+              // at most `inflight` stages outstanding
+              while (landed < s && mbar_test(full0 + 8 * lslot, luse & 1)) {
+                ++landed;
+                if (++lslot == nst) { lslot = 0; ++luse; }
+              }
+              while (s - landed >= inflight) {
+                if (!mbar_wait(full0 + 8 * lslot, luse & 1, abort_flag)) break;
+                ++landed;
+                if (++lslot == nst) { lslot = 0; ++luse; }
+              }
+              if (*abort_flag) { ok = false; break; }
+              const int which = NW == 2 ? (i & 1) : 0;
+              const int row = seg.base + seg.row0 + (NW == 2 ? i >> 1 : i) * 16;
+              const uint32_t bar = full0 + 8 * slot;
+              // rows past the last matrix and chunks past K are zero-filled by the copy engine and still counted
+              // (rows past the end of one of several matrices are the next one's: never stored)
+              mbar_expect_tx(bar, stage_bytes);
+              tma_load_3d(dst, &maps.w[which], 0, row, grp0 * (C::GB / 16) / 8, bar);
+              for (int k = 0; k < nsb; ++k) {
+                tc::tma_load_2d(dst + sb_off + k * 2048, &maps.s[which], grp0 * 2 + 128 * k, row, bar);
+                tc::tma_load_2d(dst + bb_off + k * 2048, &maps.b[which], grp0 * 2 + 128 * k, row, bar);
+              }
+              dst += stage_bytes;
+              if (++slot == nst) { slot = 0; ++use; dst = smem_base + p.off_slots; }
+            }
           }
-          while (s - landed >= inflight) {
-            if (!mbar_wait(full0 + 8 * lslot, luse & 1, abort_flag)) break;
-            ++landed;
-            if (++lslot == nst) { lslot = 0; ++luse; }
-          }
-          if (*abort_flag) break;
-          const int row0 = (b0 + 2 * irg) * 8;
-          const uint32_t bar = full0 + 8 * slot;
-#ifdef B200Q_ROWS_PROFILE
-          if (5 + 3 * s < 30 && blockIdx.x < 160) g_rows_prof[blockIdx.x][warp][5 + 3 * s] = (uint32_t)(clock64() - rp_entry);
-#endif
-          // rows past N and chunks past K are zero-filled by the copy engine and still counted
-          mbar_expect_tx(bar, STAGE_TX);
-          tma_load_3d(dst, &map_w, 0, row0, grp0 * (C::GB / 16) / 8, bar);
-#ifdef B200Q_ROWS_PROFILE
-          if (6 + 3 * s < 30 && blockIdx.x < 160) g_rows_prof[blockIdx.x][warp][6 + 3 * s] = (uint32_t)(clock64() - rp_entry);
-#endif
-          for (int i = 0; i < nsb; ++i) {
-            tc::tma_load_2d(dst + sb_off + i * 2048, &map_s, grp0 * 2 + 128 * i, row0, bar);
-            tc::tma_load_2d(dst + bb_off + i * 2048, &map_b, grp0 * 2 + 128 * i, row0, bar);
-          }
-#ifdef B200Q_ROWS_PROFILE
-          if (7 + 3 * s < 30 && blockIdx.x < 160) g_rows_prof[blockIdx.x][warp][7 + 3 * s] = (uint32_t)(clock64() - rp_entry);
-#endif
-          dst += stage_bytes;
-          if (++slot == nst) { slot = 0; ++use; dst = smem_base + p.off_slots; }
-          if (++irg == nrg) { irg = 0; ++iph; grp0 = p.ph_g0[iph < p.nph ? iph : 0]; }
         }
       }
       RP_MARK(30);
@@ -352,12 +404,19 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       asm volatile("griddepcontrol.wait;" ::: "memory");   // y may still be in use by the previous kernel
       if (lane == 0) peer_wait_previous(p.sig, p.status);  // ... or by a peer's consumer of the step before
       __syncwarp();
-      int rph = 0, rrg = 0, rslot = 0, ruse = 0;
-      for (int red = 0; red < total; ++red) {
-        if (!mbar_wait(done0 + 8 * rslot, ruse & 1, abort_flag)) break;
+      if constexpr (kGrouped) find_range();
+      int rslot = 0, ruse = 0, red = 0;
+      bool ok = true;
+      for (int at = b0; ok && next_segment(at);) {
+       const int ytok = min(lane >> 1, seg.rows - 1);
+       const long long y_off = (kGrouped ? slot_row(p.dst_slot, seg.x0 + ytok, p.per_slot) : (long long)(lane >> 1)) * p.ld + p.col0;
+       for (int rph = 0; ok && rph < p.nph; ++rph)
+       for (int rrg = 0; rrg < seg.n * NW; ++rrg) {
+        if (!mbar_wait(done0 + 8 * rslot, ruse & 1, abort_flag)) { ok = false; break; }
         if (++rslot == nst) { rslot = 0; ++ruse; }
         RP_MARK(5 + 2 * red);
         const int pbi = red % kPartialBufs;
+        ++red;
         const float4* pb = reinterpret_cast<const float4*>(smem + p.off_pbuf + (size_t)pbi * (kConsumers * MT * 512)) + lane;
         float sum[MT][4];
 #pragma unroll
@@ -392,8 +451,22 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         if (final_phase) {
           // transpose the 16 rows x 8*MT tokens through shared memory so that every lane stores 16
           // contiguous bytes of one token's row of y
-          const int row0 = (b0 + 2 * rrg) * 8;
+          const int row0 = seg.row0 + (NW == 2 ? rrg >> 1 : rrg) * 16;
           T* yt = reinterpret_cast<T*>(smem + 512);   // [16 tokens][16 rows]
+          if constexpr (W == Work::Gated) {
+            // the gate's product waits, rounded, in the half of the tile that 8 tokens leave free
+            if ((rrg & 1) == 0) {
+#pragma unroll
+              for (int c = 0; c < 4; ++c) yt[128 + (2 * t + (c & 1)) * 16 + g + (c >> 1) * 8] = Elem<T>::from_float(sum[0][c]);
+              continue;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const float gate = Elem<T>::to_float(yt[128 + (2 * t + (c & 1)) * 16 + g + (c >> 1) * 8]);
+              const float up = Elem<T>::to_float(Elem<T>::from_float(sum[0][c]));
+              sum[0][c] = __fdividef(gate, 1.f + __expf(-gate)) * up;
+            }
+          }
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -401,12 +474,12 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
               yt[(mt * 8 + 2 * t + (c & 1)) * 16 + g + (c >> 1) * 8] = Elem<T>::from_float(sum[mt][c]);
           __syncwarp();
           const int tok = lane >> 1, r8 = row0 + (lane & 1) * 8;
-          if (tok < p.M && r8 < row_end) {
+          if (tok < seg.rows && r8 < row_end) {
             const uint4 v = *reinterpret_cast<const uint4*>(yt + tok * 16 + (lane & 1) * 8);
-            const long long at = (long long)tok * p.ld + p.col0 + r8;
-            const bool vec = r8 + 8 <= row_end && ((at | p.ld) & 7) == 0;
+            const long long off = y_off + r8;
+            const bool vec = r8 + 8 <= row_end && ((off | p.ld) & 7) == 0;
             for (int q = 0; q < p.n_out; ++q) {
-              uint16_t* dst = p.y[q] + at;
+              uint16_t* dst = p.y[q] + off;
               if (vec && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
                 *reinterpret_cast<uint4*>(dst) = v;
               } else {
@@ -417,8 +490,8 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
           }
           __syncwarp();
         }
-        if (++rrg == nrg) { rrg = 0; ++rph; }
-        RP_MARK(6 + 2 * red);
+        RP_MARK(4 + 2 * red);
+       }
       }
       RP_MARK(30);
       __syncwarp();   // all of this block's stores to y were issued by this warp
@@ -454,11 +527,11 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   uint32_t woff[UW / 2];          // this lane's ldmatrix addresses inside a stage
   uint32_t soff = 0;              // scale of (row g, first group of the slice) inside a stage
   int cnt = 0;
-  int ph = 0, rg = 0, slot = 0, use = 0, pbi = 0, pbe = 0;
+  int slot = 0, use = 0, pbi = 0, pbe = 0;
   // ldmatrix roles of this lane: matrix m = lane / 8 covers rows (m & 1) * 8 .. +7 of unit (m >> 1)
   const int lm_row = (lane & 7) + ((lane >> 3) & 1) * 8, lm_unit = lane >> 4, lm_x = lane & 7;
 
-  auto setup_phase = [&]() {
+  auto setup_phase = [&](int ph, const uint16_t* x_lane) {
     cnt = p.ph_cnt[ph];
     const int g0 = warp * cnt;       // first group of this warp inside the phase
     const int u0 = g0 * UG;
@@ -485,8 +558,8 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         const int tok = mt * 8 + g;
-        const bool live = i < cnt * UG && tok < p.M;
-        const uint16_t* xp = p.x + (long long)tok * p.K + k0 + i * (4 * KW);
+        const bool live = i < cnt * UG && tok < seg.rows;
+        const uint16_t* xp = x_lane + (long long)(mt * 8) * p.K + k0 + i * (4 * KW);
         // pair q = (x_q, x_{q + NP}), the order the unpack delivers the fields in
         if constexpr (BITS == 8) {
           uint2 v = make_uint2(0, 0);
@@ -558,30 +631,36 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       sx_lo[mt] = pack_x2<T>(e0 - lo_f<T>(hi), e1 - hi_f<T>(hi));
     }
   };
-  setup_phase();
-  asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");   // the barriers exist from here on
-  {
+  const uint32_t pb_mine = smem_base + p.off_pbuf + (uint32_t)(warp * MT * 32 + lane) * 16;
+  uint32_t sb = smem_base + p.off_slots;   // stage the warp works on
+  if constexpr (kGrouped) find_range();
+  bool first = true;   // before the first stage: the barriers exist from here on
+  auto meet = [&]() {
+    first = false;
+    asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
     // The first mma.sync of a kernel is slow (the tensor pipe wakes up): issue one now, while the
     // first stage is in flight anyway.  Its result is never used.
     float d0, d1, d2, d3;
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%4,%4,%4}, {%4,%4}, {%5,%5,%5,%5};"
                  : "=f"(d0), "=f"(d1), "=f"(d2), "=f"(d3) : "r"(0u), "f"(0.0f));
-  }
-  RP_MARK(4);
-
-  const uint32_t pb_mine = smem_base + p.off_pbuf + (uint32_t)(warp * MT * 32 + lane) * 16;
-  uint32_t sb = smem_base + p.off_slots;   // stage the warp works on
-  for (int s = 0; s < total; ++s) {
-    if (!mbar_wait(full0 + 8 * slot, use & 1, abort_flag)) break;
+    RP_MARK(4);
+  };
+  int s = 0;
+  for (int at = b0; next_segment(at);) {
+  // this lane's token row of x (of the first token tile)
+  const uint16_t* x_lane =
+      p.x + (kGrouped ? slot_row(p.src_slot, seg.x0 + min(g, seg.rows - 1), p.per_slot) : (long long)g) * p.K;
+  for (int ph = 0; ph < p.nph; ++ph) {
+  setup_phase(ph, x_lane);
+  if (first) meet();
+  for (int rg = 0; rg < seg.n * NW; ++rg, ++s) {
+    if (!mbar_wait(full0 + 8 * slot, use & 1, abort_flag)) return;
     RP_MARK(5 + 3 * s);
     float out[MT][4];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int c = 0; c < 4; ++c) out[mt][c] = 0.0f;
-#ifdef B200Q_ROWS_PROFILE
-    if (!((p.inflight >> 8) & 2))
-#endif
     {
     // mma.sync results come back after many cycles: keep four independent accumulation chains going
     // per warp (two groups at a time, each group's k steps dealt round-robin to SPLIT accumulators,
@@ -664,7 +743,7 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     }
     RP_MARK(6 + 3 * s);
     // the partial buffer of this stage was read by the reducer kPartialBufs stages ago
-    if (pbe > 0 && !mbar_wait(pfree0 + 8 * pbi, (pbe - 1) & 1, abort_flag)) break;
+    if (pbe > 0 && !mbar_wait(pfree0 + 8 * pbi, (pbe - 1) & 1, abort_flag)) return;
     {
       constexpr float kOut = is_bf16<T> ? 0x1p69f : 1.0f;
       const uint32_t pa = pb_mine + (uint32_t)pbi * (kConsumers * MT * 512);
@@ -681,12 +760,10 @@ qmv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     sb += p.slot_bytes;
     if (++slot == nst) { slot = 0; ++use; sb = smem_base + p.off_slots; }
     if (++pbi == kPartialBufs) { pbi = 0; ++pbe; }
-    if (++rg == nrg) {
-      rg = 0;
-      ++ph;
-      if (ph < p.nph) setup_phase();
-    }
   }
+  }
+  }
+  if (first) meet();   // (no work for this block)
   RP_MARK(30);
 }
 
@@ -727,11 +804,12 @@ int sm_count_rows() {
   return cached[dev];
 }
 
+// `grid` blocks with at most `max_rg` row groups of a matrix each; `stages` in all per block at most.
 template <int BITS, int G, int MT>
-bool fill_plan(const QmmArgs& a, RowsPlan& pl) {
+bool fill_plan(int64_t K, int grid, int max_rg, long long stages_per_phase, RowsPlan& pl) {
   using C = Cfg<BITS, G, MT>;
   RowsParams& p = pl.prm;
-  const int groups = (int)(a.K / G);
+  const int groups = (int)(K / G);
   if (groups % kConsumers != 0) return false;   // every phase gives all 16 warps the same number of groups
   // phases of 16 * c groups, c a power of two: first as many full ones as fit, then the remainder
   p.nph = 0;
@@ -749,11 +827,7 @@ bool fill_plan(const QmmArgs& a, RowsPlan& pl) {
   p.nsb = (kConsumers * C::NGW * 2 + 127) / 128;
   if (p.nch > 256) return false;
   p.slot_bytes = (uint32_t)(p.nch + 2 * p.nsb) * 2048;
-  p.nblk8 = (int)((a.N + 7) / 8);
-  const int sms = sm_count_rows();
-  pl.grid = p.nblk8 < sms ? p.nblk8 : sms;
-  const int max_blk = (p.nblk8 + pl.grid - 1) / pl.grid;
-  const int max_rg = (max_blk + 1) / 2 + 1;
+  pl.grid = grid;
   size_t off = 1024;   // barriers, abort flag, the reducer's 512-byte output tile
   p.off_tile = (uint32_t)off;
   if (p.nph > 1) off += (size_t)max_rg * MT * 512;
@@ -762,7 +836,7 @@ bool fill_plan(const QmmArgs& a, RowsPlan& pl) {
   off = (off + 1023) / 1024 * 1024;   // swizzled tiles repeat every 1024 bytes
   p.off_slots = (uint32_t)off;
   if (off + 2 * (size_t)p.slot_bytes > kSmemLimit) return false;
-  const long long stages = (long long)max_rg * p.nph;
+  const long long stages = stages_per_phase * p.nph;
   long long nst = (long long)((kSmemLimit - off) / p.slot_bytes);
   if (nst > 16) nst = 16;
   if (nst > stages) nst = stages;
@@ -783,10 +857,13 @@ RowsPlan make_plan(const QmmArgs& a) {
   if (a.K % (16 * a.group) != 0) return pl;       // 16 warps, whole groups each (implies 128-byte row chunks)
   if (a.N > (1ll << 30)) return pl;
   const int mt = a.M > 8 ? 2 : 1;
+  pl.prm.nblk8 = (int)((a.N + 7) / 8);
+  const int grid = cmin(pl.prm.nblk8, sm_count_rows());
+  const int max_rg = ((pl.prm.nblk8 + grid - 1) / grid + 1) / 2 + 1;
   bool ok = false;
-#define B200Q_ROWS_CASE(BITS_, G_)                                                          \
-  if (a.bits == BITS_ && a.group == G_)                                                     \
-    ok = mt == 2 ? fill_plan<BITS_, G_, 2>(a, pl) : fill_plan<BITS_, G_, 1>(a, pl);
+#define B200Q_ROWS_CASE(BITS_, G_)                                                                \
+  if (a.bits == BITS_ && a.group == G_)                                                           \
+    ok = mt == 2 ? fill_plan<BITS_, G_, 2>(a.K, grid, max_rg, max_rg, pl) : fill_plan<BITS_, G_, 1>(a.K, grid, max_rg, max_rg, pl);
   B200Q_ROWS_CASE(2, 64) B200Q_ROWS_CASE(2, 128)
   B200Q_ROWS_CASE(4, 32) B200Q_ROWS_CASE(4, 64) B200Q_ROWS_CASE(4, 128)
   B200Q_ROWS_CASE(8, 32) B200Q_ROWS_CASE(8, 64) B200Q_ROWS_CASE(8, 128)
@@ -835,36 +912,41 @@ int rows_inflight(int mt, int bits, int nph) {
   return bits >= 8 ? 2 : 1;
 }
 
-template <typename T, int BITS, int G, int MT>
-int launch_rows(const QmmArgs& a, const RowsPlan& pl, cudaStream_t st) {
+// Tensor maps of one stack of matrices [rows, K].
+template <int BITS, int G>
+int encode_rows(int nch, int64_t rows, int64_t K, const void* wq, const void* scales, const void* biases, CUtensorMap* map_w,
+                CUtensorMap* map_s, CUtensorMap* map_b) {
   EncodeFn enc = rows_encode_fn();
   if (!enc) return fail(B200Q_ERR_CUDA, "[quantized_matmul] cuTensorMapEncodeTiled is not available");
-  const RowsParams& p = pl.prm;
-  CUtensorMap map_w, map_s, map_b;
   {
     // packed rows as (128 bytes, row, 128-byte chunk of the row)
-    const cuuint64_t row_bytes = (cuuint64_t)a.K * BITS / 8;
-    const cuuint64_t dims[3] = {128, (cuuint64_t)a.N, row_bytes / 128};
+    const cuuint64_t row_bytes = (cuuint64_t)K * BITS / 8;
+    const cuuint64_t dims[3] = {128, (cuuint64_t)rows, row_bytes / 128};
     const cuuint64_t strides[2] = {row_bytes, 128};
-    const cuuint32_t box[3] = {128, 16, (cuuint32_t)p.nch};
+    const cuuint32_t box[3] = {128, 16, (cuuint32_t)nch};
     const cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = enc(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint32_t*>(a.wq), dims, strides, box, estr,
+    CUresult r = enc(map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(wq), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[quantized_matmul] tensor map for the packed weights failed (%d)", (int)r);
   }
   for (int which = 0; which < 2; ++which) {
-    const cuuint64_t srow = (cuuint64_t)(a.K / G) * 2;
-    const cuuint64_t dims[2] = {srow, (cuuint64_t)a.N};
+    const cuuint64_t srow = (cuuint64_t)(K / G) * 2;
+    const cuuint64_t dims[2] = {srow, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {srow};
     const cuuint32_t box[2] = {128, 16};
     const cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(which ? &map_b : &map_s, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(which ? a.biases : a.scales),
+    CUresult r = enc(which ? map_b : map_s, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(which ? biases : scales),
                      dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[quantized_matmul] tensor map for scales / biases failed (%d)", (int)r);
   }
-  auto kern = qmv_rows_kernel<T, BITS, G, MT>;
+  return B200Q_OK;
+}
+
+template <typename T, int BITS, int G, int MT, Work W>
+int launch_kernel(const RowsMaps<W>& maps, const RowsPlan& pl, cudaStream_t st) {
+  auto kern = qmv_rows_kernel<T, BITS, G, MT, W>;
   if (pl.smem > 48 * 1024)
     B200Q_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
   cudaLaunchConfig_t cfg = {};
@@ -877,9 +959,61 @@ int launch_rows(const QmmArgs& a, const RowsPlan& pl, cudaStream_t st) {
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = pdl_enabled_rows() ? 1 : 0;
-  B200Q_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, map_w, map_s, map_b, pl.prm));
+  B200Q_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, maps, pl.prm));
   B200Q_LAUNCH_OK("qmv_rows_kernel");
   return B200Q_OK;
+}
+
+template <typename T, int BITS, int G, int MT>
+int launch_rows(const QmmArgs& a, const RowsPlan& pl, cudaStream_t st) {
+  RowsMaps<Work::Plain> maps;
+  if (int rc = encode_rows<BITS, G>(pl.prm.nch, a.N, a.K, a.wq, a.scales, a.biases, maps.w, maps.s, maps.b)) return rc;
+  return launch_kernel<T, BITS, G, MT, Work::Plain>(maps, pl, st);
+}
+
+template <int BITS, int G, Work W>
+int launch_grouped(const RowsGroup& a, const RowsPlan& pl, cudaStream_t st) {
+  RowsMaps<W> maps;
+  for (int i = 0; i < RowsMaps<W>::kN; ++i)
+    if (int rc = encode_rows<BITS, G>(pl.prm.nch, a.E * a.N, a.K, a.wq[i], a.scales[i], a.biases[i], maps.w + i, maps.s + i, maps.b + i))
+      return rc;
+  return launch_kernel<__nv_bfloat16, BITS, G, 1, W>(maps, pl, st);
+}
+
+RowsPlan make_group_plan(const RowsGroup& a) {
+  RowsPlan pl{};
+  pl.ok = false;
+  if (a.bits == 2 && a.group == 32) return pl;
+  if ((a.bits != 2 && a.bits != 4 && a.bits != 8) || a.N < 1 || a.K < 1 || a.K % (16 * a.group) != 0) return pl;
+  const int nw = a.wq[1] ? 2 : 1;
+  for (int i = 0; i < nw; ++i)
+    if ((reinterpret_cast<uintptr_t>(a.wq[i]) | reinterpret_cast<uintptr_t>(a.scales[i]) | reinterpret_cast<uintptr_t>(a.biases[i])) & 15)
+      return pl;
+  const int64_t rgs = (a.N + 15) / 16, units = a.max_tiles * rgs;
+  if (units > (1ll << 30)) return pl;
+  const int grid = (int)(units < sm_count_rows() ? units : sm_count_rows());
+  const int64_t most = (units + grid - 1) / grid;
+  const int max_rg = (int)(most < rgs ? most : rgs) * nw;
+  bool ok = false;
+#define B200Q_ROWS_CASE(BITS_, G_) \
+  if (a.bits == BITS_ && a.group == G_) ok = fill_plan<BITS_, G_, 1>(a.K, grid, max_rg, most * nw, pl);
+  B200Q_ROWS_CASE(2, 64) B200Q_ROWS_CASE(2, 128)
+  B200Q_ROWS_CASE(4, 32) B200Q_ROWS_CASE(4, 64) B200Q_ROWS_CASE(4, 128)
+  B200Q_ROWS_CASE(8, 32) B200Q_ROWS_CASE(8, 64) B200Q_ROWS_CASE(8, 128)
+#undef B200Q_ROWS_CASE
+  if (!ok) return pl;
+  RowsParams& p = pl.prm;
+  p.x = (const uint16_t*)a.x;
+  p.n_out = 1; p.ld = a.N; p.col0 = 0; p.y[0] = (uint16_t*)a.y;
+  p.N = (int)a.N; p.K = (int)a.K;
+  p.tiles = static_cast<const int4*>(a.tiles);
+  p.n_tiles = a.n_tiles;
+  p.src_slot = a.src_slot; p.dst_slot = a.dst_slot;
+  p.per_slot = (int)a.per_slot;
+  p.rgs = (int)rgs;
+  p.status = a.status;
+  pl.ok = true;
+  return pl;
 }
 
 }  // namespace
@@ -939,6 +1073,23 @@ int qmv_rows(const QmmArgs& a, cudaStream_t st) {
     rc = a.dtype == B200Q_BF16                                                                      \
              ? (pl.mt == 2 ? launch_rows<__nv_bfloat16, BITS_, G_, 2>(a, pl, st) : launch_rows<__nv_bfloat16, BITS_, G_, 1>(a, pl, st)) \
              : (pl.mt == 2 ? launch_rows<__half, BITS_, G_, 2>(a, pl, st) : launch_rows<__half, BITS_, G_, 1>(a, pl, st));
+  B200Q_ROWS_CASE(2, 64) B200Q_ROWS_CASE(2, 128)
+  B200Q_ROWS_CASE(4, 32) B200Q_ROWS_CASE(4, 64) B200Q_ROWS_CASE(4, 128)
+  B200Q_ROWS_CASE(8, 32) B200Q_ROWS_CASE(8, 64) B200Q_ROWS_CASE(8, 128)
+#undef B200Q_ROWS_CASE
+  return rc;
+}
+
+bool qmv_rows_grouped_supported(const RowsGroup& a) { return make_group_plan(a).ok; }
+
+int qmv_rows_grouped(const RowsGroup& a, cudaStream_t st) {
+  RowsPlan pl = make_group_plan(a);
+  if (!pl.ok) return fail(B200Q_ERR_UNSUPPORTED, "[gather_qmm] qmv_rows: unsupported problem");
+  pl.prm.inflight = rows_inflight(1, a.bits, pl.prm.nph);
+  int rc = B200Q_ERR_UNSUPPORTED;
+#define B200Q_ROWS_CASE(BITS_, G_)                                                                            \
+  if (a.bits == BITS_ && a.group == G_)                                                                       \
+    rc = a.wq[1] ? launch_grouped<BITS_, G_, Work::Gated>(a, pl, st) : launch_grouped<BITS_, G_, Work::Grouped>(a, pl, st);
   B200Q_ROWS_CASE(2, 64) B200Q_ROWS_CASE(2, 128)
   B200Q_ROWS_CASE(4, 32) B200Q_ROWS_CASE(4, 64) B200Q_ROWS_CASE(4, 128)
   B200Q_ROWS_CASE(8, 32) B200Q_ROWS_CASE(8, 64) B200Q_ROWS_CASE(8, 128)

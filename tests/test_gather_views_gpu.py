@@ -77,3 +77,45 @@ def test_gated_experts_native_equals_three_calls():
         y = mb.gather_qmm_swiglu(xt, gate, up, down, idx)
         assert tuple(y.shape) == (tokens, top, 1, K)
         assert torch.allclose(y.float(), ref.float(), rtol=2e-2, atol=2e-2 * float(ref.float().abs().max()))
+
+
+# Few rows per expert: tiles of up to 8 rows of the row-owning kernel.  Columns off the 16-row groups, one and two phases
+# over K, every field width it has, an expert with more rows than a tile, one row in all, two rows per pair.
+@pytest.mark.parametrize("E,tokens,top,rows,N,K,bits,group", [
+    (8, 4, 2, 1, 200, 1024, 4, 64), (64, 1, 1, 1, 16, 1024, 4, 64), (16, 16, 4, 1, 1000, 512, 4, 32), (4, 5, 1, 2, 72, 12288, 4, 64),
+    (8, 10, 2, 1, 136, 6144, 8, 128), (5, 7, 2, 1, 344, 3072, 2, 64), (32, 9, 1, 3, 64, 2048, 2, 128), (300, 500, 2, 1, 24, 512, 8, 32)])
+def test_few_rows_per_expert(E, tokens, top, rows, N, K, bits, group):
+    wq, s, b = O.quantize(make_w(70, (E, N, K), "bf16"), group, bits, "bf16")
+    x = make_x(71, (tokens, rows, K), "bf16")
+    rng = np.random.default_rng(72)
+    rhs = rng.integers(0, E, (tokens, top))
+    rhs[: min(tokens, 10)] = E - 1   # more than a tile of one expert, where there are enough
+    lhs = np.broadcast_to(np.arange(tokens)[:, None], rhs.shape)
+    ref = O.gather_qmm(O.to_f32(x, "bf16"), wq, O.to_f32(s, "bf16"), O.to_f32(b, "bf16"), lhs.ravel().astype(np.uint32),
+                       rhs.ravel().astype(np.uint32), True, group, bits, "f32")
+    args = to_torch(x, "bf16"), u32_to_torch(wq), to_torch(s, "bf16"), to_torch(b, "bf16")
+    idx = {"lhs_indices": torch.from_numpy(lhs.copy()).cuda(), "rhs_indices": torch.from_numpy(rhs).cuda()}
+    for _ in range(2):
+        y = mb.gather_qmm(*args, **idx, group_size=group, bits=bits)
+        ok, err = qmm_close(O.to_f32(from_torch(y), "bf16").reshape(ref.shape), ref)
+        assert ok, err
+
+
+@pytest.mark.parametrize("E,tokens,top,H,K,N2,bits", [(8, 4, 2, 1024, 1024, 200, 4), (16, 30, 2, 2048, 1024, 72, 4), (4, 1, 1, 3072, 6144, 16, 8),
+                                                      (6, 11, 2, 2048, 12288, 40, 4)])
+def test_few_rows_gated(E, tokens, top, H, K, N2, bits):
+    make = lambda seed, shape: O.quantize(make_w(seed, shape, "bf16"), 64, bits, "bf16")
+    dev = lambda q: (u32_to_torch(q[0]), to_torch(q[1], "bf16"), to_torch(q[2], "bf16"))
+    gate, up, down = make(80, (E, H, K)), make(81, (E, H, K)), make(82, (E, N2, H))
+    x = make_x(83, (tokens, 1, K), "bf16")
+    rhs = np.random.default_rng(84).integers(0, E, (tokens, top))
+    xt, rt = to_torch(x, "bf16")[:, None], torch.from_numpy(rhs).cuda()
+    a, u = (mb.gather_qmm(xt, *dev(q), rhs_indices=rt, bits=bits).float() for q in (gate, up))
+    h = (torch.nn.functional.silu(a) * u).to(torch.bfloat16).reshape(tokens * top, 1, H)
+    ref = O.gather_qmm(O.to_f32(from_torch(h), "bf16"), down[0], O.to_f32(down[1], "bf16"), O.to_f32(down[2], "bf16"),
+                       np.arange(tokens * top, dtype=np.uint32), rhs.ravel().astype(np.uint32), True, 64, bits, "f32")
+    for _ in range(2):
+        y = mb.gather_qmm_swiglu(xt, dev(gate), dev(up), dev(down), rt, bits=bits)
+        assert tuple(y.shape) == (tokens, top, 1, N2)
+        ok, err = qmm_close(O.to_f32(from_torch(y), "bf16").reshape(ref.shape), ref)
+        assert ok, err
