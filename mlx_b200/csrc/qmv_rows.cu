@@ -31,6 +31,10 @@
 //    Scales are applied per group to fp32 group sums, the biases come back through one small MMA
 //    against the group sums of x:  y = sum_g s_g * (sum_k x_k q_k) + sum_g b_g * (sum_k x_k).
 //    Four independent accumulation chains per warp hide the mma.sync latency.
+//  * Grouped launches (mixture-of-experts decode) walk a table of (expert, up to 8 rows) tiles: blocks take contiguous
+//    ranges of (tile, 16-row group) units, x and y rows are found through the sort's slot tables.  4 tokens, top-2 of 8
+//    experts [14336, 4096] at 4 bits, gate, up and down: 246 us on the tensor-core kernel with its sort, row copy and
+//    activation launches, 142 us here (floor 83 us: the experts' bytes); bound by the unpacking, as the plain launches.
 //  * The consumer warps leave fp32 partial tiles in shared memory; the reducer warp adds them in
 //    warp order (the result does not depend on timing), converts and stores y.
 #include <cuda.h>
@@ -315,16 +319,12 @@ qmv_rows_kernel(const __grid_constant__ RowsMaps<W> maps, const RowsParams p) {
     seg = Segment{b0 * 8, 0, (b1 - b0 + 1) >> 1, 0, p.M};
   }
   const int row_end = kGrouped ? p.N : min(b1 * 8, p.N);
-  // Walks the segments: `at` is the next unit; false when there is none.
+  // Grouped: on to the segment that starts at unit `at`; false when there is none.  (A plain launch has its one segment
+  // from the start, and every role's loop over segments folds away.)
   auto next_segment = [&](int& at) -> bool {
-    if constexpr (kGrouped) {
-      if (at >= b1) return false;
-      seg = segment_at(p, at, b1);
-      at += seg.n;
-    } else {
-      if (at > b0) return false;
-      ++at;
-    }
+    if (at >= b1) return false;
+    seg = segment_at(p, at, b1);
+    at += seg.n;
     return true;
   };
 
@@ -360,39 +360,41 @@ qmv_rows_kernel(const __grid_constant__ RowsMaps<W> maps, const RowsParams p) {
         int lslot = 0, luse = 0;      // ring position of the oldest stage not yet known to have landed
         int landed = 0, s = 0;
         uint32_t dst = smem_base + p.off_slots;
-        bool ok = true;
-        for (int at = b0; ok && next_segment(at);) {
-          for (int ph = 0; ok && ph < p.nph; ++ph) {
-            const int grp0 = p.ph_g0[ph];
-            for (int i = 0; i < seg.n * NW; ++i, ++s) {
-              // slot free: all consumer warps arrived for the stage that used it last
-              if (use > 0 && !mbar_wait(done0 + 8 * slot, (use - 1) & 1, abort_flag)) { ok = false; break; }
-              // at most `inflight` stages outstanding
-              while (landed < s && mbar_test(full0 + 8 * lslot, luse & 1)) {
-                ++landed;
-                if (++lslot == nst) { lslot = 0; ++luse; }
-              }
-              while (s - landed >= inflight) {
-                if (!mbar_wait(full0 + 8 * lslot, luse & 1, abort_flag)) break;
-                ++landed;
-                if (++lslot == nst) { lslot = 0; ++luse; }
-              }
-              if (*abort_flag) { ok = false; break; }
-              const int which = NW == 2 ? (i & 1) : 0;
-              const int row = seg.base + seg.row0 + (NW == 2 ? i >> 1 : i) * 16;
-              const uint32_t bar = full0 + 8 * slot;
-              // rows past the last matrix and chunks past K are zero-filled by the copy engine and still counted
-              // (rows past the end of one of several matrices are the next one's: never stored)
-              mbar_expect_tx(bar, stage_bytes);
-              tma_load_3d(dst, &maps.w[which], 0, row, grp0 * (C::GB / 16) / 8, bar);
-              for (int k = 0; k < nsb; ++k) {
-                tc::tma_load_2d(dst + sb_off + k * 2048, &maps.s[which], grp0 * 2 + 128 * k, row, bar);
-                tc::tma_load_2d(dst + bb_off + k * 2048, &maps.b[which], grp0 * 2 + 128 * k, row, bar);
-              }
-              dst += stage_bytes;
-              if (++slot == nst) { slot = 0; ++use; dst = smem_base + p.off_slots; }
+        int at = b0;
+        bool more = !kGrouped || next_segment(at);
+        while (more) {
+          const int nrg = seg.n * NW, end = s + nrg * p.nph;
+          int iph = 0, irg = 0, grp0 = p.ph_g0[0];
+          for (; s < end; ++s) {
+            // slot free: all consumer warps arrived for the stage that used it last
+            if (use > 0 && !mbar_wait(done0 + 8 * slot, (use - 1) & 1, abort_flag)) break;
+            // at most `inflight` stages outstanding
+            while (landed < s && mbar_test(full0 + 8 * lslot, luse & 1)) {
+              ++landed;
+              if (++lslot == nst) { lslot = 0; ++luse; }
             }
+            while (s - landed >= inflight) {
+              if (!mbar_wait(full0 + 8 * lslot, luse & 1, abort_flag)) break;
+              ++landed;
+              if (++lslot == nst) { lslot = 0; ++luse; }
+            }
+            if (*abort_flag) break;
+            const int which = NW == 2 ? (irg & 1) : 0;
+            const int row = seg.base + seg.row0 + (NW == 2 ? irg >> 1 : irg) * 16;
+            const uint32_t bar = full0 + 8 * slot;
+            // rows past the last matrix and chunks past K are zero-filled by the copy engine and still counted
+            // (rows past the end of one of several matrices are the next one's: never stored)
+            mbar_expect_tx(bar, stage_bytes);
+            tma_load_3d(dst, &maps.w[which], 0, row, grp0 * (C::GB / 16) / 8, bar);
+            for (int i = 0; i < nsb; ++i) {
+              tc::tma_load_2d(dst + sb_off + i * 2048, &maps.s[which], grp0 * 2 + 128 * i, row, bar);
+              tc::tma_load_2d(dst + bb_off + i * 2048, &maps.b[which], grp0 * 2 + 128 * i, row, bar);
+            }
+            dst += stage_bytes;
+            if (++slot == nst) { slot = 0; ++use; dst = smem_base + p.off_slots; }
+            if (++irg == nrg) { irg = 0; ++iph; grp0 = p.ph_g0[iph < p.nph ? iph : 0]; }
           }
+          more = kGrouped && s == end && next_segment(at);
         }
       }
       RP_MARK(30);
@@ -405,18 +407,19 @@ qmv_rows_kernel(const __grid_constant__ RowsMaps<W> maps, const RowsParams p) {
       if (lane == 0) peer_wait_previous(p.sig, p.status);  // ... or by a peer's consumer of the step before
       __syncwarp();
       if constexpr (kGrouped) find_range();
-      int rslot = 0, ruse = 0, red = 0;
-      bool ok = true;
-      for (int at = b0; ok && next_segment(at);) {
-       const int ytok = min(lane >> 1, seg.rows - 1);
-       const long long y_off = (kGrouped ? slot_row(p.dst_slot, seg.x0 + ytok, p.per_slot) : (long long)(lane >> 1)) * p.ld + p.col0;
-       for (int rph = 0; ok && rph < p.nph; ++rph)
-       for (int rrg = 0; rrg < seg.n * NW; ++rrg) {
-        if (!mbar_wait(done0 + 8 * rslot, ruse & 1, abort_flag)) { ok = false; break; }
+      int rslot = 0, ruse = 0, red = 0, at = b0;
+      bool more = !kGrouped || next_segment(at);
+      while (more) {
+      int rph = 0, rrg = 0;
+      const int nrg = seg.n * NW, end = red + nrg * p.nph;
+      // this lane's row of y
+      const long long y_off =
+          (kGrouped ? slot_row(p.dst_slot, seg.x0 + min(lane >> 1, seg.rows - 1), p.per_slot) : (long long)(lane >> 1)) * p.ld + p.col0;
+      for (; red < end; ++red) {
+        if (!mbar_wait(done0 + 8 * rslot, ruse & 1, abort_flag)) break;
         if (++rslot == nst) { rslot = 0; ++ruse; }
         RP_MARK(5 + 2 * red);
         const int pbi = red % kPartialBufs;
-        ++red;
         const float4* pb = reinterpret_cast<const float4*>(smem + p.off_pbuf + (size_t)pbi * (kConsumers * MT * 512)) + lane;
         float sum[MT][4];
 #pragma unroll
@@ -458,6 +461,7 @@ qmv_rows_kernel(const __grid_constant__ RowsMaps<W> maps, const RowsParams p) {
             if ((rrg & 1) == 0) {
 #pragma unroll
               for (int c = 0; c < 4; ++c) yt[128 + (2 * t + (c & 1)) * 16 + g + (c >> 1) * 8] = Elem<T>::from_float(sum[0][c]);
+              ++rrg;   // (never the last one)
               continue;
             }
 #pragma unroll
@@ -490,8 +494,10 @@ qmv_rows_kernel(const __grid_constant__ RowsMaps<W> maps, const RowsParams p) {
           }
           __syncwarp();
         }
-        RP_MARK(4 + 2 * red);
-       }
+        if (++rrg == nrg) { rrg = 0; ++rph; }
+        RP_MARK(6 + 2 * red);
+      }
+      more = kGrouped && red == end && next_segment(at);
       }
       RP_MARK(30);
       __syncwarp();   // all of this block's stores to y were issued by this warp
@@ -634,9 +640,7 @@ qmv_rows_kernel(const __grid_constant__ RowsMaps<W> maps, const RowsParams p) {
   const uint32_t pb_mine = smem_base + p.off_pbuf + (uint32_t)(warp * MT * 32 + lane) * 16;
   uint32_t sb = smem_base + p.off_slots;   // stage the warp works on
   if constexpr (kGrouped) find_range();
-  bool first = true;   // before the first stage: the barriers exist from here on
-  auto meet = [&]() {
-    first = false;
+  auto meet = [&]() {   // before the first stage: the barriers exist from here on
     asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
     // The first mma.sync of a kernel is slow (the tensor pipe wakes up): issue one now, while the
     // first stage is in flight anyway.  Its result is never used.
@@ -645,15 +649,22 @@ qmv_rows_kernel(const __grid_constant__ RowsMaps<W> maps, const RowsParams p) {
                  : "=f"(d0), "=f"(d1), "=f"(d2), "=f"(d3) : "r"(0u), "f"(0.0f));
     RP_MARK(4);
   };
-  int s = 0;
-  for (int at = b0; next_segment(at);) {
-  // this lane's token row of x (of the first token tile)
+  int at = b0;
+  if (kGrouped && !next_segment(at)) {   // no work for this block
+    meet();
+    return;
+  }
+  bool first = true, more = true;
+  while (more) {
+  // this lane's row of x (of the first token tile)
   const uint16_t* x_lane =
       p.x + (kGrouped ? slot_row(p.src_slot, seg.x0 + min(g, seg.rows - 1), p.per_slot) : (long long)g) * p.K;
-  for (int ph = 0; ph < p.nph; ++ph) {
-  setup_phase(ph, x_lane);
-  if (first) meet();
-  for (int rg = 0; rg < seg.n * NW; ++rg, ++s) {
+  const int nrg = seg.n * NW, total = nrg * p.nph;
+  int ph = 0, rg = 0;
+  setup_phase(0, x_lane);
+  if (!kGrouped || first) meet();
+  first = false;
+  for (int s = 0; s < total; ++s) {
     if (!mbar_wait(full0 + 8 * slot, use & 1, abort_flag)) return;
     RP_MARK(5 + 3 * s);
     float out[MT][4];
@@ -760,10 +771,14 @@ qmv_rows_kernel(const __grid_constant__ RowsMaps<W> maps, const RowsParams p) {
     sb += p.slot_bytes;
     if (++slot == nst) { slot = 0; ++use; sb = smem_base + p.off_slots; }
     if (++pbi == kPartialBufs) { pbi = 0; ++pbe; }
+    if (++rg == nrg) {
+      rg = 0;
+      ++ph;
+      if (ph < p.nph) setup_phase(ph, x_lane);
+    }
   }
+  more = kGrouped && next_segment(at);
   }
-  }
-  if (first) meet();   // (no work for this block)
   RP_MARK(30);
 }
 
