@@ -36,9 +36,11 @@
 //   SplitT  no transpose, bf16 and f16: W is packed along the output columns, so A is written to shared
 //           memory M-major (hi and lo)
 //
-// Few tiles (a short batch through a narrow matrix): K is split over pairs so that all SMs have
-// work; every pair leaves fp32 partial sums in the workspace and the last one to arrive adds them in
-// order.  No block ever waits for another pair.
+// Tiles are dealt to the pairs in whole waves; the K stages of the tiles that are left over are laid end to end and cut
+// into equal ranges, one per pair, so that the last wave is as short as its work (or, with few tiles, all SMs have
+// work).  A tile that is cut leaves fp32 partial sums in the workspace and the last pair to arrive adds them in order;
+// no block ever waits for another pair.  With the last wave uneven instead, 512 tokens through [28672, 8192] took four
+// waves for 3.03 waves' work.
 //
 // Grouped mode (gather_qmm): a device-side table lists (expert, first row, valid rows) for
 // every slice of up to NT rows of the expert-sorted activations; the weight tensor map spans the
@@ -142,9 +144,10 @@ struct TcParams {
   int NT;            // most tokens per tile (multiple of 32, <= 256)
   int nsb;           // x stages in shared memory (2 .. kMaxStagesB)
   int n_tiles, m_tiles;
-  int splits;        // parts of K (1 unless a tile is shared by several pairs)
-  float* partial;    // [tile][split][block of the pair][NT tokens][128 columns], splits > 1 only
-  uint32_t* counters;   // [tile][block of the pair]
+  int full;          // tiles in whole waves (all of them in grouped mode)
+  int rem, cut;      // tiles left over, and the number of pairs their stages are cut for
+  float* partial;    // [cut range, tile by tile][block of the pair][NT tokens][128 columns]
+  uint32_t* counters;   // [tile left over][block of the pair]
   int g4;            // groups per 128 fields of a row: 4, 2, 1
   int row_groups;    // groups per packed row
   int s_slots;       // chunks of scales in their ring
@@ -360,25 +363,47 @@ struct Unit {
   int x_row0;      // first activation row
   int rows, neff;  // valid activation rows, and the same rounded up to what the MMA takes
   int ks0, ks1;    // stages of K
-  int slot;        // index of the unit's partial sums
+  int parts;       // number of ranges that share the tile; with more than one:
+  int slot, slot0; // index of the unit's partial sums, and of those of the tile's first part
+  int rtile;       // index of the tile among those left over
 };
+// Pair j's range of the chunks (spc stages, whole chunks of scales) of the tiles left over.
+__device__ __forceinline__ int range_begin(const TcParams& p, int j, int chunks) { return (int)((long long)j * p.rem * chunks / p.cut); }
+// Units of the loop `for (u = pair; u < end; u += pairs)`: the pair's whole tiles, then the pieces of its range.
+__device__ __forceinline__ int units_end(const TcParams& p, int pair, int pairs) {
+  if (p.mtiles) return *p.n_mtiles * p.n_tiles;
+  if (pair >= p.cut) return p.full;
+  const int chunks = (p.K + kStageK - 1) / kStageK / p.spc, lo = range_begin(p, pair, chunks), hi = range_begin(p, pair + 1, chunks);
+  return p.full + (hi > lo ? (hi - 1) / chunks - lo / chunks + 1 : 0) * pairs;
+}
 __device__ __forceinline__ Unit unit_at(const TcParams& p, int u, int rank) {
   Unit t;
   const int kst = p.K / kStageK + (p.K % kStageK != 0);
   if (p.mtiles == nullptr) {
-    const int tile = p.splits == 1 ? u : u / p.splits, sp = u - tile * p.splits;
+    int tile = u;
+    t.ks0 = 0;
+    t.ks1 = kst;
+    t.parts = 1;
+    if (u >= p.full && p.cut > 0) {
+      const int pairs = gridDim.x >> 1, v = u - p.full, i = v / pairs, j = v - i * pairs, chunks = kst / p.spc;
+      const int lo = range_begin(p, j, chunks), hi = range_begin(p, j + 1, chunks), r = lo / chunks + i, first = r * chunks;
+      t.ks0 = (max(lo, first) - first) * p.spc;
+      t.ks1 = (min(hi, first + chunks) - first) * p.spc;
+      // the pair whose range holds chunk c is ((c + 1) * cut - 1) / (rem * chunks)
+      const long long all = (long long)p.rem * chunks;
+      const int j0 = (int)(((first + 1ll) * p.cut - 1) / all), j1 = (int)(((long long)(first + chunks) * p.cut - 1) / all);
+      t.parts = j1 - j0 + 1;
+      t.slot = j + r;           // ranges in order, one more at every tile boundary
+      t.slot0 = j0 + r;
+      t.rtile = r;
+      tile = p.full + r;
+    }
     const int tn = p.m_tiles == 1 ? tile : tile / p.m_tiles, tm = tile - tn * p.m_tiles;
     t.n0 = tn * (2 * kTileRows) + rank * kTileRows;
     t.w_row0 = t.n0;
     t.w_row_end = p.N;
     t.x_row0 = tm * p.NT;
     t.rows = min(p.M - t.x_row0, p.NT);
-    t.ks0 = 0;
-    t.ks1 = kst;
-    if (p.splits > 1) {                              // whole chunks of scales
-      t.ks0 = sp * (kst / p.spc) / p.splits * p.spc;
-      t.ks1 = (sp + 1) * (kst / p.spc) / p.splits * p.spc;
-    }
   } else {
     const int g = u / p.n_tiles, tn = u - g * p.n_tiles;
     const MTile mt = p.mtiles[g];
@@ -389,9 +414,9 @@ __device__ __forceinline__ Unit unit_at(const TcParams& p, int u, int rank) {
     t.rows = mt.rows;
     t.ks0 = 0;
     t.ks1 = kst;
+    t.parts = 1;
   }
   t.neff = (t.rows + 31) & ~31;
-  t.slot = u;
   return t;
 }
 
@@ -489,7 +514,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   __syncthreads();
   cluster_sync();
   tcgen05_fence_after();
-  const int total = p.mtiles ? *p.n_mtiles * p.n_tiles : p.n_tiles * p.m_tiles * p.splits;
+  const int total = units_end(p, pair, pairs);
   const uint32_t tmem_base = bars->tmem_base;
   const uint32_t tmem_a = tmem_base + kAccCols;
 
@@ -778,7 +803,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(leader_addr(smem_u32(&bars->acc_empty[ab])));
       };
-      if (p.splits == 1) {
+      if (t.parts == 1) {
         uint32_t r[2][16];
         load_piece(acc + c_begin, r[0]);
         for (int c0 = c_begin; c0 < c_end; c0 += 64) {
@@ -809,46 +834,58 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
             if (j < lim) __stcg(part + (size_t)(c + j) * kTileRows, __uint_as_float(v[j]));
         }
       }
-      if (p.splits > 1) {
+      if (t.parts > 1) {
         // The last of the tile's pairs to arrive (per block of the pair: each has its own 128 columns) adds
         // the parts in order and leaves them zeroed.
         __threadfence();
         asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueWarps * 32) : "memory");
-        const int tile = t.slot / p.splits;
         if (warp == kFirstEpilogue && lane == 0) {
-          uint32_t* ctr = p.counters + tile * 2 + rank;
-          const bool last = atomicAdd(ctr, 1u) == (uint32_t)p.splits - 1;
+          uint32_t* ctr = p.counters + t.rtile * 2 + rank;
+          const bool last = atomicAdd(ctr, 1u) == (uint32_t)t.parts - 1;
           if (last) *ctr = 0;
           bars->last = last;
         }
         asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueWarps * 32) : "memory");
         if (bars->last) {
+          // A warp takes whole tokens, a lane four columns of each: 16-byte loads, two tokens of four parts at a time.
           __threadfence();
-          const size_t pitch = 2 * (size_t)p.NT * kTileRows;   // from one part to the next
-          float* p0 = p.partial + ((size_t)tile * p.splits * 2 + rank) * ((size_t)p.NT * kTileRows) + quad * 32 + lane;
-          for (int c = c_begin; c < min(c_end, t.rows); c += 8) {
-            float sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            for (int s = 0; s < p.splits; s += 2) {   // 16 loads in flight
-              float a[8], b[8];
+          const size_t pitch = 2 * (size_t)p.NT * kTileRows / 4;   // from one part to the next
+          float4* p0 = reinterpret_cast<float4*>(p.partial + ((size_t)t.slot0 * 2 + rank) * ((size_t)p.NT * kTileRows)) + lane;
+          const int n4 = t.n0 + 4 * lane;
+          const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          for (int c = warp - kFirstEpilogue; c < t.rows; c += 2 * kEpilogueWarps) {
+            const int n_tok = c + kEpilogueWarps < t.rows ? 2 : 1;
+            float4* q0 = p0 + (size_t)c * (kTileRows / 4);
+            float4 sum[2] = {zero, zero};
+            for (int s = 0; s < t.parts; s += 4) {
+              float4 v[2][4];
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {           // (rows past t.rows: zeros, inside the part)
-                const float* q = p0 + s * pitch + (size_t)(c + j) * kTileRows;
-                a[j] = __ldcg(q);
-                b[j] = s + 1 < p.splits ? __ldcg(q + pitch) : 0.0f;
-              }
+              for (int k = 0; k < 2; ++k)
 #pragma unroll
-              for (int j = 0; j < 8; ++j) sum[j] = (sum[j] + a[j]) + b[j];
+                for (int i = 0; i < 4; ++i)
+                  v[k][i] = k < n_tok && s + i < t.parts ? __ldcg(q0 + (size_t)(s + i) * pitch + k * (kEpilogueWarps * kTileRows / 4)) : zero;
+#pragma unroll
+              for (int k = 0; k < 2; ++k)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) { sum[k].x += v[k][i].x; sum[k].y += v[k][i].y; sum[k].z += v[k][i].z; sum[k].w += v[k][i].w; }
             }
-            for (int s = 0; s < p.splits; ++s)
 #pragma unroll
-              for (int j = 0; j < 8; ++j) __stcg(p0 + s * pitch + (size_t)(c + j) * kTileRows, 0.0f);
-            if (n < p.N)
+            for (int k = 0; k < 2; ++k) {
+              if (k >= n_tok) break;
+              for (int s = 0; s < t.parts; ++s) __stcg(q0 + (size_t)s * pitch + k * (kEpilogueWarps * kTileRows / 4), zero);
+              const uint2 o = make_uint2(pack_pair<T>(__float_as_uint(sum[k].x), __float_as_uint(sum[k].y)),
+                                         pack_pair<T>(__float_as_uint(sum[k].z), __float_as_uint(sum[k].w)));
+              const long long at = (long long)(t.x_row0 + c + k * kEpilogueWarps) * p.ld + p.col0 + n4;
               for (int q = 0; q < p.n_out; ++q) {
-                T* yp = static_cast<T*>(p.y_out[q]) + (size_t)(t.x_row0 + c) * p.ld + p.col0 + n;
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                  if (c + j < t.rows) yp[(size_t)j * p.ld] = Elem<T>::from_float(sum[j]);
+                T* dst = static_cast<T*>(p.y_out[q]) + at;
+                if (n4 + 4 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+                  *reinterpret_cast<uint2*>(dst) = o;
+                } else {
+                  const T* e = reinterpret_cast<const T*>(&o);
+                  for (int i = 0; i < 4 && n4 + i < p.N; ++i) dst[i] = e[i];
+                }
               }
+            }
           }
         }
         asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueWarps * 32) : "memory");   // `last` may be written again
@@ -926,11 +963,12 @@ size_t fixed_smem(int bits, Form f, int cb, int slots) {
   return n;
 }
 
-// Token width of a tile and number of parts of K: the pair with the least estimated time.  A stage takes
-// the longer of its MMAs (4 cycles per token, 8 when split) and of its unpacking; a tile adds the
-// exposed part of its epilogue, and a shared tile the trip of its partial sums through L2.
+// Token width of a tile and the number of pairs that share the tiles left over from whole waves: the choice with the
+// least estimated time, in cycles.  A stage takes the longer of its MMAs (4 cycles per token, 8 when split) and of its
+// unpacking; a tile adds the exposed part of its epilogue; the last part of a cut tile to arrive reads and zeroes
+// `parts` times its fp32 sums at about 64 bytes per cycle, after a round trip through L2.
 struct TcPlan {
-  int nt, m_tiles, n_tiles, splits;
+  int nt, m_tiles, n_tiles, full, rem, cut;
 };
 TcPlan tc_plan(int64_t M, int64_t N, int64_t K, Form f) {
   TcPlan best{};
@@ -942,24 +980,35 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, Form f) {
   for (int nt = cap; nt >= 32; nt -= 32) {
     const int64_t m_tiles = (M + nt - 1) / nt;
     const int64_t tiles = m_tiles * n_tiles;
-    const double stage = f == Form::Round ? (4.0 * nt > 700 ? 4.0 * nt : 700.0) : (8.0 * nt > 1300 ? 8.0 * nt : 1300.0);
-    for (int s = 1; s == 1 || (s <= 16 && s * 4 <= kst); ++s) {
-      if (s > 1 && tiles * s > pairs) break;
-      const double waves = (double)((tiles * s + pairs - 1) / pairs);
-      const double tile = (kst + s - 1) / s * stage + (nt <= kAccCols / 2 ? 1000.0 : 1000.0 + 10.0 * nt) + (s > 1 ? 3000.0 + 8.0 * nt * s : 0.0);
-      if (waves * tile < best_t) {
-        best_t = waves * tile;
-        best = TcPlan{nt, (int)m_tiles, n_tiles, s};
+    const double stage = f == Form::Round ? (4.0 * nt > 800 ? 4.0 * nt : 800.0) : (8.0 * nt > 1300 ? 8.0 * nt : 1300.0);
+    const double exposed = nt <= kAccCols / 2 ? 1000.0 : 1000.0 + 10.0 * nt, tile = kst * stage + exposed;
+    const int64_t waves = tiles / pairs;
+    const int rem = (int)(tiles - waves * pairs);
+    // s parts per tile, on rem * s pairs; or, where that leaves pairs idle, an equal range for every pair
+    for (int s = 1; s <= 16 && (s == 1 || s * 4 <= kst); ++s) {
+      const bool all = (long long)rem * s > pairs;
+      const int cut = all ? pairs : rem * s;
+      double last = 0.0;
+      if (rem > 0 && s == 1) last = tile;
+      if (rem > 0 && s > 1) {
+        const double share = (double)rem * kst / cut, parts = all ? (double)(int)(kst / share) + 2.0 : (double)s;
+        last = (double)(int)(share + 0.999) * stage + (all ? 2.0 : 1.0) * exposed + 3000.0 + parts * (16.0 * nt + 200.0);
       }
+      const double t = waves * tile + last;
+      if (t < best_t) {
+        best_t = t;
+        best = TcPlan{nt, (int)m_tiles, n_tiles, (int)(s == 1 ? tiles : tiles - rem), s == 1 ? 0 : rem, s == 1 ? 0 : cut};
+      }
+      if (all || rem == 0) break;
     }
   }
   return best;
 }
 
+size_t counter_bytes(const TcPlan& pl) { return ((size_t)pl.rem * 2 * 4 + 255) / 256 * 256; }
 size_t split_bytes(const TcPlan& pl) {
-  if (pl.splits == 1) return 0;
-  const size_t tiles = (size_t)pl.m_tiles * pl.n_tiles;
-  return (tiles * 2 * 4 + 255) / 256 * 256 + tiles * pl.splits * 2 * pl.nt * kTileRows * 4;
+  if (pl.cut == 0) return 0;
+  return counter_bytes(pl) + (size_t)(pl.cut + pl.rem) * 2 * pl.nt * kTileRows * 4;
 }
 
 // x maps (boxes of 128, 64, 32 and 16 rows of 64 k) and the map of the packed matrix.
@@ -1077,7 +1126,10 @@ int qmm_tc(const QmmArgs& a, cudaStream_t st) {
                 (size_t)kStatusBytes, a.ws_bytes);
   const Form f = form_of(a.dtype, a.transpose);
   TcPlan pl = tc_plan(a.M, a.N, a.K, f);
-  if (a.ws_bytes < split_bytes(pl) + kStatusBytes) pl.splits = 1;   // a caller's smaller workspace: no shared tiles
+  if (a.ws_bytes < split_bytes(pl) + kStatusBytes) {   // a caller's smaller workspace: no shared tiles
+    pl.full += pl.rem;
+    pl.rem = pl.cut = 0;
+  }
   const int64_t qaxis = a.transpose ? a.K : a.N;
   TcMaps maps;
   if (int rc = encode_maps(maps, "quantized_matmul", a.x, a.M, a.K, a.dtype, a.wq, a.transpose ? a.N : a.K,
@@ -1089,12 +1141,13 @@ int qmm_tc(const QmmArgs& a, cudaStream_t st) {
   set_outputs(p, a.peers, a.y, a.N);
   p.status = reinterpret_cast<uint32_t*>(static_cast<char*>(a.ws) + a.ws_bytes - kStatusBytes);
   p.M = (int)a.M; p.N = (int)a.N; p.K = (int)a.K;
-  p.NT = pl.nt; p.m_tiles = pl.m_tiles; p.n_tiles = pl.n_tiles; p.splits = pl.splits;
+  p.NT = pl.nt; p.m_tiles = pl.m_tiles; p.n_tiles = pl.n_tiles;
+  p.full = pl.full; p.rem = pl.rem; p.cut = pl.cut;
   p.counters = static_cast<uint32_t*>(a.ws);
-  p.partial = reinterpret_cast<float*>(static_cast<char*>(a.ws) + ((size_t)pl.m_tiles * pl.n_tiles * 8 + 255) / 256 * 256);
+  p.partial = reinterpret_cast<float*>(static_cast<char*>(a.ws) + counter_bytes(pl));
   p.row_groups = (int)(qaxis / a.group);
   p.n_scales = (a.transpose ? a.N : a.K) * p.row_groups;
-  return launch_tc(a.dtype, a.bits, a.group, f, (long long)pl.m_tiles * pl.n_tiles * pl.splits, st, maps, p);
+  return launch_tc(a.dtype, a.bits, a.group, f, (long long)pl.full + pl.cut, st, maps, p);
 }
 
 int qmm_tc_grouped(const GroupedArgs& a, cudaStream_t st) {
@@ -1111,7 +1164,7 @@ int qmm_tc_grouped(const GroupedArgs& a, cudaStream_t st) {
   p.ld = a.N; p.col0 = 0;
   p.status = a.status;
   p.M = (int)a.n_rows; p.N = (int)a.N; p.K = (int)a.K;
-  p.NT = a.nt; p.m_tiles = 0; p.splits = 1;
+  p.NT = a.nt; p.m_tiles = 0;
   p.n_tiles = (int)((a.N + 2 * kTileRows - 1) / (2 * kTileRows));
   p.row_groups = (int)(a.K / a.group);
   p.n_scales = a.E * a.N * p.row_groups;

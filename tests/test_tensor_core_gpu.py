@@ -48,6 +48,14 @@ def test_k_shared_by_pairs_of_blocks(dtype, M, N, K, g, bits):
     check(dtype, M, N, K, g, bits, True, 1e-2)
 
 
+@pytest.mark.parametrize("dtype", ("bf16", "f16"))
+@pytest.mark.parametrize("M,N,K,g,bits,transpose", [(57, 19500, 1024, 64, 4, True), (40, 28601, 1152, 128, 3, True),
+                                                    (600, 6300, 1152, 32, 8, True), (300, 9728, 1032, 64, 4, False)])
+def test_tiles_left_over_from_whole_waves(dtype, M, N, K, g, bits, transpose):
+    """One to 38 tiles more than there are pairs of blocks: their stages are cut into ranges that end inside tiles."""
+    check(dtype, M, N, K, g, bits, transpose, 1e-2)
+
+
 @pytest.mark.parametrize("bits", (5, 6, 8))
 def test_experts_with_an_odd_number_of_stages(bits):
     """Nine stages per tile and several tiles per pair of blocks: the unpack warps' turns cross tile borders."""
