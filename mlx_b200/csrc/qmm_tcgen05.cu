@@ -258,33 +258,36 @@ __device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_
                                           uint32_t (&out)[16]) {
   constexpr uint32_t kMagic = 0x43004300u;  // (128.0, 128.0): 0x4300 | q == 128 + q for q < 128
   const uint32_t s2 = s_bits * 0x00010001u, b2 = b_bits * 0x00010001u;
-  // Fast form for 4- and 8-bit fields: the masked field, read as bf16, is the subnormal (or
-  // smallest normal) number q * 2^-133 (16 q * 2^-133 for a field at bits 4..7: bit 7 is the
-  // exponent's lowest bit and continues the subnormal scale exactly).  fma.rn.bf16x2 takes
-  // subnormal inputs exactly, so one fma with the scale times 2^133 (2^129) gives
-  // round(q * s + b): no shift for half of the fields, no subtraction.  It needs the scaled scale
-  // to stay finite and normal: biased exponent of s in [1, 121]; other scales (zero, subnormal,
+  // Fast form: a field inside a byte, masked in place and read as bf16, is the subnormal (or smallest normal) number
+  // q * 2^(o - 133), o its lowest bit in the byte: bit 7 is the exponent's lowest bit and continues the subnormal scale
+  // exactly.  fma.rn.bf16x2 takes subnormal inputs exactly, so one fma with the scale times 2^(133 - o) gives
+  // round(q * s + b).  A byte permute brings the bytes of fields 2j and 2j+1 into the halves of a register; a field that
+  // ends in the next byte is first shifted down (a quarter of the 3-bit fields, half of the 5- and 6-bit ones).  1.5 to
+  // 2 instructions per field (8 bits: 1) where extracting both fields, joining them and subtracting an offset took 3.5.
+  // It needs the scaled scale to stay finite and normal: biased exponent of s in [1, 121]; other scales (zero, subnormal,
   // |s| >= 2^-6 * 2, inf, nan) take the general form below.
   const uint32_t s_exp = (s_bits >> 7) & 0xFFu;
   const bool fast = __all_sync(0xFFFFFFFFu, s_exp >= 1u && s_exp <= 121u);   // one branch per warp: a predicated mixture would run both forms
-  if constexpr (BITS == 4) {
-    if (fast) {
-      const uint32_t sl = (s_bits + (133u << 7)) * 0x00010001u, sh = (s_bits + (129u << 7)) * 0x00010001u;
+  if (fast) {
+    const uint32_t s0 = (s_bits + (133u << 7)) * 0x00010001u;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t u = w[j] >> 8;
-        uint32_t p[4];   // p[i] = (w[i], w[i+4]) as bf16 pairs
-        p[0] = fma_bf16x2(w[j] & 0x000F000Fu, sl, b2);
-        p[1] = fma_bf16x2(w[j] & 0x00F000F0u, sh, b2);
-        p[2] = fma_bf16x2(u & 0x000F000Fu, sl, b2);
-        p[3] = fma_bf16x2(u & 0x00F000F0u, sh, b2);
-        out[4 * j + 0] = __byte_perm(p[0], p[1], 0x5410);
-        out[4 * j + 1] = __byte_perm(p[2], p[3], 0x5410);
-        out[4 * j + 2] = __byte_perm(p[0], p[1], 0x7632);
-        out[4 * j + 3] = __byte_perm(p[2], p[3], 0x7632);
+    for (int j = 0; j < 16; ++j) {
+      const int pl = 2 * j * BITS, ph = pl + BITS;   // first bits of the two fields
+      if constexpr (BITS == 8) {
+        out[j] = fma_bf16x2(__byte_perm(w[pl >> 5], 0u, (pl & 31) ? 0x4342 : 0x4140), s0, b2);
+      } else {
+        constexpr uint32_t m = (1u << BITS) - 1u;
+        const bool dl = (pl & 7) + BITS <= 8, dh = (ph & 7) + BITS <= 8;   // inside a byte
+        const uint32_t ol = dl ? pl & 7 : 0, oh = dh ? ph & 7 : 0;
+        const uint32_t bl = dl ? (pl >> 3) & 3 : 0, bh = (dh ? (ph >> 3) & 3 : 0) + 4;
+        const uint32_t v = __byte_perm(dl ? w[pl >> 5] : field_raw<BITS>(w, 2 * j), dh ? w[ph >> 5] : field_raw<BITS>(w, 2 * j + 1),
+                                       bl * 0x11 + bh * 0x1100);
+        out[j] = fma_bf16x2(v & (m << ol | m << (oh + 16)), s0 - (ol * 0x0080u + oh * 0x00800000u), b2);
       }
-      return;
     }
+    return;
+  }
+  if constexpr (BITS == 4) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       uint32_t p[4];
@@ -300,17 +303,6 @@ __device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_
       out[4 * j + 3] = __byte_perm(p[2], p[3], 0x7632);  // (w6, w7)
     }
   } else if constexpr (BITS == 8) {
-    if (fast) {
-      const uint32_t sl = (s_bits + (133u << 7)) * 0x00010001u;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t r0 = fma_bf16x2(w[j] & 0x00FF00FFu, sl, b2);          // (w0, w2)
-        const uint32_t r1 = fma_bf16x2((w[j] >> 8) & 0x00FF00FFu, sl, b2);   // (w1, w3)
-        out[2 * j + 0] = __byte_perm(r0, r1, 0x5410);
-        out[2 * j + 1] = __byte_perm(r0, r1, 0x7632);
-      }
-      return;
-    }
     // 8-bit values exceed the bf16 integer trick: go through float (0x4B0000qq == 2^23 + q)
     const float sf = __uint_as_float(s_bits << 16), bf = __uint_as_float(b_bits << 16);
 #pragma unroll
@@ -966,7 +958,8 @@ size_t fixed_smem(int bits, Form f, int cb, int slots) {
 // Token width of a tile and the number of pairs that share the tiles left over from whole waves: the choice with the
 // least estimated time, in cycles.  A stage takes the longer of its MMAs (4 cycles per token, 8 when split) and of its
 // unpacking; a tile adds the exposed part of its epilogue; the last part of a cut tile to arrive reads and zeroes
-// `parts` times its fp32 sums at about 64 bytes per cycle, after a round trip through L2.
+// `parts` times its fp32 sums, and all of them pass through L2 three times (1531 f16 tokens through [14336, 4096], 40
+// tiles left over: 273 us with a whole last wave, 289 us cut; 512 tokens through [28672, 8192], 2 left over: 234 / 217).
 struct TcPlan {
   int nt, m_tiles, n_tiles, full, rem, cut;
 };
@@ -992,7 +985,7 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, Form f) {
       if (rem > 0 && s == 1) last = tile;
       if (rem > 0 && s > 1) {
         const double share = (double)rem * kst / cut, parts = all ? (double)(int)(kst / share) + 2.0 : (double)s;
-        last = (double)(int)(share + 0.999) * stage + (all ? 2.0 : 1.0) * exposed + 3000.0 + parts * (16.0 * nt + 200.0);
+        last = (double)(int)(share + 0.999) * stage + (all ? 2.0 : 1.0) * exposed + 4000.0 + parts * (24.0 * nt + 200.0) + 1.2 * nt * cut;
       }
       const double t = waves * tile + last;
       if (t < best_t) {
