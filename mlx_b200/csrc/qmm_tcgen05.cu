@@ -506,9 +506,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   }
   tcgen05_fence_before();
   __syncthreads();
-  // Warps 2 and 3 fetch for this block alone: they start at once and meet the other block when they are done.
-  cluster_arrive();
-  if (warp != 2 && warp != 3) cluster_wait();
+  cluster_sync();
   tcgen05_fence_after();
   const int total = units_end(p, pair, pairs);
   const uint32_t tmem_base = bars->tmem_base;
@@ -628,8 +626,6 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         }
       }
     }
-    __syncwarp();
-    cluster_wait();
   } else if (warp == 3) {
     // ------------------------------------------------------------ scales and biases
     // Asynchronous copies straight into the ring, counted on the chunk's barrier; a lane serves four rows.
@@ -667,8 +663,6 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         if (++ss == (uint32_t)p.s_slots) { ss = 0; ps ^= 1; }
       }
     }
-    __syncwarp();
-    cluster_wait();
   } else if (warp < kFirstEpilogue) {
     // ------------------------------------------------------------ unpack
     // Everything here is counted in instructions: the warps of a scheduler make one instruction about
@@ -1099,17 +1093,6 @@ int launch_tc(int dtype, int bits, int group, Form f, long long units, cudaStrea
   long long nsb = (long long)((kSmemMax - fixed) / stage);
   p.nsb = (int)(nsb > kMaxStagesB ? kMaxStagesB : nsb);
   size_t smem = fixed + p.nsb * stage;
-  // The rest holds more scales and packed weights in flight: with few tokens an unpack warp waited 600 to 1200 cycles
-  // of a trip's 4000 for them.
-  const size_t chunk = 2 * kTileRows * (size_t)p.cb, packed = (size_t)kTileRows * 16 * bits;
-  while (2 * p.s_slots <= kMaxSlotsS && smem + p.s_slots * chunk <= kSmemMax) {
-    smem += p.s_slots * chunk;
-    p.s_slots *= 2;
-  }
-  while (p.nsp < kMaxStagesP && smem + packed <= kSmemMax) {
-    smem += packed;
-    ++p.nsp;
-  }
   // More than half of an SM's shared memory: guarantees one block per SM, so the 512-column
   // tensor-memory allocation never has to wait for a co-resident block of this kernel.
   if (smem < 120 * 1024) smem = 120 * 1024;
