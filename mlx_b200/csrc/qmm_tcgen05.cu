@@ -70,9 +70,9 @@ enum class Form { Round, Split, SplitT };
 constexpr int kTileRows = 128;    // output columns per block and tile (MMA M = 256 over the pair)
 constexpr int kStageK = 128;      // k per pipeline stage of x, W, scales
 constexpr int kMaxStagesB = 6;
-constexpr int kMaxStagesP = 16;
+constexpr int kMaxStagesP = 8;
 constexpr int kMaxSlotsA = 4;
-constexpr int kMaxSlotsS = 8;     // chunks of scales and biases
+constexpr int kMaxSlotsS = 4;     // chunks of scales and biases: 2 of four stages, else 4
 constexpr int kDoneRing = 16;     // one commit per A slot; longer than any distance a waiter can be behind
 constexpr int kTmemCols = 512;    // [0, 256) accumulators, [256, 512) A ring (4 slots of 64 columns)
 constexpr int kAccCols = 256;
@@ -91,7 +91,6 @@ struct Shape {
   static constexpr int kSets = kT ? 2 : 4;                     // sets of unpack warps, on A slots in turn
   // Packed stages: four sets hold one each while they unpack; with no more than that every set would wait for a
   // whole TMA latency after each slot.
-  // These are the fewest; what the x stages leave of the shared memory goes to more.
   static constexpr int kStagesP = kT ? (BITS == 8 ? 2 : 3) : (BITS <= 4 ? 8 : (BITS == 8 ? 5 : 6));
   static constexpr int kPRowBytes = 16 * BITS;                 // 128 fields
   static constexpr int kPStageBytes = kTileRows * kPRowBytes;
@@ -151,8 +150,7 @@ struct TcParams {
   uint32_t* counters;   // [tile left over][block of the pair]
   int g4;            // groups per 128 fields of a row: 4, 2, 1
   int row_groups;    // groups per packed row
-  int s_slots;       // chunks of scales in their ring (a power of two)
-  int nsp;           // packed stages in their ring
+  int s_slots;       // chunks of scales in their ring (2 or 4)
   int spc, cb;       // stages per chunk of scales, bytes per row of a chunk (4, 8 or 16)
   long long n_scales;   // elements of `scales`
 };
@@ -463,7 +461,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   using S = Shape<BITS, F>;
   constexpr bool kT = S::kT;
-  constexpr int kSub = S::kSub, kSlotsA = S::kSlotsA;
+  constexpr int kSub = S::kSub, kSlotsA = S::kSlotsA, kStagesP = S::kStagesP;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // carve-up: [A ring of SplitT] [B ring: nsb stages of two NT/2 * 128-byte sub-tiles] [P ring] [S ring] [barriers]
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -471,7 +469,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   const uint32_t b_stage = 2u * b_sub;
   unsigned char* ring_b = smem + S::kSmemA;
   unsigned char* ring_p = ring_b + (size_t)p.nsb * b_stage;
-  unsigned char* ring_s = ring_p + (size_t)p.nsp * S::kPStageBytes;   // per chunk: 128 rows of scales, 128 of biases
+  unsigned char* ring_s = ring_p + (size_t)kStagesP * S::kPStageBytes;   // per chunk: 128 rows of scales, 128 of biases
   unsigned char* staging = ring_s + p.s_slots * 2 * kTileRows * p.cb;    // a tile per epilogue warp
   Barriers* bars = reinterpret_cast<Barriers*>(staging + kEpilogueWarps * kStageOut);
   volatile int* abort_flag = &bars->abort_flag;
@@ -487,7 +485,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     for (int i = 0; i < 4; ++i) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.x[i]) : "memory");
   }
   if (warp == 0) {
-    for (int i = lane; i < p.nsp; i += 32) { mbar_init(smem_u32(&bars->full_p[i]), 1); mbar_init(smem_u32(&bars->empty_p[i]), S::kPArrivals); }
+    for (int i = lane; i < kStagesP; i += 32) { mbar_init(smem_u32(&bars->full_p[i]), 1); mbar_init(smem_u32(&bars->empty_p[i]), S::kPArrivals); }
     if (lane < p.s_slots) {
       mbar_init(smem_u32(&bars->full_s[lane]), 32);
       mbar_init(smem_u32(&bars->empty_s[lane]), p.spc * S::kPArrivals);
@@ -622,7 +620,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           tma_load_2d(dst, &maps.w, c0, c1, full + sp * 8);
           if constexpr (kT) c1 += kStageK; else c0 += S::kPRowBytes;
           dst += S::kPStageBytes;
-          if (++sp == (uint32_t)p.nsp) { sp = 0; pp ^= 1; dst = ring; }
+          if (++sp == (uint32_t)kStagesP) { sp = 0; pp ^= 1; dst = ring; }
         }
       }
     }
@@ -788,7 +786,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           mbar_arrive(bar_es + (c & s_mask) * 8);
         }
         sp += kSets / kSub;
-        if (sp >= (uint32_t)p.nsp) { sp -= p.nsp; pp ^= 1; }
+        if (sp >= (uint32_t)kStagesP) { sp -= kStagesP; pp ^= 1; }
       }
       it0 += n_st;
       c0 += n_st >> spc_sh;
@@ -962,17 +960,16 @@ Form form_of(int dtype, bool transpose) {
 }
 
 template <int BITS, Form F>
-size_t fixed_smem(int cb, int slots, int* nsp) {
+size_t fixed_smem(int cb, int slots) {
   using S = Shape<BITS, F>;
-  *nsp = S::kStagesP;
   return 1024 + S::kSmemA + (size_t)S::kStagesP * S::kPStageBytes + (size_t)slots * 2 * kTileRows * cb + kEpilogueWarps * kStageOut +
          sizeof(Barriers) + 64;
 }
-size_t fixed_smem(int bits, Form f, int cb, int slots, int* nsp) {
+size_t fixed_smem(int bits, Form f, int cb, int slots) {
   size_t n = 0;
   B200Q_DISPATCH_BITS(bits, BITS, {
-    n = f == Form::Round ? fixed_smem<BITS, Form::Round>(cb, slots, nsp)
-                         : (f == Form::Split ? fixed_smem<BITS, Form::Split>(cb, slots, nsp) : fixed_smem<BITS, Form::SplitT>(cb, slots, nsp));
+    n = f == Form::Round ? fixed_smem<BITS, Form::Round>(cb, slots)
+                         : (f == Form::Split ? fixed_smem<BITS, Form::Split>(cb, slots) : fixed_smem<BITS, Form::SplitT>(cb, slots));
   });
   return n;
 }
@@ -1088,7 +1085,7 @@ int launch_tc(int dtype, int bits, int group, Form f, long long units, cudaStrea
       p.spc *= 2;
   p.cb = p.spc * p.g4 * 2 < 4 ? 4 : p.spc * p.g4 * 2;
   p.s_slots = p.spc == 4 ? 2 : 4;
-  const size_t fixed = fixed_smem(bits, f, p.cb, p.s_slots, &p.nsp);
+  const size_t fixed = fixed_smem(bits, f, p.cb, p.s_slots);
   const size_t stage = (size_t)p.NT * 128;
   long long nsb = (long long)((kSmemMax - fixed) / stage);
   p.nsb = (int)(nsb > kMaxStagesB ? kMaxStagesB : nsb);
