@@ -695,8 +695,8 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
       for (; ia < (it0 + n_st) * kSub; ia += kSets) {
         const uint32_t it = ia / kSub, ks = it - it0;      // ks counts from the unit's first stage
         const uint32_t c = c0 + (ks >> spc_sh);
-        if (!mbar_wait_hot(bar_fs + (c & s_mask) * 8, (c >> s_sh) & 1u, abort_flag)) { ok = false; break; }
-        if (!mbar_wait_hot(bar_fp + sp * 8, pp, abort_flag)) { ok = false; break; }
+        const bool here = mbar_wait_hot(bar_fs + (c & s_mask) * 8, (c >> s_sh) & 1u, abort_flag) && mbar_wait_hot(bar_fp + sp * 8, pp, abort_flag);
+        if (!__all_sync(0xFFFFFFFFu, here)) { ok = false; break; }
         const uint32_t tile = p_base + sp * S::kPStageBytes;
         uint32_t at = s_row + (c & s_mask) * 2 * half_chunk + (ks & (p.spc - 1)) * 2 * p.g4;
         if (single) {
@@ -706,7 +706,10 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         const uint32_t sa = kT ? ia % kSlotsA : set;
         auto slot_free = [&]() {   // the slot's last use has been multiplied
           const uint32_t prev = ia - kSlotsA;
-          return ia < (uint32_t)kSlotsA || mbar_wait_hot(bar_done + (prev % kDoneRing) * 8, (prev / kDoneRing) & 1u, abort_flag);
+          const bool free = ia < (uint32_t)kSlotsA || mbar_wait_hot(bar_done + (prev % kDoneRing) * 8, (prev / kDoneRing) & 1u, abort_flag);
+          // The lanes poll on their own and nothing else brings them together again, which the tcgen05 instructions
+          // that follow (.sync.aligned) require.
+          return __all_sync(0xFFFFFFFFu, free) != 0;
         };
         if constexpr (F == Form::Round) {
           // One vote and one straight line for the slot's four units: every shared-memory read is under way
@@ -803,6 +806,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
       const uint32_t ab = nacc == 2 ? (tcount & 1) : 0, an = nacc == 2 ? (tcount >> 1) : tcount;
       // one warp looks, the others are held by a hardware barrier
       if (warp == kFirstEpilogue) mbar_nap<100>(smem_u32(&bars->acc_full[ab]), an & 1, abort_flag);
+      __syncwarp();
       asm volatile("bar.sync 3, %0;" ::"n"(kEpilogueWarps * 32) : "memory");
       if (*abort_flag) break;
       tcgen05_fence_after();
