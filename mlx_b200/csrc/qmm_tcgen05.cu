@@ -1167,6 +1167,7 @@ int qmm_tc(const QmmArgs& a, cudaStream_t st) {
 }
 
 int qmm_tc_grouped(const GroupedArgs& a, cudaStream_t st) {
+  if (a.bits == 8) return qmm_single_grouped(a, st);
   TcMaps maps;
   if (int rc = encode_maps(maps, "gather_qmm", a.x_sorted, a.n_rows, a.K, B200Q_BF16, a.wq, a.E * a.N, a.K * a.bits / 8, a.bits))
     return rc;
