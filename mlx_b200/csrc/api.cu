@@ -108,6 +108,7 @@ QmmArgs make_args(const void* x, const uint32_t* wq, const void* scales, const v
 // 16 rows 7424 x 1280 4 bits 13.7 / 12.4; 2816 x 2816 12.9 / 14.6.
 bool large_decode(const QmmArgs& a) {
   const int64_t weights = a.N * a.K;
+  if (a.bits == 8) return false;   // (on single blocks: slower)
   if (a.M > 8) return weights >= 9000000;
   return weights >= (a.bits == 2 || a.bits == 4 ? 160000000 : (a.bits == 6 ? 56000000 : 40000000));
 }

@@ -161,6 +161,7 @@ size_t qmm_tc_workspace_bytes(const QmmArgs& a);
 int qmm_tc(const QmmArgs& a, cudaStream_t st);
 int qmm_tc_grouped(const GroupedArgs& a, cudaStream_t st);
 // qmm_tc_single.cu: the same for 8-bit weights
+int qmm_single(const QmmArgs& a, cudaStream_t st);
 int qmm_single_grouped(const GroupedArgs& a, cudaStream_t st);
 
 }  // namespace b200q

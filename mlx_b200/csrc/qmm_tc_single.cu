@@ -1,8 +1,8 @@
-// gather_qmm with 8-bit weights: the grouped product on single thread blocks.
+// Products with 8-bit weights (bf16, transposed, dense and grouped) on single thread blocks.
 //
-// The form that pairs of blocks share (qmm_tcgen05.cu) ended with "unspecified launch failure" on an 8-bit experts
-// product (108 tokens, top-4 of 16, [10240, 2048], calls back to back), for a reason that was not found; every other width
-// and all dense products run there.  This form has no cluster, no remote barrier and no multicast commit.
+// The form that pairs of blocks share (qmm_tcgen05.cu) ended with "unspecified launch failure" on 8-bit products (9 rows
+// through [9728, 16640]; 108 tokens, top-4 of 16 experts [10240, 2048]; calls back to back), for a reason that was not
+// found; every other width runs there.  This form has no cluster, no remote barrier and no multicast commit.
 //
 // y[M, N] = x[M, K] * dequant(W[N, K])^T on the 5th-generation tensor cores.
 //
@@ -709,6 +709,60 @@ int launch(int grid, size_t smem, cudaStream_t st, const CUtensorMap& map_x, con
 }
 
 }  // namespace
+
+int qmm_single(const QmmArgs& a, cudaStream_t st) {
+  EncodeFn enc = encode_fn();
+  if (!enc) return fail(B200Q_ERR_CUDA, "[quantized_matmul] cuTensorMapEncodeTiled is not available");
+  if (!a.ws || a.ws_bytes < kStatusBytes)
+    return fail(B200Q_ERR_WORKSPACE, "[quantized_matmul] workspace of %zu bytes required, %zu given",
+                (size_t)kStatusBytes, a.ws_bytes);
+  const int nt = (int)(a.M >= 256 ? 256 : (a.M + 31) / 32 * 32);
+  CUtensorMap map_x, map_w;
+  {
+    const cuuint64_t dims[2] = {(cuuint64_t)a.K, (cuuint64_t)a.M};
+    const cuuint64_t strides[1] = {(cuuint64_t)a.K * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)kBlockK, (cuuint32_t)nt};
+    const cuuint32_t estr[2] = {1, 1};
+    CUresult r = enc(&map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(a.x), dims, strides, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[quantized_matmul] tensor map for x failed (%d)", (int)r);
+  }
+  {
+    const cuuint64_t dims[2] = {(cuuint64_t)a.K * a.bits / 8, (cuuint64_t)a.N};
+    const cuuint64_t strides[1] = {(cuuint64_t)a.K * a.bits / 8};
+    const cuuint32_t box[2] = {(cuuint32_t)(16 * a.bits), (cuuint32_t)kTileN};
+    const cuuint32_t estr[2] = {1, 1};
+    CUresult r = enc(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint32_t*>(a.wq), dims, strides, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[quantized_matmul] tensor map for w failed (%d)", (int)r);
+  }
+  TcParams p{};
+  p.scales = (const __nv_bfloat16*)a.scales;
+  p.biases = (const __nv_bfloat16*)a.biases;
+  p.y = (__nv_bfloat16*)a.y;
+  if (a.peers.n > 0) {
+    p.n_out = a.peers.n; p.ld = a.peers.ld; p.col0 = a.peers.col0;
+    for (int q = 0; q < a.peers.n; ++q) p.y_out[q] = (__nv_bfloat16*)a.peers.y[q];
+    p.sig = a.peers.sig;
+  } else {
+    p.n_out = 1; p.ld = a.N; p.col0 = 0; p.y_out[0] = (__nv_bfloat16*)a.y;
+  }
+  p.status = reinterpret_cast<uint32_t*>(static_cast<char*>(a.ws) + a.ws_bytes - kStatusBytes);
+  p.M = (int)a.M; p.N = (int)a.N; p.K = (int)a.K;
+  p.NT = nt;
+  p.nsb = x_stages(nt, (int)a.bits);
+  p.n_tiles = (int)((a.N + kTileN - 1) / kTileN);
+  p.m_tiles = (int)((a.M + nt - 1) / nt);
+  p.group_shift = a.group == 32 ? 0 : (a.group == 64 ? 1 : 2);
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long tiles = (long long)p.n_tiles * p.m_tiles;
+  const int grid = (int)(tiles < sms ? tiles : sms);
+  return launch(grid, smem_bytes(nt, a.bits), st, map_x, map_w, p);
+}
 
 int qmm_single_grouped(const GroupedArgs& a, cudaStream_t st) {
   EncodeFn enc = encode_fn();

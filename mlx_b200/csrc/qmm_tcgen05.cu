@@ -1126,6 +1126,7 @@ void set_outputs(TcParams& p, const PeerOut& peers, void* y, int64_t ld) {
 bool qmm_tc_supported(const QmmArgs& a) {
   if ((a.dtype != B200Q_BF16 && a.dtype != B200Q_F16) || a.w_batched || a.batch != 1) return false;
   if (a.M < 1 || a.N < 1 || a.K < 1 || a.M > (1 << 30) || a.N > (1 << 30)) return false;
+  if (a.bits == 8 && (a.dtype != B200Q_BF16 || !a.transpose)) return false;   // 8 bits: qmm_single
   if ((a.transpose ? a.K : a.N) % kStageK != 0 || a.K % 8 != 0) return false;
   // TMA: 16-byte aligned bases and row pitches
   if ((reinterpret_cast<uintptr_t>(a.x) & 15) || (reinterpret_cast<uintptr_t>(a.wq) & 15)) return false;
@@ -1137,6 +1138,7 @@ size_t qmm_tc_workspace_bytes(const QmmArgs& a) {
 }
 
 int qmm_tc(const QmmArgs& a, cudaStream_t st) {
+  if (a.bits == 8) return qmm_single(a, st);
   if (!a.ws || a.ws_bytes < kStatusBytes)
     return fail(B200Q_ERR_WORKSPACE, "[quantized_matmul] workspace of %zu bytes required, %zu given",
                 (size_t)kStatusBytes, a.ws_bytes);

@@ -19,7 +19,8 @@ def check(dtype, M, N, K, g, bits, transpose, rel):
     w = make_w(M + N, (N, K) if transpose else (K, N), dtype)
     wq, s, b = O.quantize(w, g, bits, dtype)
     x = make_x(M + K, (M, K), dtype)
-    assert mb.qmm_kernel_name(DT[dtype], M, N, K, g, bits, transpose) == "qmm_tcgen05"
+    if bits != 8 or (dtype == "bf16" and transpose):
+        assert mb.qmm_kernel_name(DT[dtype], M, N, K, g, bits, transpose) == "qmm_tcgen05"
     ref = O.qmm_f32_from(x, wq, s, b, dtype, transpose=transpose, group_size=g, bits=bits)
     args = (to_torch(x, dtype), u32_to_torch(wq), to_torch(s, dtype), to_torch(b, dtype))
     for _ in range(2):   # the second call finds the counters and partial sums the first has left
