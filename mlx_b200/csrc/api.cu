@@ -101,18 +101,6 @@ QmmArgs make_args(const void* x, const uint32_t* wq, const void* scales, const v
   return a;
 }
 
-// Decode shapes of the register-path kernel that the tensor-core kernel does faster: it costs 8 us whatever the matrix
-// and then reads 4 to 5 million weights per us of any width, the register path 3 to 3.5 million of 3, 5, 6 and 8 bits (half of
-// that with more than 8 rows) and 4.2 million of 2 and 4 bits.  Measured in us, register path / tensor cores: 1 row 28672 x 8192
-// 3 bits 70 / 50, 6 bits 77 / 61; 14336 x 4096 3 bits 27 / 21, 6 bits 27.5 / 24.7; 5376 x 5376 3 bits 16.9 / 18.5;
-// 16 rows 7424 x 1280 4 bits 13.7 / 12.4; 2816 x 2816 12.9 / 14.6.
-bool large_decode(const QmmArgs& a) {
-  const int64_t weights = a.N * a.K;
-  if (a.bits == 8) return false;   // (on single blocks: slower)
-  if (a.M > 8) return weights >= 9000000;
-  return weights >= (a.bits == 2 || a.bits == 4 ? 160000000 : (a.bits == 6 ? 56000000 : 40000000));
-}
-
 int run_qmm(const QmmArgs& a, cudaStream_t st) {
   if (a.batch == 0 || a.M == 0 || a.N == 0) return B200Q_OK;
   if (a.K == 0) {
@@ -127,7 +115,7 @@ int run_qmm(const QmmArgs& a, cudaStream_t st) {
     // f16 tiles cost twice as much (weights split in two): there only 8-bit weights.
     case Path::QmvRows:
       return a.M > 16 && (a.dtype == B200Q_BF16 || a.bits == 8) && qmm_tc_supported(a) ? qmm_tc(a, st) : qmv_rows(a, st);
-    case Path::Qmv: return qmv_override() == 0 && large_decode(a) && qmm_tc_supported(a) ? qmm_tc(a, st) : qmv_mma(a, st);
+    case Path::Qmv: return qmv_mma(a, st);
     case Path::Tc: return qmm_tc(a, st);
     case Path::Qvm: return qvm(a, st);
     default: return qmm_generic(a, st);

@@ -150,7 +150,7 @@ struct TcParams {
   uint32_t* counters;   // [tile left over][block of the pair]
   int g4;            // groups per 128 fields of a row: 4, 2, 1
   int row_groups;    // groups per packed row
-  int s_slots;       // chunks of scales in their ring (2 or 4)
+  int s_slots;       // chunks of scales in their ring
   int spc, cb;       // stages per chunk of scales, bytes per row of a chunk (4, 8 or 16)
   long long n_scales;   // elements of `scales`
 };
@@ -253,39 +253,40 @@ __device__ __forceinline__ void split32(const uint32_t (&w)[BITS], float s, floa
 // Unpacks 32 consecutive BITS-wide fields (BITS words, LSB-first bit stream) of one row into
 // 16 bf16x2 registers in natural k order, applying w = s*q + b (one rounding).  s and b are
 // the raw bf16 bit patterns.
-// Fast form: a field inside a byte, masked in place and read as bf16, is the subnormal (or smallest normal) number
-// q * 2^(o - 133), o its lowest bit in the byte: bit 7 is the exponent's lowest bit and continues the subnormal scale
-// exactly.  fma.rn.bf16x2 takes subnormal inputs exactly, so one fma with the scale times 2^(133 - o) gives
-// round(q * s + b).  A byte permute brings the bytes of fields 2j and 2j+1 into the halves of a register; a field that
-// ends in the next byte is first shifted down (a quarter of the 3-bit fields, half of the 5- and 6-bit ones).  1.5 to
-// 2 instructions per field (8 bits: 1) where extracting both fields, joining them and subtracting an offset took 3.5.
-// It needs the scaled scale to stay finite and normal: biased exponent of s in [1, 121]; other scales (zero, subnormal,
-// |s| >= 2^-6 * 2, inf, nan) take the general form.
-__device__ __forceinline__ bool scale_has_room(uint32_t s) { return (s & 0x7FFFu) - 0x80u < (122u << 7) - 0x80u; }
 template <int BITS>
-__device__ __forceinline__ void dequant32_fast(const uint32_t (&w)[BITS], uint32_t s_bits, uint32_t b_bits, uint32_t (&out)[16]) {
-  const uint32_t b2 = b_bits * 0x00010001u;
-  const uint32_t s0 = (s_bits + (133u << 7)) * 0x00010001u;
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const int pl = 2 * j * BITS, ph = pl + BITS;   // first bits of the two fields
-    if constexpr (BITS == 8) {
-      out[j] = fma_bf16x2(__byte_perm(w[pl >> 5], 0u, (pl & 31) ? 0x4342 : 0x4140), s0, b2);
-    } else {
-      constexpr uint32_t m = (1u << BITS) - 1u;
-      const bool dl = (pl & 7) + BITS <= 8, dh = (ph & 7) + BITS <= 8;   // inside a byte
-      const uint32_t ol = dl ? pl & 7 : 0, oh = dh ? ph & 7 : 0;
-      const uint32_t bl = dl ? (pl >> 3) & 3 : 0, bh = (dh ? (ph >> 3) & 3 : 0) + 4;
-      const uint32_t v = __byte_perm(dl ? w[pl >> 5] : field_raw<BITS>(w, 2 * j), dh ? w[ph >> 5] : field_raw<BITS>(w, 2 * j + 1),
-                                     bl * 0x11 + bh * 0x1100);
-      out[j] = fma_bf16x2(v & (m << ol | m << (oh + 16)), s0 - (ol * 0x0080u + oh * 0x00800000u), b2);
-    }
-  }
-}
-template <int BITS>
-__device__ __forceinline__ void dequant32_any(const uint32_t (&w)[BITS], uint32_t s_bits, uint32_t b_bits, uint32_t (&out)[16]) {
+__device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_bits, uint32_t b_bits,
+                                          uint32_t (&out)[16]) {
   constexpr uint32_t kMagic = 0x43004300u;  // (128.0, 128.0): 0x4300 | q == 128 + q for q < 128
   const uint32_t s2 = s_bits * 0x00010001u, b2 = b_bits * 0x00010001u;
+  // Fast form: a field inside a byte, masked in place and read as bf16, is the subnormal (or smallest normal) number
+  // q * 2^(o - 133), o its lowest bit in the byte: bit 7 is the exponent's lowest bit and continues the subnormal scale
+  // exactly.  fma.rn.bf16x2 takes subnormal inputs exactly, so one fma with the scale times 2^(133 - o) gives
+  // round(q * s + b).  A byte permute brings the bytes of fields 2j and 2j+1 into the halves of a register; a field that
+  // ends in the next byte is first shifted down (a quarter of the 3-bit fields, half of the 5- and 6-bit ones).  1.5 to
+  // 2 instructions per field (8 bits: 1) where extracting both fields, joining them and subtracting an offset took 3.5.
+  // It needs the scaled scale to stay finite and normal: biased exponent of s in [1, 121]; other scales (zero, subnormal,
+  // |s| >= 2^-6 * 2, inf, nan) take the general form below.
+  const uint32_t s_exp = (s_bits >> 7) & 0xFFu;
+  const bool fast = __all_sync(0xFFFFFFFFu, s_exp >= 1u && s_exp <= 121u);   // one branch per warp: a predicated mixture would run both forms
+  if (fast) {
+    const uint32_t s0 = (s_bits + (133u << 7)) * 0x00010001u;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int pl = 2 * j * BITS, ph = pl + BITS;   // first bits of the two fields
+      if constexpr (BITS == 8) {
+        out[j] = fma_bf16x2(__byte_perm(w[pl >> 5], 0u, (pl & 31) ? 0x4342 : 0x4140), s0, b2);
+      } else {
+        constexpr uint32_t m = (1u << BITS) - 1u;
+        const bool dl = (pl & 7) + BITS <= 8, dh = (ph & 7) + BITS <= 8;   // inside a byte
+        const uint32_t ol = dl ? pl & 7 : 0, oh = dh ? ph & 7 : 0;
+        const uint32_t bl = dl ? (pl >> 3) & 3 : 0, bh = (dh ? (ph >> 3) & 3 : 0) + 4;
+        const uint32_t v = __byte_perm(dl ? w[pl >> 5] : field_raw<BITS>(w, 2 * j), dh ? w[ph >> 5] : field_raw<BITS>(w, 2 * j + 1),
+                                       bl * 0x11 + bh * 0x1100);
+        out[j] = fma_bf16x2(v & (m << ol | m << (oh + 16)), s0 - (ol * 0x0080u + oh * 0x00800000u), b2);
+      }
+    }
+    return;
+  }
   if constexpr (BITS == 4) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -484,19 +485,18 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.x[i]) : "memory");
   }
-  if (warp == 0) {
-    for (int i = lane; i < kStagesP; i += 32) { mbar_init(smem_u32(&bars->full_p[i]), 1); mbar_init(smem_u32(&bars->empty_p[i]), S::kPArrivals); }
-    if (lane < p.s_slots) {
-      mbar_init(smem_u32(&bars->full_s[lane]), 32);
-      mbar_init(smem_u32(&bars->empty_s[lane]), p.spc * S::kPArrivals);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStagesP; ++i) { mbar_init(smem_u32(&bars->full_p[i]), 1); mbar_init(smem_u32(&bars->empty_p[i]), S::kPArrivals); }
+    for (int i = 0; i < p.s_slots; ++i) {
+      mbar_init(smem_u32(&bars->full_s[i]), 32);
+      mbar_init(smem_u32(&bars->empty_s[i]), p.spc * S::kPArrivals);
     }
-    if (lane < p.nsb) mbar_init(smem_u32(&bars->full_b[lane]), 1);
-    if (lane < kSlotsA) mbar_init(smem_u32(&bars->full_a[lane]), 2 * kUnpackWarps / S::kSets);
-    if (lane < kDoneRing) mbar_init(smem_u32(&bars->done[lane]), 1);
-    if (lane < 2) { mbar_init(smem_u32(&bars->acc_full[lane]), 1); mbar_init(smem_u32(&bars->acc_empty[lane]), 2 * kEpilogueWarps); }
-    if (lane == 0) bars->abort_flag = 0;
+    for (int i = 0; i < p.nsb; ++i) mbar_init(smem_u32(&bars->full_b[i]), 1);
+    for (int i = 0; i < kSlotsA; ++i) mbar_init(smem_u32(&bars->full_a[i]), 2 * kUnpackWarps / S::kSets);
+    for (int i = 0; i < kDoneRing; ++i) mbar_init(smem_u32(&bars->done[i]), 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&bars->acc_full[i]), 1); mbar_init(smem_u32(&bars->acc_empty[i]), 2 * kEpilogueWarps); }
+    bars->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    __syncwarp();
   }
   if (warp == 1) {
     tcgen05_alloc(smem_u32(&bars->tmem_base), kTmemCols);
@@ -677,7 +677,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     const uint32_t t_slot = tmem_a + ((uint32_t)(quad * 32) << 16) + set * 64;   // (transpose) as many slots as sets
     // offset of unit un's value in a chunk row's stage: one value per 1, 2 or 4 units
     const int gsh = p.g4 == 4 ? 0 : (p.g4 == 2 ? 1 : 2);
-    const uint32_t s_mask = p.s_slots - 1, s_sh = 31 - __clz(p.s_slots);
+    const uint32_t s_mask = p.s_slots - 1, s_sh = p.s_slots == 2 ? 1 : 2;
     const uint32_t spc_sh = p.spc == 4 ? 2 : (p.spc == 2 ? 1 : 0), half_chunk = (uint32_t)kTileRows * p.cb;
     const bool single = p.spc * p.g4 == 1;   // a chunk is one value: the odd or the even half of the copied word
     const uint32_t s_row = smem_u32(ring_s) + row * p.cb;
@@ -686,7 +686,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     const uint32_t bar_fp = smem_u32(&bars->full_p[0]), bar_ep = smem_u32(&bars->empty_p[0]);
     const uint32_t bar_fs = smem_u32(&bars->full_s[0]), bar_es = smem_u32(&bars->empty_s[0]);
     uint32_t it0 = 0, c0 = 0;              // stages and chunks of the units before this one
-    uint32_t ia = set, sp = set / kSub, pp = 0;
+    uint32_t ia = set;
     bool ok = true;
     for (int u = pair; ok && u < total; u += pairs) {
       const Unit t = unit_at(p, u, rank);
@@ -694,9 +694,9 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
       const uint32_t o_row = kT ? min(t.n0 / kTileRows, p.row_groups - 1) : (uint32_t)min(t.w_row0 + row, t.w_row_end - 1) * p.row_groups + t.ks0;
       for (; ia < (it0 + n_st) * kSub; ia += kSets) {
         const uint32_t it = ia / kSub, ks = it - it0;      // ks counts from the unit's first stage
-        const uint32_t c = c0 + (ks >> spc_sh);
-        const bool here = mbar_wait_hot(bar_fs + (c & s_mask) * 8, (c >> s_sh) & 1u, abort_flag) && mbar_wait_hot(bar_fp + sp * 8, pp, abort_flag);
-        if (!__all_sync(0xFFFFFFFFu, here)) { ok = false; break; }
+        const uint32_t c = c0 + (ks >> spc_sh), sp = it % kStagesP;
+        if (!mbar_wait_hot(bar_fs + (c & s_mask) * 8, (c >> s_sh) & 1u, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_hot(bar_fp + sp * 8, (it / kStagesP) & 1u, abort_flag)) { ok = false; break; }
         const uint32_t tile = p_base + sp * S::kPStageBytes;
         uint32_t at = s_row + (c & s_mask) * 2 * half_chunk + (ks & (p.spc - 1)) * 2 * p.g4;
         if (single) {
@@ -707,40 +707,20 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         auto slot_free = [&]() {   // the slot's last use has been multiplied
           const uint32_t prev = ia - kSlotsA;
           const bool free = ia < (uint32_t)kSlotsA || mbar_wait_hot(bar_done + (prev % kDoneRing) * 8, (prev / kDoneRing) & 1u, abort_flag);
-          // The lanes poll on their own and nothing else brings them together again, which the tcgen05 instructions
-          // that follow (.sync.aligned) require.
-          return __all_sync(0xFFFFFFFFu, free) != 0;
+          return __all_sync(0xFFFFFFFFu, free) != 0;   // the tcgen05 instructions that follow need the whole warp
         };
         if constexpr (F == Form::Round) {
-          // One vote and one straight line for the slot's four units: every shared-memory read is under way
-          // before it is needed (a unit at a time, each waited for its own: 1575 cycles per trip at 4 bits).
-          uint32_t sv[4], bv[4], w[2][BITS], vals[16];
 #pragma unroll
           for (int un = 0; un < 4; ++un) {
-            sv[un] = lds_u16(at + 2 * (un >> gsh));
-            bv[un] = lds_u16(at + 2 * (un >> gsh) + half_chunk);
-          }
-          load_fields<BITS>(tile, row, 0, w[0]);
-          if (__all_sync(0xFFFFFFFFu, scale_has_room(sv[0]) && scale_has_room(sv[1]) && scale_has_room(sv[2]) && scale_has_room(sv[3]))) {
-#pragma unroll
-            for (int un = 0; un < 4; ++un) {
-              if (un < 3) load_fields<BITS>(tile, row, un + 1, w[(un + 1) & 1]);
-              dequant32_fast<BITS>(w[un & 1], sv[un], bv[un], vals);
-              if (un == 0) {
-                if (!slot_free()) { ok = false; break; }
-                tcgen05_fence_after();
-              }
-              tcgen05_st_x16(t_slot + un * 16, vals);
+            uint32_t w[BITS], vals[16];
+            load_fields<BITS>(tile, row, un, w);
+            const uint32_t v = at + 2 * (un >> gsh);
+            dequant32<BITS>(w, lds_u16(v), lds_u16(v + half_chunk), vals);
+            if (un == 0) {
+              if (!slot_free()) { ok = false; break; }
+              tcgen05_fence_after();
             }
-          } else {
-            if (!slot_free()) { ok = false; break; }
-            tcgen05_fence_after();
-#pragma unroll
-            for (int un = 0; un < 4; ++un) {
-              load_fields<BITS>(tile, row, un, w[0]);
-              dequant32_any<BITS>(w[0], sv[un], bv[un], vals);
-              tcgen05_st_x16(t_slot + un * 16, vals);
-            }
+            tcgen05_st_x16(t_slot + un * 16, vals);
           }
         } else if constexpr (F == Form::Split) {
 #pragma unroll
@@ -788,8 +768,6 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           mbar_arrive(bar_ep + sp * 8);
           mbar_arrive(bar_es + (c & s_mask) * 8);
         }
-        sp += kSets / kSub;
-        if (sp >= (uint32_t)kStagesP) { sp -= kStagesP; pp ^= 1; }
       }
       it0 += n_st;
       c0 += n_st >> spc_sh;
@@ -806,10 +784,10 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
       const uint32_t ab = nacc == 2 ? (tcount & 1) : 0, an = nacc == 2 ? (tcount >> 1) : tcount;
       // one warp looks, the others are held by a hardware barrier
       if (warp == kFirstEpilogue) mbar_nap<100>(smem_u32(&bars->acc_full[ab]), an & 1, abort_flag);
-      __syncwarp();
       asm volatile("bar.sync 3, %0;" ::"n"(kEpilogueWarps * 32) : "memory");
       if (*abort_flag) break;
       tcgen05_fence_after();
+      const int n = t.n0 + quad * 32 + lane;
       const int c_begin = chalf * (t.neff >> 1), c_end = c_begin + (t.neff >> 1);
       const uint32_t acc = tmem_base + ab * (kAccCols / 2) + lane_field;
       // after the last load the accumulator is free for another tile's MMAs

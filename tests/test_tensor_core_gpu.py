@@ -86,18 +86,3 @@ def test_autograd_worker_thread():
     ref = O.qmm_f32_from(dy, wq, s, b, "bf16", transpose=False, group_size=64, bits=4)
     ok, err = qmm_close(O.to_f32(from_torch(dx), "bf16"), ref)
     assert ok, err
-
-
-@pytest.mark.parametrize("M,N,K,g,bits", [(1, 9800, 4096, 64, 3), (8, 13700, 4096, 32, 6), (16, 3600, 2560, 64, 4), (9, 9001, 1024, 128, 5)])
-def test_large_decode_shapes(M, N, K, g, bits):
-    """Decode products that are named after the register path and run on the tensor cores: just above the sizes from
-    which they do."""
-    w = make_w(M + N, (N, K), "bf16")
-    wq, s, b = O.quantize(w, g, bits, "bf16")
-    x = make_x(M + K, (M, K), "bf16")
-    ref = O.qmm_f32_from(x, wq, s, b, "bf16", transpose=True, group_size=g, bits=bits)
-    args = (to_torch(x, "bf16"), u32_to_torch(wq), to_torch(s, "bf16"), to_torch(b, "bf16"))
-    for _ in range(2):
-        y = mb.quantized_matmul(*args, transpose=True, group_size=g, bits=bits)
-        ok, err = qmm_close(O.to_f32(from_torch(y), "bf16"), ref, 1e-2)
-        assert ok, err
