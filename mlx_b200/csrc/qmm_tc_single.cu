@@ -1,8 +1,7 @@
 // Products with 8-bit weights (bf16, transposed, dense and grouped) on single thread blocks.
 //
-// The form that pairs of blocks share (qmm_tcgen05.cu) ended with "unspecified launch failure" on 8-bit products (9 rows
-// through [9728, 16640]; 108 tokens, top-4 of 16 experts [10240, 2048]; calls back to back), for a reason that was not
-// found; every other width runs there.  This form has no cluster, no remote barrier and no multicast commit.
+// The form that pairs of blocks share (qmm_tcgen05.cu) failed on 8-bit products (9 rows through [9728, 16640]; 108
+// tokens, top-4 of 16 experts [10240, 2048]) while its ring of five packed stages had a race; this form has no cluster.
 //
 // y[M, N] = x[M, K] * dequant(W[N, K])^T on the 5th-generation tensor cores.
 //

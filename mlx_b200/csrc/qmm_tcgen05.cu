@@ -696,6 +696,12 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         const uint32_t it = ia / kSub, ks = it - it0;      // ks counts from the unit's first stage
         const uint32_t c = c0 + (ks >> spc_sh), sp = it % kStagesP;
         if (!mbar_wait_hot(bar_fs + (c & s_mask) * 8, (c >> s_sh) & 1u, abort_flag)) { ok = false; break; }
+        // Where a ring slot passes from one set to another (its length no multiple of the stages per turn), a set can
+        // come to it before the slot's previous stage, another set's, has landed.  The parity asked for is then that of
+        // the use before, which reads as complete: so the previous use is waited for first.
+        if constexpr (S::kStagesP % (kSets / kSub > 0 ? kSets / kSub : 1) != 0) {
+          if (it >= (uint32_t)kStagesP && !mbar_wait_hot(bar_fp + sp * 8, ((it / kStagesP) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+        }
         if (!mbar_wait_hot(bar_fp + sp * 8, (it / kStagesP) & 1u, abort_flag)) { ok = false; break; }
         const uint32_t tile = p_base + sp * S::kPStageBytes;
         uint32_t at = s_row + (c & s_mask) * 2 * half_chunk + (ks & (p.spc - 1)) * 2 * p.g4;
