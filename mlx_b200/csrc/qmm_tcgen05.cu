@@ -698,9 +698,12 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         if (!mbar_wait_hot(bar_fs + (c & s_mask) * 8, (c >> s_sh) & 1u, abort_flag)) { ok = false; break; }
         // Where a ring slot passes from one set to another (its length no multiple of the stages per turn), a set can
         // come to it before the slot's previous stage, another set's, has landed.  The parity asked for is then that of
-        // the use before, which reads as complete: so the previous use is waited for first.
+        // the use before, which reads as complete.  So such rings wait first until the set's own A slot has been multiplied:
+        // products run in order, and the slot's previous stage is an earlier one.
         if constexpr (S::kStagesP % (kSets / kSub > 0 ? kSets / kSub : 1) != 0) {
-          if (it >= (uint32_t)kStagesP && !mbar_wait_hot(bar_fp + sp * 8, ((it / kStagesP) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+          static_assert(S::kStagesP > kSlotsA / kSub, "the previous stage of a ring slot is not after that of the A slot");
+          const uint32_t prev = ia - kSlotsA;
+          if (ia >= (uint32_t)kSlotsA && !mbar_wait_hot(bar_done + (prev % kDoneRing) * 8, (prev / kDoneRing) & 1u, abort_flag)) { ok = false; break; }
         }
         if (!mbar_wait_hot(bar_fp + sp * 8, (it / kStagesP) & 1u, abort_flag)) { ok = false; break; }
         const uint32_t tile = p_base + sp * S::kPStageBytes;
