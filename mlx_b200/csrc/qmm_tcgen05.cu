@@ -152,6 +152,7 @@ struct TcParams {
   int row_groups;    // groups per packed row
   int s_slots;       // chunks of scales in their ring
   int spc, cb;       // stages per chunk of scales, bytes per row of a chunk (4, 8 or 16)
+  int narrow;        // scales or biases are not aligned to cb: 2-byte loads
   long long n_scales;   // elements of `scales`
 };
 
@@ -342,6 +343,9 @@ __device__ __forceinline__ float bits_to_float(uint32_t v) {
 template <int N>
 __device__ __forceinline__ void cp_async(uint32_t dst, const void* src, int n) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(N), "r"(n) : "memory");
+}
+__device__ __forceinline__ void st_shared_u16(uint32_t at, unsigned short v) {
+  asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(v) : "memory");
 }
 __device__ __forceinline__ void st_shared_v4(uint32_t at, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
@@ -644,7 +648,13 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           if constexpr (kT) o = (long long)min(ks * kStageK + lane + 32 * i, p.K - 1) * p.row_groups + min(t.n0 / kTileRows * p.g4, p.row_groups - p.g4);
           else o = (long long)min(t.w_row0 + lane + 32 * i, t.w_row_end - 1) * p.row_groups + ks * p.g4;
           const uint32_t d = dst + 32 * i * p.cb;
-          if (p.cb == 16) {
+          if (p.narrow) {   // scales or biases at any 2-byte address (an expert's slice of a stack of odd size): one stage, value by value
+            const uint32_t at = d + (p.g4 == 1 ? (uint32_t)(o & 1) * 2 : 0);   // a lone value lies where the copied word would have it
+            for (int e = 0; e < p.g4; ++e) {
+              st_shared_u16(at + 2 * e, __ldg(p.scales + o + e));
+              st_shared_u16(at + half_chunk + 2 * e, __ldg(p.biases + o + e));
+            }
+          } else if (p.cb == 16) {
             cp_async<16>(d, p.scales + o, 16);
             cp_async<16>(d + half_chunk, p.biases + o, 16);
           } else if (p.cb == 8) {
@@ -657,7 +667,8 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
             cp_async<4>(d + half_chunk, p.biases + w, n);
           }
         }
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->full_s[ss])) : "memory");
+        if (p.narrow) mbar_arrive(smem_u32(&bars->full_s[ss]));
+        else asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->full_s[ss])) : "memory");
         if (++ss == (uint32_t)p.s_slots) { ss = 0; ps ^= 1; }
       }
     }
@@ -1075,6 +1086,7 @@ int launch_tc(int dtype, int bits, int group, Form f, long long units, cudaStrea
            ((reinterpret_cast<uintptr_t>(p.scales) | reinterpret_cast<uintptr_t>(p.biases)) % (4 * p.spc * p.g4)) == 0)
       p.spc *= 2;
   p.cb = p.spc * p.g4 * 2 < 4 ? 4 : p.spc * p.g4 * 2;
+  p.narrow = (reinterpret_cast<uintptr_t>(p.scales) | reinterpret_cast<uintptr_t>(p.biases)) % p.cb != 0;   // (only with chunks of one stage)
   p.s_slots = p.spc == 4 ? 2 : 4;
   const size_t fixed = fixed_smem(bits, f, p.cb, p.s_slots);
   const size_t stage = (size_t)p.NT * 128;

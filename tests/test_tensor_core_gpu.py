@@ -73,6 +73,29 @@ def test_experts_with_an_odd_number_of_stages(bits):
         assert ok, (e, err)
 
 
+def at_odd_address(t):
+    """The same values, contiguous, 2 bytes past a 16-byte boundary: a slice of a flat buffer."""
+    flat = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)
+    assert flat.data_ptr() % 16 == 0
+    return flat[1:1 + t.numel()].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("bits", (2, 3, 4, 5, 6, 8))
+@pytest.mark.parametrize("E,tokens,N,K,g", [(2, 90, 65, 128, 128), (3, 70, 300, 640, 64), (4, 200, 200, 1152, 32), (3, 40, 65, 384, 128)])
+def test_experts_with_scales_at_odd_addresses(bits, E, tokens, N, K, g):
+    wq, s, b = O.quantize(make_w(7, (E, N, K), "bf16"), g, bits, "bf16")
+    x = to_torch(make_x(8, (tokens, 1, K), "bf16"), "bf16")
+    st, bt = at_odd_address(to_torch(s, "bf16")), at_odd_address(to_torch(b, "bf16"))
+    rhs = torch.arange(tokens, device="cuda") * 5 % E
+    for _ in range(2):   # through plain arrays of pairs, then through views of them
+        y = mb.gather_qmm(x, u32_to_torch(wq), st, bt, rhs_indices=rhs, group_size=g, bits=bits)
+        for e in range(E):
+            rows = torch.nonzero(rhs == e).flatten()
+            ref = O.qmm_f32_from(from_torch(x[rows, 0]), wq[e], s[e], b[e], "bf16", transpose=True, group_size=g, bits=bits)
+            ok, err = qmm_close(O.to_f32(from_torch(y[rows, 0]), "bf16"), ref)
+            assert ok, (e, err)
+
+
 def test_autograd_worker_thread():
     """The backward pass runs in a thread of its own, which has made no CUDA call yet."""
     from mlx_b200 import grad
