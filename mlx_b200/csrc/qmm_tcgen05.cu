@@ -1128,8 +1128,7 @@ bool qmm_tc_supported(const QmmArgs& a) {
   if (a.bits == 8 && (a.dtype != B200Q_BF16 || !a.transpose)) return false;   // 8 bits: qmm_single
   if ((a.transpose ? a.K : a.N) % kStageK != 0 || a.K % 8 != 0) return false;
   // TMA: 16-byte aligned bases and row pitches
-  if ((reinterpret_cast<uintptr_t>(a.x) & 15) || (reinterpret_cast<uintptr_t>(a.wq) & 15)) return false;
-  return !((reinterpret_cast<uintptr_t>(a.scales) | reinterpret_cast<uintptr_t>(a.biases)) & 7);
+  return !((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.wq)) & 15);
 }
 
 size_t qmm_tc_workspace_bytes(const QmmArgs& a) {

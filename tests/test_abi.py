@@ -94,6 +94,17 @@ def test_sharded_rejects_on_host():
     assert lib.b200q_peer_wait(None, dummy, dummy, None) == _lib.ERR_INVALID_ARGUMENT
 
 
+@pytest.mark.parametrize("scales", (4096, 4098))
+def test_scales_need_no_alignment_for_the_tensor_cores(scales):
+    """64 rows of bf16 go to the tensor-core kernel whatever the address of scales and biases, plain and sharded: without
+    a workspace it is that kernel's refusal that comes back (before any CUDA call)."""
+    lib = _lib.load()
+    d, s = ctypes.c_void_p(4096), ctypes.c_void_p(scales)
+    one = (ctypes.c_void_p * 1)(4096)
+    assert lib.b200q_qmm_sharded(d, d, s, s, one, 1, 256, 0, _lib.BF16, 64, 256, 256, 64, 4, None, 0, None) == _lib.ERR_WORKSPACE
+    assert lib.b200q_qmm(d, d, s, s, d, _lib.BF16, 1, 64, 256, 256, 64, 4, 1, 0, None, 0, None) == _lib.ERR_WORKSPACE
+
+
 def test_gather_sharded_rejects_on_host():
     lib = _lib.load()
     dummy = ctypes.c_void_p(4096)

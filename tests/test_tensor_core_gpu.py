@@ -96,6 +96,19 @@ def test_experts_with_scales_at_odd_addresses(bits, E, tokens, N, K, g):
             assert ok, (e, err)
 
 
+@pytest.mark.parametrize("bits", (3, 4, 8))
+@pytest.mark.parametrize("dtype,transpose,rel", [("bf16", True, 1e-2), ("f16", True, 2e-3), ("bf16", False, 6e-3), ("f16", False, 2e-3)])
+@pytest.mark.parametrize("M,N,K,g", [(40, 384, 640, 32), (64, 128, 1152, 128), (300, 256, 512, 64)])
+def test_scales_at_odd_addresses(bits, dtype, transpose, rel, M, N, K, g):
+    wq, s, b = O.quantize(make_w(M, (N, K) if transpose else (K, N), dtype), g, bits, dtype)
+    x = make_x(K, (M, K), dtype)
+    ref = O.qmm_f32_from(x, wq, s, b, dtype, transpose=transpose, group_size=g, bits=bits)
+    y = mb.quantized_matmul(to_torch(x, dtype), u32_to_torch(wq), at_odd_address(to_torch(s, dtype)), at_odd_address(to_torch(b, dtype)),
+                            transpose=transpose, group_size=g, bits=bits)
+    ok, err = qmm_close(O.to_f32(from_torch(y), dtype), ref, rel)
+    assert ok, err
+
+
 def test_autograd_worker_thread():
     """The backward pass runs in a thread of its own, which has made no CUDA call yet."""
     from mlx_b200 import grad
