@@ -1142,7 +1142,8 @@ int qmm_tc(const QmmArgs& a, cudaStream_t st) {
                 (size_t)kStatusBytes, a.ws_bytes);
   const Form f = form_of(a.dtype, a.transpose);
   TcPlan pl = tc_plan(a.M, a.N, a.K, f);
-  if (a.ws_bytes < split_bytes(pl) + kStatusBytes) {   // a caller's smaller workspace: no shared tiles
+  // a caller's smaller workspace, or one that the 16-byte accesses to the partial sums do not fit: no shared tiles
+  if (a.ws_bytes < split_bytes(pl) + kStatusBytes || (reinterpret_cast<uintptr_t>(a.ws) & 15)) {
     pl.full += pl.rem;
     pl.rem = pl.cut = 0;
   }

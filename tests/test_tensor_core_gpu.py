@@ -109,6 +109,27 @@ def test_scales_at_odd_addresses(bits, dtype, transpose, rel, M, N, K, g):
     assert ok, err
 
 
+def test_workspace_off_a_16_byte_boundary():
+    """A caller's workspace may lie anywhere a 4-byte word may; its tiles are then not shared between pairs of blocks."""
+    import ctypes
+
+    from mlx_b200 import _lib
+
+    lib, P = _lib.load(), lambda t: ctypes.c_void_p(t.data_ptr())
+    M, N, K, g, bits = 57, 512, 8192, 64, 4   # few tiles, a long K
+    wq, s, b = O.quantize(make_w(1, (N, K), "bf16"), g, bits, "bf16")
+    x = make_x(2, (M, K), "bf16")
+    need = lib.b200q_qmm_workspace_bytes(_lib.BF16, 1, M, N, K, g, bits, 1)
+    ws = torch.zeros(need + 256, dtype=torch.uint8, device="cuda")[8:8 + need]
+    xt, wt, st, bt = to_torch(x, "bf16"), u32_to_torch(wq), to_torch(s, "bf16"), to_torch(b, "bf16")
+    y = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    _lib.check(lib.b200q_qmm(P(xt), P(wt), P(st), P(bt), P(y), _lib.BF16, 1, M, N, K, g, bits, 1, 0, P(ws), need, stream))
+    ok, err = qmm_close(O.to_f32(from_torch(y), "bf16"), O.qmm_f32_from(x, wq, s, b, "bf16", transpose=True, group_size=g, bits=bits))
+    assert ok, err
+    assert int(ws.max()) == 0
+
+
 def test_autograd_worker_thread():
     """The backward pass runs in a thread of its own, which has made no CUDA call yet."""
     from mlx_b200 import grad
