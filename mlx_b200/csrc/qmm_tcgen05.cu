@@ -169,6 +169,7 @@ struct __align__(8) Barriers {
   uint64_t acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   int abort_flag, last;
+  int landed[2];   // of a tile (even, odd): its accumulator is complete, as the epilogue warp that waits for it found
 };
 
 // ------------------------------------------------------------------------------------ unpacking
@@ -802,10 +803,16 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     for (int u = pair; u < total; u += pairs, ++tcount) {
       const Unit t = unit_at(p, u, rank);
       const uint32_t ab = nacc == 2 ? (tcount & 1) : 0, an = nacc == 2 ? (tcount >> 1) : tcount;
-      // one warp looks, the others are held by a hardware barrier
-      if (warp == kFirstEpilogue) mbar_nap<100>(smem_u32(&bars->acc_full[ab]), an & 1, abort_flag);
+      // One warp looks, the others are held by a hardware barrier.  All go by what it found: the abort flag may be
+      // raised between two warps' looks at it, and a warp that left alone would keep the others at the next barrier.
+      // (Two words: the one of two tiles ago has been read by all who have passed the last tile's barrier.)
+      if (warp == kFirstEpilogue) {
+        const bool landed = __all_sync(0xFFFFFFFFu, mbar_nap<100>(smem_u32(&bars->acc_full[ab]), an & 1, abort_flag));
+        if (lane == 0) bars->landed[tcount & 1] = landed;
+        __syncwarp();
+      }
       asm volatile("bar.sync 3, %0;" ::"n"(kEpilogueWarps * 32) : "memory");
-      if (*abort_flag) break;
+      if (!bars->landed[tcount & 1]) break;
       tcgen05_fence_after();
       const int n = t.n0 + quad * 32 + lane;
       const int c_begin = chalf * (t.neff >> 1), c_end = c_begin + (t.neff >> 1);
