@@ -348,6 +348,14 @@ __device__ __forceinline__ void cp_async(uint32_t dst, const void* src, int n) {
 __device__ __forceinline__ void st_shared_u16(uint32_t at, unsigned short v) {
   asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(v) : "memory");
 }
+// The same for scales or biases that are not aligned to a row's chunk (an expert's slice of a stack of odd size): one stage,
+// value by value; a lone value goes where the copied word would have it.  (Out of line: the ordinary loop stays short.)
+__device__ __noinline__ void copy_values(uint32_t dst, uint32_t bias_off, const unsigned short* s, const unsigned short* b, int n) {
+  for (int e = 0; e < n; ++e) {
+    st_shared_u16(dst + 2 * e, __ldg(s + e));
+    st_shared_u16(dst + bias_off + 2 * e, __ldg(b + e));
+  }
+}
 __device__ __forceinline__ void st_shared_v4(uint32_t at, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
@@ -643,19 +651,24 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
       for (int ks = t.ks0; ks < t.ks1; ks += p.spc) {
         if (!mbar_nap<100>(smem_u32(&bars->empty_s[ss]), ps ^ 1, abort_flag)) { ok = false; break; }
         const uint32_t dst = smem_u32(ring_s) + ss * 2 * half_chunk + lane * p.cb;
+        auto row_at = [&](int i) -> long long {   // rows past the end: results are never stored (transpose), x is zero (no transpose)
+          if constexpr (kT) return (long long)min(ks * kStageK + lane + 32 * i, p.K - 1) * p.row_groups + min(t.n0 / kTileRows * p.g4, p.row_groups - p.g4);
+          else return (long long)min(t.w_row0 + lane + 32 * i, t.w_row_end - 1) * p.row_groups + ks * p.g4;
+        };
+        if (p.narrow) {
+          for (int i = 0; i < 4; ++i) {
+            const long long o = row_at(i);
+            copy_values(dst + 32 * i * p.cb + (p.g4 == 1 ? (uint32_t)(o & 1) * 2 : 0), half_chunk, p.scales + o, p.biases + o, p.g4);
+          }
+          mbar_arrive(smem_u32(&bars->full_s[ss]));
+          if (++ss == (uint32_t)p.s_slots) { ss = 0; ps ^= 1; }
+          continue;
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          long long o;   // rows past the end: results are never stored (transpose), x is zero (no transpose)
-          if constexpr (kT) o = (long long)min(ks * kStageK + lane + 32 * i, p.K - 1) * p.row_groups + min(t.n0 / kTileRows * p.g4, p.row_groups - p.g4);
-          else o = (long long)min(t.w_row0 + lane + 32 * i, t.w_row_end - 1) * p.row_groups + ks * p.g4;
+          const long long o = row_at(i);
           const uint32_t d = dst + 32 * i * p.cb;
-          if (p.narrow) {   // scales or biases at any 2-byte address (an expert's slice of a stack of odd size): one stage, value by value
-            const uint32_t at = d + (p.g4 == 1 ? (uint32_t)(o & 1) * 2 : 0);   // a lone value lies where the copied word would have it
-            for (int e = 0; e < p.g4; ++e) {
-              st_shared_u16(at + 2 * e, __ldg(p.scales + o + e));
-              st_shared_u16(at + half_chunk + 2 * e, __ldg(p.biases + o + e));
-            }
-          } else if (p.cb == 16) {
+          if (p.cb == 16) {
             cp_async<16>(d, p.scales + o, 16);
             cp_async<16>(d + half_chunk, p.biases + o, 16);
           } else if (p.cb == 8) {
@@ -668,8 +681,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
             cp_async<4>(d + half_chunk, p.biases + w, n);
           }
         }
-        if (p.narrow) mbar_arrive(smem_u32(&bars->full_s[ss]));
-        else asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->full_s[ss])) : "memory");
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->full_s[ss])) : "memory");
         if (++ss == (uint32_t)p.s_slots) { ss = 0; ps ^= 1; }
       }
     }
