@@ -719,7 +719,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
       for (; ia < (it0 + n_st) * kSub; ia += kSets) {
         const uint32_t it = ia / kSub, ks = it - it0;      // ks counts from the unit's first stage
         const uint32_t c = c0 + (ks >> spc_sh), sp = it % kStagesP;
-        if (!mbar_wait_hot(bar_fs + (c & s_mask) * 8, (c >> s_sh) & 1u, abort_flag)) { ok = false; break; }
+        bool got = mbar_wait_hot(bar_fs + (c & s_mask) * 8, (c >> s_sh) & 1u, abort_flag);
         // Where a ring slot passes from one set to another (its length no multiple of the stages per turn), a set can
         // come to it before the slot's previous stage, another set's, has landed.  The parity asked for is then that of
         // the use before, which reads as complete.  So such rings wait first until the set's own A slot has been multiplied:
@@ -727,9 +727,11 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         if constexpr (S::kStagesP % (kSets / kSub > 0 ? kSets / kSub : 1) != 0) {
           static_assert(S::kStagesP > kSlotsA / kSub, "the previous stage of a ring slot is not after that of the A slot");
           const uint32_t prev = ia - kSlotsA;
-          if (ia >= (uint32_t)kSlotsA && !mbar_wait_hot(bar_done + (prev % kDoneRing) * 8, (prev / kDoneRing) & 1u, abort_flag)) { ok = false; break; }
+          got = got && (ia < (uint32_t)kSlotsA || mbar_wait_hot(bar_done + (prev % kDoneRing) * 8, (prev / kDoneRing) & 1u, abort_flag));
         }
-        if (!mbar_wait_hot(bar_fp + sp * 8, (it / kStagesP) & 1u, abort_flag)) { ok = false; break; }
+        got = got && mbar_wait_hot(bar_fp + sp * 8, (it / kStagesP) & 1u, abort_flag);
+        // A wait may run out for some of the lanes only.  They stay (what they unpack is never stored) until the vote below:
+        // the votes and tcgen05 instructions from here on need the whole warp.
         const uint32_t tile = p_base + sp * S::kPStageBytes;
         uint32_t at = s_row + (c & s_mask) * 2 * half_chunk + (ks & (p.spc - 1)) * 2 * p.g4;
         if (single) {
@@ -739,8 +741,8 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         const uint32_t sa = kT ? ia % kSlotsA : set;
         auto slot_free = [&]() {   // the slot's last use has been multiplied
           const uint32_t prev = ia - kSlotsA;
-          const bool free = ia < (uint32_t)kSlotsA || mbar_wait_hot(bar_done + (prev % kDoneRing) * 8, (prev / kDoneRing) & 1u, abort_flag);
-          return __all_sync(0xFFFFFFFFu, free) != 0;   // the tcgen05 instructions that follow need the whole warp
+          const bool free = got && (ia < (uint32_t)kSlotsA || mbar_wait_hot(bar_done + (prev % kDoneRing) * 8, (prev / kDoneRing) & 1u, abort_flag));
+          return __all_sync(0xFFFFFFFFu, free) != 0;
         };
         if constexpr (F == Form::Round) {
 #pragma unroll
