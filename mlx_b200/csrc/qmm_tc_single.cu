@@ -504,7 +504,7 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     if (vec) prefetch();
     int cur_chunk = -1;
     bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < total_tiles && !*abort_flag; tile += gridDim.x) {
+    for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
       const int row = row_of(tile);
       const unsigned short* sc = reinterpret_cast<const unsigned short*>(p.scales) + (size_t)row * row_groups;
       const unsigned short* bi = reinterpret_cast<const unsigned short*>(p.biases) + (size_t)row * row_groups;
@@ -533,7 +533,8 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
           s_q[1] = __ldg(sc + g1); b_q[1] = __ldg(bi + g1);
         }
         TC_T0();
-        if (!TC_WAIT16(smem_u32(&bars->full_p[sp]), pp, abort_flag)) { ok = false; break; }
+        // (A wait may run out for some of the lanes only; they stay until the vote below, before anything is stored.)
+        bool got = TC_WAIT16(smem_u32(&bars->full_p[sp]), pp, abort_flag);
         TC_ACC(pw0);
         const unsigned char* src0 = ring_p + sp * kPStageBytes + row_in_tile * kPRowBytes + half * (8 * BITS);
         bool freed = false;
@@ -567,12 +568,14 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
           asm volatile("" ::"r"(vals[0]), "r"(vals[5]), "r"(vals[10]), "r"(vals[15]));
 #endif
           TC_ACC(pw3);
+          __syncwarp();   // the lanes' scales may have taken both forms; a tcgen05.st needs the whole warp
           if (q == 0) {
             TC_T0();
             if (it >= (uint32_t)kStagesA) {   // the stage that used this A slot last has been multiplied
               const uint32_t prev = it - (uint32_t)kStagesA;
-              if (!TC_WAIT16(smem_u32(&bars->done[prev % kDoneRing]), (prev / kDoneRing) & 1u, abort_flag)) { ok = false; break; }
+              got = got && TC_WAIT16(smem_u32(&bars->done[prev % kDoneRing]), (prev / kDoneRing) & 1u, abort_flag);
             }
+            if (!__all_sync(0xFFFFFFFFu, got)) { ok = false; break; }
             TC_ACC(pw2);
             tcgen05_fence_after();
             freed = true;
@@ -602,10 +605,10 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     const int chalf = (warp - (2 + kDequantWarps)) >> 2;  // which half of the token columns
     const uint32_t lane_field = (uint32_t)(quad * 32) << 16;
     uint32_t tcount = 0;
-    for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x, ++tcount) {
+    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++tcount) {
       const TileCoord tc_ = tile_coord(p, tile);
       TC_T0();
-      if (!mbar_wait(smem_u32(&bars->acc_full), tcount & 1, abort_flag)) break;
+      if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&bars->acc_full), tcount & 1, abort_flag))) break;
       TC_ACC(pw0);
       tcgen05_fence_after();
       const int n = tc_.n0 + quad * 32 + lane;
@@ -655,6 +658,7 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   }
 
   // ---- teardown: everyone meets, then the allocating warp returns the tensor memory
+  __syncwarp();
   tcgen05_fence_before();
   __syncthreads();
   if (threadIdx.x == 0 && *abort_flag) atomicMax(&p.status[0], 3u);
