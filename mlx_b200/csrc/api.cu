@@ -2,7 +2,9 @@
 //
 // Kernel selection for b200q_qmm (the role of QuantizedMatmul::eval_gpu's dispatch,
 // mlx/backend/cuda/quantized/quantized.cpp:106-136):
-//   bf16, f16, transpose, M <= 16, bits 2/4/8, K % (16 * group) == 0 -> qmv_rows (HBM-bound decode)
+//   bf16, f16, transpose, M <= 32, bits 2/4/8, K % (16 * group) == 0 -> qmv_rows (HBM-bound decode; above 16 rows in
+//       two passes.  bf16 keeps the weights' exact value there, which one tensor-core tile of 17 to 32 rows rounds: the
+//       result is off by 1.7e-3 of its norm against 2.2e-3)
 //   bf16, transpose, M <= 16, K % 128 == 0 (any width)           -> qmv_mma     (register-path decode)
 //   bf16, f16, transpose, K % 128 == 0                           -> qmm_tcgen05 (TMA + tcgen05 + TMEM)
 //   bf16, f16, transpose == 0, M > 16, N % 128 == 0              -> qmm_tcgen05 (fewer rows waste half of the 32-token tile)
@@ -110,11 +112,7 @@ int run_qmm(const QmmArgs& a, cudaStream_t st) {
   if (!a.x || !a.wq || !a.scales || !a.biases || !a.y)
     return fail(B200Q_ERR_INVALID_ARGUMENT, "[quantized_matmul] null pointer");
   switch (choose(a)) {
-    // 17 to 32 rows: the row-owning kernel would read W twice; one tensor-core tile does it in 18 us against 27
-    // (14336 x 4096, 4 bits) and in 25 against 50 (4096 x 14336, 8 bits).
-    // f16 tiles cost twice as much (weights split in two): there only 8-bit weights.
-    case Path::QmvRows:
-      return a.M > 16 && (a.dtype == B200Q_BF16 || a.bits == 8) && qmm_tc_supported(a) ? qmm_tc(a, st) : qmv_rows(a, st);
+    case Path::QmvRows: return qmv_rows(a, st);
     case Path::Qmv: return qmv_mma(a, st);
     case Path::Tc: return qmm_tc(a, st);
     case Path::Qvm: return qvm(a, st);

@@ -197,6 +197,21 @@ def test_row_owning_kernel_two_passes(M, N, K, bits, g):
     run_case("bf16", M, N, K, g, bits, seed=M + N, expect_kernel=("qmv_rows",))
 
 
+@pytest.mark.parametrize("bits,g", [(4, 64), (8, 64), (8, 128)])
+@pytest.mark.parametrize("M", (16, 17, 24, 32))
+def test_row_owning_kernel_does_not_round_weights(bits, g, M):
+    """Up to 32 rows only the result is rounded, to 8 bits: an error of 2^-8 / sqrt(3) binades over the root mean square
+    of the mantissas, which lies between 1.36 (spread evenly over their logarithm) and 1.53 (evenly): 1.5e-3 to 1.66e-3 of the
+    result's norm.  Weights rounded to 8 bits as well add as much again in the square: 2.1e-3 and more."""
+    N, K = 512, 4096
+    wq, s, b = O.quantize(make_w(M, (N, K), "bf16"), g, bits, "bf16")
+    x = make_x(bits, (M, K), "bf16")
+    ref = O.qmm_f32_from(x, wq, s, b, "bf16", transpose=True, group_size=g, bits=bits).astype(np.float64)
+    y = mb.quantized_matmul(to_torch(x, "bf16"), u32_to_torch(wq), to_torch(s, "bf16"), to_torch(b, "bf16"), group_size=g, bits=bits)
+    err = np.linalg.norm(O.to_f32(from_torch(y), "bf16") - ref) / np.linalg.norm(ref)
+    assert err < 1.8e-3, err
+
+
 def test_kernel_selection_by_token_count():
     """The selection a caller sees for C2's matrix as the token count grows."""
     name = lambda M, **kw: mb.qmm_kernel_name(torch.bfloat16, M, 14336, 4096, kw.get("g", 64), kw.get("bits", 4))
