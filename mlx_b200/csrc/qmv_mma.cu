@@ -95,7 +95,9 @@ __device__ __forceinline__ void load_chunk(const uint32_t* __restrict__ p, uint3
     uint2 v = ldg_nc_u64(p);
     w[0] = v.x; w[1] = v.y;
   } else if constexpr (BITS == 6) {
-    // (through L1: three loads share each 32-byte sector)
+    // 3, 5 and 6 words: through L1, since several loads share each 32-byte sector.  Against loads past L1 (device us, one
+    // row): 6 bits [4096, 11008] 28.0 -> 22.8, [28672, 8192] 74.4 -> 69.9; 3 bits [4096, 11008] 26.0 -> 21.6; matrices of
+    // 17 M weights and less the same.
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       const uint2 v = __ldg(reinterpret_cast<const uint2*>(p) + i);
@@ -104,50 +106,6 @@ __device__ __forceinline__ void load_chunk(const uint32_t* __restrict__ p, uint3
   } else {
 #pragma unroll
     for (int i = 0; i < BITS; ++i) w[i] = __ldg(p + i);
-  }
-}
-
-// 3-, 5- and 6-bit fields straddle bytes and words.  A chunk's 32 fields are taken in pairs (e, e + 16), which lie
-// 2 * BITS whole bytes apart: one byte permute (`window`) brings the two bytes that hold field e into the low half of
-// a register and those of field e + 16 into the high half, at the same bit offset.  A field that ends inside the
-// first byte is masked in place and read as the bf16 subnormal q * 2^(off - 133); the others are shifted down
-// first; one fma with s * 2^(133 - off) gives s*q+b, rounded once.  Between 3 and 4 instructions per pair
-// instead of 6 (extracting both fields, joining them, subtracting an offset).
-__host__ __device__ constexpr bool straddles(int bits) { return bits == 3 || bits == 5 || bits == 6; }
-template <int BITS>
-__device__ __forceinline__ uint32_t window(const uint32_t (&w)[BITS], int by, bool one_byte) {
-  const int b2 = by + 2 * BITS, i0 = by >> 2, i1 = b2 >> 2, r0 = by & 3, r1 = b2 & 3;
-  if (r0 != 3 && r1 != 3) return __byte_perm(w[i0], w[i1], r0 | (r0 + 1) << 4 | (r1 + 4) << 8 | (r1 + 5) << 12);
-  if (one_byte) return __byte_perm(w[i0], w[i1], r0 | r0 << 4 | (r1 + 4) << 8 | (r1 + 4) << 12);
-  const uint32_t lo = r0 == 3 ? __funnelshift_r(w[i0], w[(i0 + 1) % BITS], 24) : w[i0];
-  const uint32_t hi = r1 == 3 ? __funnelshift_r(w[i1], w[(i1 + 1) % BITS], 24) : w[i1];
-  const int q0 = r0 == 3 ? 0 : r0, q1 = r1 == 3 ? 0 : r1;
-  return __byte_perm(lo, hi, q0 | (q0 + 1) << 4 | (q1 + 4) << 8 | (q1 + 5) << 12);
-}
-// A scale times 2^133 has to stay finite and normal: biased exponent 1 to 121 (else the general form).
-__device__ __forceinline__ bool scale_has_room(uint32_t s) { return (s & 0x7FFFu) - 0x80u < (122u << 7) - 0x80u; }
-// Pairs e = 4c .. 4c+3 of a chunk.  s, b: raw bf16 bits.
-template <int BITS>
-__device__ __forceinline__ void dequant_pairs(const uint32_t (&w)[BITS], int c, uint32_t s, uint32_t b, bool fast, uint32_t (&P)[4]) {
-  constexpr uint32_t kM = ((1u << BITS) - 1u) * 0x00010001u;
-  if (fast) {
-    const uint32_t s0 = (s + (133u << 7)) * 0x00010001u, b2 = b * 0x00010001u;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int by = (BITS * (4 * c + i)) >> 3, off = (BITS * (4 * c + i)) & 7;
-      const bool direct = off + BITS <= 8;
-      const uint32_t v = window<BITS>(w, by, direct);
-      if (direct) P[i] = fma_bf16x2(v & (kM << off), s0 - (uint32_t)off * 0x00800080u, b2);
-      else P[i] = fma_bf16x2((v >> off) & kM, s0, b2);
-    }
-  } else {
-    const float sf = __uint_as_float(s << 16), bf = __uint_as_float(b << 16);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int by = (BITS * (4 * c + i)) >> 3, off = (BITS * (4 * c + i)) & 7;
-      const uint32_t v = (window<BITS>(w, by, off + BITS <= 8) >> off) & kM;
-      P[i] = pack_bf16x2(fmaf((float)(v & 0xFFFFu), sf, bf), fmaf((float)(v >> 16), sf, bf));
-    }
   }
 }
 
@@ -181,6 +139,20 @@ __device__ __forceinline__ void dequant_block(const uint32_t (&w)[BITS], int c, 
       float a = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7540 | i)) - 8388608.0f;
       float d = __uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7540 | i)) - 8388608.0f;
       P[i] = pack_bf16x2(fmaf(a, sf, bf), fmaf(d, sf, bf));
+    }
+  } else {
+    // 3/5/6-bit fields straddle words: extract each field with a funnel shift.
+    constexpr uint32_t mask = (1u << BITS) - 1u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int e0 = 8 * c + i, e1 = e0 + 4;
+      const int w0 = (e0 * BITS) >> 5, s0 = (e0 * BITS) & 31;
+      const int w1 = (e1 * BITS) >> 5, s1 = (e1 * BITS) & 31;
+      uint32_t f0 = (s0 + BITS > 32) ? __funnelshift_r(w[w0], w[(w0 + 1) % BITS], s0) : (w[w0] >> s0);
+      uint32_t f1 = (s1 + BITS > 32) ? __funnelshift_r(w[w1], w[(w1 + 1) % BITS], s1) : (w[w1] >> s1);
+      uint32_t t = lop3_and_or(f0, mask, kMagic);
+      asm("bfi.b32 %0, %1, %2, 16, %3;" : "=r"(t) : "r"(f1), "r"(t), "n"(BITS));
+      P[i] = fma_bf16x2(sub_bf16x2(t, kMagic), s2, b2);
     }
   }
 }
@@ -301,15 +273,8 @@ qmv_mma_kernel(const QmvParams p) {
           if (j < per_mt) {
             const int ln = j & 31, c = (j >> 5) & 3, kb = j >> 7;
             const int tok = mt * 8 + (ln >> 2);
-            const __nv_bfloat16* xc = p.x + (int64_t)tok * p.K + kb * 128 + 32 * (ln & 3);
-            if (tok < p.M) {
-              if constexpr (straddles(BITS)) {   // pairs (k, k + 16)
-                const uint2 l = __ldg(reinterpret_cast<const uint2*>(xc) + c), h = __ldg(reinterpret_cast<const uint2*>(xc + 16) + c);
-                v[u] = make_uint4(l.x, l.y, h.x, h.y);
-              } else {                           // pairs (k, k + 4)
-                v[u] = __ldg(reinterpret_cast<const uint4*>(xc) + c);
-              }
-            }
+            const int k8 = kb * 128 + 32 * (ln & 3) + 8 * c;
+            if (tok < p.M) v[u] = __ldg(reinterpret_cast<const uint4*>(p.x + (int64_t)tok * p.K + k8));
           }
         }
 #pragma unroll
@@ -317,7 +282,7 @@ qmv_mma_kernel(const QmvParams p) {
           const int j = base + u * kThreads;
           if (j < per_mt) {
             uint4 o;
-            o.x = __byte_perm(v[u].x, v[u].z, 0x5410);  // (x0, x4), or (x0, x16) ...
+            o.x = __byte_perm(v[u].x, v[u].z, 0x5410);  // (x0, x4)
             o.y = __byte_perm(v[u].x, v[u].z, 0x7632);  // (x1, x5)
             o.z = __byte_perm(v[u].y, v[u].w, 0x5410);  // (x2, x6)
             o.w = __byte_perm(v[u].y, v[u].w, 0x7632);  // (x3, x7)
@@ -374,12 +339,6 @@ qmv_mma_kernel(const QmvParams p) {
         bf[j] = 0.0f;
       }
     }
-    bool fast = true;   // straddling widths: every scale of the warp's step has room for the short form
-    if constexpr (straddles(BITS)) {
-#pragma unroll
-      for (int j = 0; j < NLD; ++j) fast = fast && scale_has_room(sbuf[slot][j] & 0xFFFFu);
-      fast = __all_sync(0xFFFFFFFFu, fast);
-    }
     const uint4* xk = xs_lane + pkb * 128;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -389,15 +348,9 @@ qmv_mma_kernel(const QmvParams p) {
 #pragma unroll
       for (int a = 0; a < RT; ++a) {
         uint32_t P0[4], P1[4];
-        if constexpr (straddles(BITS)) {
-          const uint32_t sb0 = sbuf[slot][2 * a], sb1 = sbuf[slot][2 * a + 1];
-          dequant_pairs<BITS>(wbuf[slot][2 * a], c, sb0 & 0xFFFFu, sb0 >> 16, fast, P0);
-          dequant_pairs<BITS>(wbuf[slot][2 * a + 1], c, sb1 & 0xFFFFu, sb1 >> 16, fast, P1);
-        } else {
-          dequant_block<BITS>(wbuf[slot][2 * a], c, s2[2 * a], b2[2 * a], sf[2 * a], bf[2 * a], P0);
-          dequant_block<BITS>(wbuf[slot][2 * a + 1], c, s2[2 * a + 1], b2[2 * a + 1], sf[2 * a + 1],
-                              bf[2 * a + 1], P1);
-        }
+        dequant_block<BITS>(wbuf[slot][2 * a], c, s2[2 * a], b2[2 * a], sf[2 * a], bf[2 * a], P0);
+        dequant_block<BITS>(wbuf[slot][2 * a + 1], c, s2[2 * a + 1], b2[2 * a + 1], sf[2 * a + 1],
+                            bf[2 * a + 1], P1);
 #pragma unroll
         for (int b = 0; b < MT; ++b) {
           mma_bf16(acc[a][b], P0[0], P1[0], P0[1], P1[1], xf[b].x, xf[b].y);
