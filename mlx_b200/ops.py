@@ -54,20 +54,32 @@ class _Workspaces:
 
     quantized_matmul and gather_qmm keep separate buffers: the matmul kernels rely on
     counters that start at zero and are left at zero, while gather_qmm uses its buffer as
-    plain scratch (sorted indices, tile table, gathered rows)."""
+    plain scratch (sorted indices, tile table, gathered rows).
+
+    A buffer that has become too small is kept: a CUDA graph captured before goes on using it.
+    Every new one is at least twice as large, so that the old ones never add up to more than it."""
 
     def __init__(self):
         self._bufs = {}
+        self._outgrown = []   # (key, buffer)
 
     def get(self, dev: torch.device, nbytes: int, op: str) -> torch.Tensor:
         key = (dev.index, torch.cuda.current_stream(dev).cuda_stream, op)
         buf = self._bufs.get(key)
         if buf is None or buf.numel() < nbytes:
+            nbytes = max(nbytes, 256)
+            if buf is not None:
+                self._outgrown.append((key, buf))
+                nbytes = max(nbytes, 2 * buf.numel())
             with torch.cuda.device(dev):
-                buf = torch.zeros(max(nbytes, 256), dtype=torch.uint8, device=dev)
+                buf = torch.zeros(nbytes, dtype=torch.uint8, device=dev)
             self._bufs[key] = buf
             _front.scratch(dev.index, key[1], _SCRATCH_OPS[op], buf.data_ptr(), buf.numel())
         return buf
+
+    def all(self):
+        """Every (key, buffer) that a kernel may still be using."""
+        return list(self._bufs.items()) + self._outgrown
 
 
 _workspaces = _Workspaces()
@@ -113,7 +125,7 @@ def check_status(device: Optional[torch.device] = None) -> None:
     the last check.  The operators themselves never synchronise; call this where the results are
     about to be consumed on the host, or set B200Q_CHECK_STATUS=1 to have every operator call do
     it before it returns (debugging: it serialises host and device)."""
-    for (dev_index, stream_ptr, op), ws in list(_workspaces._bufs.items()):
+    for (dev_index, stream_ptr, op), ws in _workspaces.all():
         if device is not None and torch.device(device).index not in (None, dev_index):
             continue
         read_workspace_status(ws, stream_ptr, op)
