@@ -50,3 +50,33 @@ def test_graph_replay_after_the_workspace_has_grown():
     st.synchronize()
     assert torch.allclose(y.float(), ref.float(), rtol=1e-2, atol=1e-2 * float(ref.float().abs().max()))
     assert all(int((o != 0x55).sum()) == 0 for o in others)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("transpose", (True, False))
+def test_first_tensor_core_call_of_a_thread_inside_a_capture(transpose):
+    import threading
+
+    M, N, K = 64, 256, 256
+    G = torch.Generator(device="cuda").manual_seed(1)
+    w = mb.quantize(torch.randn(N, K, generator=G, device="cuda", dtype=torch.bfloat16) * 0.02)
+    x = torch.randn(M, N if not transpose else K, generator=G, device="cuda", dtype=torch.bfloat16)
+    ref = mb.quantized_matmul(x, *w, transpose=transpose)
+    torch.cuda.synchronize()
+    out, errors = [], []
+
+    def capture():
+        try:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                out.append(mb.quantized_matmul(x, *w, transpose=transpose))
+            graph.replay()
+            torch.cuda.synchronize()
+        except Exception as e:   # noqa: BLE001
+            errors.append(e)
+
+    t = threading.Thread(target=capture)
+    t.start()
+    t.join()
+    assert not errors, errors
+    assert torch.equal(out[0], ref)
