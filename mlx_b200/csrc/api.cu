@@ -34,6 +34,20 @@ int fail(int code, const char* fmt, ...) {
 
 void count_launch(int n) { g_launches += (uint64_t)n; }
 
+// cuTensorMapEncodeTiled is a driver call and needs a current context, which a thread that has not yet
+// made a runtime call that touches the device (an autograd worker) does not have.  cudaSetDevice makes one current; unlike
+// cudaFree(nullptr), the customary way, it may also be called while the thread's stream is being captured.
+int bind_context() {
+  static thread_local bool bound = false;
+  if (!bound) {
+    int dev = 0;
+    B200Q_CUDA_OK(cudaGetDevice(&dev));
+    B200Q_CUDA_OK(cudaSetDevice(dev));
+  }
+  bound = true;
+  return B200Q_OK;
+}
+
 namespace {
 
 enum class Path { QmvRows, Qmv, Tc, Qvm, Generic };

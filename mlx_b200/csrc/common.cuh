@@ -18,6 +18,8 @@ namespace b200q {
 // Records a formatted message in the calling thread's error slot and returns `code`.
 int fail(int code, const char* fmt, ...);
 void count_launch(int n = 1);
+// Makes the device's context current for the calling thread; to be called before cuTensorMapEncodeTiled.
+int bind_context();
 
 #define B200Q_CUDA_OK(expr)                                                          \
   do {                                                                               \

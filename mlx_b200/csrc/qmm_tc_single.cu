@@ -716,6 +716,7 @@ int launch(int grid, size_t smem, cudaStream_t st, const CUtensorMap& map_x, con
 int qmm_single(const QmmArgs& a, cudaStream_t st) {
   EncodeFn enc = encode_fn();
   if (!enc) return fail(B200Q_ERR_CUDA, "[quantized_matmul] cuTensorMapEncodeTiled is not available");
+  if (int rc = bind_context()) return rc;
   if (!a.ws || a.ws_bytes < kStatusBytes)
     return fail(B200Q_ERR_WORKSPACE, "[quantized_matmul] workspace of %zu bytes required, %zu given",
                 (size_t)kStatusBytes, a.ws_bytes);
@@ -770,6 +771,7 @@ int qmm_single(const QmmArgs& a, cudaStream_t st) {
 int qmm_single_grouped(const GroupedArgs& a, cudaStream_t st) {
   EncodeFn enc = encode_fn();
   if (!enc) return fail(B200Q_ERR_CUDA, "[gather_qmm] cuTensorMapEncodeTiled is not available");
+  if (int rc = bind_context()) return rc;
   const int nt = a.nt;
   CUtensorMap map_x, map_w;
   {

@@ -933,6 +933,7 @@ int encode_rows(int nch, int64_t rows, int64_t K, const void* wq, const void* sc
                 CUtensorMap* map_s, CUtensorMap* map_b) {
   EncodeFn enc = rows_encode_fn();
   if (!enc) return fail(B200Q_ERR_CUDA, "[quantized_matmul] cuTensorMapEncodeTiled is not available");
+  if (int rc = bind_context()) return rc;
   {
     // packed rows as (128 bytes, row, 128-byte chunk of the row)
     const cuuint64_t row_bytes = (cuuint64_t)K * BITS / 8;

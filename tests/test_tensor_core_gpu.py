@@ -143,3 +143,28 @@ def test_autograd_worker_thread():
     ref = O.qmm_f32_from(dy, wq, s, b, "bf16", transpose=False, group_size=64, bits=4)
     ok, err = qmm_close(O.to_f32(from_torch(dx), "bf16"), ref)
     assert ok, err
+
+
+@pytest.mark.parametrize("M,bits,dtype,transpose", [(8, 4, "bf16", False), (8, 8, "f16", False), (64, 8, "bf16", False), (64, 4, "f16", True)])
+def test_every_kernel_as_the_first_call_of_an_autograd_worker(M, bits, dtype, transpose):
+    """A process of its own, so that nothing has used its worker thread before; the backward product is the row-owning
+    kernel, the one for 8-bit weights, or the one for pairs of blocks."""
+    import os
+    import subprocess
+    import sys
+
+    code = f"""
+import torch, mlx_b200 as mb
+from mlx_b200 import grad
+G = torch.Generator(device="cuda").manual_seed(1)
+dt = {DT[dtype]}
+w = mb.quantize(torch.randn(1024, 2048, generator=G, device="cuda", dtype=dt) * 0.02, 64, {bits})
+x = torch.randn({M}, {2048 if transpose else 1024}, generator=G, device="cuda", dtype=dt, requires_grad=True)
+dy = torch.randn({M}, {1024 if transpose else 2048}, generator=G, device="cuda", dtype=dt)
+dx, = torch.autograd.grad(grad.quantized_matmul(x, *w, {transpose}, 64, {bits}), x, dy)
+assert torch.equal(dx, mb.quantized_matmul(dy, *w, {not transpose}, 64, {bits}))
+print("worker-ok")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    res = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0 and "worker-ok" in res.stdout, res.stdout + res.stderr
