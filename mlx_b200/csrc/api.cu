@@ -369,7 +369,7 @@ int sharded_impl(const void* x, const uint32_t* wq, const void* scales, const vo
     if (int rc = qmv_mma(a, st)) return rc;
     return signal_only();
   }
-  if (a.K > 0 && qmm_tc_supported(a)) {
+  if (a.dtype == B200Q_BF16 && a.K > 0 && qmm_tc_supported(a)) {
     // Large results over more than four ranks: the product stores its block locally, a copy kernel
     // moves it to the other ranks with 16-byte accesses and signals (see peer_push_kernel).
     const int pm = push_mode();

@@ -105,6 +105,15 @@ def test_scales_need_no_alignment_for_the_tensor_cores(scales):
     assert lib.b200q_qmm(d, d, s, s, d, _lib.BF16, 1, 64, 256, 256, 64, 4, 1, 0, None, 0, None) == _lib.ERR_WORKSPACE
 
 
+@pytest.mark.parametrize("M", (4, 64))
+def test_sharded_takes_bfloat16_only(M):
+    lib = _lib.load()
+    d, one = ctypes.c_void_p(4096), (ctypes.c_void_p * 1)(4096)
+    for dtype in (_lib.F16, _lib.F32):
+        rc = lib.b200q_qmm_sharded(d, d, d, d, one, 1, 256, 0, dtype, M, 256, 256, 64, 4, None, 0, None)
+        assert rc == _lib.ERR_UNSUPPORTED and "only bfloat16" in _lib.last_error()
+
+
 def test_gather_sharded_rejects_on_host():
     lib = _lib.load()
     dummy = ctypes.c_void_p(4096)
