@@ -504,6 +504,8 @@ int swiglu_impl(const void* x, const uint32_t* wq_gate, const void* scales_gate,
     return fail(B200Q_ERR_INVALID_ARGUMENT, "[gather_qmm_swiglu] negative dimension.");
   if (K1 % group_size != 0 || (K1 * bits) % 32 != 0 || H % group_size != 0 || (H * bits) % 32 != 0)
     return fail(B200Q_ERR_INVALID_ARGUMENT, "[gather_qmm_swiglu] The shapes of the weight and scales are incompatible based on bits and group_size");
+  if (x_batch > UINT32_MAX || M > INT32_MAX || H > INT32_MAX || K1 > INT32_MAX || N2 > INT32_MAX)
+    return fail(B200Q_ERR_UNSUPPORTED, "[gather_qmm_swiglu] No implementation for problem shape: dimension too large.");
   if (n_idx == 0 || M == 0 || N2 == 0) return B200Q_OK;
   if (!x || !wq_gate || !scales_gate || !biases_gate || !wq_up || !scales_up || !biases_up || !wq_down || !scales_down ||
       !biases_down || !y || (pairs.simple && (!pairs.lhs.data || !pairs.rhs.data)))
@@ -610,6 +612,10 @@ extern "C" int b200q_gather_qmm_indexed(const void* x, const uint32_t* wq, const
     return fail(B200Q_ERR_INVALID_ARGUMENT, "[gather_qmm] bad index view");
   if (!valid_group(group_size) || !valid_bits(bits) || K % group_size != 0)
     return fail(B200Q_ERR_INVALID_ARGUMENT, "[gather_qmm] unsupported group size %d, bits %d or K", group_size, bits);
+  if (x_batch < 0 || E < 0 || M < 0 || N < 0 || K < 0)
+    return fail(B200Q_ERR_INVALID_ARGUMENT, "[gather_qmm] negative dimension.");
+  if (x_batch > UINT32_MAX || E > UINT32_MAX || M > INT32_MAX || N > INT32_MAX || K > INT32_MAX)
+    return fail(B200Q_ERR_UNSUPPORTED, "[gather_qmm] No implementation for problem shape: dimension too large.");
   if (n_idx == 0 || M == 0 || N == 0) return B200Q_OK;
   const bool aligned = !((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wq) |
                           reinterpret_cast<uintptr_t>(ws) | reinterpret_cast<uintptr_t>(y)) & 15);

@@ -126,6 +126,35 @@ def test_gather_sharded_rejects_on_host():
     assert call(2, 0, 0, 4, K=96) == _lib.ERR_INVALID_ARGUMENT  # K not a multiple of the group
 
 
+class Index(ctypes.Structure):
+    _fields_ = [("data", ctypes.c_void_p), ("elem_bytes", ctypes.c_int), ("stride", ctypes.c_int64 * 4)]
+
+
+def test_index_views_reject_on_host():
+    """The dimension checks of the plain entry, before any CUDA call."""
+    lib, d = _lib.load(), ctypes.c_void_p(4096)
+    idx = Index(4096, 8, (ctypes.c_int64 * 4)(0, 0, 0, 1))
+
+    def call(shape=(1, 1, 1, 8), elem=8, **kw):
+        idx.elem_bytes = elem
+        a = dict(x_batch=8, E=4, M=1, N=128, K=256, group=64, bits=4, ws=1 << 24)
+        a.update(kw)
+        return lib.b200q_gather_qmm_indexed(d, d, d, d, ctypes.byref(idx), ctypes.byref(idx), (ctypes.c_int64 * 4)(*shape), d, _lib.BF16,
+                                            a["x_batch"], a["E"], a["M"], a["N"], a["K"], a["group"], a["bits"], d, a["ws"], None)
+
+    assert call(elem=2) == _lib.ERR_INVALID_ARGUMENT
+    assert call(shape=(1, 1, -1, 8)) == _lib.ERR_INVALID_ARGUMENT
+    assert call(group=48) == _lib.ERR_INVALID_ARGUMENT
+    assert call(bits=7) == _lib.ERR_INVALID_ARGUMENT
+    for kw in (dict(x_batch=-1), dict(E=-4), dict(M=-1), dict(N=-128), dict(K=-256)):
+        assert call(**kw) == _lib.ERR_INVALID_ARGUMENT, kw
+    assert call(x_batch=1 << 33) == _lib.ERR_UNSUPPORTED
+    assert call(K=1 << 33) == _lib.ERR_UNSUPPORTED
+    assert call(K=96, group=32) == _lib.ERR_UNSUPPORTED      # the sort-by-expert path wants multiples of 128
+    assert call(ws=256) == _lib.ERR_WORKSPACE
+    assert call(shape=(1, 1, 0, 8)) == 0
+
+
 def test_embedding_and_gated_mlp_reject_on_host():
     lib = _lib.load()
     d = ctypes.c_void_p(4096)
