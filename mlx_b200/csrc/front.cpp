@@ -12,6 +12,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 #include <cstring>
 #include <vector>
@@ -59,8 +60,11 @@ const Tensor* tensor(PyObject* o) {
 bool integer(PyObject* o, int dflt, int* out) {
   if (o == Py_None) { *out = dflt; return true; }
   if (!PyLong_CheckExact(o)) return false;
-  *out = (int)PyLong_AsLong(o);
-  return !PyErr_Occurred();
+  int overflow = 0;
+  const long v = PyLong_AsLongAndOverflow(o, &overflow);
+  if (overflow != 0 || v < INT_MIN || v > INT_MAX) return false;   // the Python form says what is wrong with it
+  *out = (int)v;
+  return true;
 }
 bool affine(PyObject* o) { return PyUnicode_Check(o) && PyUnicode_CompareWithASCIIString(o, "affine") == 0; }
 

@@ -48,6 +48,21 @@ def test_quantized_matmul_errors():
         mb.quantized_matmul(torch.zeros(2, 9), w, s, b, transpose=False)
 
 
+@pytest.mark.parametrize("big", (2**32 + 64, 2**70, -2**70))
+def test_parameters_beyond_an_int(big):
+    x, w, s = torch.zeros(2, 256, dtype=torch.bfloat16), u32(8, 32), torch.zeros(8, 4, dtype=torch.bfloat16)
+    idx, w3, s3 = torch.zeros(2, dtype=torch.int64), u32(2, 8, 32), torch.zeros(2, 8, 4, dtype=torch.bfloat16)
+    for kw in (dict(group_size=big), dict(bits=big)):
+        with pytest.raises(ValueError):
+            mb.quantize(x, **kw)
+        with pytest.raises(ValueError):
+            mb.quantized_matmul(x, w, s, s, **kw)
+        with pytest.raises(ValueError):
+            mb.gather_qmm(x[:, None], w3, s3, s3, rhs_indices=idx, **kw)
+        with pytest.raises(ValueError):
+            mb.dequantize(w, s, s, **kw)
+
+
 def test_dequantize_errors():
     w, s, b = u32(8, 32), torch.zeros(8, 4), torch.zeros(8, 4)
     with pytest.raises(ValueError):
