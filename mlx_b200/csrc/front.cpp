@@ -218,6 +218,8 @@ PyObject* py_qmm_grad(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Tensor y;
   if (!qmm_args(a, n, t, &transpose, &group, &bits)) return none();
   if (t[2]->requires_grad() || t[3]->requires_grad()) return none();
+  for (const Tensor* u : t)   // forward-mode differentiation: the Python form's autograd.Function says that it has none
+    if (u->_fw_grad(0).defined()) return none();
   {
     at::AutoDispatchBelowAutograd below;
     if (!qmm_run(*t[0], *t[1], *t[2], *t[3], transpose, group, bits, &y)) return none();

@@ -91,3 +91,15 @@ def test_gather_qmm_vjp_matches_dense_autograd(transpose):
     for got, ref in ((ds, rs), (db, rb)):
         assert got.shape == ref.shape and float((got.double() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
     assert not ds[2].any() and not db[2].any()       # an expert no pair names gets no gradient
+
+
+@pytest.mark.parametrize("requires_grad", (False, True))
+def test_forward_mode_is_refused(requires_grad):
+    """A tangent is never dropped silently (grad.jvp is the form that takes one)."""
+    import torch.autograd.forward_ad as fwd
+
+    w = mb.quantize(torch.randn(256, 256, device="cuda", dtype=torch.bfloat16))
+    x = torch.randn(4, 256, device="cuda", dtype=torch.bfloat16, requires_grad=requires_grad)
+    grad.quantized_matmul(x, *w)   # (the scratch buffer is there: the native form takes ordinary calls)
+    with fwd.dual_level(), pytest.raises(RuntimeError):
+        grad.quantized_matmul(fwd.make_dual(x, torch.ones_like(x)), *w)
