@@ -156,6 +156,8 @@ quantize_kernel(const T* __restrict__ w, uint32_t* __restrict__ wq, T* __restric
     const float l = __shfl_sync(0xffffffffu, lo[k], src), h = __shfl_sync(0xffffffffu, hi[k], src);
     if (lane / Q::kPerIter == k) { w_min = l; w_max = h; }
   }
+  // The reference's comparisons pass over NaN and start from (inf, -inf); a minimum is NaN only where all of the group is.
+  if (w_min != w_min) { w_min = INFINITY; w_max = -INFINITY; }
   constexpr float n_bins = (float)((1 << BITS) - 1);
   const float eps = 1e-7f;
   const bool mask = fabsf(w_min) > fabsf(w_max);

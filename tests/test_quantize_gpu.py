@@ -62,6 +62,36 @@ def test_quantize_bit_exact_vs_oracle(dtype, g, bits):
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("g", GROUPS)
 @pytest.mark.parametrize("bits", BITS)
+def test_quantize_groups_with_nan(dtype, g, bits):
+    """The reference's minimum and maximum are comparisons: they pass over NaN and start from (inf, -inf).  A NaN among
+    numbers leaves scale and bias as they are without it; a group of nothing but NaN has bias -inf; fields of NaN are 0."""
+    rng = np.random.default_rng(g + bits)
+    w = (0.02 * rng.standard_normal((12, 4 * g))).astype(np.float32)
+    clean = w.copy()
+    w[1, :g] = np.nan
+    w[2, g:2 * g] = np.nan
+    for r in range(3, 12):   # some of a group, in odd and even places
+        at = rng.choice(g, size=1 + 5 * (r - 3) % (g - 2), replace=False)
+        clean[r, at] = clean[r, (set(range(g)) - set(at)).pop()]
+        w[r, at] = np.nan
+    got = [from_torch(t) for t in mb.quantize(to_torch(O.to_dtype(w, dtype), dtype), g, bits)]
+    ref = O.quantize(O.to_dtype(clean, dtype), g, bits, dtype)
+    s, b = O.to_f32(got[1], dtype), O.to_f32(got[2], dtype)
+    alone = [(1, 0), (2, 1)]
+    for r, k in alone:
+        assert np.isnan(s[r, k]) and b[r, k] == -np.inf
+        words = g * bits // 32
+        assert not got[0][r, k * words:(k + 1) * words].any()
+        s[r, k], b[r, k] = O.to_f32(ref[1], dtype)[r, k], O.to_f32(ref[2], dtype)[r, k]
+    assert np.array_equal(s, O.to_f32(ref[1], dtype)) and np.array_equal(b, O.to_f32(ref[2], dtype))
+    q = lambda x: np.unpackbits(np.ascontiguousarray(x).view(np.uint8), axis=-1, bitorder="little").reshape(12, 4 * g, bits)
+    assert np.array_equal(q(got[0]).any(-1) & ~np.isnan(w), q(ref[0]).any(-1) & ~np.isnan(w))
+    assert not q(got[0])[np.isnan(w)].any()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("g", GROUPS)
+@pytest.mark.parametrize("bits", BITS)
 def test_dequantize_bit_exact_vs_oracle(dtype, g, bits):
     rng = np.random.default_rng(2000 + g + bits)
     w = O.to_dtype(edge_matrix(rng, 33, 1024, g), dtype)
