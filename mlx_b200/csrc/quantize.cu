@@ -44,9 +44,13 @@ __device__ __forceinline__ void store8(T* __restrict__ p, const float (&v)[8]) {
 // constant.  About 12 instructions per value, none on the quarter-rate conversion unit (which rint and
 // the float-to-int conversion used).
 // 28672 x 8192 bf16, groups of 64 (device time): to 4 bits 321 -> 136 us (4.4 TB/s), to 8 bits 401 -> 152; f32 99.
-template <int GROUP>
+// Up to 2^22 values a warp takes one row: there the blocks are few and it is one warp's chain that takes the time (four
+// rows / one, us: 256 x 1024 bf16 to 4 bits 3.7 / 2.5, f32 to 8 bits 4.3 / 2.6; 1024 x 1024 3.9 / 3.0; 2048 x 2048 6.2 /
+// 6.0; 4096 x 4096 13.5 / 16.3).  Groups of 32 have two rows per warp and keep them (64 x 1024 2.5 / 2.4, 2048 x 2048 5.1 / 5.6).
+constexpr int64_t kSmall = 1 << 22;
+template <int GROUP, bool SMALL>
 struct QuantShape {
-  static constexpr int kIter = GROUP == 32 ? 2 : 4;         // 512-value rows per warp: at most one group per lane
+  static constexpr int kIter = GROUP == 32 ? 2 : (SMALL ? 1 : 4);   // 512-value rows per warp: at most one group per lane
   static constexpr int kLanes = GROUP / 16;                 // lanes per group
   static constexpr int kPerIter = 512 / GROUP;              // groups per row
 };
@@ -117,11 +121,11 @@ __device__ __forceinline__ void minmax16(const Pack16<T>& d, float& lo, float& h
   }
 }
 
-template <typename T, int BITS, int GROUP>
+template <typename T, int BITS, int GROUP, bool SMALL>
 __global__ void __launch_bounds__(256)
 quantize_kernel(const T* __restrict__ w, uint32_t* __restrict__ wq, T* __restrict__ scales,
                 T* __restrict__ biases, int64_t n) {
-  using Q = QuantShape<GROUP>;
+  using Q = QuantShape<GROUP, SMALL>;
   constexpr int IT = Q::kIter;
   const int lane = threadIdx.x & 31;
   const int64_t base = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * (IT * 512);
@@ -334,20 +338,22 @@ __device__ __forceinline__ void store_chunk(T* __restrict__ dst, uint2 bits, T s
   }
 }
 
-// Chunks of 8 values per thread, a block apart: enough loads in flight for HBM.  28672 x 8192 bf16, groups of 64: from
-// 4 bits 134 -> 99 us (6.1 TB/s), from 3 bits 138 -> 111.
+// CHUNKS chunks of 8 values per thread, a block apart: four keep enough loads in flight for HBM.  28672 x 8192 bf16,
+// groups of 64: from 4 bits 134 -> 99 us (6.1 TB/s), from 3 bits 138 -> 111.  One up to 2^22 values (f32: 2^23), where one
+// thread's chain takes the time (four / one, us: 256 x 1024 f16 from 3 bits 2.2 / 1.5, f32 3.0 / 1.8; 2048 x 2048 4.0 / 3.2;
+// 2048 x 4096 f16 5.7 / 5.5, from 4 bits 5.0 / 5.6, f32 12.7 / 11.6).
 constexpr int kDequantChunks = 4;
 
-template <typename T, int BITS>
+template <typename T, int BITS, int CHUNKS>
 __global__ void __launch_bounds__(256)
 dequantize_kernel(const uint32_t* __restrict__ wq, const T* __restrict__ scales,
                   const T* __restrict__ biases, T* __restrict__ out, int64_t n_chunks,
                   int group_shift /* log2(group/8) */, int64_t n_words) {
-  const int64_t c0 = (int64_t)blockIdx.x * (256 * kDequantChunks) + threadIdx.x;
-  uint2 bits[kDequantChunks];
-  T s[kDequantChunks], b[kDequantChunks];
+  const int64_t c0 = (int64_t)blockIdx.x * (256 * CHUNKS) + threadIdx.x;
+  uint2 bits[CHUNKS];
+  T s[CHUNKS], b[CHUNKS];
 #pragma unroll
-  for (int i = 0; i < kDequantChunks; ++i) {
+  for (int i = 0; i < CHUNKS; ++i) {
     const int64_t c = c0 + 256 * i;
     if (c < n_chunks) {
       bits[i] = chunk_bits<BITS>(wq, c, n_words);
@@ -356,7 +362,7 @@ dequantize_kernel(const uint32_t* __restrict__ wq, const T* __restrict__ scales,
     }
   }
 #pragma unroll
-  for (int i = 0; i < kDequantChunks; ++i) {
+  for (int i = 0; i < CHUNKS; ++i) {
     const int64_t c = c0 + 256 * i;
     if (c < n_chunks) store_chunk<T, BITS>(out + c * 8, bits[i], s[i], b[i]);
   }
@@ -368,14 +374,18 @@ int launch_quantize(const T* w, int64_t n_elems, int group, int bits, uint32_t* 
   if (n_elems == 0) return B200Q_OK;
   bool done = false;
   B200Q_DISPATCH_BITS(bits, BITS, {
-    auto go = [&](auto gtag) {
+    auto go = [&](auto gtag, auto small) {
       constexpr int G = decltype(gtag)::value;
-      constexpr int64_t per_block = 8 * QuantShape<G>::kIter * 512;
-      quantize_kernel<T, BITS, G><<<(unsigned)((n_elems + per_block - 1) / per_block), 256, 0, st>>>(w, wq, s, b, n_elems);
+      constexpr int64_t per_block = 8 * QuantShape<G, small>::kIter * 512;
+      quantize_kernel<T, BITS, G, small><<<(unsigned)((n_elems + per_block - 1) / per_block), 256, 0, st>>>(w, wq, s, b, n_elems);
     };
-    if (group == 32) go(std::integral_constant<int, 32>{});
-    else if (group == 64) go(std::integral_constant<int, 64>{});
-    else go(std::integral_constant<int, 128>{});
+    auto pick = [&](auto small) {
+      if (group == 64) go(std::integral_constant<int, 64>{}, small);
+      else go(std::integral_constant<int, 128>{}, small);
+    };
+    if (group == 32) go(std::integral_constant<int, 32>{}, std::false_type{});
+    else if (n_elems <= kSmall) pick(std::true_type{});
+    else pick(std::false_type{});
     done = true;
   });
   if (!done) return fail(B200Q_ERR_INVALID_ARGUMENT, "[quantize] unsupported bits %d", bits);
@@ -388,12 +398,15 @@ int launch_dequantize(const uint32_t* wq, const T* s, const T* b, int64_t n_elem
                       int bits, T* out, cudaStream_t st) {
   const int64_t n_chunks = n_elems / 8;
   if (n_chunks == 0) return B200Q_OK;
-  const unsigned grid = (unsigned)((n_chunks + 256 * kDequantChunks - 1) / (256 * kDequantChunks));
+  const bool small = n_elems <= (sizeof(T) == 4 ? 2 : 1) * kSmall;
+  const int64_t per_block = 256 * (small ? 1 : kDequantChunks);
+  const unsigned grid = (unsigned)((n_chunks + per_block - 1) / per_block);
   const int gshift = group == 32 ? 2 : (group == 64 ? 3 : 4);
   const int64_t n_words = n_elems * bits / 32;
   bool done = false;
   B200Q_DISPATCH_BITS(bits, BITS, {
-    dequantize_kernel<T, BITS><<<grid, 256, 0, st>>>(wq, s, b, out, n_chunks, gshift, n_words);
+    if (small) dequantize_kernel<T, BITS, 1><<<grid, 256, 0, st>>>(wq, s, b, out, n_chunks, gshift, n_words);
+    else dequantize_kernel<T, BITS, kDequantChunks><<<grid, 256, 0, st>>>(wq, s, b, out, n_chunks, gshift, n_words);
     done = true;
   });
   if (!done) return fail(B200Q_ERR_INVALID_ARGUMENT, "[dequantize] unsupported bits %d", bits);

@@ -157,6 +157,22 @@ def test_quantize_rounding_ties_and_extremes(dtype, g, bits):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("g,bits", [(32, 3), (64, 4), (128, 6), (64, 8), (32, 2), (128, 5)])
+@pytest.mark.parametrize("rows", (2048, 2049))
+def test_both_forms_at_their_border(dtype, g, bits, rows):
+    """Matrices of up to 2^22 values and larger ones are cut differently; ties among the values, the last block ragged."""
+    K = 2048
+    rng = np.random.default_rng(rows + bits)
+    w = (0.02 * rng.standard_normal((rows, K))).astype(np.float32)
+    w[::3] = rng.integers(0, 2 * (1 << bits) - 1, size=w[::3].shape) * 0.5
+    wd = O.to_dtype(w, dtype)
+    ref, got = O.quantize(wd, g, bits, dtype), mb.quantize(to_torch(wd, dtype), g, bits)
+    for r, t in zip(ref, got):
+        assert same(r, from_torch(t))
+    assert same(O.dequantize(*ref, g, bits, dtype), from_torch(mb.dequantize(*got, g, bits)))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("g,bits", [(32, 3), (64, 4), (128, 6), (64, 8), (32, 2), (128, 5)])
 def test_quantized_embedding_bit_exact_vs_oracle(dtype, g, bits):
     """QuantizedEmbedding look-up (python/mlx/nn/layers/quantized.py:149-158) = the oracle's
     dequantize of the indexed rows; negative ids count from the end, out-of-range ids give zeros."""
