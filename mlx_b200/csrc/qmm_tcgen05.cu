@@ -138,6 +138,7 @@ struct TcParams {
   void* y_out[kMaxPeers];
   int n_out;
   long long ld, col0;
+  int y_align;       // bytes that the start of every row of every output is a multiple of: 16, 8 or 2
   PeerSignal sig;    // completion signal towards the ranks that receive y (n == 0: none)
   uint32_t* status;
   int M, N, K;
@@ -448,7 +449,31 @@ __device__ __forceinline__ void stage_piece(uint32_t stg, int lane, const uint32
     stmatrix_x4_trans(at + i * 512, pack_pair<T>(r[4 * i], r[4 * i + 1]), pack_pair<T>(r[4 * i + 2], r[4 * i + 3]),
                       pack_pair<T>(r[8 + 4 * i], r[8 + 4 * i + 1]), pack_pair<T>(r[8 + 4 * i + 2], r[8 + 4 * i + 3]));
 }
+// 32 tokens straight from the accumulator, for rows of y off 8-byte boundaries (an output head of any size): a lane has a
+// column, and the warp stores 64 contiguous bytes per token.  Through the staging tile such rows went out as eight 2-byte
+// stores per lane, each instruction in 32 places (4 bits, us: 700
+// tokens through [32001, 4096] 201 -> 150, 2048 through [14301, 2048] 167 -> 117).
 template <typename T>
+__device__ __forceinline__ void store_columns(const TcParams& p, const Unit& t, const uint32_t (&v)[32], int n, int c, int lim) {
+  if (n >= p.N) return;
+  for (int q = 0; q < p.n_out; ++q) {
+    T* y = static_cast<T*>(p.y_out[q]) + p.col0 + n;
+    if (p.dst_row == nullptr) {
+      y += (long long)(t.x_row0 + c) * p.ld;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        if (j < lim) *y = Elem<T>::from_float(__uint_as_float(v[j]));
+        y += p.ld;
+      }
+    } else {
+      const int* row = p.dst_row + t.x_row0 + c;
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < lim) y[(long long)row[j] * p.ld] = Elem<T>::from_float(__uint_as_float(v[j]));
+    }
+  }
+}
+template <typename T, bool ROWS16>
 __device__ __forceinline__ void store_chunk(const TcParams& p, const Unit& t, uint32_t stg, int lane, int n0, int c, int lim) {
   const int n = n0 + (lane & 3) * 8;
   const bool whole = n + 8 <= p.N;
@@ -460,8 +485,11 @@ __device__ __forceinline__ void store_chunk(const TcParams& p, const Unit& t, ui
     const long long at = (long long)(p.dst_row ? p.dst_row[m] : m) * p.ld + p.col0 + n;
     for (int q = 0; q < p.n_out; ++q) {
       T* dst = static_cast<T*>(p.y_out[q]) + at;
-      if (whole && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+      if (ROWS16 && whole) {
         *reinterpret_cast<uint4*>(dst) = v;
+      } else if (whole) {
+        reinterpret_cast<uint2*>(dst)[0] = make_uint2(v.x, v.y);
+        reinterpret_cast<uint2*>(dst)[1] = make_uint2(v.z, v.w);
       } else {
         const T* e = reinterpret_cast<const T*>(&v);
         for (int j = 0; j < 8 && n + j < p.N; ++j) dst[j] = e[j];
@@ -470,7 +498,9 @@ __device__ __forceinline__ void store_chunk(const TcParams& p, const Unit& t, ui
   }
 }
 
-template <typename T, int BITS, Form F>
+// ROWS16: the rows of y start on 16-byte boundaries (an instantiation of its own: the registers of the other stores cost the
+// ordinary products 2 to 4 %).
+template <typename T, int BITS, Form F, bool ROWS16>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   using S = Shape<BITS, F>;
@@ -837,7 +867,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(leader_addr(smem_u32(&bars->acc_empty[ab])));
       };
-      if (t.parts == 1) {
+      if (t.parts == 1 && (ROWS16 || p.y_align == 8)) {
         uint32_t r[2][16];
         load_piece(acc + c_begin, r[0]);
         for (int c0 = c_begin; c0 < c_end; c0 += 64) {
@@ -852,7 +882,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
             }
           }
           __syncwarp();
-          store_chunk<T>(p, t, stg, lane, t.n0 + quad * 32, c0, min(min(t.rows, c_end) - c0, 64));
+          store_chunk<T, ROWS16>(p, t, stg, lane, t.n0 + quad * 32, c0, min(min(t.rows, c_end) - c0, 64));
           __syncwarp();   // the staging tile may be written again
         }
       } else {
@@ -863,6 +893,11 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           tcgen05_wait_ld();
           if (c + 32 >= c_end) release();
           const int lim = min(t.rows, c_end) - c;  // valid columns of this chunk
+          if (!ROWS16 && t.parts == 1) {
+            store_columns<T>(p, t, v, n, c, lim);
+            __syncwarp();   // the next load needs the whole warp
+            continue;
+          }
 #pragma unroll
           for (int j = 0; j < 32; ++j)
             if (j < lim) __stcg(part + (size_t)(c + j) * kTileRows, __uint_as_float(v[j]));
@@ -1066,7 +1101,7 @@ int encode_maps(TcMaps& m, const char* tag, const void* x, int64_t x_rows, int64
 
 // Once per kernel, device and thread.
 int allow_smem(const void* kernel) {
-  constexpr int kMost = 32;   // instantiations: 24
+  constexpr int kMost = 64;   // instantiations: 48
   static thread_local const void* done[64][kMost];
   static thread_local int count[64];
   int dev = 0;
@@ -1081,16 +1116,26 @@ int allow_smem(const void* kernel) {
 
 template <typename T, int BITS, Form F>
 int launch_one(unsigned grid, size_t smem, cudaStream_t st, const TcMaps& maps, const TcParams& p) {
-  if (int rc = allow_smem((const void*)qmm_tc_kernel<T, BITS, F>)) return rc;
   // A plain launch: programmatic stream serialization would hide about 2 us of set-up, but clusters launched that way
   // faulted (once in some hundred thousand launches here) for a reason that was not found.
-  qmm_tc_kernel<T, BITS, F><<<grid, kThreads, smem, st>>>(maps, p);
-  B200Q_LAUNCH_OK("qmm_tc_kernel");
-  return B200Q_OK;
+  auto go = [&](auto kernel) -> int {
+    if (int rc = allow_smem((const void*)kernel)) return rc;
+    kernel<<<grid, kThreads, smem, st>>>(maps, p);
+    B200Q_LAUNCH_OK("qmm_tc_kernel");
+    return B200Q_OK;
+  };
+  return p.y_align == 16 ? go(qmm_tc_kernel<T, BITS, F, true>) : go(qmm_tc_kernel<T, BITS, F, false>);
+}
+
+int row_alignment(const TcParams& p) {
+  uintptr_t at = (uintptr_t)p.ld * 2 | (uintptr_t)p.col0 * 2;
+  for (int q = 0; q < p.n_out; ++q) at |= reinterpret_cast<uintptr_t>(p.y_out[q]);
+  return (at & 15) == 0 ? 16 : ((at & 7) == 0 ? 8 : 2);
 }
 
 // Completes the parameters that depend on the shape of the kernel and launches it for `units` units of work.
 int launch_tc(int dtype, int bits, int group, Form f, long long units, cudaStream_t st, const TcMaps& maps, TcParams& p) {
+  p.y_align = row_alignment(p);
   p.g4 = kTileRows / group;
   p.spc = 1;
   if (f != Form::SplitT)

@@ -109,6 +109,31 @@ def test_scales_at_odd_addresses(bits, dtype, transpose, rel, M, N, K, g):
     assert ok, err
 
 
+@pytest.mark.parametrize("dtype", ("bf16", "f16"))
+@pytest.mark.parametrize("M,N", [(33, 129), (40, 132), (100, 250), (257, 517), (300, 34), (600, 9477)])
+def test_rows_of_y_off_16_byte_boundaries(dtype, M, N):
+    """Widths that are no multiple of 8 (an output head): columns stored one by one; nothing past the last one."""
+    import ctypes
+
+    from mlx_b200 import _lib
+
+    lib, P, K, g, bits = _lib.load(), lambda t: ctypes.c_void_p(t.data_ptr()), 384, 64, 4
+    wq, s, b = O.quantize(make_w(M, (N, K), dtype), g, bits, dtype)
+    x = make_x(N, (M, K), dtype)
+    ref = O.qmm_f32_from(x, wq, s, b, dtype, transpose=True, group_size=g, bits=bits)
+    xt, wt, st, bt = to_torch(x, dtype), u32_to_torch(wq), to_torch(s, dtype), to_torch(b, dtype)
+    dt = {"bf16": _lib.BF16, "f16": _lib.F16}[dtype]
+    ws = torch.zeros(lib.b200q_qmm_workspace_bytes(dt, 1, M, N, K, g, bits, 1), dtype=torch.uint8, device="cuda")
+    for before in (0, 1, 8):   # y itself at 16, 2 and 16 bytes past a boundary
+        flat = torch.full((before + M * N + 64,), 7.0, dtype=DT[dtype], device="cuda")
+        y = flat[before:before + M * N].view(M, N)
+        _lib.check(lib.b200q_qmm(P(xt), P(wt), P(st), P(bt), P(y), dt, 1, M, N, K, g, bits, 1, 0, P(ws), ws.numel(),
+                                 ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        ok, err = qmm_close(O.to_f32(from_torch(y), dtype), ref, 1e-2 if dtype == "bf16" else 2e-3)
+        assert ok, err
+        assert bool((flat[:before] == 7).all()) and bool((flat[before + M * N:] == 7).all())
+
+
 def test_workspace_off_a_16_byte_boundary():
     """A caller's workspace may lie anywhere a 4-byte word may; its tiles are then not shared between pairs of blocks."""
     import ctypes
