@@ -32,9 +32,13 @@
 // How W becomes the A operand (Form):
 //   Round   bf16, transpose: s*q+b rounded once to bf16 (one fma.rn.bf16x2 per pair), in tensor memory
 //   Split   f16, transpose: s*q+b in fp32, split into two f16 numbers hi + lo, two MMAs per k step: the
-//           product keeps the weights' fp32 value (to 2^-22), as the CUDA-core kernel did
+//           product keeps the weights' fp32 value (split32 says how closely), as the CUDA-core kernel did
 //   SplitT  no transpose, bf16 and f16: W is packed along the output columns, so A is written to shared
 //           memory M-major (hi and lo)
+// In two parts a weight beyond 65504 (f16), an infinite one and an infinite x give NaN where the weight itself gives a number
+// or an infinity.  Where the epilogue warps of a block of the split forms have stored a result that is not finite, they go over
+// the block's tiles once more at the end, when nobody waits for them any more, and compute such elements in fp32 from the weights
+// themselves (repair).
 //
 // Tiles are dealt to the pairs in whole waves; the K stages of the tiles that are left over are laid end to end and cut
 // into equal ranges, one per pair, so that the last wave is as short as its work (or, with few tiles, all SMs have
@@ -134,6 +138,8 @@ struct TcParams {
   const int* dst_row;       // output row of every activation row
   const unsigned short* scales;
   const unsigned short* biases;
+  const void* x;            // split forms, for `repair`: x and the packed weights
+  const uint32_t* wq;
   // output buffers (one, or one per GPU of an N-sharded layer), row pitch and first column
   void* y_out[kMaxPeers];
   int n_out;
@@ -170,6 +176,8 @@ struct __align__(8) Barriers {
   uint64_t acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   int abort_flag, last;
+  int odd;         // split forms: a result was not finite
+  uint32_t ended;  // pieces of cut tiles (by their number among this pair's) that this block has summed
   int landed[2];   // of a tile (even, odd): its accumulator is complete, as the epilogue warp that waits for it found
 };
 
@@ -225,7 +233,10 @@ __device__ __forceinline__ uint32_t field_raw(const uint32_t (&w)[BITS], int e) 
 }
 
 // s*q+b of 32 consecutive fields in fp32, split into hi + lo numbers of T (16 registers of pairs each, in
-// order).  bf16: hi is the value cut off after 8 bits, lo the rounded rest; f16: both rounded.
+// order).  bf16: hi is the value cut off after 8 bits, lo the rounded rest, 2^-17 of the value is lost; f16: both rounded, what
+// is lost is 2^-22 of the value from 1/8 up and at most 2^-25 below (against 64 bits the products' errors are those of
+// fp32 weights to three digits, for weights of 1e-4 to 1: the rounding of the result is far larger).  f16 numbers end at
+// 65504: a larger weight gives inf - inf, which the epilogue finds (repair).
 template <int BITS, typename T>
 __device__ __forceinline__ void split32(const uint32_t (&w)[BITS], float s, float b, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
   constexpr uint32_t mask = (1u << BITS) - 1u;
@@ -246,9 +257,9 @@ __device__ __forceinline__ void split32(const uint32_t (&w)[BITS], float s, floa
       const float l1 = v[1] - __uint_as_float(__float_as_uint(v[1]) & 0xFFFF0000u);
       asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo[j]) : "f"(l1), "f"(l0));
     } else {
-      asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(hi[j]) : "f"(v[1]), "f"(v[0]));
+      asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(hi[j]) : "f"(v[1]), "f"(v[0]));
       const float2 h2 = __half22float2(*reinterpret_cast<const __half2*>(&hi[j]));
-      asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(lo[j]) : "f"(v[1] - h2.y), "f"(v[0] - h2.x));
+      asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo[j]) : "f"(v[1] - h2.y), "f"(v[0] - h2.x));
     }
   }
 }
@@ -441,6 +452,12 @@ __device__ __forceinline__ void load_piece(uint32_t tmem, uint32_t (&r)[16]) {  
   tcgen05_ld_16x16(tmem, r);
   tcgen05_ld_16x16(tmem + (16u << 16), r + 8);
 }
+// Nonzero where one of a pair of numbers is not finite.
+template <typename T>
+__device__ __forceinline__ uint32_t odd_pair(uint32_t v) {
+  constexpr bool kBf = std::is_same<T, __nv_bfloat16>::value;
+  return ((v & (kBf ? 0x7F807F80u : 0x7C007C00u)) + (kBf ? 0x00800080u : 0x04000400u)) & 0x80008000u;   // an exponent of ones carries
+}
 template <typename T>
 __device__ __forceinline__ void stage_piece(uint32_t stg, int lane, const uint32_t (&r)[16]) {
   const uint32_t row = lane & 7, at = stg + row * 64 + ((((uint32_t)lane >> 3) ^ (row >> 1)) << 4);
@@ -453,9 +470,15 @@ __device__ __forceinline__ void stage_piece(uint32_t stg, int lane, const uint32
 // column, and the warp stores 64 contiguous bytes per token.  Through the staging tile such rows went out as eight 2-byte
 // stores per lane, each instruction in 32 places (4 bits, us: 700
 // tokens through [32001, 4096] 201 -> 150, 2048 through [14301, 2048] 167 -> 117).
-template <typename T>
-__device__ __forceinline__ void store_columns(const TcParams& p, const Unit& t, const uint32_t (&v)[32], int n, int c, int lim) {
-  if (n >= p.N) return;
+// Returns nonzero (WATCH) where a result is not finite, as store_chunk does.
+template <typename T, bool WATCH>
+__device__ __forceinline__ uint32_t store_columns(const TcParams& p, const Unit& t, const uint32_t (&v)[32], int n, int c, int lim) {
+  if (n >= p.N) return 0;
+  uint32_t odd = 0;
+  if constexpr (WATCH) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) odd |= odd_pair<T>(pack_pair<T>(j < lim ? v[j] : 0u, j + 1 < lim ? v[j + 1] : 0u));
+  }
   for (int q = 0; q < p.n_out; ++q) {
     T* y = static_cast<T*>(p.y_out[q]) + p.col0 + n;
     if (p.dst_row == nullptr) {
@@ -472,15 +495,18 @@ __device__ __forceinline__ void store_columns(const TcParams& p, const Unit& t, 
         if (j < lim) y[(long long)row[j] * p.ld] = Elem<T>::from_float(__uint_as_float(v[j]));
     }
   }
+  return odd;
 }
-template <typename T, bool ROWS16>
-__device__ __forceinline__ void store_chunk(const TcParams& p, const Unit& t, uint32_t stg, int lane, int n0, int c, int lim) {
+template <typename T, bool ROWS16, bool WATCH>
+__device__ __forceinline__ uint32_t store_chunk(const TcParams& p, const Unit& t, uint32_t stg, int lane, int n0, int c, int lim) {
   const int n = n0 + (lane & 3) * 8;
   const bool whole = n + 8 <= p.N;
-  if (n >= p.N) return;
+  uint32_t odd = 0;
+  if (n >= p.N) return odd;
   for (int tok = lane >> 2; tok < lim; tok += 8) {
     uint4 v;
     lds_v4(stg + tok * 64 + (((lane & 3) ^ ((tok >> 1) & 3)) << 4), v.x, v.y, v.z, v.w);
+    if constexpr (WATCH) odd |= odd_pair<T>(v.x) | odd_pair<T>(v.y) | odd_pair<T>(v.z) | odd_pair<T>(v.w);
     const int m = t.x_row0 + c + tok;
     const long long at = (long long)(p.dst_row ? p.dst_row[m] : m) * p.ld + p.col0 + n;
     for (int q = 0; q < p.n_out; ++q) {
@@ -496,6 +522,28 @@ __device__ __forceinline__ void store_chunk(const TcParams& p, const Unit& t, ui
       }
     }
   }
+  return odd;
+}
+
+// The elements of a tile that are not finite, from the weights themselves in fp32, by the epilogue warps.
+template <typename T, int BITS, bool TRANSPOSED>
+__device__ __forceinline__ void repair(const TcParams& p, int n0, int x_row0, int rows) {
+  const int64_t row_words = (TRANSPOSED ? (int64_t)p.K : (int64_t)p.N) * BITS / 32;
+  const int group = kTileRows / p.g4;
+  for (int i = threadIdx.x - 32 * kFirstEpilogue; i < rows * kTileRows; i += 32 * kEpilogueWarps) {
+    const int n = n0 + (i & (kTileRows - 1));
+    if (n >= p.N) continue;
+    const long long m = x_row0 + i / kTileRows;
+    T* y = static_cast<T*>(p.y_out[0]) + m * p.N + n;
+    if (fabsf(Elem<T>::to_float(*y)) < INFINITY) continue;
+    float sum = 0.0f;
+    for (int k = 0; k < p.K && sum == sum; ++k) {
+      const int64_t r = TRANSPOSED ? n : k, sc = r * p.row_groups + (TRANSPOSED ? k : n) / group;
+      const float w = fmaf((float)stream_get<BITS>(p.wq + r * row_words, TRANSPOSED ? k : n), bits_to_float<T>(p.scales[sc]), bits_to_float<T>(p.biases[sc]));
+      sum = fmaf(Elem<T>::to_float(static_cast<const T*>(p.x)[m * p.K + k]), w, sum);
+    }
+    *y = Elem<T>::from_float(sum);
+  }
 }
 
 // ROWS16: the rows of y start on 16-byte boundaries (an instantiation of its own: the registers of the other stores cost the
@@ -504,7 +552,7 @@ template <typename T, int BITS, Form F, bool ROWS16>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   using S = Shape<BITS, F>;
-  constexpr bool kT = S::kT;
+  constexpr bool kT = S::kT, kSplit = F != Form::Round;
   constexpr int kSub = S::kSub, kSlotsA = S::kSlotsA, kStagesP = S::kStagesP;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // carve-up: [A ring of SplitT] [B ring: nsb stages of two NT/2 * 128-byte sub-tiles] [P ring] [S ring] [barriers]
@@ -539,6 +587,8 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     for (int i = 0; i < kDoneRing; ++i) mbar_init(smem_u32(&bars->done[i]), 1);
     for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&bars->acc_full[i]), 1); mbar_init(smem_u32(&bars->acc_empty[i]), 2 * kEpilogueWarps); }
     bars->abort_flag = 0;
+    bars->odd = 0;
+    bars->ended = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -882,7 +932,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
             }
           }
           __syncwarp();
-          store_chunk<T, ROWS16>(p, t, stg, lane, t.n0 + quad * 32, c0, min(min(t.rows, c_end) - c0, 64));
+          if (store_chunk<T, ROWS16, kSplit>(p, t, stg, lane, t.n0 + quad * 32, c0, min(min(t.rows, c_end) - c0, 64))) bars->odd = 1;
           __syncwarp();   // the staging tile may be written again
         }
       } else {
@@ -894,7 +944,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           if (c + 32 >= c_end) release();
           const int lim = min(t.rows, c_end) - c;  // valid columns of this chunk
           if (!ROWS16 && t.parts == 1) {
-            store_columns<T>(p, t, v, n, c, lim);
+            if (store_columns<T, kSplit>(p, t, v, n, c, lim)) bars->odd = 1;
             __syncwarp();   // the next load needs the whole warp
             continue;
           }
@@ -916,6 +966,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         }
         asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueWarps * 32) : "memory");
         if (bars->last) {
+          if (kSplit && warp == kFirstEpilogue && lane == 0) bars->ended |= 1u << ((u - p.full) / pairs & 31);
           // A warp takes whole tokens, a lane four columns of each: 16-byte loads, two tokens of four parts at a time.
           __threadfence();
           const size_t pitch = 2 * (size_t)p.NT * kTileRows / 4;   // from one part to the next
@@ -944,6 +995,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
               for (int s = 0; s < t.parts; ++s) __stcg(q0 + (size_t)s * pitch + k * (kEpilogueWarps * kTileRows / 4), zero);
               const uint2 o = make_uint2(pack_pair<T>(__float_as_uint(sum[k].x), __float_as_uint(sum[k].y)),
                                          pack_pair<T>(__float_as_uint(sum[k].z), __float_as_uint(sum[k].w)));
+              if (kSplit && (odd_pair<T>(o.x) | odd_pair<T>(o.y)) != 0) bars->odd = 1;
               const long long at = (long long)(t.x_row0 + c + k * kEpilogueWarps) * p.ld + p.col0 + n4;
               for (int q = 0; q < p.n_out; ++q) {
                 T* dst = static_cast<T*>(p.y_out[q]) + at;
@@ -958,6 +1010,16 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           }
         }
         asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueWarps * 32) : "memory");   // `last` may be written again
+      }
+    }
+    if constexpr (kSplit) {
+      __syncwarp();
+      asm volatile("bar.sync 3, %0;" ::"n"(kEpilogueWarps * 32) : "memory");   // every result and every `odd` is there
+      if (bars->odd != 0) {
+        for (int u = pair; u < total; u += pairs) {
+          const Unit t = unit_at(p, u, rank);
+          if (t.parts == 1 || (bars->ended >> ((u - p.full) / pairs & 31) & 1)) repair<T, BITS, !kT>(p, t.n0, t.x_row0, t.rows);
+        }
       }
     }
   }
@@ -1212,6 +1274,8 @@ int qmm_tc(const QmmArgs& a, cudaStream_t st) {
   TcParams p{};
   p.scales = (const unsigned short*)a.scales;
   p.biases = (const unsigned short*)a.biases;
+  p.x = a.x;
+  p.wq = a.wq;
   set_outputs(p, a.peers, a.y, a.N);
   p.status = reinterpret_cast<uint32_t*>(static_cast<char*>(a.ws) + a.ws_bytes - kStatusBytes);
   p.M = (int)a.M; p.N = (int)a.N; p.K = (int)a.K;

@@ -4,6 +4,7 @@ split in two, packed along the output columns), against the oracle's fp32 accumu
 Sizes: one stage of 128 k and odd numbers of stages, token counts around 32, 128 and 256, output columns that
 end inside a block's or a pair's half of a tile, one scale per stage at an odd position of its 4-byte
 word, and few tiles with a long K (K shared by several pairs of thread blocks)."""
+import numpy as np
 import pytest
 import torch
 
@@ -153,6 +154,71 @@ def test_workspace_off_a_16_byte_boundary():
     ok, err = qmm_close(O.to_f32(from_torch(y), "bf16"), O.qmm_f32_from(x, wq, s, b, "bf16", transpose=True, group_size=g, bits=bits))
     assert ok, err
     assert int(ws.max()) == 0
+
+
+def dense(wq, s, b, g, bits, dtype):
+    """The weights in 64 bits."""
+    K = wq.shape[-1] * 32 // bits
+    stream = np.unpackbits(np.ascontiguousarray(wq).view(np.uint8), axis=-1, bitorder="little").reshape(wq.shape[0], K, bits)
+    q = (stream.astype(np.float64) * 2.0 ** np.arange(bits)).sum(-1)
+    wide = lambda t: np.repeat(O.to_f32(t, dtype).astype(np.float64), g, -1)
+    return q * wide(s) + wide(b)
+
+
+SPLIT = [("f16", True, 40, 257, 640, 64, 4), ("f16", True, 57, 512, 8192, 64, 4), ("f16", True, 300, 132, 512, 32, 3),
+         ("f16", False, 64, 256, 392, 64, 6), ("f16", False, 300, 384, 1032, 128, 4), ("bf16", False, 64, 256, 392, 64, 4)]
+
+
+@pytest.mark.parametrize("dtype,transpose,M,N,K,g,bits", SPLIT[:5])
+def test_weights_beyond_the_range_of_half(dtype, transpose, M, N, K, g, bits):
+    """Scales and biases are half precision, s*q+b need not be: some weights of a few rows lie between 65504 and 700000, x
+    is small enough for every result to be a half.  Whole tiles, tiles shared between pairs of blocks, columns stored one by one."""
+    rng = np.random.default_rng(M + K)
+    rows, cols = (N, K) if transpose else (K, N)
+    wq, s, b = O.quantize(make_w(M, (rows, cols), dtype), g, bits, dtype)
+    sf = O.to_f32(s, dtype).copy()
+    for r in rng.choice(rows, size=4, replace=False):
+        sf[r, rng.integers(sf.shape[1])] = rng.uniform(2e4, 4e4)
+    s = O.to_dtype(sf, dtype)
+    w = dense(wq, s, b, g, bits, dtype)
+    assert (np.abs(w) > 131008).any() and np.isfinite(w).all()
+    x = O.to_dtype((rng.standard_normal((M, K)) * 1e-4).astype(np.float32), dtype)
+    xf = O.to_f32(x, dtype).astype(np.float64)
+    ref = xf @ (w.T if transpose else w)
+    size = np.abs(xf) @ np.abs(w.T if transpose else w)
+    got = mb.quantized_matmul(to_torch(x, dtype), u32_to_torch(wq), to_torch(s, dtype), to_torch(b, dtype), transpose=transpose,
+                              group_size=g, bits=bits)
+    got = O.to_f32(from_torch(got), dtype).astype(np.float64)
+    # the result's rounding (2^-11 of it, 2^-25 where it is subnormal), and fp32 sums of K terms of that size in any order
+    assert (np.abs(got - ref) <= 2.0 ** -11 * np.abs(ref) + 2.0 ** -25 + K * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("dtype,transpose,M,N,K,g,bits", SPLIT)
+def test_activations_and_weights_that_are_not_finite(dtype, transpose, M, N, K, g, bits):
+    """One infinity in a row of x times a weight is an infinity of the sign of both; so is one infinite bias; NaN stays NaN.
+    The next call finds the workspace clear."""
+    rng = np.random.default_rng(M + N)
+    rows, cols = (N, K) if transpose else (K, N)
+    wq, s, b = O.quantize(make_w(N, (rows, cols), dtype), g, bits, dtype)
+    xf = rng.standard_normal((M, K)).astype(np.float32)
+    xf[1, 3], xf[2, K - 1], xf[5, 7] = np.inf, -np.inf, np.nan
+    bf = O.to_f32(b, dtype).copy()
+    bf[rows - 2, 0] = np.inf
+    x, b = O.to_dtype(xf, dtype), O.to_dtype(bf, dtype)
+    w = dense(wq, s, b, g, bits, dtype)
+    with np.errstate(invalid="ignore"):
+        ref = O.to_f32(x, dtype).astype(np.float64) @ (w.T if transpose else w)
+    odd = ~np.isfinite(ref)
+    assert odd.any() and not odd.all()
+    for _ in range(2):
+        got = mb.quantized_matmul(to_torch(x, dtype), u32_to_torch(wq), to_torch(s, dtype), to_torch(b, dtype), transpose=transpose,
+                                  group_size=g, bits=bits)
+        got = O.to_f32(from_torch(got), dtype)
+        assert np.array_equal(got[odd], ref[odd].astype(np.float32), equal_nan=True)
+        ok, err = qmm_close(got[~odd], ref[~odd], 6e-3 if dtype == "bf16" else 2e-3)
+        assert ok, err
+    from mlx_b200 import ops
+    assert int(ops._workspaces.get(torch.device("cuda", torch.cuda.current_device()), 0, "qmm").max()) == 0
 
 
 def test_autograd_worker_thread():
