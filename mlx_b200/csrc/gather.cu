@@ -197,10 +197,18 @@ bool fast_supported(int dtype, int64_t n_idx, int64_t x_batch, int64_t E, int64_
 }
 
 
-// Experts with few rows go through the row-owning decode kernel: it reads a matrix at 1.6 times the rate at which the
-// tensor-core kernel unpacks one (8 experts [14336, 4096] at 4 bits), takes the rows of x where they lie and needs no
-// second launch for a gated pair.  At more than about four rows per expert on average the tiles of 8 rows begin to
-// split experts, and every part reads the matrix again.
+// Experts with few rows go through the row-owning decode kernel: it does not round the weights (error against 64 bits 1.65e-3
+// of the result, tensor cores 2.2e-3), reads a matrix at up to 1.6 times the rate at which the tensor-core kernel unpacks
+// one, takes the rows of x where they lie and needs no second launch for a gated pair.  At more than about four rows per
+// expert the tiles of 8 rows begin to split experts, and every part reads the matrix again.  Measured (us, this kernel / tensor
+// cores, uniform routing):
+//   4 bits  16 experts [7168, 4096], 16 to 64 rows 56 to 76 / 77 to 101; 8 [14336, 4096], 32 rows 75 / 101;
+//           16 [2048, 2048], 16 and 64 rows 21 and 27 / 26 and 27; 32 [4096, 2048], 64 and 128 rows 63 and 77 / 56 and 63;
+//           64 [2048, 2048], 64 and 256 rows 51 and 75 / 48 and 63; 64 [1024, 1024], 256 rows 41 / 29
+//   2 bits  64 [2048, 2048], 64 and 256 rows 48 and 69 / 62 and 83
+//   8 bits  (the other side is qmm_tc_single.cu) 64 [2048, 2048], 256 rows 70 / 135
+// With short K the tensor cores would be up to 1.4 times as fast at 4 bits; the line stays for the weights' sake.  All rows on
+// one expert, which the host cannot see, is this kernel's worst case: 64 [2048, 2048], 256 rows 39 us, tensor cores 20 to 30.
 bool few_rows(int64_t n_rows, int64_t E) { return n_rows <= 4 * E; }
 
 RowsGroup rows_group(const FastLayout& L, char* base, int64_t E, int64_t M, int64_t N, int64_t K, int group, int bits, uint32_t* status) {

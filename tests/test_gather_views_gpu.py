@@ -119,3 +119,21 @@ def test_few_rows_gated(E, tokens, top, H, K, N2, bits):
         assert tuple(y.shape) == (tokens, top, 1, N2)
         ok, err = qmm_close(O.to_f32(from_torch(y), "bf16").reshape(ref.shape), ref)
         assert ok, err
+
+
+@pytest.mark.parametrize("bits,rows", [(2, 32), (4, 32), (4, 33), (8, 32), (8, 33)])
+@pytest.mark.parametrize("skew", (False, True))
+def test_both_sides_of_the_rule_for_few_rows(bits, rows, skew):
+    """8 experts: the last number of rows that takes the row-owning kernel and the first that does not; routing spread
+    evenly, and all rows on one expert."""
+    E, N, K, g = 8, 264, 1024, 64
+    wq, s, b = O.quantize(make_w(90, (E, N, K), "bf16"), g, bits, "bf16")
+    x = make_x(91, (rows, 1, K), "bf16")
+    rhs = np.full(rows, 5) if skew else np.arange(rows) * 3 % E
+    ref = O.gather_qmm(O.to_f32(x, "bf16"), wq, O.to_f32(s, "bf16"), O.to_f32(b, "bf16"), np.arange(rows, dtype=np.uint32),
+                       rhs.astype(np.uint32), True, g, bits, "f32")
+    for _ in range(2):
+        y = mb.gather_qmm(to_torch(x, "bf16"), u32_to_torch(wq), to_torch(s, "bf16"), to_torch(b, "bf16"),
+                          rhs_indices=torch.from_numpy(rhs).cuda(), group_size=g, bits=bits)
+        ok, err = qmm_close(O.to_f32(from_torch(y), "bf16").reshape(ref.shape), ref)
+        assert ok, err
