@@ -13,10 +13,10 @@
 // operand that has to be dequantised (W) is the 128-row A operand and is re-used by up
 // to 256 tokens per instruction, and the operand that streams unchanged (x) is B.
 //
-//   thread A: TMA  --packed W tile [128 rows x 128 k, 16*bits bytes per row]-->  smem ring P
+//   thread A: TMA  --packed W tile [128 rows x 128 k, 128 bytes per row]-->  smem ring P
 //   16 dequant warps (4 TMEM lane quadrants x 4 quarters of the 128-k stage): one thread per
-//        weight row (= one TMEM lane) unpacks 32 k, applies s*q+b in bf16x2 (4- and 8-bit:
-//        mask + one fma on the field read as a subnormal bf16; other widths shift/lop3/prmt),
+//        weight row (= one TMEM lane) unpacks 32 k, applies s*q+b in bf16x2 (mask + one fma on
+//        the field read as a subnormal bf16),
 //        tcgen05.st into the A ring in TMEM; scales and biases come as 16-byte chunks per row
 //   thread B: TMA  --two x sub-tiles [NT tokens x 64 k], 128B-swizzled K-major-->  smem ring B
 //   1 thread: tcgen05.mma.kind::f16 (A from TMEM, B from smem descriptors), fp32
@@ -30,7 +30,7 @@
 //
 // Grouped mode (gather_qmm): a device-side table lists (expert, first row, valid rows) for
 // every NT-row slice of the expert-sorted activations; the weight tensor map spans the
-// stacked experts [E*N, K*bits/8].
+// stacked experts [E*N, K].
 //
 // TMEM columns (512 allocated): [0, 256) accumulator, [256, 512) A ring of 4 stages
 // (128 k of bf16 = 64 columns each).  One CTA per SM (persistent), tiles are taken
@@ -59,9 +59,10 @@ constexpr int kBlockK = 64;       // k per x sub-tile (one 128-byte swizzle row 
 constexpr int kStageK = 128;      // k per pipeline stage: two x sub-tiles, one packed tile, 8 MMAs
 constexpr int kStagesA = 4;       // A ring in TMEM (64 columns each)
 constexpr int kMaxStagesB = 6;    // x stages in shared memory: as many as fit (3 at 256 tokens)
-constexpr int kMaxStagesP = 4;    // packed W tiles in shared memory
-// Packed stages: 16 * bits bytes per row and stage; next to three 64 KB x stages 35 KB remain.
-__host__ __device__ constexpr int stages_p(int bits) { return bits <= 4 ? 4 : (bits == 5 ? 3 : 2); }
+constexpr int kBits = 8;
+constexpr int kPRowBytes = 16 * kBits;   // packed bytes of 128 k of a row
+constexpr int kPStageBytes = kTileN * kPRowBytes;
+constexpr int kStagesP = 2;       // packed W tiles in shared memory: next to three 64 KB x stages 35 KB remain
 constexpr size_t kSmemMax = 227 * 1024;
 constexpr int kDoneRing = 12;
 constexpr int kAccCols = 256;
@@ -97,19 +98,6 @@ __device__ __forceinline__ void one_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uin
       : "memory");
 }
 
-// Waits of the three single-thread roles.
-#ifndef B200Q_TC_PARK
-#define TC_WAIT1 mbar_wait_spin
-#else
-#define TC_WAIT1 mbar_wait
-#endif
-// Waits of the dequant warps.
-#ifdef B200Q_TC_DQ_SPIN
-#define TC_WAIT16 mbar_wait_spin
-#else
-#define TC_WAIT16 mbar_wait
-#endif
-
 // Shared-memory matrix descriptor of a K-major, 128-byte-swizzled operand tile whose
 // rows are 128 bytes (64 bf16): 8-row groups are 1024 bytes apart (SBO), descriptor
 // version 1 (sm_100), layout type 2 = SWIZZLE_128B.  `addr` may point 32*j bytes into
@@ -143,8 +131,7 @@ struct TcParams {
   const int* dst_row;       // output row of every activation row
   const __nv_bfloat16* scales;
   const __nv_bfloat16* biases;
-  __nv_bfloat16* y;
-  // plain mode: output buffers (one, or one per GPU of an N-sharded layer), row pitch and first column
+  // output buffers (one, or one per GPU of an N-sharded layer), row pitch and first column
   __nv_bfloat16* y_out[kMaxPeers];
   int n_out;
   long long ld, col0;
@@ -158,7 +145,7 @@ struct TcParams {
 };
 
 struct __align__(8) Barriers {
-  uint64_t full_p[kMaxStagesP], empty_p[kMaxStagesP];
+  uint64_t full_p[kStagesP], empty_p[kStagesP];
   uint64_t full_b[kMaxStagesB];
   uint64_t full_a[kStagesA];
   // One commit per stage: stage `it` (counted across tiles) arrives on done[it % kDoneRing] when its
@@ -171,93 +158,37 @@ struct __align__(8) Barriers {
   int abort_flag;
 };
 
-// Unpacks 32 consecutive BITS-wide fields (BITS words, LSB-first bit stream) of one row into
-// 16 bf16x2 registers in natural k order, applying w = s*q + b (one rounding).  s and b are
-// the raw bf16 bit patterns.
-template <int BITS>
-__device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_bits, uint32_t b_bits,
-                                          uint32_t (&out)[16]) {
-  constexpr uint32_t kMagic = 0x43004300u;  // (128.0, 128.0): 0x4300 | q == 128 + q for q < 128
-  const uint32_t s2 = s_bits * 0x00010001u, b2 = b_bits * 0x00010001u;
-  // Fast form for 4- and 8-bit fields: the masked field, read as bf16, is the subnormal (or
-  // smallest normal) number q * 2^-133 (16 q * 2^-133 for a field at bits 4..7: bit 7 is the
-  // exponent's lowest bit and continues the subnormal scale exactly).  fma.rn.bf16x2 takes
-  // subnormal inputs exactly, so one fma with the scale times 2^133 (2^129) gives
-  // round(q * s + b): no shift for half of the fields, no subtraction.  It needs the scaled scale
-  // to stay finite and normal: biased exponent of s in [1, 121]; other scales (zero, subnormal,
-  // |s| >= 2^-6 * 2, inf, nan) take the general form below.
+// Unpacks 32 consecutive fields (8 words) of one row into 16 bf16x2 registers in natural k order, applying w = s*q + b (one
+// rounding).  s and b are the raw bf16 bit patterns.
+__device__ __forceinline__ void dequant32(const uint32_t (&w)[kBits], uint32_t s_bits, uint32_t b_bits, uint32_t (&out)[16]) {
+  const uint32_t b2 = b_bits * 0x00010001u;
+  // Fast form: the masked field, read as bf16, is the subnormal (or smallest normal) number q * 2^-133 (bit 7 is the
+  // exponent's lowest bit and continues the subnormal scale exactly).  fma.rn.bf16x2 takes subnormal inputs exactly, so
+  // one fma with the scale times 2^133 gives round(q * s + b).  It needs the scaled scale to stay finite and normal:
+  // biased exponent of s in [1, 121]; other scales (zero, subnormal, |s| >= 2^-6 * 2, inf, nan) take the general form.
   const uint32_t s_exp = (s_bits >> 7) & 0xFFu;
-  const bool fast = s_exp >= 1u && s_exp <= 121u;
-  if constexpr (BITS == 4) {
-    if (fast) {
-      const uint32_t sl = (s_bits + (133u << 7)) * 0x00010001u, sh = (s_bits + (129u << 7)) * 0x00010001u;
+  if (s_exp >= 1u && s_exp <= 121u) {
+    const uint32_t sl = (s_bits + (133u << 7)) * 0x00010001u;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t u = w[j] >> 8;
-        uint32_t p[4];   // p[i] = (w[i], w[i+4]) as bf16 pairs
-        p[0] = fma_bf16x2(w[j] & 0x000F000Fu, sl, b2);
-        p[1] = fma_bf16x2(w[j] & 0x00F000F0u, sh, b2);
-        p[2] = fma_bf16x2(u & 0x000F000Fu, sl, b2);
-        p[3] = fma_bf16x2(u & 0x00F000F0u, sh, b2);
-        out[4 * j + 0] = __byte_perm(p[0], p[1], 0x5410);
-        out[4 * j + 1] = __byte_perm(p[2], p[3], 0x5410);
-        out[4 * j + 2] = __byte_perm(p[0], p[1], 0x7632);
-        out[4 * j + 3] = __byte_perm(p[2], p[3], 0x7632);
-      }
-      return;
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t r0 = fma_bf16x2(w[j] & 0x00FF00FFu, sl, b2);          // (w0, w2)
+      const uint32_t r1 = fma_bf16x2((w[j] >> 8) & 0x00FF00FFu, sl, b2);   // (w1, w3)
+      out[2 * j + 0] = __byte_perm(r0, r1, 0x5410);
+      out[2 * j + 1] = __byte_perm(r0, r1, 0x7632);
     }
+    return;
+  }
+  // through float (0x4B0000qq == 2^23 + q)
+  const float sf = __uint_as_float(s_bits << 16), bf = __uint_as_float(b_bits << 16);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      uint32_t p[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        // p[i] = (q[i], q[i+4]) as bf16 pairs
-        const uint32_t t = lop3_and_or(w[j] >> (4 * i), 0x000F000Fu, kMagic);
-        p[i] = fma_bf16x2(sub_bf16x2(t, kMagic), s2, b2);
-      }
-      out[4 * j + 0] = __byte_perm(p[0], p[1], 0x5410);  // (w0, w1)
-      out[4 * j + 1] = __byte_perm(p[2], p[3], 0x5410);  // (w2, w3)
-      out[4 * j + 2] = __byte_perm(p[0], p[1], 0x7632);  // (w4, w5)
-      out[4 * j + 3] = __byte_perm(p[2], p[3], 0x7632);  // (w6, w7)
-    }
-  } else if constexpr (BITS == 8) {
-    if (fast) {
-      const uint32_t sl = (s_bits + (133u << 7)) * 0x00010001u;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t r0 = fma_bf16x2(w[j] & 0x00FF00FFu, sl, b2);          // (w0, w2)
-        const uint32_t r1 = fma_bf16x2((w[j] >> 8) & 0x00FF00FFu, sl, b2);   // (w1, w3)
-        out[2 * j + 0] = __byte_perm(r0, r1, 0x5410);
-        out[2 * j + 1] = __byte_perm(r0, r1, 0x7632);
-      }
-      return;
-    }
-    // 8-bit values exceed the bf16 integer trick: go through float (0x4B0000qq == 2^23 + q)
-    const float sf = __uint_as_float(s_bits << 16), bf = __uint_as_float(b_bits << 16);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const uint32_t word = w[j >> 1];
-      const int b0 = (j & 1) * 2;
-      const float q0 = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540 | b0)) - 8388608.0f;
-      const float q1 = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540 | (b0 + 1))) - 8388608.0f;
-      uint32_t d;
-      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(fmaf(q1, sf, bf)), "f"(fmaf(q0, sf, bf)));
-      out[j] = d;
-    }
-  } else {
-    constexpr uint32_t mask = (1u << BITS) - 1u;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      uint32_t f[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int e = 2 * j + h, wi = (e * BITS) >> 5, sh = (e * BITS) & 31;
-        f[h] = (sh + BITS > 32) ? __funnelshift_r(w[wi], w[(wi + 1) % BITS], sh) : (w[wi] >> sh);
-      }
-      const uint32_t lo = lop3_and_or(f[0], mask, 0x4300u), hi = lop3_and_or(f[1], mask, 0x4300u);
-      const uint32_t t = __byte_perm(lo, hi, 0x5410);
-      out[j] = fma_bf16x2(sub_bf16x2(t, kMagic), s2, b2);
-    }
+  for (int j = 0; j < 16; ++j) {
+    const uint32_t word = w[j >> 1];
+    const int b0 = (j & 1) * 2;
+    const float q0 = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540 | b0)) - 8388608.0f;
+    const float q1 = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540 | (b0 + 1))) - 8388608.0f;
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(fmaf(q1, sf, bf)), "f"(fmaf(q0, sf, bf)));
+    out[j] = d;
   }
 }
 
@@ -289,18 +220,10 @@ __device__ __forceinline__ TileCoord tile_coord(const TcParams& p, int tile) {
   return t;
 }
 
-#ifdef B200Q_PROFILE
-__device__ uint32_t g_tc_prof[64];
-#endif
 
-template <int BITS>
 __global__ void __launch_bounds__(kThreads, 1)
 qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
               const TcParams p) {
-  // A packed stage holds 128 k of every row (16*BITS bytes, a multiple of 16 for every width).
-  constexpr int kPRowBytes = 16 * BITS;
-  constexpr int kStagesP = stages_p(BITS);
-  constexpr int kPStageBytes = kTileN * kPRowBytes;
   const int kStagesB = p.nsb;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // carve-up: [B ring: nsb stages of two NT*128-byte sub-tiles (1024-aligned)] [P ring] [barriers]
@@ -314,20 +237,6 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#ifdef B200Q_PROFILE
-  // Tuning builds (plain mode only): thread block 0 leaves per-role wait cycles / 16 in a buffer of
-  // its own (g_tc_prof), which a test harness reads back with cudaMemcpyFromSymbol.
-  uint32_t* dbg = g_tc_prof;
-  long long pw0 = 0, pw1 = 0, pw2 = 0, pw3 = 0, pw4 = 0, pt = 0;
-  const long long prof_entry = clock64();
-#define TC_T0() pt = clock64()
-#define TC_ACC(v) v += clock64() - pt
-#define TC_OUT(slot, v) if (blockIdx.x == 0 && lane == 0 && p.mtiles == nullptr) dbg[slot] = (uint32_t)((v) >> 4)
-#else
-#define TC_T0()
-#define TC_ACC(v)
-#define TC_OUT(slot, v)
-#endif
   const int kstages = p.K / kStageK;
   const int total_tiles = p.mtiles ? *p.n_mtiles * p.n_tiles : p.n_tiles * p.m_tiles;
 
@@ -360,12 +269,10 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         const TileCoord tc_ = tile_coord(p, tile);
         bool ok = true;
         for (int ks = 0; ks < kstages; ++ks) {
-          TC_T0();
           if (it >= (uint32_t)kStagesB) {   // the stage that used this slot last has been multiplied
             const uint32_t prev = it - (uint32_t)kStagesB;
-            if (!TC_WAIT1(smem_u32(&bars->done[prev % kDoneRing]), (prev / kDoneRing) & 1u, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_spin(smem_u32(&bars->done[prev % kDoneRing]), (prev / kDoneRing) & 1u, abort_flag)) { ok = false; break; }
           }
-          TC_ACC(pw1);
           const uint32_t bar = smem_u32(&bars->full_b[sb]);
           const uint32_t dst = smem_u32(ring_b + sb * b_stage_pitch);
           mbar_expect_tx(bar, b_stage_bytes);
@@ -376,7 +283,6 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         }
         if (!ok) break;
       }
-      TC_OUT(1, pw1); TC_OUT(2, clock64() - prof_entry);
     }
   } else if (warp == kProducerPWarp) {
     // ------------------------------------------------------------ TMA producer: packed W tiles (P ring).
@@ -388,9 +294,7 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         const TileCoord tc_ = tile_coord(p, tile);
         bool ok = true;
         for (int ks = 0; ks < kstages; ++ks) {
-          TC_T0();
-          if (!TC_WAIT1(smem_u32(&bars->empty_p[sp]), pp ^ 1, abort_flag)) { ok = false; break; }
-          TC_ACC(pw0);
+          if (!mbar_wait_spin(smem_u32(&bars->empty_p[sp]), pp ^ 1, abort_flag)) { ok = false; break; }
           mbar_expect_tx(smem_u32(&bars->full_p[sp]), kPStageBytes);
           tma_load_2d(smem_u32(ring_p + sp * kPStageBytes), &map_w, ks * kPRowBytes, tc_.w_row0,
                       smem_u32(&bars->full_p[sp]));
@@ -398,7 +302,6 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         }
         if (!ok) break;
       }
-      TC_OUT(0, pw0);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
@@ -410,21 +313,14 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       // MMA: the stage is released 128 cycles later.)
       bool commit_due = false;
       for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x, ++tcount) {
-        TC_T0();
-        if (!TC_WAIT1(smem_u32(&bars->acc_empty), (tcount & 1) ^ 1, abort_flag)) break;
-        TC_ACC(pw2);
+        if (!mbar_wait_spin(smem_u32(&bars->acc_empty), (tcount & 1) ^ 1, abort_flag)) break;
         tcgen05_fence_after();
         bool ok = true;
         for (int ks = 0; ks < kstages; ++ks) {
-          TC_T0();
-          if (!TC_WAIT1(smem_u32(&bars->full_a[sa]), pa, abort_flag)) { ok = false; break; }
-          TC_ACC(pw0);
-          TC_T0();
-          if (!TC_WAIT1(smem_u32(&bars->full_b[sb]), pb, abort_flag)) { ok = false; break; }
-          TC_ACC(pw1);
+          if (!mbar_wait_spin(smem_u32(&bars->full_a[sa]), pa, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_spin(smem_u32(&bars->full_b[sb]), pb, abort_flag)) { ok = false; break; }
           tcgen05_fence_after();
           const uint32_t b_addr = smem_u32(ring_b + sb * b_stage_pitch);
-          TC_T0();
 #pragma unroll
           for (int kk = 0; kk < kStageK / 16; ++kk) {
             one_mma_ts(tmem_acc, tmem_a + sa * 64 + kk * 8,
@@ -437,7 +333,6 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
               commit_due = false;
             }
           }
-          TC_ACC(pw3);
           commit_due = true;
           ++itm;
           if (++sa == (uint32_t)kStagesA) { sa = 0; pa ^= 1; }
@@ -450,7 +345,6 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         }
         one_commit(smem_u32(&bars->acc_full));
       }
-      TC_OUT(4, pw0); TC_OUT(5, pw1); TC_OUT(6, pw2); TC_OUT(7, clock64() - prof_entry); TC_OUT(14, pw3); TC_OUT(15, pw4);
     }
   } else if (warp < 2 + kDequantWarps) {
     // ------------------------------------------------------------ dequant: one thread per weight row
@@ -532,62 +426,35 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
           s_q[0] = __ldg(sc + g0); b_q[0] = __ldg(bi + g0);
           s_q[1] = __ldg(sc + g1); b_q[1] = __ldg(bi + g1);
         }
-        TC_T0();
         // (A wait may run out for some of the lanes only; they stay until the vote below, before anything is stored.)
-        bool got = TC_WAIT16(smem_u32(&bars->full_p[sp]), pp, abort_flag);
-        TC_ACC(pw0);
-        const unsigned char* src0 = ring_p + sp * kPStageBytes + row_in_tile * kPRowBytes + half * (8 * BITS);
+        bool got = mbar_wait(smem_u32(&bars->full_p[sp]), pp, abort_flag);
+        const unsigned char* src0 = ring_p + sp * kPStageBytes + row_in_tile * kPRowBytes + half * (8 * kBits);
         bool freed = false;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          // this thread's 32 fields of quarter 2 * half + q: BITS words of its row
-          uint32_t w[BITS];
+          // this thread's 32 fields of quarter 2 * half + q: 8 words of its row
+          uint32_t w[kBits];
           {
-            const unsigned char* src = src0 + q * (4 * BITS);
-            if constexpr (BITS == 4) {
-              const uint4 v = *reinterpret_cast<const uint4*>(src);
-              w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-            } else if constexpr (BITS == 8) {
-              const uint4 v = *reinterpret_cast<const uint4*>(src), u = *reinterpret_cast<const uint4*>(src + 16);
-              w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w; w[4] = u.x; w[5] = u.y; w[6] = u.z; w[7] = u.w;
-            } else if constexpr (BITS == 2 || BITS == 6) {
-#pragma unroll
-              for (int i = 0; i < BITS / 2; ++i) {
-                const uint2 v = *reinterpret_cast<const uint2*>(src + 8 * i);
-                w[2 * i] = v.x; w[2 * i + 1] = v.y;
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < BITS; ++i) w[i] = *reinterpret_cast<const uint32_t*>(src + 4 * i);
-            }
+            const unsigned char* src = src0 + q * (4 * kBits);
+            const uint4 v = *reinterpret_cast<const uint4*>(src), u = *reinterpret_cast<const uint4*>(src + 16);
+            w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w; w[4] = u.x; w[5] = u.y; w[6] = u.z; w[7] = u.w;
           }
           uint32_t vals[16];
-          TC_T0();
-          dequant32<BITS>(w, s_q[q], b_q[q], vals);
-#ifdef B200Q_PROFILE
-          asm volatile("" ::"r"(vals[0]), "r"(vals[5]), "r"(vals[10]), "r"(vals[15]));
-#endif
-          TC_ACC(pw3);
+          dequant32(w, s_q[q], b_q[q], vals);
           __syncwarp();   // the lanes' scales may have taken both forms; a tcgen05.st needs the whole warp
           if (q == 0) {
-            TC_T0();
             if (it >= (uint32_t)kStagesA) {   // the stage that used this A slot last has been multiplied
               const uint32_t prev = it - (uint32_t)kStagesA;
-              got = got && TC_WAIT16(smem_u32(&bars->done[prev % kDoneRing]), (prev / kDoneRing) & 1u, abort_flag);
+              got = got && mbar_wait(smem_u32(&bars->done[prev % kDoneRing]), (prev / kDoneRing) & 1u, abort_flag);
             }
             if (!__all_sync(0xFFFFFFFFu, got)) { ok = false; break; }
-            TC_ACC(pw2);
             tcgen05_fence_after();
             freed = true;
           }
-          TC_T0();
           tcgen05_st_x16(tmem_a + lane_field + sa * 64 + (2 * half + q) * 16, vals);
-          TC_ACC(pw4);
         }
         if (!freed) break;
-        TC_T0();
         publish(sa);
-        TC_ACC(pw1);
         // The packed stage is released only here, after the stores that consume the unpacked
         // registers have been issued: the shared-memory reads above have then returned for every
         // lane, so the refill of the stage cannot overtake them.
@@ -596,9 +463,6 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       }
       ++tcount;
     }
-    if (warp == 2) { TC_OUT(8, pw0); TC_OUT(9, pw1); TC_OUT(10, pw2); TC_OUT(11, clock64() - prof_entry); }
-    TC_OUT(16 + dq, pw2); TC_OUT(32 + dq, pw0);
-    if (warp == 2) { TC_OUT(48, pw3); TC_OUT(49, pw4); }
   } else if (warp < kProducerPWarp) {
     // ------------------------------------------------------------ epilogue
     const int quad = warp & 3;
@@ -607,9 +471,7 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     uint32_t tcount = 0;
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++tcount) {
       const TileCoord tc_ = tile_coord(p, tile);
-      TC_T0();
       if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&bars->acc_full), tcount & 1, abort_flag))) break;
-      TC_ACC(pw0);
       tcgen05_fence_after();
       const int n = tc_.n0 + quad * 32 + lane;
       const int m0 = tc_.x_row0;
@@ -654,7 +516,6 @@ qmm_single_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         if (lane == 0) mbar_arrive(smem_u32(&bars->acc_empty));
       }
     }
-    if (warp == 2 + kDequantWarps) { TC_OUT(12, pw0); TC_OUT(13, clock64() - prof_entry); }
   }
 
   // ---- teardown: everyone meets, then the allocating warp returns the tensor memory
@@ -688,14 +549,14 @@ EncodeFn encode_fn() {
   return fn;
 }
 
-int x_stages(int nt, int bits) {
-  const size_t fixed = 1024 + (size_t)stages_p(bits) * kTileN * 16 * bits + sizeof(Barriers) + 64;
+int x_stages(int nt) {
+  const size_t fixed = 1024 + (size_t)kStagesP * kPStageBytes + sizeof(Barriers) + 64;
   const size_t n = (kSmemMax - fixed) / ((size_t)nt * 256);
   return n >= 6 ? 6 : (n >= 4 ? 4 : (n >= 3 ? 3 : 2));   // a divisor of the length of the `done` ring
 }
 
-size_t smem_bytes(int nt, int bits) {
-  const size_t need = 1024 + (size_t)x_stages(nt, bits) * nt * 256 + (size_t)stages_p(bits) * kTileN * 16 * bits +
+size_t smem_bytes(int nt) {
+  const size_t need = 1024 + (size_t)x_stages(nt) * nt * 256 + (size_t)kStagesP * kPStageBytes +
                       sizeof(Barriers) + 64;
   // More than half of an SM's shared memory: guarantees one CTA per SM, so the 512-column
   // tensor-memory allocation never has to wait for a co-resident CTA of this kernel.
@@ -703,10 +564,9 @@ size_t smem_bytes(int nt, int bits) {
   return need > one_per_sm ? need : one_per_sm;
 }
 
-// Launches the kernel instantiated for `bits`.
 int launch(int grid, size_t smem, cudaStream_t st, const CUtensorMap& map_x, const CUtensorMap& map_w, const TcParams& p) {
-  B200Q_CUDA_OK(cudaFuncSetAttribute(qmm_single_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  qmm_single_kernel<8><<<grid, kThreads, smem, st>>>(map_x, map_w, p);
+  B200Q_CUDA_OK(cudaFuncSetAttribute(qmm_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  qmm_single_kernel<<<grid, kThreads, smem, st>>>(map_x, map_w, p);
   B200Q_LAUNCH_OK("qmm_single_kernel");
   return B200Q_OK;
 }
@@ -733,9 +593,9 @@ int qmm_single(const QmmArgs& a, cudaStream_t st) {
     if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[quantized_matmul] tensor map for x failed (%d)", (int)r);
   }
   {
-    const cuuint64_t dims[2] = {(cuuint64_t)a.K * a.bits / 8, (cuuint64_t)a.N};
-    const cuuint64_t strides[1] = {(cuuint64_t)a.K * a.bits / 8};
-    const cuuint32_t box[2] = {(cuuint32_t)(16 * a.bits), (cuuint32_t)kTileN};
+    const cuuint64_t dims[2] = {(cuuint64_t)a.K * kBits / 8, (cuuint64_t)a.N};
+    const cuuint64_t strides[1] = {(cuuint64_t)a.K * kBits / 8};
+    const cuuint32_t box[2] = {(cuuint32_t)kPRowBytes, (cuuint32_t)kTileN};
     const cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint32_t*>(a.wq), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -745,7 +605,6 @@ int qmm_single(const QmmArgs& a, cudaStream_t st) {
   TcParams p{};
   p.scales = (const __nv_bfloat16*)a.scales;
   p.biases = (const __nv_bfloat16*)a.biases;
-  p.y = (__nv_bfloat16*)a.y;
   if (a.peers.n > 0) {
     p.n_out = a.peers.n; p.ld = a.peers.ld; p.col0 = a.peers.col0;
     for (int q = 0; q < a.peers.n; ++q) p.y_out[q] = (__nv_bfloat16*)a.peers.y[q];
@@ -756,7 +615,7 @@ int qmm_single(const QmmArgs& a, cudaStream_t st) {
   p.status = reinterpret_cast<uint32_t*>(static_cast<char*>(a.ws) + a.ws_bytes - kStatusBytes);
   p.M = (int)a.M; p.N = (int)a.N; p.K = (int)a.K;
   p.NT = nt;
-  p.nsb = x_stages(nt, (int)a.bits);
+  p.nsb = x_stages(nt);
   p.n_tiles = (int)((a.N + kTileN - 1) / kTileN);
   p.m_tiles = (int)((a.M + nt - 1) / nt);
   p.group_shift = a.group == 32 ? 0 : (a.group == 64 ? 1 : 2);
@@ -765,7 +624,7 @@ int qmm_single(const QmmArgs& a, cudaStream_t st) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = (long long)p.n_tiles * p.m_tiles;
   const int grid = (int)(tiles < sms ? tiles : sms);
-  return launch(grid, smem_bytes(nt, a.bits), st, map_x, map_w, p);
+  return launch(grid, smem_bytes(nt), st, map_x, map_w, p);
 }
 
 int qmm_single_grouped(const GroupedArgs& a, cudaStream_t st) {
@@ -785,9 +644,9 @@ int qmm_single_grouped(const GroupedArgs& a, cudaStream_t st) {
     if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[gather_qmm] tensor map for x failed (%d)", (int)r);
   }
   {
-    const cuuint64_t dims[2] = {(cuuint64_t)a.K * a.bits / 8, (cuuint64_t)(a.E * a.N)};
-    const cuuint64_t strides[1] = {(cuuint64_t)a.K * a.bits / 8};
-    const cuuint32_t box[2] = {(cuuint32_t)(16 * a.bits), (cuuint32_t)kTileN};
+    const cuuint64_t dims[2] = {(cuuint64_t)a.K * kBits / 8, (cuuint64_t)(a.E * a.N)};
+    const cuuint64_t strides[1] = {(cuuint64_t)a.K * kBits / 8};
+    const cuuint32_t box[2] = {(cuuint32_t)kPRowBytes, (cuuint32_t)kTileN};
     const cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint32_t*>(a.wq), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -800,7 +659,6 @@ int qmm_single_grouped(const GroupedArgs& a, cudaStream_t st) {
   p.dst_row = a.dst_row;
   p.scales = (const __nv_bfloat16*)a.scales;
   p.biases = (const __nv_bfloat16*)a.biases;
-  p.y = (__nv_bfloat16*)a.y;
   if (a.peers.n > 0) {
     p.n_out = a.peers.n;
     for (int q = 0; q < a.peers.n; ++q) p.y_out[q] = (__nv_bfloat16*)a.peers.y[q];
@@ -812,7 +670,7 @@ int qmm_single_grouped(const GroupedArgs& a, cudaStream_t st) {
   p.status = a.status;
   p.M = (int)a.n_rows; p.N = (int)a.N; p.K = (int)a.K;
   p.NT = nt;
-  p.nsb = x_stages(nt, (int)a.bits);
+  p.nsb = x_stages(nt);
   p.n_tiles = (int)((a.N + kTileN - 1) / kTileN);
   p.m_tiles = 0;
   p.group_shift = a.group == 32 ? 0 : (a.group == 64 ? 1 : 2);
@@ -821,7 +679,7 @@ int qmm_single_grouped(const GroupedArgs& a, cudaStream_t st) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = (long long)p.n_tiles * a.max_mtiles;  // upper bound; the kernel reads the exact count
   const int grid = (int)(tiles < sms ? tiles : sms);
-  return launch(grid, smem_bytes(nt, a.bits), st, map_x, map_w, p);
+  return launch(grid, smem_bytes(nt), st, map_x, map_w, p);
 }
 
 }  // namespace b200q
