@@ -1,7 +1,7 @@
 // Native form of the operator front-end for the calls a program makes every step: contiguous tensors of one
 // type on the current device.  ops.py's Python form costs 25 to 30 us per call (attribute look-ups,
 // torch functions and a ctypes call with 17 arguments), several times what the decode kernels take; this
-// one about 3 us.  Anything out of the ordinary - a cast, a copy, a broadcast, an error to report - makes a
+// one 4 to 7 us.  Anything out of the ordinary - a cast, a copy, a broadcast, an error to report - makes a
 // function here return None, and the caller goes through the Python form, which handles all of it.
 #include <Python.h>
 

@@ -143,7 +143,7 @@ bool qmv_mma_supported(const QmmArgs& a);
 size_t qmv_mma_workspace_bytes(const QmmArgs& a);
 int qmv_mma(const QmmArgs& a, cudaStream_t st);
 
-// qmv_rows.cu : decode path, bits 2/4/8, every CTA owns whole weight rows (bulk-copy ring, no scratch)
+// qmv_rows.cu : decode path, bf16 and f16, bits 2/4/8, every CTA owns whole weight rows (bulk-copy ring, no scratch)
 bool qmv_rows_supported(const QmmArgs& a);
 int qmv_rows(const QmmArgs& a, cudaStream_t st);
 // Promise that weights are not written by the stream operation preceding a matmul (see qmv_rows.cu).
@@ -155,7 +155,7 @@ bool qvm_supported(const QmmArgs& a);
 size_t qvm_workspace_bytes(const QmmArgs& a);
 int qvm(const QmmArgs& a, cudaStream_t st);
 
-// qmm_tcgen05.cu : prefill path (TMA + tcgen05 + TMEM), transpose only, bf16
+// qmm_tcgen05.cu : products with many rows (TMA + tcgen05 + TMEM); 8 bits only bf16 and transposed (qmm_tc_single.cu)
 bool qmm_tc_supported(const QmmArgs& a);
 size_t qmm_tc_workspace_bytes(const QmmArgs& a);
 int qmm_tc(const QmmArgs& a, cudaStream_t st);

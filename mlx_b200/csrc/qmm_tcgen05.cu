@@ -71,6 +71,17 @@ using namespace tc;
 
 enum class Form { Round, Split, SplitT };
 
+// The widths of this kernel (8 bits: qmm_tc_single.cu).
+#define DISPATCH_WIDTH(bits, BITS, ...)                     \
+  switch (bits) {                                           \
+    case 2: { constexpr int BITS = 2; __VA_ARGS__; } break; \
+    case 3: { constexpr int BITS = 3; __VA_ARGS__; } break; \
+    case 4: { constexpr int BITS = 4; __VA_ARGS__; } break; \
+    case 5: { constexpr int BITS = 5; __VA_ARGS__; } break; \
+    case 6: { constexpr int BITS = 6; __VA_ARGS__; } break; \
+    default: break;                                         \
+  }
+
 constexpr int kTileRows = 128;    // output columns per block and tile (MMA M = 256 over the pair)
 constexpr int kStageK = 128;      // k per pipeline stage of x, W, scales
 constexpr int kMaxStagesB = 6;
@@ -95,7 +106,7 @@ struct Shape {
   static constexpr int kSets = kT ? 2 : 4;                     // sets of unpack warps, on A slots in turn
   // Packed stages: four sets hold one each while they unpack; with no more than that every set would wait for a
   // whole TMA latency after each slot.
-  static constexpr int kStagesP = kT ? (BITS == 8 ? 2 : 3) : (BITS <= 4 ? 8 : (BITS == 8 ? 5 : 6));
+  static constexpr int kStagesP = kT ? 3 : (BITS <= 4 ? 8 : 6);
   static constexpr int kPRowBytes = 16 * BITS;                 // 128 fields
   static constexpr int kPStageBytes = kTileRows * kPRowBytes;
   static constexpr int kSmemA = kT ? kSlotsA * 32768 : 0;      // 64 k x 128 columns, hi and lo
@@ -205,9 +216,6 @@ __device__ __forceinline__ void load_fields(uint32_t tile, int r, int u, uint32_
     lds_v2(tile + r * 32 + ((((u >> 1) ^ (r >> 2)) & 1) << 4) + (u & 1) * 8, w[0], w[1]);
   } else if constexpr (BITS == 4) {   // 64-byte swizzle
     lds_v4(tile + r * 64 + (((u ^ (r >> 1)) & 3) << 4), w[0], w[1], w[2], w[3]);
-  } else if constexpr (BITS == 8) {   // 128-byte swizzle
-    lds_v4(tile + r * 128 + (((2 * u) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
-    lds_v4(tile + r * 128 + (((2 * u + 1) ^ (r & 7)) << 4), w[4], w[5], w[6], w[7]);
   } else if constexpr (BITS == 6) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) lds_v2(tile + r * 96 + u * 24 + 8 * i, w[2 * i], w[2 * i + 1]);
@@ -246,9 +254,7 @@ __device__ __forceinline__ void split32(const uint32_t (&w)[BITS], float s, floa
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int e = 2 * j + h;
-      uint32_t f;   // 0x4B0000qq is 2^23 + q exactly
-      if constexpr (BITS == 8) f = __byte_perm(w[e >> 2], 0x4B000000u, 0x7540 | (e & 3));
-      else f = lop3_and_or(field_raw<BITS>(w, e), mask, 0x4B000000u);
+      const uint32_t f = lop3_and_or(field_raw<BITS>(w, e), mask, 0x4B000000u);   // 0x4B0000qq is 2^23 + q exactly
       v[h] = fmaf(__uint_as_float(f) - 8388608.0f, s, b);
     }
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
@@ -277,7 +283,7 @@ __device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_
   // exactly.  fma.rn.bf16x2 takes subnormal inputs exactly, so one fma with the scale times 2^(133 - o) gives
   // round(q * s + b).  A byte permute brings the bytes of fields 2j and 2j+1 into the halves of a register; a field that
   // ends in the next byte is first shifted down (a quarter of the 3-bit fields, half of the 5- and 6-bit ones).  1.5 to
-  // 2 instructions per field (8 bits: 1) where extracting both fields, joining them and subtracting an offset took 3.5.
+  // 2 instructions per field where extracting both fields, joining them and subtracting an offset took 3.5.
   // It needs the scaled scale to stay finite and normal: biased exponent of s in [1, 121]; other scales (zero, subnormal,
   // |s| >= 2^-6 * 2, inf, nan) take the general form below.
   const uint32_t s_exp = (s_bits >> 7) & 0xFFu;
@@ -287,17 +293,13 @@ __device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       const int pl = 2 * j * BITS, ph = pl + BITS;   // first bits of the two fields
-      if constexpr (BITS == 8) {
-        out[j] = fma_bf16x2(__byte_perm(w[pl >> 5], 0u, (pl & 31) ? 0x4342 : 0x4140), s0, b2);
-      } else {
-        constexpr uint32_t m = (1u << BITS) - 1u;
-        const bool dl = (pl & 7) + BITS <= 8, dh = (ph & 7) + BITS <= 8;   // inside a byte
-        const uint32_t ol = dl ? pl & 7 : 0, oh = dh ? ph & 7 : 0;
-        const uint32_t bl = dl ? (pl >> 3) & 3 : 0, bh = (dh ? (ph >> 3) & 3 : 0) + 4;
-        const uint32_t v = __byte_perm(dl ? w[pl >> 5] : field_raw<BITS>(w, 2 * j), dh ? w[ph >> 5] : field_raw<BITS>(w, 2 * j + 1),
-                                       bl * 0x11 + bh * 0x1100);
-        out[j] = fma_bf16x2(v & (m << ol | m << (oh + 16)), s0 - (ol * 0x0080u + oh * 0x00800000u), b2);
-      }
+      constexpr uint32_t m = (1u << BITS) - 1u;
+      const bool dl = (pl & 7) + BITS <= 8, dh = (ph & 7) + BITS <= 8;   // inside a byte
+      const uint32_t ol = dl ? pl & 7 : 0, oh = dh ? ph & 7 : 0;
+      const uint32_t bl = dl ? (pl >> 3) & 3 : 0, bh = (dh ? (ph >> 3) & 3 : 0) + 4;
+      const uint32_t v = __byte_perm(dl ? w[pl >> 5] : field_raw<BITS>(w, 2 * j), dh ? w[ph >> 5] : field_raw<BITS>(w, 2 * j + 1),
+                                     bl * 0x11 + bh * 0x1100);
+      out[j] = fma_bf16x2(v & (m << ol | m << (oh + 16)), s0 - (ol * 0x0080u + oh * 0x00800000u), b2);
     }
     return;
   }
@@ -315,19 +317,6 @@ __device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_
       out[4 * j + 1] = __byte_perm(p[2], p[3], 0x5410);  // (w2, w3)
       out[4 * j + 2] = __byte_perm(p[0], p[1], 0x7632);  // (w4, w5)
       out[4 * j + 3] = __byte_perm(p[2], p[3], 0x7632);  // (w6, w7)
-    }
-  } else if constexpr (BITS == 8) {
-    // 8-bit values exceed the bf16 integer trick: go through float (0x4B0000qq == 2^23 + q)
-    const float sf = __uint_as_float(s_bits << 16), bf = __uint_as_float(b_bits << 16);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const uint32_t word = w[j >> 1];
-      const int b0 = (j & 1) * 2;
-      const float q0 = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540 | b0)) - 8388608.0f;
-      const float q1 = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540 | (b0 + 1))) - 8388608.0f;
-      uint32_t d;
-      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(fmaf(q1, sf, bf)), "f"(fmaf(q0, sf, bf)));
-      out[j] = d;
     }
   } else {
     constexpr uint32_t mask = (1u << BITS) - 1u;
@@ -1078,7 +1067,7 @@ size_t fixed_smem(int cb, int slots) {
 }
 size_t fixed_smem(int bits, Form f, int cb, int slots) {
   size_t n = 0;
-  B200Q_DISPATCH_BITS(bits, BITS, {
+  DISPATCH_WIDTH(bits, BITS, {
     n = f == Form::Round ? fixed_smem<BITS, Form::Round>(cb, slots)
                          : (f == Form::Split ? fixed_smem<BITS, Form::Split>(cb, slots) : fixed_smem<BITS, Form::SplitT>(cb, slots));
   });
@@ -1154,7 +1143,7 @@ int encode_maps(TcMaps& m, const char* tag, const void* x, int64_t x_rows, int64
   const cuuint64_t strides[1] = {(cuuint64_t)w_row_bytes};
   const cuuint32_t box[2] = {(cuuint32_t)(16 * bits), (cuuint32_t)kTileRows};
   const CUtensorMapSwizzle sw = bits == 2 ? CU_TENSOR_MAP_SWIZZLE_32B : (bits == 4 ? CU_TENSOR_MAP_SWIZZLE_64B
-                                : (bits == 8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE));
+                                : CU_TENSOR_MAP_SWIZZLE_NONE);
   CUresult r = enc(&m.w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(wq), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[%s] tensor map for w failed (%d)", tag, (int)r);
@@ -1163,7 +1152,7 @@ int encode_maps(TcMaps& m, const char* tag, const void* x, int64_t x_rows, int64
 
 // Once per kernel, device and thread.
 int allow_smem(const void* kernel) {
-  constexpr int kMost = 64;   // instantiations: 48
+  constexpr int kMost = 64;   // instantiations: 40
   static thread_local const void* done[64][kMost];
   static thread_local int count[64];
   int dev = 0;
@@ -1178,8 +1167,9 @@ int allow_smem(const void* kernel) {
 
 template <typename T, int BITS, Form F>
 int launch_one(unsigned grid, size_t smem, cudaStream_t st, const TcMaps& maps, const TcParams& p) {
-  // A plain launch: programmatic stream serialization would hide about 2 us of set-up, but clusters launched that way
-  // faulted (once in some hundred thousand launches here) for a reason that was not found.
+  // A plain launch: programmatic stream serialization would hide about 2 us of set-up.  It was taken back after a launch
+  // that failed once, while a ring of packed stages could still be read before its stage had landed (see the unpack warps); it
+  // has not been tried again since.
   auto go = [&](auto kernel) -> int {
     if (int rc = allow_smem((const void*)kernel)) return rc;
     kernel<<<grid, kThreads, smem, st>>>(maps, p);
@@ -1218,7 +1208,7 @@ int launch_tc(int dtype, int bits, int group, Form f, long long units, cudaStrea
   const long long pairs = sm_pairs();
   const unsigned grid = 2u * (unsigned)(units < pairs ? units : pairs);
   int rc = fail(B200Q_ERR_UNSUPPORTED, "[quantized_matmul] unsupported bits %d", bits);
-  B200Q_DISPATCH_BITS(bits, BITS, {
+  DISPATCH_WIDTH(bits, BITS, {
     if (f == Form::Round) rc = launch_one<__nv_bfloat16, BITS, Form::Round>(grid, smem, st, maps, p);
     else if (f == Form::Split) rc = launch_one<__half, BITS, Form::Split>(grid, smem, st, maps, p);
     else if (dtype == B200Q_BF16) rc = launch_one<__nv_bfloat16, BITS, Form::SplitT>(grid, smem, st, maps, p);
@@ -1251,6 +1241,7 @@ bool qmm_tc_supported(const QmmArgs& a) {
 }
 
 size_t qmm_tc_workspace_bytes(const QmmArgs& a) {
+  if (a.bits == 8) return kStatusBytes;   // qmm_single
   return split_bytes(tc_plan(a.M, a.N, a.K, form_of(a.dtype, a.transpose))) + kStatusBytes;
 }
 
