@@ -6,9 +6,8 @@
 //       two passes.  bf16 keeps the weights' exact value there, which one tensor-core tile of 17 to 32 rows rounds: the
 //       result is off by 1.7e-3 of its norm against 2.2e-3)
 //   bf16, transpose, M <= 16, K % 128 == 0 (any width)           -> qmv_mma     (register-path decode)
-//   bf16, f16, transpose, K % 128 == 0                           -> qmm_tcgen05 (TMA + tcgen05 + TMEM; bf16 with 8
-//       bits: qmm_tc_single.cu, f16 with 8 bits: qmm_generic)
-//   bf16, f16, transpose == 0, M > 16, N % 128 == 0, not 8 bits  -> qmm_tcgen05 (fewer rows waste half of the 32-token tile)
+//   bf16, f16, transpose, K % 128 == 0                           -> qmm_tcgen05 (TMA + tcgen05 + TMEM)
+//   bf16, f16, transpose == 0, M > 16, N % 128 == 0              -> qmm_tcgen05 (fewer rows waste half of the 32-token tile)
 //   transpose == 0, M <= 4, bits 2/4/8                           -> qvm
 //   everything else                                              -> qmm_generic
 #include <cstdlib>

@@ -155,13 +155,10 @@ bool qvm_supported(const QmmArgs& a);
 size_t qvm_workspace_bytes(const QmmArgs& a);
 int qvm(const QmmArgs& a, cudaStream_t st);
 
-// qmm_tcgen05.cu : products with many rows (TMA + tcgen05 + TMEM); 8 bits only bf16 and transposed (qmm_tc_single.cu)
+// qmm_tcgen05.cu : products with many rows (TMA + tcgen05 + TMEM)
 bool qmm_tc_supported(const QmmArgs& a);
 size_t qmm_tc_workspace_bytes(const QmmArgs& a);
 int qmm_tc(const QmmArgs& a, cudaStream_t st);
 int qmm_tc_grouped(const GroupedArgs& a, cudaStream_t st);
-// qmm_tc_single.cu: the same for 8-bit weights
-int qmm_single(const QmmArgs& a, cudaStream_t st);
-int qmm_single_grouped(const GroupedArgs& a, cudaStream_t st);
 
 }  // namespace b200q

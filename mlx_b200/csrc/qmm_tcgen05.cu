@@ -71,17 +71,6 @@ using namespace tc;
 
 enum class Form { Round, Split, SplitT };
 
-// The widths of this kernel (8 bits: qmm_tc_single.cu).
-#define DISPATCH_WIDTH(bits, BITS, ...)                     \
-  switch (bits) {                                           \
-    case 2: { constexpr int BITS = 2; __VA_ARGS__; } break; \
-    case 3: { constexpr int BITS = 3; __VA_ARGS__; } break; \
-    case 4: { constexpr int BITS = 4; __VA_ARGS__; } break; \
-    case 5: { constexpr int BITS = 5; __VA_ARGS__; } break; \
-    case 6: { constexpr int BITS = 6; __VA_ARGS__; } break; \
-    default: break;                                         \
-  }
-
 constexpr int kTileRows = 128;    // output columns per block and tile (MMA M = 256 over the pair)
 constexpr int kStageK = 128;      // k per pipeline stage of x, W, scales
 constexpr int kMaxStagesB = 6;
@@ -106,7 +95,13 @@ struct Shape {
   static constexpr int kSets = kT ? 2 : 4;                     // sets of unpack warps, on A slots in turn
   // Packed stages: four sets hold one each while they unpack; with no more than that every set would wait for a
   // whole TMA latency after each slot.
-  static constexpr int kStagesP = kT ? 3 : (BITS <= 4 ? 8 : 6);
+  // 8 bits: 16 KB a stage.  Eight where the tile's x leaves room (up to 128 tokens), else four; both whole turns of the
+  // sets.  Against single blocks with two packed stages and whole tiles, which bf16 ran on before (us): 64 rows through
+  // [4096, 4096] 40 -> 20, 512 42 -> 23, 4096 141 -> 105; 35 through [1280, 22784] 196 -> 27; against CUDA cores: f16, 512
+  // rows through [4096, 3584] 1090 -> 35, transpose=False, 300 through [4096, 4096] 1415 -> 56 (errors against 64 bits equal
+  // to three digits: f16 2.08e-4, bf16 1.66e-3).
+  static constexpr int kStagesP = kT ? (BITS == 8 ? 2 : 3) : (BITS <= 4 || BITS == 8 ? 8 : 6);
+  static constexpr int kFewStagesP = BITS == 8 && !kT ? 4 : kStagesP;
   static constexpr int kPRowBytes = 16 * BITS;                 // 128 fields
   static constexpr int kPStageBytes = kTileRows * kPRowBytes;
   static constexpr int kSmemA = kT ? kSlotsA * 32768 : 0;      // 64 k x 128 columns, hi and lo
@@ -160,7 +155,8 @@ struct TcParams {
   uint32_t* status;
   int M, N, K;
   int NT;            // most tokens per tile (multiple of 32, <= 256)
-  int nsb;           // x stages in shared memory (2 .. kMaxStagesB)
+  int nsb;           // x stages in shared memory (1 .. kMaxStagesB)
+  int nsp;           // packed stages, 8 bits only: 8 or 4
   int n_tiles, m_tiles;
   int full;          // tiles in whole waves (all of them in grouped mode)
   int rem, cut;      // tiles left over, and the number of pairs their stages are cut for
@@ -216,6 +212,9 @@ __device__ __forceinline__ void load_fields(uint32_t tile, int r, int u, uint32_
     lds_v2(tile + r * 32 + ((((u >> 1) ^ (r >> 2)) & 1) << 4) + (u & 1) * 8, w[0], w[1]);
   } else if constexpr (BITS == 4) {   // 64-byte swizzle
     lds_v4(tile + r * 64 + (((u ^ (r >> 1)) & 3) << 4), w[0], w[1], w[2], w[3]);
+  } else if constexpr (BITS == 8) {   // 128-byte swizzle
+    lds_v4(tile + r * 128 + (((2 * u) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+    lds_v4(tile + r * 128 + (((2 * u + 1) ^ (r & 7)) << 4), w[4], w[5], w[6], w[7]);
   } else if constexpr (BITS == 6) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) lds_v2(tile + r * 96 + u * 24 + 8 * i, w[2 * i], w[2 * i + 1]);
@@ -254,7 +253,9 @@ __device__ __forceinline__ void split32(const uint32_t (&w)[BITS], float s, floa
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int e = 2 * j + h;
-      const uint32_t f = lop3_and_or(field_raw<BITS>(w, e), mask, 0x4B000000u);   // 0x4B0000qq is 2^23 + q exactly
+      uint32_t f;   // 0x4B0000qq is 2^23 + q exactly
+      if constexpr (BITS == 8) f = __byte_perm(w[e >> 2], 0x4B000000u, 0x7540 | (e & 3));
+      else f = lop3_and_or(field_raw<BITS>(w, e), mask, 0x4B000000u);
       v[h] = fmaf(__uint_as_float(f) - 8388608.0f, s, b);
     }
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
@@ -283,7 +284,7 @@ __device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_
   // exactly.  fma.rn.bf16x2 takes subnormal inputs exactly, so one fma with the scale times 2^(133 - o) gives
   // round(q * s + b).  A byte permute brings the bytes of fields 2j and 2j+1 into the halves of a register; a field that
   // ends in the next byte is first shifted down (a quarter of the 3-bit fields, half of the 5- and 6-bit ones).  1.5 to
-  // 2 instructions per field where extracting both fields, joining them and subtracting an offset took 3.5.
+  // 2 instructions per field (8 bits: 1) where extracting both fields, joining them and subtracting an offset took 3.5.
   // It needs the scaled scale to stay finite and normal: biased exponent of s in [1, 121]; other scales (zero, subnormal,
   // |s| >= 2^-6 * 2, inf, nan) take the general form below.
   const uint32_t s_exp = (s_bits >> 7) & 0xFFu;
@@ -293,6 +294,10 @@ __device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       const int pl = 2 * j * BITS, ph = pl + BITS;   // first bits of the two fields
+      if constexpr (BITS == 8) {
+        out[j] = fma_bf16x2(__byte_perm(w[pl >> 5], 0u, (pl & 31) ? 0x4342 : 0x4140), s0, b2);
+        continue;
+      }
       constexpr uint32_t m = (1u << BITS) - 1u;
       const bool dl = (pl & 7) + BITS <= 8, dh = (ph & 7) + BITS <= 8;   // inside a byte
       const uint32_t ol = dl ? pl & 7 : 0, oh = dh ? ph & 7 : 0;
@@ -317,6 +322,16 @@ __device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_
       out[4 * j + 1] = __byte_perm(p[2], p[3], 0x5410);  // (w2, w3)
       out[4 * j + 2] = __byte_perm(p[0], p[1], 0x7632);  // (w4, w5)
       out[4 * j + 3] = __byte_perm(p[2], p[3], 0x7632);  // (w6, w7)
+    }
+  } else if constexpr (BITS == 8) {
+    // beyond the bf16 integers: through float (0x4B0000qq == 2^23 + q)
+    const float sf = __uint_as_float(s_bits << 16), bf = __uint_as_float(b_bits << 16);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int b0 = (j & 1) * 2;
+      const float q0 = __uint_as_float(__byte_perm(w[j >> 1], 0x4B000000u, 0x7540 | b0)) - 8388608.0f;
+      const float q1 = __uint_as_float(__byte_perm(w[j >> 1], 0x4B000000u, 0x7540 | (b0 + 1))) - 8388608.0f;
+      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(out[j]) : "f"(fmaf(q1, sf, bf)), "f"(fmaf(q0, sf, bf)));
     }
   } else {
     constexpr uint32_t mask = (1u << BITS) - 1u;
@@ -542,7 +557,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   using S = Shape<BITS, F>;
   constexpr bool kT = S::kT, kSplit = F != Form::Round;
-  constexpr int kSub = S::kSub, kSlotsA = S::kSlotsA, kStagesP = S::kStagesP;
+  constexpr int kSub = S::kSub, kSlotsA = S::kSlotsA;
+  constexpr bool kRingFixed = S::kStagesP == S::kFewStagesP;
+  const uint32_t nsp = kRingFixed ? S::kStagesP : p.nsp;   // packed stages; where not fixed, a power of two
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // carve-up: [A ring of SplitT] [B ring: nsb stages of two NT/2 * 128-byte sub-tiles] [P ring] [S ring] [barriers]
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -550,7 +567,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   const uint32_t b_stage = 2u * b_sub;
   unsigned char* ring_b = smem + S::kSmemA;
   unsigned char* ring_p = ring_b + (size_t)p.nsb * b_stage;
-  unsigned char* ring_s = ring_p + (size_t)kStagesP * S::kPStageBytes;   // per chunk: 128 rows of scales, 128 of biases
+  unsigned char* ring_s = ring_p + (size_t)nsp * S::kPStageBytes;   // per chunk: 128 rows of scales, 128 of biases
   unsigned char* staging = ring_s + p.s_slots * 2 * kTileRows * p.cb;    // a tile per epilogue warp
   Barriers* bars = reinterpret_cast<Barriers*>(staging + kEpilogueWarps * kStageOut);
   volatile int* abort_flag = &bars->abort_flag;
@@ -566,7 +583,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     for (int i = 0; i < 4; ++i) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.x[i]) : "memory");
   }
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kStagesP; ++i) { mbar_init(smem_u32(&bars->full_p[i]), 1); mbar_init(smem_u32(&bars->empty_p[i]), S::kPArrivals); }
+    for (int i = 0; i < (int)nsp; ++i) { mbar_init(smem_u32(&bars->full_p[i]), 1); mbar_init(smem_u32(&bars->empty_p[i]), S::kPArrivals); }
     for (int i = 0; i < p.s_slots; ++i) {
       mbar_init(smem_u32(&bars->full_s[i]), 32);
       mbar_init(smem_u32(&bars->empty_s[i]), p.spc * S::kPArrivals);
@@ -702,7 +719,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           tma_load_2d(dst, &maps.w, c0, c1, full + sp * 8);
           if constexpr (kT) c1 += kStageK; else c0 += S::kPRowBytes;
           dst += S::kPStageBytes;
-          if (++sp == (uint32_t)kStagesP) { sp = 0; pp ^= 1; dst = ring; }
+          if (++sp == nsp) { sp = 0; pp ^= 1; dst = ring; }
         }
       }
     }
@@ -774,7 +791,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     const uint32_t spc_sh = p.spc == 4 ? 2 : (p.spc == 2 ? 1 : 0), half_chunk = (uint32_t)kTileRows * p.cb;
     const bool single = p.spc * p.g4 == 1;   // a chunk is one value: the odd or the even half of the copied word
     const uint32_t s_row = smem_u32(ring_s) + row * p.cb;
-    const uint32_t p_base = smem_u32(ring_p);
+    const uint32_t p_base = smem_u32(ring_p), p_sh = nsp == 8 ? 3 : 2;
     const uint32_t bar_a = leader_addr(smem_u32(&bars->full_a[0])), bar_done = smem_u32(&bars->done[0]);
     const uint32_t bar_fp = smem_u32(&bars->full_p[0]), bar_ep = smem_u32(&bars->empty_p[0]);
     const uint32_t bar_fs = smem_u32(&bars->full_s[0]), bar_es = smem_u32(&bars->empty_s[0]);
@@ -787,18 +804,18 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
       const uint32_t o_row = kT ? min(t.n0 / kTileRows, p.row_groups - 1) : (uint32_t)min(t.w_row0 + row, t.w_row_end - 1) * p.row_groups + t.ks0;
       for (; ia < (it0 + n_st) * kSub; ia += kSets) {
         const uint32_t it = ia / kSub, ks = it - it0;      // ks counts from the unit's first stage
-        const uint32_t c = c0 + (ks >> spc_sh), sp = it % kStagesP;
+        const uint32_t c = c0 + (ks >> spc_sh), sp = kRingFixed ? it % S::kStagesP : it & (nsp - 1);
         bool got = mbar_wait_hot(bar_fs + (c & s_mask) * 8, (c >> s_sh) & 1u, abort_flag);
         // Where a ring slot passes from one set to another (its length no multiple of the stages per turn), a set can
         // come to it before the slot's previous stage, another set's, has landed.  The parity asked for is then that of
         // the use before, which reads as complete.  So such rings wait first until the set's own A slot has been multiplied:
         // products run in order, and the slot's previous stage is an earlier one.
         if constexpr (S::kStagesP % (kSets / kSub > 0 ? kSets / kSub : 1) != 0) {
-          static_assert(S::kStagesP > kSlotsA / kSub, "the previous stage of a ring slot is not after that of the A slot");
+          static_assert(kRingFixed && S::kStagesP > kSlotsA / kSub, "the previous stage of a ring slot is not after that of the A slot");
           const uint32_t prev = ia - kSlotsA;
           got = got && (ia < (uint32_t)kSlotsA || mbar_wait_hot(bar_done + (prev % kDoneRing) * 8, (prev / kDoneRing) & 1u, abort_flag));
         }
-        got = got && mbar_wait_hot(bar_fp + sp * 8, (it / kStagesP) & 1u, abort_flag);
+        got = got && mbar_wait_hot(bar_fp + sp * 8, (kRingFixed ? it / S::kStagesP : it >> p_sh) & 1u, abort_flag);
         // A wait may run out for some of the lanes only.  They stay (what they unpack is never stored) until the vote below:
         // the votes and tcgen05 instructions from here on need the whole warp.
         const uint32_t tile = p_base + sp * S::kPStageBytes;
@@ -1060,16 +1077,16 @@ Form form_of(int dtype, bool transpose) {
 }
 
 template <int BITS, Form F>
-size_t fixed_smem(int cb, int slots) {
+size_t fixed_smem(int cb, int slots, bool few) {
   using S = Shape<BITS, F>;
-  return 1024 + S::kSmemA + (size_t)S::kStagesP * S::kPStageBytes + (size_t)slots * 2 * kTileRows * cb + kEpilogueWarps * kStageOut +
+  return 1024 + S::kSmemA + (size_t)(few ? S::kFewStagesP : S::kStagesP) * S::kPStageBytes + (size_t)slots * 2 * kTileRows * cb + kEpilogueWarps * kStageOut +
          sizeof(Barriers) + 64;
 }
-size_t fixed_smem(int bits, Form f, int cb, int slots) {
+size_t fixed_smem(int bits, Form f, int cb, int slots, bool few) {
   size_t n = 0;
-  DISPATCH_WIDTH(bits, BITS, {
-    n = f == Form::Round ? fixed_smem<BITS, Form::Round>(cb, slots)
-                         : (f == Form::Split ? fixed_smem<BITS, Form::Split>(cb, slots) : fixed_smem<BITS, Form::SplitT>(cb, slots));
+  B200Q_DISPATCH_BITS(bits, BITS, {
+    n = f == Form::Round ? fixed_smem<BITS, Form::Round>(cb, slots, few)
+                         : (f == Form::Split ? fixed_smem<BITS, Form::Split>(cb, slots, few) : fixed_smem<BITS, Form::SplitT>(cb, slots, few));
   });
   return n;
 }
@@ -1143,7 +1160,7 @@ int encode_maps(TcMaps& m, const char* tag, const void* x, int64_t x_rows, int64
   const cuuint64_t strides[1] = {(cuuint64_t)w_row_bytes};
   const cuuint32_t box[2] = {(cuuint32_t)(16 * bits), (cuuint32_t)kTileRows};
   const CUtensorMapSwizzle sw = bits == 2 ? CU_TENSOR_MAP_SWIZZLE_32B : (bits == 4 ? CU_TENSOR_MAP_SWIZZLE_64B
-                                : CU_TENSOR_MAP_SWIZZLE_NONE);
+                                : (bits == 8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE));
   CUresult r = enc(&m.w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(wq), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(B200Q_ERR_CUDA, "[%s] tensor map for w failed (%d)", tag, (int)r);
@@ -1152,7 +1169,7 @@ int encode_maps(TcMaps& m, const char* tag, const void* x, int64_t x_rows, int64
 
 // Once per kernel, device and thread.
 int allow_smem(const void* kernel) {
-  constexpr int kMost = 64;   // instantiations: 40
+  constexpr int kMost = 64;   // instantiations: 48
   static thread_local const void* done[64][kMost];
   static thread_local int count[64];
   int dev = 0;
@@ -1197,8 +1214,10 @@ int launch_tc(int dtype, int bits, int group, Form f, long long units, cudaStrea
   p.cb = p.spc * p.g4 * 2 < 4 ? 4 : p.spc * p.g4 * 2;
   p.narrow = (reinterpret_cast<uintptr_t>(p.scales) | reinterpret_cast<uintptr_t>(p.biases)) % p.cb != 0;   // (only with chunks of one stage)
   p.s_slots = p.spc == 4 ? 2 : 4;
-  const size_t fixed = fixed_smem(bits, f, p.cb, p.s_slots);
   const size_t stage = (size_t)p.NT * 128;
+  const bool few = fixed_smem(bits, f, p.cb, p.s_slots, false) + 3 * stage > kSmemMax;   // three stages of x come first
+  p.nsp = few ? 4 : 8;
+  const size_t fixed = fixed_smem(bits, f, p.cb, p.s_slots, few);
   long long nsb = (long long)((kSmemMax - fixed) / stage);
   p.nsb = (int)(nsb > kMaxStagesB ? kMaxStagesB : nsb);
   size_t smem = fixed + p.nsb * stage;
@@ -1208,7 +1227,7 @@ int launch_tc(int dtype, int bits, int group, Form f, long long units, cudaStrea
   const long long pairs = sm_pairs();
   const unsigned grid = 2u * (unsigned)(units < pairs ? units : pairs);
   int rc = fail(B200Q_ERR_UNSUPPORTED, "[quantized_matmul] unsupported bits %d", bits);
-  DISPATCH_WIDTH(bits, BITS, {
+  B200Q_DISPATCH_BITS(bits, BITS, {
     if (f == Form::Round) rc = launch_one<__nv_bfloat16, BITS, Form::Round>(grid, smem, st, maps, p);
     else if (f == Form::Split) rc = launch_one<__half, BITS, Form::Split>(grid, smem, st, maps, p);
     else if (dtype == B200Q_BF16) rc = launch_one<__nv_bfloat16, BITS, Form::SplitT>(grid, smem, st, maps, p);
@@ -1234,19 +1253,16 @@ void set_outputs(TcParams& p, const PeerOut& peers, void* y, int64_t ld) {
 bool qmm_tc_supported(const QmmArgs& a) {
   if ((a.dtype != B200Q_BF16 && a.dtype != B200Q_F16) || a.w_batched || a.batch != 1) return false;
   if (a.M < 1 || a.N < 1 || a.K < 1 || a.M > (1 << 30) || a.N > (1 << 30)) return false;
-  if (a.bits == 8 && (a.dtype != B200Q_BF16 || !a.transpose)) return false;   // 8 bits: qmm_single
   if ((a.transpose ? a.K : a.N) % kStageK != 0 || a.K % 8 != 0) return false;
   // TMA: 16-byte aligned bases and row pitches
   return !((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.wq)) & 15);
 }
 
 size_t qmm_tc_workspace_bytes(const QmmArgs& a) {
-  if (a.bits == 8) return kStatusBytes;   // qmm_single
   return split_bytes(tc_plan(a.M, a.N, a.K, form_of(a.dtype, a.transpose))) + kStatusBytes;
 }
 
 int qmm_tc(const QmmArgs& a, cudaStream_t st) {
-  if (a.bits == 8) return qmm_single(a, st);
   if (!a.ws || a.ws_bytes < kStatusBytes)
     return fail(B200Q_ERR_WORKSPACE, "[quantized_matmul] workspace of %zu bytes required, %zu given",
                 (size_t)kStatusBytes, a.ws_bytes);
@@ -1280,7 +1296,6 @@ int qmm_tc(const QmmArgs& a, cudaStream_t st) {
 }
 
 int qmm_tc_grouped(const GroupedArgs& a, cudaStream_t st) {
-  if (a.bits == 8) return qmm_single_grouped(a, st);
   TcMaps maps;
   if (int rc = encode_maps(maps, "gather_qmm", a.x_sorted, a.n_rows, a.K, B200Q_BF16, a.wq, a.E * a.N, a.K * a.bits / 8, a.bits))
     return rc;

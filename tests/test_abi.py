@@ -77,6 +77,15 @@ def test_kernel_selection_names():
     assert lib.b200q_qmm_workspace_bytes(_lib.BF16, 1, 16, 14336, 4096, 64, 4, 1) > 14336 * 64
 
 
+def test_eight_bit_products_with_many_rows_are_tensor_core_products():
+    lib = _lib.load()
+    name = lambda M, N, K, dt, tr: lib.b200q_qmm_kernel_name(dt, 1, M, N, K, 64, 8, tr).decode()
+    for dt in (_lib.BF16, _lib.F16):
+        assert name(64, 4096, 4096, dt, 1) == "qmm_tcgen05" and name(64, 4096, 4096, dt, 0) == "qmm_tcgen05"
+        assert name(16, 4096, 4096, dt, 0) == "qmm_generic" and name(64, 4096, 192, dt, 1) == "qmm_generic"
+    assert name(64, 4096, 4096, _lib.F32, 1) == "qmm_generic"
+
+
 def test_sharded_rejects_on_host():
     """b200q_qmm_sharded validates its output description before any CUDA call."""
     lib = _lib.load()
