@@ -76,7 +76,7 @@ constexpr int kStageK = 128;      // k per pipeline stage of x, W, scales
 constexpr int kMaxStagesB = 6;
 constexpr int kMaxStagesP = 8;
 constexpr int kMaxSlotsA = 4;
-constexpr int kMaxSlotsS = 4;     // chunks of scales and biases: 2 of four stages, else 4
+constexpr int kMaxSlotsS = 8;     // chunks of scales and biases
 constexpr int kDoneRing = 16;     // one commit per A slot; longer than any distance a waiter can be behind
 constexpr int kTmemCols = 512;    // [0, 256) accumulators, [256, 512) A ring (4 slots of 64 columns)
 constexpr int kAccCols = 256;
@@ -164,7 +164,7 @@ struct TcParams {
   uint32_t* counters;   // [tile left over][block of the pair]
   int g4;            // groups per 128 fields of a row: 4, 2, 1
   int row_groups;    // groups per packed row
-  int s_slots;       // chunks of scales in their ring
+  int s_slots;       // chunks of scales in their ring (a power of two)
   int spc, cb;       // stages per chunk of scales, bytes per row of a chunk (4, 8 or 16)
   int narrow;        // scales or biases are not aligned to cb: 2-byte loads
   long long n_scales;   // elements of `scales`
@@ -183,6 +183,7 @@ struct __align__(8) Barriers {
   uint64_t acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   int abort_flag, last;
+  int help;        // the pair's last unit is a tile that this block is the last to add up: all warps that can take part
   int odd;         // split forms: a result was not finite
   uint32_t ended;  // pieces of cut tiles (by their number among this pair's) that this block has summed
   int landed[2];   // of a tile (even, odd): its accumulator is complete, as the epilogue warp that waits for it found
@@ -274,30 +275,24 @@ __device__ __forceinline__ void split32(const uint32_t (&w)[BITS], float s, floa
 // Unpacks 32 consecutive BITS-wide fields (BITS words, LSB-first bit stream) of one row into
 // 16 bf16x2 registers in natural k order, applying w = s*q + b (one rounding).  s and b are
 // the raw bf16 bit patterns.
+// Fast form: a field inside a byte, masked in place and read as bf16, is the subnormal (or smallest normal) number
+// q * 2^(o - 133), o its lowest bit in the byte: bit 7 is the exponent's lowest bit and continues the subnormal scale
+// exactly.  fma.rn.bf16x2 takes subnormal inputs exactly, so one fma with the scale times 2^(133 - o) gives
+// round(q * s + b).  A byte permute brings the bytes of fields 2j and 2j+1 into the halves of a register; a field that
+// ends in the next byte is first shifted down (a quarter of the 3-bit fields, half of the 5- and 6-bit ones).  1.5 to
+// 2 instructions per field (8 bits: 1) where extracting both fields, joining them and subtracting an offset took 3.5.
+// It needs the scaled scale to stay finite and normal: biased exponent of s in [1, 121]; other scales (zero, subnormal,
+// |s| >= 2^-6 * 2, inf, nan) take the general form.
+__device__ __forceinline__ bool scale_has_room(uint32_t s_bits) { return (s_bits & 0x7FFFu) - 0x80u < (122u << 7) - 0x80u; }
 template <int BITS>
-__device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_bits, uint32_t b_bits,
-                                          uint32_t (&out)[16]) {
-  constexpr uint32_t kMagic = 0x43004300u;  // (128.0, 128.0): 0x4300 | q == 128 + q for q < 128
-  const uint32_t s2 = s_bits * 0x00010001u, b2 = b_bits * 0x00010001u;
-  // Fast form: a field inside a byte, masked in place and read as bf16, is the subnormal (or smallest normal) number
-  // q * 2^(o - 133), o its lowest bit in the byte: bit 7 is the exponent's lowest bit and continues the subnormal scale
-  // exactly.  fma.rn.bf16x2 takes subnormal inputs exactly, so one fma with the scale times 2^(133 - o) gives
-  // round(q * s + b).  A byte permute brings the bytes of fields 2j and 2j+1 into the halves of a register; a field that
-  // ends in the next byte is first shifted down (a quarter of the 3-bit fields, half of the 5- and 6-bit ones).  1.5 to
-  // 2 instructions per field (8 bits: 1) where extracting both fields, joining them and subtracting an offset took 3.5.
-  // It needs the scaled scale to stay finite and normal: biased exponent of s in [1, 121]; other scales (zero, subnormal,
-  // |s| >= 2^-6 * 2, inf, nan) take the general form below.
-  const uint32_t s_exp = (s_bits >> 7) & 0xFFu;
-  const bool fast = __all_sync(0xFFFFFFFFu, s_exp >= 1u && s_exp <= 121u);   // one branch per warp: a predicated mixture would run both forms
-  if (fast) {
-    const uint32_t s0 = (s_bits + (133u << 7)) * 0x00010001u;
+__device__ __forceinline__ void dequant32_fast(const uint32_t (&w)[BITS], uint32_t s_bits, uint32_t b_bits, uint32_t (&out)[16]) {
+  const uint32_t b2 = b_bits * 0x00010001u, s0 = (s_bits + (133u << 7)) * 0x00010001u;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int pl = 2 * j * BITS, ph = pl + BITS;   // first bits of the two fields
-      if constexpr (BITS == 8) {
-        out[j] = fma_bf16x2(__byte_perm(w[pl >> 5], 0u, (pl & 31) ? 0x4342 : 0x4140), s0, b2);
-        continue;
-      }
+  for (int j = 0; j < 16; ++j) {
+    const int pl = 2 * j * BITS, ph = pl + BITS;   // first bits of the two fields
+    if constexpr (BITS == 8) {
+      out[j] = fma_bf16x2(__byte_perm(w[pl >> 5], 0u, (pl & 31) ? 0x4342 : 0x4140), s0, b2);
+    } else {
       constexpr uint32_t m = (1u << BITS) - 1u;
       const bool dl = (pl & 7) + BITS <= 8, dh = (ph & 7) + BITS <= 8;   // inside a byte
       const uint32_t ol = dl ? pl & 7 : 0, oh = dh ? ph & 7 : 0;
@@ -306,8 +301,12 @@ __device__ __forceinline__ void dequant32(const uint32_t (&w)[BITS], uint32_t s_
                                      bl * 0x11 + bh * 0x1100);
       out[j] = fma_bf16x2(v & (m << ol | m << (oh + 16)), s0 - (ol * 0x0080u + oh * 0x00800000u), b2);
     }
-    return;
   }
+}
+template <int BITS>
+__device__ __forceinline__ void dequant32_any(const uint32_t (&w)[BITS], uint32_t s_bits, uint32_t b_bits, uint32_t (&out)[16]) {
+  constexpr uint32_t kMagic = 0x43004300u;  // (128.0, 128.0): 0x4300 | q == 128 + q for q < 128
+  const uint32_t s2 = s_bits * 0x00010001u, b2 = b_bits * 0x00010001u;
   if constexpr (BITS == 4) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -389,7 +388,7 @@ struct Unit {
   int rtile;       // index of the tile among those left over
 };
 // Pair j's range of the chunks (spc stages, whole chunks of scales) of the tiles left over.
-__device__ __forceinline__ int range_begin(const TcParams& p, int j, int chunks) { return (int)((long long)j * p.rem * chunks / p.cut); }
+__device__ __forceinline__ int range_begin(const TcParams& p, int j, int chunks) { return (int)((uint32_t)(j * p.rem * chunks) / (uint32_t)p.cut); }   // (tc_plan keeps it below 2^31)
 // Units of the loop `for (u = pair; u < end; u += pairs)`: the pair's whole tiles, then the pieces of its range.
 __device__ __forceinline__ int units_end(const TcParams& p, int pair, int pairs) {
   if (p.mtiles) return *p.n_mtiles * p.n_tiles;
@@ -411,8 +410,8 @@ __device__ __forceinline__ Unit unit_at(const TcParams& p, int u, int rank) {
       t.ks0 = (max(lo, first) - first) * p.spc;
       t.ks1 = (min(hi, first + chunks) - first) * p.spc;
       // the pair whose range holds chunk c is ((c + 1) * cut - 1) / (rem * chunks)
-      const long long all = (long long)p.rem * chunks;
-      const int j0 = (int)(((first + 1ll) * p.cut - 1) / all), j1 = (int)(((long long)(first + chunks) * p.cut - 1) / all);
+      const uint32_t all = p.rem * chunks;
+      const int j0 = (int)((uint32_t)((first + 1) * p.cut - 1) / all), j1 = (int)((uint32_t)((first + chunks) * p.cut - 1) / all);
       t.parts = j1 - j0 + 1;
       t.slot = j + r;           // ranges in order, one more at every tile boundary
       t.slot0 = j0 + r;
@@ -529,6 +528,55 @@ __device__ __forceinline__ uint32_t store_chunk(const TcParams& p, const Unit& t
   return odd;
 }
 
+// A cut tile's fp32 sums, part by part in order, by NW warps of the last block to arrive, which leave them zeroed.  A warp
+// takes whole tokens, a lane four columns of each: 16-byte loads, two tokens of four parts at a time.  Returns nonzero (WATCH)
+// where a result is not finite.
+template <typename T, int NW, bool WATCH>
+__device__ __forceinline__ uint32_t sum_parts(const TcParams& p, const Unit& t, int rank, int warp, int lane) {
+  uint32_t odd = 0;
+  __threadfence();
+  const size_t pitch = 2 * (size_t)p.NT * kTileRows / 4;   // from one part to the next
+  float4* p0 = reinterpret_cast<float4*>(p.partial + ((size_t)t.slot0 * 2 + rank) * ((size_t)p.NT * kTileRows)) + lane;
+  const int n4 = t.n0 + 4 * lane;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (int c = warp; c < t.rows; c += 2 * NW) {
+    const int n_tok = c + NW < t.rows ? 2 : 1;
+    float4* q0 = p0 + (size_t)c * (kTileRows / 4);
+    float4 sum[2] = {zero, zero};
+    for (int s = 0; s < t.parts; s += 4) {
+      float4 v[2][4];
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          v[k][i] = k < n_tok && s + i < t.parts ? __ldcg(q0 + (size_t)(s + i) * pitch + k * (NW * kTileRows / 4)) : zero;
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { sum[k].x += v[k][i].x; sum[k].y += v[k][i].y; sum[k].z += v[k][i].z; sum[k].w += v[k][i].w; }
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (k >= n_tok) break;
+      for (int s = 0; s < t.parts; ++s) __stcg(q0 + (size_t)s * pitch + k * (NW * kTileRows / 4), zero);
+      const uint2 o = make_uint2(pack_pair<T>(__float_as_uint(sum[k].x), __float_as_uint(sum[k].y)),
+                                 pack_pair<T>(__float_as_uint(sum[k].z), __float_as_uint(sum[k].w)));
+      if constexpr (WATCH) odd |= odd_pair<T>(o.x) | odd_pair<T>(o.y);
+      const long long at = (long long)(t.x_row0 + c + k * NW) * p.ld + p.col0 + n4;
+      for (int q = 0; q < p.n_out; ++q) {
+        T* dst = static_cast<T*>(p.y_out[q]) + at;
+        if (n4 + 4 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+          *reinterpret_cast<uint2*>(dst) = o;
+        } else {
+          const T* e = reinterpret_cast<const T*>(&o);
+          for (int i = 0; i < 4 && n4 + i < p.N; ++i) dst[i] = e[i];
+        }
+      }
+    }
+  }
+  return odd;
+}
+
 // The elements of a tile that are not finite, from the weights themselves in fp32, by the epilogue warps.
 template <typename T, int BITS, bool TRANSPOSED>
 __device__ __forceinline__ void repair(const TcParams& p, int n0, int x_row0, int rows) {
@@ -554,7 +602,7 @@ __device__ __forceinline__ void repair(const TcParams& p, int n0, int x_row0, in
 // ordinary products 2 to 4 %).
 template <typename T, int BITS, Form F, bool ROWS16>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
+qmm_tc_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcParams p) {
   using S = Shape<BITS, F>;
   constexpr bool kT = S::kT, kSplit = F != Form::Round;
   constexpr int kSub = S::kSub, kSlotsA = S::kSlotsA;
@@ -582,20 +630,24 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.x[i]) : "memory");
   }
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < (int)nsp; ++i) { mbar_init(smem_u32(&bars->full_p[i]), 1); mbar_init(smem_u32(&bars->empty_p[i]), S::kPArrivals); }
-    for (int i = 0; i < p.s_slots; ++i) {
-      mbar_init(smem_u32(&bars->full_s[i]), 32);
-      mbar_init(smem_u32(&bars->empty_s[i]), p.spc * S::kPArrivals);
+  if (warp == 0) {   // a lane per barrier of each kind: one thread after another took 0.7 us
+    if (lane < (int)nsp) { mbar_init(smem_u32(&bars->full_p[lane]), 1); mbar_init(smem_u32(&bars->empty_p[lane]), S::kPArrivals); }
+    if (lane < p.s_slots) {
+      mbar_init(smem_u32(&bars->full_s[lane]), 32);
+      mbar_init(smem_u32(&bars->empty_s[lane]), p.spc * S::kPArrivals);
     }
-    for (int i = 0; i < p.nsb; ++i) mbar_init(smem_u32(&bars->full_b[i]), 1);
-    for (int i = 0; i < kSlotsA; ++i) mbar_init(smem_u32(&bars->full_a[i]), 2 * kUnpackWarps / S::kSets);
-    for (int i = 0; i < kDoneRing; ++i) mbar_init(smem_u32(&bars->done[i]), 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&bars->acc_full[i]), 1); mbar_init(smem_u32(&bars->acc_empty[i]), 2 * kEpilogueWarps); }
-    bars->abort_flag = 0;
-    bars->odd = 0;
-    bars->ended = 0;
+    if (lane < p.nsb) mbar_init(smem_u32(&bars->full_b[lane]), 1);
+    if (lane < kSlotsA) mbar_init(smem_u32(&bars->full_a[lane]), 2 * kUnpackWarps / S::kSets);
+    if (lane < kDoneRing) mbar_init(smem_u32(&bars->done[lane]), 1);
+    if (lane < 2) { mbar_init(smem_u32(&bars->acc_full[lane]), 1); mbar_init(smem_u32(&bars->acc_empty[lane]), 2 * kEpilogueWarps); }
+    if (lane == 0) {
+      bars->abort_flag = 0;
+      bars->odd = 0;
+      bars->ended = 0;
+      bars->help = 0;
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    __syncwarp();
   }
   if (warp == 1) {
     tcgen05_alloc(smem_u32(&bars->tmem_base), kTmemCols);
@@ -603,7 +655,10 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   }
   tcgen05_fence_before();
   __syncthreads();
-  cluster_sync();
+  // Warps 2 and 3 fetch for this block alone: they start at once and meet the other block when they are done.  (33 rows through
+  // [4096, 4096], clock marks: first packed stage used 5.1 us after entry, now 4.1 to 5.2; first MMA 7.0 -> 6.0.)
+  cluster_arrive();
+  if (warp != 2 && warp != 3) cluster_wait();
   tcgen05_fence_after();
   const int total = units_end(p, pair, pairs);
   const uint32_t tmem_base = bars->tmem_base;
@@ -723,6 +778,8 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         }
       }
     }
+    __syncwarp();
+    cluster_wait();
   } else if (warp == 3) {
     // ------------------------------------------------------------ scales and biases
     // Asynchronous copies straight into the ring, counted on the chunk's barrier; a lane serves four rows.
@@ -771,6 +828,8 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         if (++ss == (uint32_t)p.s_slots) { ss = 0; ps ^= 1; }
       }
     }
+    __syncwarp();
+    cluster_wait();
   } else if (warp < kFirstEpilogue) {
     // ------------------------------------------------------------ unpack
     // Everything here is counted in instructions: the warps of a scheduler make one instruction about
@@ -787,7 +846,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     const uint32_t t_slot = tmem_a + ((uint32_t)(quad * 32) << 16) + set * 64;   // (transpose) as many slots as sets
     // offset of unit un's value in a chunk row's stage: one value per 1, 2 or 4 units
     const int gsh = p.g4 == 4 ? 0 : (p.g4 == 2 ? 1 : 2);
-    const uint32_t s_mask = p.s_slots - 1, s_sh = p.s_slots == 2 ? 1 : 2;
+    const uint32_t s_mask = p.s_slots - 1, s_sh = 31 - __clz(p.s_slots);
     const uint32_t spc_sh = p.spc == 4 ? 2 : (p.spc == 2 ? 1 : 0), half_chunk = (uint32_t)kTileRows * p.cb;
     const bool single = p.spc * p.g4 == 1;   // a chunk is one value: the odd or the even half of the copied word
     const uint32_t s_row = smem_u32(ring_s) + row * p.cb;
@@ -831,17 +890,37 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           return __all_sync(0xFFFFFFFFu, free) != 0;
         };
         if constexpr (F == Form::Round) {
+          // One vote and one straight line for the slot's four units: every shared-memory read is under way before it is
+          // needed.  With a vote per unit, after which its words and scales were read: 512 tokens through [28672, 8192] at 3 bits 216
+          // us, now 209; 57 rows through [4096, 11008] 26.6, now 24.6 (with the shorter set-up and the helpers' sums below).
+          uint32_t sv[4], bv[4], w[2][BITS], vals[16];
 #pragma unroll
           for (int un = 0; un < 4; ++un) {
-            uint32_t w[BITS], vals[16];
-            load_fields<BITS>(tile, row, un, w);
-            const uint32_t v = at + 2 * (un >> gsh);
-            dequant32<BITS>(w, lds_u16(v), lds_u16(v + half_chunk), vals);
-            if (un == 0) {
-              if (!slot_free()) { ok = false; break; }
-              tcgen05_fence_after();
+            sv[un] = lds_u16(at + 2 * (un >> gsh));
+            bv[un] = lds_u16(at + 2 * (un >> gsh) + half_chunk);
+          }
+          load_fields<BITS>(tile, row, 0, w[0]);
+          if (__all_sync(0xFFFFFFFFu, scale_has_room(sv[0]) && scale_has_room(sv[1]) && scale_has_room(sv[2]) && scale_has_room(sv[3]))) {
+#pragma unroll
+            for (int un = 0; un < 4; ++un) {
+              if (un < 3) load_fields<BITS>(tile, row, un + 1, w[(un + 1) & 1]);
+              dequant32_fast<BITS>(w[un & 1], sv[un], bv[un], vals);
+              if (un == 0) {
+                if (!slot_free()) { ok = false; break; }
+                tcgen05_fence_after();
+              }
+              tcgen05_st_x16(t_slot + un * 16, vals);
             }
-            tcgen05_st_x16(t_slot + un * 16, vals);
+          } else if (slot_free()) {
+            tcgen05_fence_after();
+#pragma unroll
+            for (int un = 0; un < 4; ++un) {
+              load_fields<BITS>(tile, row, un, w[0]);
+              dequant32_any<BITS>(w[0], sv[un], bv[un], vals);
+              tcgen05_st_x16(t_slot + un * 16, vals);
+            }
+          } else {
+            ok = false;
           }
         } else if constexpr (F == Form::Split) {
 #pragma unroll
@@ -960,8 +1039,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         }
       }
       if (t.parts > 1) {
-        // The last of the tile's pairs to arrive (per block of the pair: each has its own 128 columns) adds
-        // the parts in order and leaves them zeroed.
+        // The last of the tile's pairs to arrive (per block of the pair: each has its own 128 columns) adds the parts.
         __threadfence();
         asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueWarps * 32) : "memory");
         if (warp == kFirstEpilogue && lane == 0) {
@@ -973,55 +1051,30 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueWarps * 32) : "memory");
         if (bars->last) {
           if (kSplit && warp == kFirstEpilogue && lane == 0) bars->ended |= 1u << ((u - p.full) / pairs & 31);
-          // A warp takes whole tokens, a lane four columns of each: 16-byte loads, two tokens of four parts at a time.
-          __threadfence();
-          const size_t pitch = 2 * (size_t)p.NT * kTileRows / 4;   // from one part to the next
-          float4* p0 = reinterpret_cast<float4*>(p.partial + ((size_t)t.slot0 * 2 + rank) * ((size_t)p.NT * kTileRows)) + lane;
-          const int n4 = t.n0 + 4 * lane;
-          const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          for (int c = warp - kFirstEpilogue; c < t.rows; c += 2 * kEpilogueWarps) {
-            const int n_tok = c + kEpilogueWarps < t.rows ? 2 : 1;
-            float4* q0 = p0 + (size_t)c * (kTileRows / 4);
-            float4 sum[2] = {zero, zero};
-            for (int s = 0; s < t.parts; s += 4) {
-              float4 v[2][4];
-#pragma unroll
-              for (int k = 0; k < 2; ++k)
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                  v[k][i] = k < n_tok && s + i < t.parts ? __ldcg(q0 + (size_t)(s + i) * pitch + k * (kEpilogueWarps * kTileRows / 4)) : zero;
-#pragma unroll
-              for (int k = 0; k < 2; ++k)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) { sum[k].x += v[k][i].x; sum[k].y += v[k][i].y; sum[k].z += v[k][i].z; sum[k].w += v[k][i].w; }
-            }
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              if (k >= n_tok) break;
-              for (int s = 0; s < t.parts; ++s) __stcg(q0 + (size_t)s * pitch + k * (kEpilogueWarps * kTileRows / 4), zero);
-              const uint2 o = make_uint2(pack_pair<T>(__float_as_uint(sum[k].x), __float_as_uint(sum[k].y)),
-                                         pack_pair<T>(__float_as_uint(sum[k].z), __float_as_uint(sum[k].w)));
-              if (kSplit && (odd_pair<T>(o.x) | odd_pair<T>(o.y)) != 0) bars->odd = 1;
-              const long long at = (long long)(t.x_row0 + c + k * kEpilogueWarps) * p.ld + p.col0 + n4;
-              for (int q = 0; q < p.n_out; ++q) {
-                T* dst = static_cast<T*>(p.y_out[q]) + at;
-                if (n4 + 4 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
-                  *reinterpret_cast<uint2*>(dst) = o;
-                } else {
-                  const T* e = reinterpret_cast<const T*>(&o);
-                  for (int i = 0; i < 4 && n4 + i < p.N; ++i) dst[i] = e[i];
-                }
-              }
-            }
+          if (u + pairs >= total) {
+            if (warp == kFirstEpilogue && lane == 0) bars->help = 1;   // below, with the unpack warps
+          } else if (sum_parts<T, kEpilogueWarps, kSplit>(p, t, rank, warp - kFirstEpilogue, lane)) {
+            bars->odd = 1;
           }
         }
         asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueWarps * 32) : "memory");   // `last` may be written again
       }
     }
+  }
+  if (warp >= kFirstUnpack) {
+    // A pair's last unit, where it is part of a cut tile and this block the last of the tile's, is added up by the unpack warps
+    // too, which have nothing left to do.
+    constexpr int kAll = kUnpackWarps + kEpilogueWarps;
+    __syncwarp();
+    asm volatile("bar.sync 4, %0;" ::"n"(kAll * 32) : "memory");
+    if (bars->help) {
+      const int u = pair + (total - 1 - pair) / pairs * pairs;
+      if (sum_parts<T, kAll, kSplit>(p, unit_at(p, u, rank), rank, warp - kFirstUnpack, lane)) bars->odd = 1;
+    }
     if constexpr (kSplit) {
       __syncwarp();
-      asm volatile("bar.sync 3, %0;" ::"n"(kEpilogueWarps * 32) : "memory");   // every result and every `odd` is there
-      if (bars->odd != 0) {
+      asm volatile("bar.sync 4, %0;" ::"n"(kAll * 32) : "memory");   // every result and every `odd` is there
+      if (warp >= kFirstEpilogue && bars->odd != 0) {
         for (int u = pair; u < total; u += pairs) {
           const Unit t = unit_at(p, u, rank);
           if (t.parts == 1 || (bars->ended >> ((u - p.full) / pairs & 31) & 1)) repair<T, BITS, !kT>(p, t.n0, t.x_row0, t.rows);
@@ -1114,7 +1167,7 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, Form f) {
     const int64_t waves = tiles / pairs;
     const int rem = (int)(tiles - waves * pairs);
     // s parts per tile, on rem * s pairs; or, where that leaves pairs idle, an equal range for every pair
-    for (int s = 1; s <= 16 && (s == 1 || s * 4 <= kst); ++s) {
+    for (int s = 1; s <= 16 && (s == 1 || (s * 4 <= kst && (long long)pairs * pairs * (kst + 1) < INT32_MAX)); ++s) {
       const bool all = (long long)rem * s > pairs;
       const int cut = all ? pairs : rem * s;
       double last = 0.0;
@@ -1221,6 +1274,12 @@ int launch_tc(int dtype, int bits, int group, Form f, long long units, cudaStrea
   long long nsb = (long long)((kSmemMax - fixed) / stage);
   p.nsb = (int)(nsb > kMaxStagesB ? kMaxStagesB : nsb);
   size_t smem = fixed + p.nsb * stage;
+  // What is left holds more chunks of scales.
+  const size_t chunk = 2 * kTileRows * (size_t)p.cb;
+  while (2 * p.s_slots <= kMaxSlotsS && smem + p.s_slots * chunk <= kSmemMax) {
+    smem += p.s_slots * chunk;
+    p.s_slots *= 2;
+  }
   // More than half of an SM's shared memory: guarantees one block per SM, so the 512-column
   // tensor-memory allocation never has to wait for a co-resident block of this kernel.
   if (smem < 120 * 1024) smem = 120 * 1024;
