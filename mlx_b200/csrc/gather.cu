@@ -165,16 +165,17 @@ int pick_nt(int64_t n_rows, int64_t E) {
 
 struct FastLayout {
   size_t hdr, sorted, lhs, dst, mtiles, xs, total;
-  int64_t n_rows, max_mtiles, max_few;   // max_few: tiles of kRowsTile rows
+  int64_t n_rows, max_mtiles, max_few;   // max_few: tiles of rows_tile rows, at most
   int nt;
 };
 
 FastLayout fast_layout(int64_t n_idx, int64_t E, int64_t M, int64_t K) {
+  constexpr int kLeast = 4;   // rows of the smallest tile that rows_tile gives
   FastLayout L{};
   L.n_rows = n_idx * M;
   L.nt = pick_nt(L.n_rows, E);
   L.max_mtiles = L.n_rows / L.nt + E + 1;
-  L.max_few = L.n_rows / kRowsTile + (E < L.n_rows ? E : L.n_rows);
+  L.max_few = L.n_rows / kLeast + (E < L.n_rows ? E : L.n_rows);
   size_t off = 0;
   L.hdr = off; off += align256(sizeof(Header));
   L.sorted = off; off += align256((size_t)n_idx * 4);
@@ -215,7 +216,7 @@ RowsGroup rows_group(const FastLayout& L, char* base, int64_t E, int64_t M, int6
   RowsGroup r{};
   r.tiles = base + L.mtiles;
   r.n_tiles = &reinterpret_cast<Header*>(base + L.hdr)->n_mtiles;
-  r.max_tiles = L.max_few;
+  r.max_tiles = L.n_rows / rows_tile(bits, group) + (E < L.n_rows ? E : L.n_rows);
   r.per_slot = M; r.E = E; r.N = N; r.K = K;
   r.group = group; r.bits = bits;
   r.status = status;
@@ -244,7 +245,7 @@ int run_grouped(const void* x, const uint32_t* wq, const void* scales, const voi
   set_matrix(r, 0, wq, scales, biases);
   if (!peers && few_rows(L.n_rows, E_total) && qmv_rows_grouped_supported(r)) {
     gather_sort_kernel<<<1, 1024, 0, st>>>(pairs, (int)n_idx, (uint32_t)x_batch, (uint32_t)E_total, (uint32_t)e_lo, (uint32_t)E_local,
-                                           (int)M, kRowsTile, hdr, sorted, slhs, mt, y, (size_t)M * N * 2, status);
+                                           (int)M, rows_tile(bits, group_size), hdr, sorted, slhs, mt, y, (size_t)M * N * 2, status);
     B200Q_LAUNCH_OK("gather_sort_kernel");
     r.x = x; r.src_slot = slhs; r.y = y; r.dst_slot = sorted;
     return qmv_rows_grouped(r, st);
@@ -444,7 +445,7 @@ extern "C" int b200q_gather_qmm_chain(const void* x, const uint32_t* wq1, const 
   set_matrix(r2, 0, wq2, scales2, biases2);
   if (few_rows(L.n_rows, E) && qmv_rows_grouped_supported(r1) && qmv_rows_grouped_supported(r2)) {
     gather_sort_kernel<<<1, 1024, 0, st>>>(plain_pairs(lhs_idx, rhs_idx), (int)n_idx, (uint32_t)x_batch, (uint32_t)E, 0u, (uint32_t)E,
-                                           (int)M, kRowsTile, hdr, sorted, slhs, mt, y, (size_t)M * N2 * 2, status);
+                                           (int)M, rows_tile(bits, group_size), hdr, sorted, slhs, mt, y, (size_t)M * N2 * 2, status);
     B200Q_LAUNCH_OK("gather_sort_kernel");
     r1.x = x; r1.src_slot = slhs; r1.y = h;
     if (int rc = qmv_rows_grouped(r1, st)) return rc;
@@ -544,7 +545,7 @@ int swiglu_impl(const void* x, const uint32_t* wq_gate, const void* scales_gate,
   set_matrix(r1, 1, wq_up, scales_up, biases_up);
   set_matrix(r2, 0, wq_down, scales_down, biases_down);
   if (few_rows(L.n_rows, E) && qmv_rows_grouped_supported(r1) && qmv_rows_grouped_supported(r2)) {
-    gather_sort_kernel<<<1, 1024, 0, st>>>(pairs, (int)n_idx, (uint32_t)x_batch, (uint32_t)E, 0u, (uint32_t)E, (int)M, kRowsTile, hdr,
+    gather_sort_kernel<<<1, 1024, 0, st>>>(pairs, (int)n_idx, (uint32_t)x_batch, (uint32_t)E, 0u, (uint32_t)E, (int)M, rows_tile(bits, group_size), hdr,
                                            sorted, slhs, mt, y, (size_t)M * N2 * 2, status);
     B200Q_LAUNCH_OK("gather_sort_kernel");
     r1.x = x; r1.src_slot = slhs; r1.y = hg;

@@ -105,9 +105,9 @@ struct GroupedArgs {
   PeerOut peers;            // n > 0: every result row is stored into all of these [n_rows, N] buffers
 };
 
-// The row-owning decode kernel over the experts that have rows, for tiles of up to 8 expert-sorted rows.  With a
-// second matrix the result is silu(x W0^T) * (x W1^T).
-constexpr int kRowsTile = 8;
+// The row-owning decode kernel over the experts that have rows, for tiles of up to 8 expert-sorted rows (rows_tile: 4 where
+// groups of 32 take columns of their own).  With a second matrix the result is silu(x W0^T) * (x W1^T).
+int rows_tile(int bits, int group);
 struct RowsGroup {
   const void* x;            // bf16 rows of K
   const uint32_t* wq[2];    // [E, N, K*bits/32]; the second may be null
@@ -143,7 +143,7 @@ bool qmv_mma_supported(const QmmArgs& a);
 size_t qmv_mma_workspace_bytes(const QmmArgs& a);
 int qmv_mma(const QmmArgs& a, cudaStream_t st);
 
-// qmv_rows.cu : decode path, bf16 and f16, bits 2/4/8, every CTA owns whole weight rows (bulk-copy ring, no scratch)
+// qmv_rows.cu : decode path, bf16 and f16, every CTA owns whole weight rows (bulk-copy ring, no scratch)
 bool qmv_rows_supported(const QmmArgs& a);
 int qmv_rows(const QmmArgs& a, cudaStream_t st);
 // Promise that weights are not written by the stream operation preceding a matmul (see qmv_rows.cu).

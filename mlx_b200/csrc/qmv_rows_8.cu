@@ -1,0 +1,8 @@
+// The row-owning decode kernel for 8-bit weights.
+#include "qmv_rows.cuh"
+
+namespace b200q {
+namespace rows {
+template int launch_rows<8>(const RowsPlan& pl, cudaStream_t st);
+}
+}  // namespace b200q
