@@ -1051,7 +1051,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcPar
         asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueWarps * 32) : "memory");
         if (bars->last) {
           if (kSplit && warp == kFirstEpilogue && lane == 0) bars->ended |= 1u << ((u - p.full) / pairs & 31);
-          if (u + pairs >= total) {
+          if (!kSplit && u + pairs >= total) {
             if (warp == kFirstEpilogue && lane == 0) bars->help = 1;   // below, with the unpack warps
           } else if (sum_parts<T, kEpilogueWarps, kSplit>(p, t, rank, warp - kFirstEpilogue, lane)) {
             bars->odd = 1;
@@ -1061,20 +1061,23 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcPar
       }
     }
   }
-  if (warp >= kFirstUnpack) {
-    // A pair's last unit, where it is part of a cut tile and this block the last of the tile's, is added up by the unpack warps
-    // too, which have nothing left to do.
-    constexpr int kAll = kUnpackWarps + kEpilogueWarps;
-    __syncwarp();
-    asm volatile("bar.sync 4, %0;" ::"n"(kAll * 32) : "memory");
-    if (bars->help) {
-      const int u = pair + (total - 1 - pair) / pairs * pairs;
-      if (sum_parts<T, kAll, kSplit>(p, unit_at(p, u, rank), rank, warp - kFirstUnpack, lane)) bars->odd = 1;
-    }
-    if constexpr (kSplit) {
+  if constexpr (!kSplit) {
+    if (warp >= kFirstUnpack) {
+      // A pair's last unit, where it is part of a cut tile and this block the last of the tile's, is added up by the unpack warps
+      // too, which have nothing left to do.  (The split forms' loops have no registers for it: 1531 f16 tokens 275 -> 279 us.)
+      constexpr int kAll = kUnpackWarps + kEpilogueWarps;
       __syncwarp();
-      asm volatile("bar.sync 4, %0;" ::"n"(kAll * 32) : "memory");   // every result and every `odd` is there
-      if (warp >= kFirstEpilogue && bars->odd != 0) {
+      asm volatile("bar.sync 4, %0;" ::"n"(kAll * 32) : "memory");
+      if (bars->help) {
+        const int u = pair + (total - 1 - pair) / pairs * pairs;
+        sum_parts<T, kAll, false>(p, unit_at(p, u, rank), rank, warp - kFirstUnpack, lane);
+      }
+    }
+  } else {
+    if (warp >= kFirstEpilogue) {
+      __syncwarp();
+      asm volatile("bar.sync 3, %0;" ::"n"(kEpilogueWarps * 32) : "memory");   // every result and every `odd` is there
+      if (bars->odd != 0) {
         for (int u = pair; u < total; u += pairs) {
           const Unit t = unit_at(p, u, rank);
           if (t.parts == 1 || (bars->ended >> ((u - p.full) / pairs & 31) & 1)) repair<T, BITS, !kT>(p, t.n0, t.x_row0, t.rows);

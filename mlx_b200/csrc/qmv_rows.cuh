@@ -354,6 +354,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       __syncwarp();
       asm volatile("bar.arrive 2, 64;" ::: "memory");   // the scales warp does not wait for the others
+      asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");
       // ================================= loader warp ==========================================
       // Without the caller's promise the weights may have been written by the previous kernel.
       if (kGrouped || !p.early) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -381,14 +382,14 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
                         pairs && lane_row + 1 < rows ? 2 * bytes : bytes, bar);
             dst += p.slot_bytes;
             if (++slot == nst) { slot = 0; ++use; dst -= nst * p.slot_bytes; }
-            // One stage; the rest once x is in registers, which would else wait behind a ring full of weights (one row of x
-            // through [14336, 4096]: 8400 cycles instead of 3000).
-            if (!met) { met = true; asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory"); }
+            // One stage; the rest once the consumers have asked for x, which would else wait behind a ring full of weights (one row of
+            // x through [14336, 4096]: 8400 cycles instead of 3000), or, with x of 9 to 16 tokens, once they have it (16 rows: 14.1 us
+            // against 15.1; 3 rows of f16 through [11008, 4096] at 8 bits the other way, 12.3 and 11.65).
+            if (!met) { met = true; asm volatile("bar.sync 4, %0;" ::"r"(32 * (p.n_active + 1)) : "memory"); }
           }
         }
         more = kGrouped && ok && next_segment(at);
       }
-      if (!met) asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
       if (!ok) {   // the copies in flight still write to this block's shared memory
         for (int i = 0; i < nst; ++i) {
           const int n = use + (i < slot ? 1 : 0);
@@ -658,6 +659,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
             }
           }
         }
+        if (MT == 1 && first) asm volatile("bar.arrive 4, %0;" ::"r"(32 * (p.n_active + 1)) : "memory");   // x is on its way
         // Group sums of x by MMAs with x as the other operand (tokens as rows, times ones; summing by adds took 9 instructions
         // per register, most of the 3000 cycles between a launch's start and its first product).  Lane t keeps groups 2t, 2t+1.
         float e[MT][2];
@@ -706,6 +708,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
           sx_hi[mt] = hi;
           sx_lo[mt] = pack_x2<T>(e0 - lo_f<T>(hi), e1 - hi_f<T>(hi));
         }
+        if (MT == 2 && first) asm volatile("bar.arrive 4, %0;" ::"r"(32 * (p.n_active + 1)) : "memory");
         if (first) { meet(); first = false; }
         // ldmatrix roles of this lane: matrix m = lane / 8 covers rows (m & 1) * 8 .. +7 of unit (m >> 1)
         // (row i of the MMA's upper half is row 2i of the stage, of its lower half row 2i + 1)
@@ -723,7 +726,10 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
           for (int gq = 0; gq < NGW; gq += 2) {
             if (gq < lim) {
               float acc[2][MT][4];
-              uint32_t sl2 = 0, sh2 = 0;
+              // (a group past the row's end multiplies what is there with x registers that are zero, and with a zero scale)
+              uint32_t sl2, sh2;
+              auto read_scales = [&]() { sl2 = lds_u32(sa + 2 * gq); sh2 = lds_u32(sa + s8 + 2 * gq); };
+              if constexpr (BITS == 8) read_scales();   // (8 rows through [14336, 4096]: 15.2 us before the words, 16.4 after; 4 bits the other way)
               // units iu, iu + 1 of both groups (of one unit each: both at once); a few words at a time, for registers
               constexpr int UB = UG == 1 ? 1 : 2;
 #pragma unroll
@@ -736,10 +742,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
 #pragma unroll
                   for (int u = 0; u < 2; ++u) ldmatrix_x4(wa + ((gq + u) * UG + i0u) * 16, wl[u][0], wh[u][0], wl[u][UB - 1], wh[u][UB - 1]);
                 }
-                if (i0u == 0) {   // (a group past the row's end multiplies what is there with x registers that are zero, and with a zero scale)
-                  sl2 = lds_u32(sa + 2 * gq);
-                  sh2 = lds_u32(sa + s8 + 2 * gq);
-                }
+                if (BITS != 8 && i0u == 0) read_scales();
 #pragma unroll
                 for (int iu = i0u; iu < i0u + UB; ++iu) {
 #pragma unroll
@@ -844,6 +847,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
             xs[j][nt][0] = d[0];
             xs[j][nt][1] = d[1];
           }
+          if (nt == 0 && first) asm volatile("bar.arrive 4, %0;" ::"r"(32 * (p.n_active + 1)) : "memory");   // x is on its way
           const int E = exponent(quad_max(m));
           const uint32_t e1 = (uint32_t)((is_bf16<T> ? 127 : 15) + E);
 #pragma unroll
