@@ -354,7 +354,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       __syncwarp();
       asm volatile("bar.arrive 2, 64;" ::: "memory");   // the scales warp does not wait for the others
-      asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");
+      if (MT == 1) asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");
       // ================================= loader warp ==========================================
       // Without the caller's promise the weights may have been written by the previous kernel.
       if (kGrouped || !p.early) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -385,7 +385,11 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
             // One stage; the rest once the consumers have asked for x, which would else wait behind a ring full of weights (one row of
             // x through [14336, 4096]: 8400 cycles instead of 3000), or, with x of 9 to 16 tokens, once they have it (16 rows: 14.1 us
             // against 15.1; 3 rows of f16 through [11008, 4096] at 8 bits the other way, 12.3 and 11.65).
-            if (!met) { met = true; asm volatile("bar.sync 4, %0;" ::"r"(32 * (p.n_active + 1)) : "memory"); }
+            if (!met) {
+              met = true;
+              if (MT == 2) asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+              else asm volatile("bar.sync 4, %0;" ::"r"(32 * (p.n_active + 1)) : "memory");
+            }
           }
         }
         more = kGrouped && ok && next_segment(at);
@@ -708,7 +712,6 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
           sx_hi[mt] = hi;
           sx_lo[mt] = pack_x2<T>(e0 - lo_f<T>(hi), e1 - hi_f<T>(hi));
         }
-        if (MT == 2 && first) asm volatile("bar.arrive 4, %0;" ::"r"(32 * (p.n_active + 1)) : "memory");
         if (first) { meet(); first = false; }
         // ldmatrix roles of this lane: matrix m = lane / 8 covers rows (m & 1) * 8 .. +7 of unit (m >> 1)
         // (row i of the MMA's upper half is row 2i of the stage, of its lower half row 2i + 1)
@@ -847,7 +850,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
             xs[j][nt][0] = d[0];
             xs[j][nt][1] = d[1];
           }
-          if (nt == 0 && first) asm volatile("bar.arrive 4, %0;" ::"r"(32 * (p.n_active + 1)) : "memory");   // x is on its way
+          if (MT == 1 && nt == 0 && first) asm volatile("bar.arrive 4, %0;" ::"r"(32 * (p.n_active + 1)) : "memory");   // x is on its way
           const int E = exponent(quad_max(m));
           const uint32_t e1 = (uint32_t)((is_bf16<T> ? 127 : 15) + E);
 #pragma unroll
