@@ -84,7 +84,6 @@ constexpr int kUnpackWarps = 16;
 constexpr int kEpilogueWarps = 8;
 constexpr int kFirstUnpack = 4, kFirstEpilogue = kFirstUnpack + kUnpackWarps;
 constexpr int kThreads = 32 * (kFirstEpilogue + kEpilogueWarps);   // 896
-constexpr int kStageOut = 4096;    // bytes of the epilogue's staging tile per warp: 64 tokens x 32 columns
 constexpr size_t kSmemMax = 227 * 1024;
 
 template <int BITS, Form F>
@@ -105,6 +104,10 @@ struct Shape {
   static constexpr int kPRowBytes = 16 * BITS;                 // 128 fields
   static constexpr int kPStageBytes = kTileRows * kPRowBytes;
   static constexpr int kSmemA = kT ? kSlotsA * 32768 : 0;      // 64 k x 128 columns, hi and lo
+  // Tokens (x 32 columns, 64 bytes) of the epilogue's staging tile per warp.  SplitT, whose A ring takes 96 KB: half as many, so that
+  // 256 tokens of x have two stages at 5, 6 and 8 bits too.
+  static constexpr int kOutTok = kT ? 32 : 64;
+  static constexpr int kStageOut = kOutTok * 64;
   static constexpr int kPArrivals = kSub * kUnpackWarps / kSets;   // of a packed stage: every set that takes one of its slots
 };
 
@@ -617,7 +620,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcPar
   unsigned char* ring_p = ring_b + (size_t)p.nsb * b_stage;
   unsigned char* ring_s = ring_p + (size_t)nsp * S::kPStageBytes;   // per chunk: 128 rows of scales, 128 of biases
   unsigned char* staging = ring_s + p.s_slots * 2 * kTileRows * p.cb;    // a tile per epilogue warp
-  Barriers* bars = reinterpret_cast<Barriers*>(staging + kEpilogueWarps * kStageOut);
+  Barriers* bars = reinterpret_cast<Barriers*>(staging + kEpilogueWarps * S::kStageOut);
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -976,7 +979,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcPar
     // ------------------------------------------------------------ epilogue
     const int quad = warp & 3;
     const int chalf = (warp - kFirstEpilogue) >> 2;  // which half of the token columns
-    const uint32_t stg = smem_u32(staging) + (warp - kFirstEpilogue) * kStageOut;
+    const uint32_t stg = smem_u32(staging) + (warp - kFirstEpilogue) * S::kStageOut;
     const uint32_t lane_field = (uint32_t)(quad * 32) << 16;
     uint32_t tcount = 0;
     for (int u = pair; u < total; u += pairs, ++tcount) {
@@ -1005,9 +1008,9 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcPar
       if (t.parts == 1 && (ROWS16 || p.y_align == 8)) {
         uint32_t r[2][16];
         load_piece(acc + c_begin, r[0]);
-        for (int c0 = c_begin; c0 < c_end; c0 += 64) {
+        for (int c0 = c_begin; c0 < c_end; c0 += S::kOutTok) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
+          for (int i = 0; i < S::kOutTok / 16; ++i) {
             const int c = c0 + 16 * i;
             if (c < c_end) {                             // (halves are whole 16-column pieces)
               tcgen05_wait_ld16(r[i & 1]);
@@ -1017,7 +1020,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcPar
             }
           }
           __syncwarp();
-          if (store_chunk<T, ROWS16, kSplit>(p, t, stg, lane, t.n0 + quad * 32, c0, min(min(t.rows, c_end) - c0, 64))) bars->odd = 1;
+          if (store_chunk<T, ROWS16, kSplit>(p, t, stg, lane, t.n0 + quad * 32, c0, min(min(t.rows, c_end) - c0, S::kOutTok))) bars->odd = 1;
           __syncwarp();   // the staging tile may be written again
         }
       } else {
@@ -1135,7 +1138,7 @@ Form form_of(int dtype, bool transpose) {
 template <int BITS, Form F>
 size_t fixed_smem(int cb, int slots, bool few) {
   using S = Shape<BITS, F>;
-  return 1024 + S::kSmemA + (size_t)(few ? S::kFewStagesP : S::kStagesP) * S::kPStageBytes + (size_t)slots * 2 * kTileRows * cb + kEpilogueWarps * kStageOut +
+  return 1024 + S::kSmemA + (size_t)(few ? S::kFewStagesP : S::kStagesP) * S::kPStageBytes + (size_t)slots * 2 * kTileRows * cb + kEpilogueWarps * S::kStageOut +
          sizeof(Barriers) + 64;
 }
 size_t fixed_smem(int bits, Form f, int cb, int slots, bool few) {
