@@ -2,9 +2,10 @@
 //
 // Kernel selection for b200q_qmm (the role of QuantizedMatmul::eval_gpu's dispatch,
 // mlx/backend/cuda/quantized/quantized.cpp:106-136):
-//   bf16, f16, transpose, M <= 32, bits 2/4/8, K % (16 * group) == 0 -> qmv_rows (HBM-bound decode; above 16 rows in
-//       two passes.  bf16 keeps the weights' exact value there, which one tensor-core tile of 17 to 32 rows rounds: the
-//       result is off by 1.7e-3 of its norm against 2.2e-3)
+//   bf16, f16, transpose, K % 128 == 0, few rows                 -> qmv_rows (HBM-bound decode).  2, 4 and 8 bits: M <= 16, and
+//       up to 32 in two passes where K % (16 * group) == 0 (bf16 keeps the weights' exact value there, which one tensor-core
+//       tile of 17 to 32 rows rounds: the result is off by 1.7e-3 of its norm against 2.2e-3); 3, 5 and 6 bits, and 2 bits in
+//       groups of 32: M <= 16, 8, 4 in groups of 128, 64, 32
 //   bf16, transpose, M <= 16, K % 128 == 0 (any width)           -> qmv_mma     (register-path decode)
 //   bf16, f16, transpose, K % 128 == 0                           -> qmm_tcgen05 (TMA + tcgen05 + TMEM)
 //   bf16, f16, transpose == 0, M > 16, N % 128 == 0              -> qmm_tcgen05 (fewer rows waste half of the 32-token tile)
