@@ -199,18 +199,21 @@ bool fast_supported(int dtype, int64_t n_idx, int64_t x_batch, int64_t E, int64_
 
 
 // Experts with few rows go through the row-owning decode kernel: it does not round the weights (error against 64 bits 1.65e-3
-// of the result, tensor cores 2.2e-3), reads a matrix at up to 1.6 times the rate at which the tensor-core kernel unpacks
-// one, takes the rows of x where they lie and needs no second launch for a gated pair.  At more than about four rows per
-// expert the tiles of 8 rows begin to split experts, and every part reads the matrix again.  Measured (us, this kernel / tensor
-// cores, uniform routing):
-//   4 bits  16 experts [7168, 4096], 16 to 64 rows 56 to 76 / 77 to 101; 8 [14336, 4096], 32 rows 75 / 101;
-//           16 [2048, 2048], 16 and 64 rows 21 and 27 / 26 and 27; 32 [4096, 2048], 64 and 128 rows 63 and 77 / 56 and 63;
-//           64 [2048, 2048], 64 and 256 rows 51 and 75 / 48 and 63; 64 [1024, 1024], 256 rows 41 / 29
-//   2 bits  64 [2048, 2048], 64 and 256 rows 48 and 69 / 62 and 83
-//   8 bits  (the other side is qmm_tc_single.cu) 64 [2048, 2048], 256 rows 70 / 135
-// With short K the tensor cores would be up to 1.4 times as fast at 4 bits; the line stays for the weights' sake.  All rows on
-// one expert, which the host cannot see, is this kernel's worst case: 64 [2048, 2048], 256 rows 39 us, tensor cores 20 to 30.
-bool few_rows(int64_t n_rows, int64_t E) { return n_rows <= 4 * E; }
+// of the result, tensor cores 2.2e-3), takes the rows of x where they lie and needs no second launch for a gated pair.  Beyond a tile's
+// rows (8; 4 where groups of 32 take MMA columns) every part of an expert reads the matrix again.  Measured at 5, 6 and 8 rows per
+// expert (us, this kernel / tensor cores, uniform routing):
+//   2 bits  64 [2048, 2048] 49, 52, 60 / 84; 8 [14336, 4096] 54, 54, 70 / 145
+//   4 bits  16 [2048, 2048] 20, 21, 24 / 26; 64 [2048, 2048] 51, 54, 65 / 59; 8 [14336, 4096] 57, 60, 74 / 97
+//   8 bits  64 [2048, 2048] 59, 60, 77 / 63; 8 [14336, 4096] 95, 96, 114 / 106
+//   3 bits, groups of 128   64 [2048, 2048] 52, 57, 68 / 62; 8 [14336, 4096] 68, 68, 89 / 100
+//   6 bits  64 [2048, 2048] 71, 77, 92 / 70 (4 rows: 69); 8 [14336, 4096] 123, 123, 147 / 118 (4 rows: 109)
+//   6 bits, groups of 32   64 [2048, 2048] 105, 125, 152 / 75; 16 [4096, 2048] gated, 2 rows 105 / 140
+// All rows on one expert, which the host cannot see: 64 [2048, 2048] at 4 bits, 256 rows 28.
+bool few_rows(int64_t n_rows, int64_t E, int bits, int group) {
+  const bool runs = bits == 3 || bits == 5 || bits == 6 || (bits == 2 && group == 32);
+  const int64_t most = runs && group == 32 ? 2 : (bits == 2 ? 8 : (bits == 5 || bits == 6 ? 4 : 6));
+  return n_rows <= most * E;
+}
 
 RowsGroup rows_group(const FastLayout& L, char* base, int64_t E, int64_t M, int64_t N, int64_t K, int group, int bits, uint32_t* status) {
   RowsGroup r{};
@@ -243,7 +246,7 @@ int run_grouped(const void* x, const uint32_t* wq, const void* scales, const voi
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(base + L.xs);
   RowsGroup r = rows_group(L, base, E_local, M, N, K, group_size, bits, status);
   set_matrix(r, 0, wq, scales, biases);
-  if (!peers && few_rows(L.n_rows, E_total) && qmv_rows_grouped_supported(r)) {
+  if (!peers && few_rows(L.n_rows, E_total, bits, group_size) && qmv_rows_grouped_supported(r)) {
     gather_sort_kernel<<<1, 1024, 0, st>>>(pairs, (int)n_idx, (uint32_t)x_batch, (uint32_t)E_total, (uint32_t)e_lo, (uint32_t)E_local,
                                            (int)M, rows_tile(bits, group_size), hdr, sorted, slhs, mt, y, (size_t)M * N * 2, status);
     B200Q_LAUNCH_OK("gather_sort_kernel");
@@ -443,7 +446,7 @@ extern "C" int b200q_gather_qmm_chain(const void* x, const uint32_t* wq1, const 
   RowsGroup r1 = rows_group(L, base, E, M, N1, K1, group_size, bits, status), r2 = rows_group(L, base, E, M, N2, N1, group_size, bits, status);
   set_matrix(r1, 0, wq1, scales1, biases1);
   set_matrix(r2, 0, wq2, scales2, biases2);
-  if (few_rows(L.n_rows, E) && qmv_rows_grouped_supported(r1) && qmv_rows_grouped_supported(r2)) {
+  if (few_rows(L.n_rows, E, bits, group_size) && qmv_rows_grouped_supported(r1) && qmv_rows_grouped_supported(r2)) {
     gather_sort_kernel<<<1, 1024, 0, st>>>(plain_pairs(lhs_idx, rhs_idx), (int)n_idx, (uint32_t)x_batch, (uint32_t)E, 0u, (uint32_t)E,
                                            (int)M, rows_tile(bits, group_size), hdr, sorted, slhs, mt, y, (size_t)M * N2 * 2, status);
     B200Q_LAUNCH_OK("gather_sort_kernel");
@@ -544,7 +547,7 @@ int swiglu_impl(const void* x, const uint32_t* wq_gate, const void* scales_gate,
   set_matrix(r1, 0, wq_gate, scales_gate, biases_gate);
   set_matrix(r1, 1, wq_up, scales_up, biases_up);
   set_matrix(r2, 0, wq_down, scales_down, biases_down);
-  if (few_rows(L.n_rows, E) && qmv_rows_grouped_supported(r1) && qmv_rows_grouped_supported(r2)) {
+  if (few_rows(L.n_rows, E, bits, group_size) && qmv_rows_grouped_supported(r1) && qmv_rows_grouped_supported(r2)) {
     gather_sort_kernel<<<1, 1024, 0, st>>>(pairs, (int)n_idx, (uint32_t)x_batch, (uint32_t)E, 0u, (uint32_t)E, (int)M, rows_tile(bits, group_size), hdr,
                                            sorted, slhs, mt, y, (size_t)M * N2 * 2, status);
     B200Q_LAUNCH_OK("gather_sort_kernel");

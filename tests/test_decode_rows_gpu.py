@@ -126,3 +126,24 @@ def test_experts(bits, g, K, gated):
             if len(rows):
                 ref = O.qmm_f32_from(from_torch(x[rows, 0, 0]), wq[e].view(np.uint32), s[e], b[e], "bf16", transpose=True, group_size=g, bits=bits)
                 assert norm_error(O.to_f32(from_torch(y[rows, 0, 0]), "bf16"), ref) < limit("bf16", ref.size)
+
+
+@pytest.mark.parametrize("bits,g,line", [(2, 64, 8), (4, 64, 6), (8, 64, 6), (3, 128, 6), (6, 64, 4), (6, 32, 2), (2, 32, 2)])
+@pytest.mark.parametrize("beyond", (0, 1))
+def test_experts_on_both_sides_of_the_rule_for_few_rows(bits, g, line, beyond):
+    """The last row count of the row-owning kernel (tiles full, an expert with more rows than a tile's) and the first of the
+    tensor-core kernel, which rounds the weights."""
+    E, N, K = 3, 100, 384
+    rows = line * E + beyond
+    wq, s, b = O.quantize(make_w(bits, (E, N, K), "bf16"), g, bits, "bf16")
+    x = make_x(line, (rows, 1, K), "bf16")
+    idx = np.sort(np.arange(rows) % (E + 1)) % E   # expert 0 has about twice the others' rows
+    y = mb.gather_qmm(to_torch(x, "bf16"), u32_to_torch(wq), to_torch(s, "bf16"), to_torch(b, "bf16"),
+                      rhs_indices=torch.from_numpy(idx.astype(np.int64)).cuda(), group_size=g, bits=bits)
+    for e in range(E):
+        mine = np.flatnonzero(idx == e)
+        ref = O.qmm_f32_from(x[mine, 0], wq[e], s[e], b[e], "bf16", transpose=True, group_size=g, bits=bits)
+        got = O.to_f32(from_torch(y[torch.from_numpy(mine).cuda(), 0]), "bf16")
+        assert qmm_close(got, ref, 1e-2)[0]
+        if not beyond:
+            assert norm_error(got, ref) < limit("bf16", ref.size)
