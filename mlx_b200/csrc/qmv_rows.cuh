@@ -43,6 +43,7 @@
 #pragma once
 #include <type_traits>
 
+#include "bounded_wait.h"
 #include "common.cuh"
 #include "kernels.h"
 #include "qmv_rows.h"
@@ -162,18 +163,11 @@ __device__ __forceinline__ void sts_rows(uint32_t addr, float a, float b) {
 
 // Bounded wait that never parks the thread (try_wait may suspend it for a hardware-chosen time) and leaves issue slots to
 // the warps that share the scheduler.
-__device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  for (uint32_t i = 0; i < (1u << 23); ++i) {
-    if (mbar_test(bar, parity)) return true;
-    if ((i & 255u) == 255u && *abort_flag) return false;
-    __nanosleep(20);
-  }
-  *abort_flag = 1;
-  return false;
-}
+constexpr uint32_t kStatusRanOut = 7;
 // For a whole warp: all lanes go on or none.
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  return __all_sync(0xFFFFFFFFu, wait_for(bar, parity, abort_flag));
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status) {
+  return __all_sync(0xFFFFFFFFu, bounded_wait([=] { return mbar_test(bar, parity); }, [] { __nanosleep(20); }, 1u << 23, abort_flag,
+                                              status, kStatusRanOut));
 }
 
 // ---- units: one packed word -> NP registers of two subnormals each; register i holds fields (i, i + NP) of the word
@@ -371,7 +365,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
           const uint32_t off = (uint32_t)ph * p.phase_bytes, bytes = min(p.phase_bytes, p.row_bytes - off);
           for (int rg = 0; rg < nrg; ++rg) {
             // slot free: all consumer warps arrived for the stage that used it last
-            if (use > 0 && !warp_wait(done0 + 8 * slot, (use - 1) & 1, abort_flag)) { ok = false; break; }
+            if (use > 0 && !warp_wait(done0 + 8 * slot, (use - 1) & 1, abort_flag, p.status)) { ok = false; break; }
             const int row = seg.row0 + (NW == 2 ? rg >> 1 : rg) * 16, rows = min(16, p.N - row);
             const uint32_t bar = full0 + 8 * slot;
             if (lane == 0) mbar_expect_tx(bar, rows * bytes);
@@ -416,7 +410,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         for (int ph = 0; ok && ph < p.nph; ++ph) {
           const int g0 = ph * p.phase_groups, bytes = 2 * min(p.phase_groups, p.groups - g0), all = p.s_bytes;   // (zeros beyond the row)
           for (int rg = 0; rg < nrg; ++rg) {
-            if (use > 0 && !warp_wait(done0 + 8 * slot, (use - 1) & 1, abort_flag)) { ok = false; break; }
+            if (use > 0 && !warp_wait(done0 + 8 * slot, (use - 1) & 1, abort_flag, p.status)) { ok = false; break; }
             const int row = seg.row0 + (NW == 2 ? rg >> 1 : rg) * 16, which = NW == 2 ? rg & 1 : 0;
             const long long src = ((long long)(seg.base + min(row + r, p.N - 1)) * p.groups + g0) * 2;
             const char* s = reinterpret_cast<const char*>(p.scales[which]) + src;
@@ -467,7 +461,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         for (; red < end; ++red) {
           const int pbi = buffer_of(rrg, red);
           if (MT == 2 || (NW == 2 ? pbi >> 1 : pbi) == mine) {
-            if (!warp_wait(pfull0 + 8 * pbi, (MT == 2 || NW == 2 ? uses >> 1 : uses) & 1, abort_flag)) break;
+            if (!warp_wait(pfull0 + 8 * pbi, (MT == 2 || NW == 2 ? uses >> 1 : uses) & 1, abort_flag, p.status)) break;
             ++uses;
             float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
             if (tok < seg.rows) {
@@ -547,10 +541,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         __threadfence_system();
         asm volatile("bar.sync 3, 64;" ::: "memory");
       }
-      if (mine == 0 && lane == 0) {
-        peer_signal_tail(p.sig);
-        if (*abort_flag && p.status) atomicMax(&p.status[0], 7u);
-      }
+      if (mine == 0 && lane == 0) peer_signal_tail(p.sig);
     }
     return;
   }
@@ -718,7 +709,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         const uint32_t w_off = (lane & 7) * p.pitch + ((lane >> 3) & 1) * p.phase_bytes + (i0 * UG + (lane >> 4)) * 16;
         const uint32_t s_off = p.off_scales + g * p.spitch + 2 * i0, s8 = p.shalf;
         for (int rg = 0; rg < nrg; ++rg) {
-          if (!warp_wait(full0 + 8 * slot, use & 1, abort_flag)) return;
+          if (!warp_wait(full0 + 8 * slot, use & 1, abort_flag, p.status)) return;
           float out[MT][4];
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt)
@@ -792,7 +783,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
           }
           // the partial buffer has been read by its reducer
           const int pbi = buffer_of(rg, nth);
-          if (!warp_wait(pfree0 + 8 * pbi, (pphase >> pbi & 1) ^ 1, abort_flag)) return;
+          if (!warp_wait(pfree0 + 8 * pbi, (pphase >> pbi & 1) ^ 1, abort_flag, p.status)) return;
           pphase ^= 1u << pbi;
           ++nth;
           const uint32_t pa = pb_mine + (uint32_t)pbi * p.pbuf_bytes;
@@ -876,7 +867,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         const uint32_t c0 = 2 * ((2 * t) & (ng - 1)), c1 = 2 * ((2 * t + 1) & (ng - 1));   // byte offsets of the columns' groups in a chunk
         const uint32_t s_off = p.off_scales + g * p.spitch + 2 * (i0 << sh), s8 = p.shalf;
         for (int rg = 0; rg < nrg; ++rg) {
-          if (!warp_wait(full0 + 8 * slot, use & 1, abort_flag)) return;
+          if (!warp_wait(full0 + 8 * slot, use & 1, abort_flag, p.status)) return;
           float out[NT][4];
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt)
@@ -921,7 +912,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
           }
           // the partial buffer has been read by its reducer
           const int pbi = buffer_of(rg, nth);
-          if (!warp_wait(pfree0 + 8 * pbi, (pphase >> pbi & 1) ^ 1, abort_flag)) return;
+          if (!warp_wait(pfree0 + 8 * pbi, (pphase >> pbi & 1) ^ 1, abort_flag, p.status)) return;
           pphase ^= 1u << pbi;
           ++nth;
           const uint32_t pa = pb_mine + (uint32_t)pbi * p.pbuf_bytes;

@@ -24,3 +24,13 @@ def test_shim_compiles_and_validates(tmp_path):
     subprocess.run(cmd, check=True, capture_output=True, text=True)
     res = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert res.returncode == 0 and "SHIM-OK" in res.stdout, res.stdout + res.stderr
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_a_wait_that_runs_out_is_reported_by_the_role_that_waited(tmp_path):
+    """The decode kernel's wait, on the CPU: no order in which the roles of a block end may lose the report."""
+    exe = str(tmp_path / "bounded_wait_check")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "mlx_b200", "csrc"),
+                    os.path.join(ROOT, "tests", "bounded_wait_check.cpp"), "-o", exe], check=True, capture_output=True, text=True)
+    res = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert res.returncode == 0 and "WAIT-OK" in res.stdout, res.stdout + res.stderr
