@@ -164,10 +164,11 @@ __device__ __forceinline__ void sts_rows(uint32_t addr, float a, float b) {
 // Bounded wait that never parks the thread (try_wait may suspend it for a hardware-chosen time) and leaves issue slots to
 // the warps that share the scheduler.
 constexpr uint32_t kStatusRanOut = 7;
-// For a whole warp: all lanes go on or none.
+// For a whole warp: all lanes go on or none.  0.65 s from the last beat: the word after the abort flag, which changes while a
+// role waits for a peer's flag.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status) {
   return __all_sync(0xFFFFFFFFu, bounded_wait([=] { return mbar_test(bar, parity); }, [] { __nanosleep(20); }, 1u << 23, abort_flag,
-                                              status, kStatusRanOut));
+                                              reinterpret_cast<volatile uint32_t*>(abort_flag) + 1, status, kStatusRanOut));
 }
 
 // ---- units: one packed word -> NP registers of two subnormals each; register i holds fields (i, i + NP) of the word
@@ -288,10 +289,11 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
   static_assert(!kGrouped || MT == 1, "grouped tiles have up to 8 rows");
   extern __shared__ __align__(1024) unsigned char smem[];
   // header: [0, 128) "stage landed" barriers | [128, 256) "stage consumed" barriers |
-  //         [256, 288) "partial buffer free" barriers | [288, 320) "partial buffer full" | 320: abort flag
+  //         [256, 288) "partial buffer free" barriers | [288, 320) "partial buffer full" | 320: abort flag, beat
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t full0 = smem_base, done0 = smem_base + 128, pfree0 = smem_base + 256, pfull0 = smem_base + 288;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 320);
+  volatile uint32_t* beat = reinterpret_cast<volatile uint32_t*>(smem + 324);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -344,7 +346,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         mbar_init(pfree0 + 8 * lane, MT);
         mbar_init(pfull0 + 8 * lane, p.n_active);
       }
-      if (lane == 0) *abort_flag = 0;
+      if (lane == 0) { *abort_flag = 0; *beat = 0; }
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       __syncwarp();
       asm volatile("bar.arrive 2, 64;" ::: "memory");   // the scales warp does not wait for the others
@@ -404,12 +406,18 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
       const int r = lane >> 1;   // two lanes per row, pieces in turn
       uint32_t ds = smem_base + p.off_slots + p.off_scales + (r >> 1) * p.spitch + (r & 1) * p.shalf;
       const uint32_t db = 8 * p.spitch;
-      bool more = !kGrouped || next_segment(at), ok = true;
+      bool more = !kGrouped || next_segment(at), ok = true, met = !more;
+      // Its first wait comes after the consumers' for the kernel before and for a peer, which may be longer than its own may be.
+      auto meet_consumers = [&]() {
+        if (!met) asm volatile("bar.sync 5, 64;" ::: "memory");
+        met = true;
+      };
       while (more) {
         const int nrg = seg.n * NW;
         for (int ph = 0; ok && ph < p.nph; ++ph) {
           const int g0 = ph * p.phase_groups, bytes = 2 * min(p.phase_groups, p.groups - g0), all = p.s_bytes;   // (zeros beyond the row)
           for (int rg = 0; rg < nrg; ++rg) {
+            if (use > 0) meet_consumers();
             if (use > 0 && !warp_wait(done0 + 8 * slot, (use - 1) & 1, abort_flag, p.status)) { ok = false; break; }
             const int row = seg.row0 + (NW == 2 ? rg >> 1 : rg) * 16, which = NW == 2 ? rg & 1 : 0;
             const long long src = ((long long)(seg.base + min(row + r, p.N - 1)) * p.groups + g0) * 2;
@@ -438,6 +446,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         }
         more = kGrouped && ok && next_segment(at);
       }
+      meet_consumers();
       asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
       // ================================= reducer warps ========================================
@@ -447,7 +456,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
       const int mine = warp - (kConsumers + 1), mt = MT == 2 ? mine : 0;
       asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
       asm volatile("griddepcontrol.wait;" ::: "memory");   // y may still be in use by the previous kernel
-      if (lane == 0) peer_wait_previous(p.sig, p.status);  // ... or by a peer's consumer of the step before
+      if (lane == 0) peer_wait_previous(p.sig, p.status, beat);  // ... or by a peer's consumer of the step before
       __syncwarp();
       if constexpr (kGrouped) find_range();
       const int r4 = 4 * (lane & 3), tok = mt * 8 + g;
@@ -563,7 +572,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (p.sig.wait_flag != nullptr && p.sig.wait_x) {   // x is the gathered output of the previous exchange step
-    if (lane == 0) peer_wait_previous(p.sig, p.status);
+    if (lane == 0) peer_wait_previous(p.sig, p.status, beat);
     __syncwarp();
   }
   if constexpr (kGrouped) find_range();
@@ -572,6 +581,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
     meet();
     return;
   }
+  if (warp == 0) asm volatile("bar.arrive 5, 64;" ::: "memory");   // the scales warp may wait for stages from now on
   constexpr uint32_t kOne = is_bf16<T> ? 0x00800080u : 0x04000400u;      // one binary place of both halves
   constexpr uint32_t kOnes = is_bf16<T> ? 0x3F803F80u : 0x3C003C00u;     // (1, 1)
   constexpr float kOut = is_bf16<T> ? 0x1p69f : 1.0f;

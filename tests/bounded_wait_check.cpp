@@ -16,13 +16,14 @@ static void expect(const char* what, bool ok) {
 int main() {
   auto never = [] { return false; };
   auto idle = [] {};
+  volatile uint32_t beat = 0;
   {
     // the role that ends the block has gone by the flag before the last role's wait runs out: that one reports
     volatile int abort_flag = 0;
     uint32_t status = 0;
-    expect("a role that is done goes on", bounded_wait([] { return true; }, idle, 1000, &abort_flag, &status, 7));
+    expect("a role that is done goes on", bounded_wait([] { return true; }, idle, 1000, &abort_flag, &beat, &status, 7));
     expect("nothing to report yet", abort_flag == 0 && status == 0);
-    expect("the last wait runs out", !bounded_wait(never, idle, 1000, &abort_flag, &status, 7));
+    expect("the last wait runs out", !bounded_wait(never, idle, 1000, &abort_flag, &beat, &status, 7));
     expect("its expiry is in the status word", status == 7);
     expect("the others are told", abort_flag == 1);
   }
@@ -31,12 +32,25 @@ int main() {
     volatile int abort_flag = 1;
     uint32_t status = 9;
     int naps = 0;
-    expect("the flag ends a wait", !bounded_wait(never, [&] { ++naps; }, 1u << 20, &abort_flag, &status, 7));
+    expect("the flag ends a wait", !bounded_wait(never, [&] { ++naps; }, 1u << 20, &abort_flag, &beat, &status, 7));
     expect("soon", naps < 256);
     abort_flag = 0;
-    bounded_wait(never, idle, 10, &abort_flag, &status, 7);
+    bounded_wait(never, idle, 10, &abort_flag, &beat, &status, 7);
     expect("a larger code stays", status == 9);
-    expect("without a status word", !bounded_wait(never, idle, 10, &abort_flag, (uint32_t*)nullptr, 7));
+    expect("without a status word", !bounded_wait(never, idle, 10, &abort_flag, &beat, (uint32_t*)nullptr, 7));
+  }
+  {
+    // while another role waits for a peer, with a limit of its own, those that wait for it go on; then the count starts again
+    volatile int abort_flag = 0;
+    uint32_t status = 0;
+    int naps = 0;
+    auto peer = [&] {
+      if (++naps < 100000) beat = naps;
+    };
+    expect("landed at last", bounded_wait([&] { return naps >= 100200; }, peer, 1000, &abort_flag, &beat, &status, 7));
+    naps = 0;
+    expect("no beat, no end", !bounded_wait(never, peer, 1000, &abort_flag, &beat, &status, 7));
+    expect("the looks count from the last beat", naps > 100000 && naps < 102000 && status == 7);
   }
   if (!bad) std::printf("WAIT-OK\n");
   return bad;
