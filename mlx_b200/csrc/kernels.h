@@ -40,8 +40,8 @@ struct PeerOut {
 
 #ifdef __CUDACC__
 // Called by one lane of every warp that is about to touch what the previous exchange step's
-// consumers may still be using.  Returns false when the bound ran out (status word set).  `beat` changes while it waits.
-__device__ __forceinline__ bool peer_wait_previous(const PeerSignal& ps, uint32_t* status, volatile uint32_t* beat) {
+// consumers may still be using.  Returns false when the bound ran out (status word set).
+__device__ __forceinline__ bool peer_wait_previous(const PeerSignal& ps, uint32_t* status) {
   if (ps.wait_flag == nullptr) return true;
   const uint32_t expected = *reinterpret_cast<const volatile uint32_t*>(ps.epoch);
   const long long t0 = clock64();
@@ -49,12 +49,10 @@ __device__ __forceinline__ bool peer_wait_previous(const PeerSignal& ps, uint32_
     uint32_t v;
     asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(ps.wait_flag) : "memory");
     if ((int32_t)(v - expected) >= 0) return true;
-    const long long t = clock64();
-    if (t - t0 > ps.wait_limit) {
+    if (clock64() - t0 > ps.wait_limit) {
       if (status) { atomicMax(&status[0], 6u); status[1] = v; }
       return false;
     }
-    *beat = (uint32_t)t;
     __nanosleep(100);
   }
 }

@@ -161,14 +161,17 @@ __device__ __forceinline__ void sts_rows(uint32_t addr, float a, float b) {
   asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
 }
 
-// Bounded wait that never parks the thread (try_wait may suspend it for a hardware-chosen time) and leaves issue slots to
-// the warps that share the scheduler.
-constexpr uint32_t kStatusRanOut = 7;
-// For a whole warp: all lanes go on or none.  0.65 s from the last beat: the word after the abort flag, which changes while a
-// role waits for a peer's flag.
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status) {
-  return __all_sync(0xFFFFFFFFu, bounded_wait([=] { return mbar_test(bar, parity); }, [] { __nanosleep(20); }, 1u << 23, abort_flag,
-                                              reinterpret_cast<volatile uint32_t*>(abort_flag) + 1, status, kStatusRanOut));
+// Bounded wait (0.65 s) that never parks the thread (try_wait may suspend it for a hardware-chosen time) and leaves issue slots to
+// the warps that share the scheduler.  For a whole warp: all lanes go on or none.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xFFFFFFFFu, bounded_wait([=] { return mbar_test(bar, parity); }, [] { __nanosleep(20); }, [] { return false; }, 1u << 23,
+                                              abort_flag));
+}
+// The same for the loader and the scales warp, which start before the others and count from when those go: the word after the flag.
+// (Hardware barriers for that, before their first wait, cost decode 5 to 10 %.)
+__device__ __forceinline__ bool early_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xFFFFFFFFu, bounded_wait([=] { return mbar_test(bar, parity); }, [] { __nanosleep(20); }, [=] { return abort_flag[1] == 0; },
+                                              1u << 23, abort_flag));
 }
 
 // ---- units: one packed word -> NP registers of two subnormals each; register i holds fields (i, i + NP) of the word
@@ -289,11 +292,10 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
   static_assert(!kGrouped || MT == 1, "grouped tiles have up to 8 rows");
   extern __shared__ __align__(1024) unsigned char smem[];
   // header: [0, 128) "stage landed" barriers | [128, 256) "stage consumed" barriers |
-  //         [256, 288) "partial buffer free" barriers | [288, 320) "partial buffer full" | 320: abort flag, beat
+  //         [256, 288) "partial buffer free" barriers | [288, 320) "partial buffer full" | 320: abort flag, "all go"
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t full0 = smem_base, done0 = smem_base + 128, pfree0 = smem_base + 256, pfull0 = smem_base + 288;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 320);
-  volatile uint32_t* beat = reinterpret_cast<volatile uint32_t*>(smem + 324);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -346,7 +348,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         mbar_init(pfree0 + 8 * lane, MT);
         mbar_init(pfull0 + 8 * lane, p.n_active);
       }
-      if (lane == 0) { *abort_flag = 0; *beat = 0; }
+      if (lane == 0) abort_flag[0] = abort_flag[1] = 0;
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       __syncwarp();
       asm volatile("bar.arrive 2, 64;" ::: "memory");   // the scales warp does not wait for the others
@@ -367,7 +369,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
           const uint32_t off = (uint32_t)ph * p.phase_bytes, bytes = min(p.phase_bytes, p.row_bytes - off);
           for (int rg = 0; rg < nrg; ++rg) {
             // slot free: all consumer warps arrived for the stage that used it last
-            if (use > 0 && !warp_wait(done0 + 8 * slot, (use - 1) & 1, abort_flag, p.status)) { ok = false; break; }
+            if (use > 0 && !early_wait(done0 + 8 * slot, (use - 1) & 1, abort_flag)) { ok = false; break; }
             const int row = seg.row0 + (NW == 2 ? rg >> 1 : rg) * 16, rows = min(16, p.N - row);
             const uint32_t bar = full0 + 8 * slot;
             if (lane == 0) mbar_expect_tx(bar, rows * bytes);
@@ -406,19 +408,13 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
       const int r = lane >> 1;   // two lanes per row, pieces in turn
       uint32_t ds = smem_base + p.off_slots + p.off_scales + (r >> 1) * p.spitch + (r & 1) * p.shalf;
       const uint32_t db = 8 * p.spitch;
-      bool more = !kGrouped || next_segment(at), ok = true, met = !more;
-      // Its first wait comes after the consumers' for the kernel before and for a peer, which may be longer than its own may be.
-      auto meet_consumers = [&]() {
-        if (!met) asm volatile("bar.sync 5, 64;" ::: "memory");
-        met = true;
-      };
+      bool more = !kGrouped || next_segment(at), ok = true;
       while (more) {
         const int nrg = seg.n * NW;
         for (int ph = 0; ok && ph < p.nph; ++ph) {
           const int g0 = ph * p.phase_groups, bytes = 2 * min(p.phase_groups, p.groups - g0), all = p.s_bytes;   // (zeros beyond the row)
           for (int rg = 0; rg < nrg; ++rg) {
-            if (use > 0) meet_consumers();
-            if (use > 0 && !warp_wait(done0 + 8 * slot, (use - 1) & 1, abort_flag, p.status)) { ok = false; break; }
+            if (use > 0 && !early_wait(done0 + 8 * slot, (use - 1) & 1, abort_flag)) { ok = false; break; }
             const int row = seg.row0 + (NW == 2 ? rg >> 1 : rg) * 16, which = NW == 2 ? rg & 1 : 0;
             const long long src = ((long long)(seg.base + min(row + r, p.N - 1)) * p.groups + g0) * 2;
             const char* s = reinterpret_cast<const char*>(p.scales[which]) + src;
@@ -446,7 +442,6 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         }
         more = kGrouped && ok && next_segment(at);
       }
-      meet_consumers();
       asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
       // ================================= reducer warps ========================================
@@ -454,10 +449,11 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
       // keep running sums while K is walked in phases).  A lane has four consecutive rows of a token.  Each of the two warps takes
       // every other row group, or (MT = 2) eight of the tokens: one warp took longer per stage than the products.
       const int mine = warp - (kConsumers + 1), mt = MT == 2 ? mine : 0;
-      asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
       asm volatile("griddepcontrol.wait;" ::: "memory");   // y may still be in use by the previous kernel
-      if (lane == 0) peer_wait_previous(p.sig, p.status, beat);  // ... or by a peer's consumer of the step before
+      if (lane == 0) peer_wait_previous(p.sig, p.status);  // ... or by a peer's consumer of the step before
       __syncwarp();
+      asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+      abort_flag[1] = 1;   // all go: every role that waits for something outside the block has done so (a store in the consumers: 10 %)
       if constexpr (kGrouped) find_range();
       const int r4 = 4 * (lane & 3), tok = mt * 8 + g;
       int red = 0, uses = 0, at = b0;
@@ -470,7 +466,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         for (; red < end; ++red) {
           const int pbi = buffer_of(rrg, red);
           if (MT == 2 || (NW == 2 ? pbi >> 1 : pbi) == mine) {
-            if (!warp_wait(pfull0 + 8 * pbi, (MT == 2 || NW == 2 ? uses >> 1 : uses) & 1, abort_flag, p.status)) break;
+            if (!warp_wait(pfull0 + 8 * pbi, (MT == 2 || NW == 2 ? uses >> 1 : uses) & 1, abort_flag)) break;
             ++uses;
             float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
             if (tok < seg.rows) {
@@ -550,7 +546,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         __threadfence_system();
         asm volatile("bar.sync 3, 64;" ::: "memory");
       }
-      if (mine == 0 && lane == 0) peer_signal_tail(p.sig);
+      if (lane == 0) end_of_role([&] { if (mine == 0) peer_signal_tail(p.sig); }, abort_flag, p.status, 7u);
     }
     return;
   }
@@ -572,7 +568,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (p.sig.wait_flag != nullptr && p.sig.wait_x) {   // x is the gathered output of the previous exchange step
-    if (lane == 0) peer_wait_previous(p.sig, p.status, beat);
+    if (lane == 0) peer_wait_previous(p.sig, p.status);
     __syncwarp();
   }
   if constexpr (kGrouped) find_range();
@@ -581,7 +577,6 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
     meet();
     return;
   }
-  if (warp == 0) asm volatile("bar.arrive 5, 64;" ::: "memory");   // the scales warp may wait for stages from now on
   constexpr uint32_t kOne = is_bf16<T> ? 0x00800080u : 0x04000400u;      // one binary place of both halves
   constexpr uint32_t kOnes = is_bf16<T> ? 0x3F803F80u : 0x3C003C00u;     // (1, 1)
   constexpr float kOut = is_bf16<T> ? 0x1p69f : 1.0f;
@@ -719,7 +714,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         const uint32_t w_off = (lane & 7) * p.pitch + ((lane >> 3) & 1) * p.phase_bytes + (i0 * UG + (lane >> 4)) * 16;
         const uint32_t s_off = p.off_scales + g * p.spitch + 2 * i0, s8 = p.shalf;
         for (int rg = 0; rg < nrg; ++rg) {
-          if (!warp_wait(full0 + 8 * slot, use & 1, abort_flag, p.status)) return;
+          if (!warp_wait(full0 + 8 * slot, use & 1, abort_flag)) return;
           float out[MT][4];
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt)
@@ -793,7 +788,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
           }
           // the partial buffer has been read by its reducer
           const int pbi = buffer_of(rg, nth);
-          if (!warp_wait(pfree0 + 8 * pbi, (pphase >> pbi & 1) ^ 1, abort_flag, p.status)) return;
+          if (!warp_wait(pfree0 + 8 * pbi, (pphase >> pbi & 1) ^ 1, abort_flag)) return;
           pphase ^= 1u << pbi;
           ++nth;
           const uint32_t pa = pb_mine + (uint32_t)pbi * p.pbuf_bytes;
@@ -877,7 +872,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         const uint32_t c0 = 2 * ((2 * t) & (ng - 1)), c1 = 2 * ((2 * t + 1) & (ng - 1));   // byte offsets of the columns' groups in a chunk
         const uint32_t s_off = p.off_scales + g * p.spitch + 2 * (i0 << sh), s8 = p.shalf;
         for (int rg = 0; rg < nrg; ++rg) {
-          if (!warp_wait(full0 + 8 * slot, use & 1, abort_flag, p.status)) return;
+          if (!warp_wait(full0 + 8 * slot, use & 1, abort_flag)) return;
           float out[NT][4];
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt)
@@ -922,7 +917,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
           }
           // the partial buffer has been read by its reducer
           const int pbi = buffer_of(rg, nth);
-          if (!warp_wait(pfree0 + 8 * pbi, (pphase >> pbi & 1) ^ 1, abort_flag, p.status)) return;
+          if (!warp_wait(pfree0 + 8 * pbi, (pphase >> pbi & 1) ^ 1, abort_flag)) return;
           pphase ^= 1u << pbi;
           ++nth;
           const uint32_t pa = pb_mine + (uint32_t)pbi * p.pbuf_bytes;

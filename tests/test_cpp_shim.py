@@ -27,8 +27,8 @@ def test_shim_compiles_and_validates(tmp_path):
 
 
 @pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
-def test_a_wait_that_runs_out_is_reported_by_the_role_that_waited(tmp_path):
-    """The decode kernel's wait, on the CPU: no order in which the roles of a block end may lose the report."""
+def test_a_wait_that_runs_out_is_reported_whichever_role_ends_last(tmp_path):
+    """The waits of the decode kernel's roles and their end, on the CPU: no order in which they end may lose the report."""
     exe = str(tmp_path / "bounded_wait_check")
     subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "mlx_b200", "csrc"),
                     os.path.join(ROOT, "tests", "bounded_wait_check.cpp"), "-o", exe], check=True, capture_output=True, text=True)
