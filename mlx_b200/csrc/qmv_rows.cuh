@@ -36,8 +36,8 @@
 //              (token, group of the 128) has x in the lanes of its group and zeros in the others.  M = 1 fills one tile of 8 columns
 //              for any group size.
 //  * The consumer warps leave fp32 partial sums in shared memory; a reducer warp adds them in
-//    warp order (the result does not depend on timing), converts and stores y.  A sum that is not finite (an infinite x: the
-//    factored form cannot give the sign) is computed again from the weights themselves.
+//    warp order (the result does not depend on timing), converts and stores y.  What is not finite (an infinite x: the
+//    factored form cannot give the sign) is computed again from the weights themselves at the end, unless its token's x has a NaN.
 //  * Grouped launches (mixture-of-experts decode) walk a table of (expert, up to 8 rows) tiles: blocks take contiguous
 //    ranges of (tile, 16-row group) units, x and y rows are found through the sort's slot tables.
 #pragma once
@@ -267,20 +267,41 @@ __device__ __forceinline__ long long slot_row(const int* table, int r, int per) 
   return (long long)table[q] * per + (r - q * per);
 }
 
-// One element from the weights themselves, in fp32, by a warp.
+// One element from the weights themselves, in fp32, by a warp, until a lane's sum is a NaN.
 template <typename T, int BITS>
 __device__ __forceinline__ float exact_dot(const RowsParams& p, int which, long long row, const uint16_t* x, int lane) {
   const uint32_t* w = p.wq[which] + row * (p.row_bytes / 4);
   const uint16_t *s = p.scales[which] + row * p.groups, *b = p.biases[which] + row * p.groups;
-  const int group = p.K / p.groups;
+  const int sh = 31 - __clz(p.K / p.groups);   // (32 neighbouring k are of one group)
   float sum = 0.0f;
+#pragma unroll 1
   for (int k = lane; k < p.K; k += 32) {
-    const int gi = k / group;
+    const int gi = k >> sh;
     sum = fmaf(lo_f<T>(x[k]), fmaf((float)stream_get<BITS>(w, k), lo_f<T>(s[gi]), lo_f<T>(b[gi])), sum);
+    if (__any_sync(0xFFFFFFFFu, sum != sum)) break;
   }
 #pragma unroll
   for (int d = 16; d; d >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, d);
   return sum;
+}
+template <typename T>
+__device__ __forceinline__ bool not_finite(uint16_t v) {
+  constexpr uint16_t kExp = is_bf16<T> ? 0x7F80 : 0x7C00;
+  return (v & kExp) == kExp;
+}
+__device__ __forceinline__ float gated(float a, float b) { return __fdividef(a, 1.f + __expf(-a)) * b; }
+// Whether K values at x, a whole number of 128 on a 16-byte boundary, have a NaN among them, by a warp.
+template <typename T>
+__device__ __forceinline__ bool has_nan(const uint16_t* x, int K, int lane) {
+  constexpr uint32_t kInf = is_bf16<T> ? 0x7F807F80u : 0x7C007C00u;
+  uint32_t found = 0;
+#pragma unroll 1
+  for (int k = 8 * lane; k < K; k += 256) {
+    const uint4 v = *reinterpret_cast<const uint4*>(x + k);
+    found |= __vcmpgtu2(v.x & 0x7FFF7FFFu, kInf) | __vcmpgtu2(v.y & 0x7FFF7FFFu, kInf) | __vcmpgtu2(v.z & 0x7FFF7FFFu, kInf) |
+             __vcmpgtu2(v.w & 0x7FFF7FFFu, kInf);
+  }
+  return __any_sync(0xFFFFFFFFu, found != 0);
 }
 
 // SHAPE: units: the group size; runs: tiles of 8 columns.  MT: units: tiles of 8 tokens.
@@ -457,7 +478,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
       if constexpr (kGrouped) find_range();
       const int r4 = 4 * (lane & 3), tok = mt * 8 + g;
       int red = 0, uses = 0, at = b0;
-      bool more = !kGrouped || next_segment(at);
+      bool more = !kGrouped || next_segment(at), odd = false;   // odd: a sum of this lane's was not finite
       while (more) {
         int rph = 0, rrg = 0;
         const int nrg = seg.n * NW, end = red + nrg * p.nph;
@@ -496,22 +517,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
             if (final_phase) {
               const int row0 = seg.row0 + (NW == 2 ? rrg >> 1 : rrg) * 16, r = row0 + r4;
               const bool live = tok < seg.rows && r < row_end;
-              const bool odd = live && !(fabsf(sum.x) + fabsf(sum.y) + fabsf(sum.z) + fabsf(sum.w) < INFINITY);
-              for (uint32_t bad = __ballot_sync(0xFFFFFFFFu, odd); bad; bad &= bad - 1) {
-                const int who = __ffs(bad) - 1;
-                const long long xr = kGrouped ? slot_row(p.src_slot, seg.x0 + (who >> 2), p.per_slot) : mt * 8 + (who >> 2);
-#pragma unroll 1
-                for (int c = 0; c < 4; ++c) {
-                  const int rr = min(row0 + 4 * (who & 3) + c, p.N - 1);
-                  const float v = exact_dot<T, BITS>(p, NW == 2 ? rrg & 1 : 0, seg.base + rr, p.x + xr * p.K, lane);
-                  if (lane == who) {
-                    if (c == 0) sum.x = v;
-                    else if (c == 1) sum.y = v;
-                    else if (c == 2) sum.z = v;
-                    else sum.w = v;
-                  }
-                }
-              }
+              odd = odd || (live && !(fabsf(sum.x) + fabsf(sum.y) + fabsf(sum.z) + fabsf(sum.w) < INFINITY));
               uint2 v = make_uint2(pack_x2<T>(sum.x, sum.y), pack_x2<T>(sum.z, sum.w));
               bool store = live;
               if constexpr (W == Work::Gated) {
@@ -519,9 +525,8 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
                   gate = v;
                   store = false;
                 } else {
-                  auto silu = [](float a, float b) { return __fdividef(a, 1.f + __expf(-a)) * b; };
-                  v.x = pack_x2<T>(silu(lo_f<T>(gate.x), lo_f<T>(v.x)), silu(hi_f<T>(gate.x), hi_f<T>(v.x)));
-                  v.y = pack_x2<T>(silu(lo_f<T>(gate.y), lo_f<T>(v.y)), silu(hi_f<T>(gate.y), hi_f<T>(v.y)));
+                  v.x = pack_x2<T>(gated(lo_f<T>(gate.x), lo_f<T>(v.x)), gated(hi_f<T>(gate.x), hi_f<T>(v.x)));
+                  v.y = pack_x2<T>(gated(lo_f<T>(gate.y), lo_f<T>(v.y)), gated(hi_f<T>(gate.y), hi_f<T>(v.y)));
                 }
               }
               if (store) {
@@ -541,6 +546,48 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
           if (++rrg == nrg) { rrg = 0; ++rph; }
         }
         more = kGrouped && red == end && next_segment(at);
+      }
+      // What this warp has stored that is not finite, once more from the weights: here, where no role waits for it any more.
+      // (In the loop above one row of x with a NaN was N sums of K products that the block's other roles waited for.)
+      if (__any_sync(0xFFFFFFFFu, odd)) {
+        at = b0;
+        more = !kGrouped || next_segment(at);
+        while (more) {
+          uint32_t looked = 0, nans = 0;   // a bit per token of the warp's eight: x has been looked at, has a NaN
+          const long long y_off = (kGrouped ? slot_row(p.dst_slot, seg.x0 + min(tok, seg.rows - 1), p.per_slot) : (long long)tok) * p.ld + p.col0;
+          for (int rg = MT == 2 ? 0 : mine; rg < seg.n; rg += MT == 2 ? 1 : 2) {
+            const int row0 = seg.row0 + rg * 16;
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+              const int r = row0 + r4 + c;
+              bool again = tok < seg.rows && r < row_end;
+              if (again) again = not_finite<T>(p.y[0][y_off + r]);
+#pragma unroll 1
+              for (uint32_t bad = __ballot_sync(0xFFFFFFFFu, again); bad; bad &= bad - 1) {
+                const int who = __ffs(bad) - 1;
+                const uint32_t bit = 1u << (who >> 2);
+                const uint16_t* x = p.x + (kGrouped ? slot_row(p.src_slot, seg.x0 + (who >> 2), p.per_slot) : mt * 8 + (who >> 2)) * p.K;
+                if (!(looked & bit)) {
+                  looked |= bit;
+                  if (has_nan<T>(x, p.K, lane)) nans |= bit;
+                }
+                if (nans & bit) continue;   // a NaN, as it stands
+                const long long row = seg.base + row0 + 4 * (who & 3) + c;
+                float v = 0.0f;
+#pragma unroll 1
+                for (int i = 0; i < NW; ++i) {
+                  const float before = v;
+                  v = lo_f<T>(pack_x2<T>(exact_dot<T, BITS>(p, i, row, x, lane), 0.0f));
+                  if (i == 1) v = gated(before, v);
+                }
+                if (lane == who)
+                  for (int q = 0; q < p.n_out; ++q) p.y[q][y_off + r] = (uint16_t)pack_x2<T>(v, 0.0f);
+              }
+            }
+          }
+          more = kGrouped && next_segment(at);
+        }
+        __syncwarp();
       }
       if (p.sig.n > 0) {   // all of this block's stores to y were issued by these two warps
         __threadfence_system();

@@ -95,6 +95,72 @@ def test_infinite_and_largest_activations(dtype, top, bits, g):
     assert qmm_close(got[3:], ref, 1e-2)[0]
 
 
+@pytest.mark.parametrize("bits,g", [(4, 64), (6, 128), (2, 32)])
+@pytest.mark.parametrize("dtype", ("bf16", "f16"))
+def test_nan_costs_no_time(dtype, bits, g):
+    """A NaN in a row of x, the last element of it, leaves the launch as long as it is: nothing is computed again for what stays NaN.
+    (Every output once more from the weights is a hundred times the product; the bound is far from both.)  Other rows are as without."""
+    M, N, K = 4, 14336, 4096
+    x = torch.randn(M, K, device="cuda").to(DT[dtype])
+    w = mb.quantize((torch.randn(N, K, device="cuda") * 0.02).to(DT[dtype]), g, bits)
+    bad = x.clone()
+    bad[:3, -1] = float("nan")
+    ref, got = (mb.quantized_matmul(v, *w, group_size=g, bits=bits) for v in (x, bad))
+    assert got[:3].isnan().all() and torch.equal(got[3], ref[3])
+
+    def us(v):
+        t = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(10):
+                mb.quantized_matmul(v, *w, group_size=g, bits=bits)
+            b.record()
+            b.synchronize()
+            t.append(a.elapsed_time(b) * 100)
+        return min(t)
+
+    assert us(bad) < 8 * us(x), (us(bad), us(x))
+
+
+@pytest.mark.parametrize("bits,g", [(4, 64), (3, 64), (8, 128)])
+def test_sums_that_are_not_finite_in_several_tiles(bits, g):
+    """Infinities in some of 16 rows, which two warps sum, and in rows of a gated expert layer: each result is the weights' sign times
+    infinity, and rows without one keep their bits."""
+    M, N, K = 16, 270, 4352
+    if bits == 3:
+        M = 8
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    w = mb.quantize(torch.randn(N, K, device="cuda", dtype=torch.bfloat16) * 0.02, g, bits)
+    ref = mb.quantized_matmul(x, *w, group_size=g, bits=bits)
+    W = mb.dequantize(*w, g, bits).float()
+    rows = [1, M - 2]
+    bad = x.clone()
+    for i in rows:
+        bad[i, 300 * i] = float("-inf")
+    got = mb.quantized_matmul(bad, *w, group_size=g, bits=bits)
+    for i in range(M):
+        if i in rows:
+            sign = W[:, 300 * i]
+            assert torch.equal(got[i][sign != 0], torch.where(sign > 0, float("-inf"), float("inf")).bfloat16()[sign != 0])
+        else:
+            assert torch.equal(got[i], ref[i])
+    E = 3
+    G = torch.Generator(device="cuda").manual_seed(bits)
+    mk = lambda a, c: mb.quantize(torch.randn(E, a, c, generator=G, device="cuda", dtype=torch.bfloat16) * 0.02, g, bits)
+    gate, up = mk(256, K), mk(256, K)
+    down = mk(K, 256)
+    xe = x[:6].view(6, 1, 1, K).clone()
+    idx = torch.tensor([0, 1, 2, 0, 1, 2], device="cuda").view(6, 1)
+    ref = mb.gather_qmm_swiglu(xe, gate, up, down, idx, group_size=g, bits=bits)
+    xe[4, 0, 0, 7] = float("inf")
+    xe[2, 0, 0, 9] = float("nan")
+    got = mb.gather_qmm_swiglu(xe, gate, up, down, idx, group_size=g, bits=bits)
+    assert got[2].isnan().all() and not got[4].isfinite().any()
+    for i in (0, 1, 3, 5):
+        assert torch.equal(got[i], ref[i])
+
+
 @pytest.mark.parametrize("bits,g,K", [(3, 32, 640), (6, 64, 1152), (5, 128, 1280), (2, 32, 384), (4, 128, 1792), (8, 64, 4224)])
 @pytest.mark.parametrize("gated", (False, True))
 def test_experts(bits, g, K, gated):
