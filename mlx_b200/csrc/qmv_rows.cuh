@@ -24,7 +24,7 @@
 //    that several pairs share); the offsets' powers of two go into x.  The integer pipe, which issues at half rate, bounds the
 //    unpacking: 5 operations per 8 four-bit weights, 3 per 4 eight-bit, 9 per 16 two-bit, 26 to 34 per 32 of 3, 5 and 6 bits.
 //    To keep the products inside fp32's range whatever the magnitude of x, every token row of a
-//    warp's K slice is multiplied by a power of two that brings its largest element to about 2^64
+//    warp's K slice is multiplied by a power of two, 2^126 at most, that brings its largest element to about 2^126
 //    (less where the field sits some bits up) when it is put into registers, and the warp's sums
 //    are multiplied back by the matching power of two before they leave the warp: exact.
 //  * Scales are applied per group to fp32 group sums:  y = sum_g s_g * (sum_k x_k q_k) + sum_g b_g * (sum_k x_k).
@@ -626,13 +626,14 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
   }
   constexpr uint32_t kOne = is_bf16<T> ? 0x00800080u : 0x04000400u;      // one binary place of both halves
   constexpr uint32_t kOnes = is_bf16<T> ? 0x3F803F80u : 0x3C003C00u;     // (1, 1)
-  constexpr float kOut = is_bf16<T> ? 0x1p69f : 1.0f;
-  // x is multiplied by 2^E so that its largest element, whose bits are `m`, lands at or below 2^65 (f16: 2^15; the powers of two
-  // below that the fields ask for stay normal numbers)
+  constexpr float kOut = is_bf16<T> ? 0x1p8f : 1.0f;
+  // x is multiplied by 2^E, E up to 126, so that its largest element, whose bits are `m`, lands at or below 2^127 (f16: 2^15): with the
+  // weights' 2^-133 the sums are within 2^-7 of true units for x up to 1, and results down to the smallest numbers keep their bits.
+  // (The powers of two below that the fields ask for stay normal numbers; sums beyond fp32 end up infinite and are computed again.)
   auto exponent = [](uint32_t m) -> int {
     if constexpr (is_bf16<T>) {
-      const int E = 191 - (int)(m >> 7);
-      return E < -62 ? -62 : (E > 120 ? 120 : E);
+      const int E = 253 - (int)(m >> 7);
+      return E < -2 ? -2 : (E > 126 ? 126 : E);
     } else {
       const int E = 29 - (int)(m >> 10);
       return E < -8 ? -8 : (E > 15 ? 15 : E);
@@ -651,9 +652,9 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
     m = __vmaxu2(m, __shfl_xor_sync(0xFFFFFFFFu, m, 2));
     return max(m & 0xFFFFu, m >> 16);
   };
-  // The weights come out as field * 2^-133 (f16: 2^-24): sums are true value * 2^(E - 133).  2^(64 - E) is applied when they
-  // leave the warp, 2^69 with it (f16: 2^(24 - E)).
-  auto unscale_of = [](int E) { return __uint_as_float((uint32_t)(127 + (is_bf16<T> ? 64 : 24) - E) << 23); };
+  // The weights come out as field * 2^-133 (f16: 2^-24): sums are true value * 2^(E - 133).  2^(125 - E) is applied when they
+  // leave the warp, 2^8 with it (f16: 2^(24 - E)).
+  auto unscale_of = [](int E) { return __uint_as_float((uint32_t)(127 + (is_bf16<T> ? 125 : 24) - E) << 23); };
 
   int slot = 0, use = 0, nth = 0;
   uint32_t pphase = 0;   // per partial buffer: parity of its uses so far
@@ -671,7 +672,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
         constexpr int NGW = C::NGW, NP = C::NP, UG = C::UG, UW = C::UW, KW = C::KW;
         uint32_t X[UW][MT][NP];         // B fragments of this warp's K slice, pre-scaled
         uint32_t sx_hi[MT], sx_lo[MT];  // scaled group sums of x for groups 2t, 2t+1 of the slice (hi / lo parts)
-        float unscale[MT][2];           // per output token (2t, 2t+1 of tile mt): what brings the warp's sums back to true units / 2^69
+        float unscale[MT][2];           // per output token (2t, 2t+1 of tile mt): what brings the warp's sums back to true units / kOut
         const uint16_t* xr[MT];
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) {

@@ -95,6 +95,23 @@ def test_infinite_and_largest_activations(dtype, top, bits, g):
     assert qmm_close(got[3:], ref, 1e-2)[0]
 
 
+@pytest.mark.parametrize("bits,g", [(3, 64), (6, 32), (2, 32), (4, 64), (8, 128)])
+@pytest.mark.parametrize("x_exp,s_exp", [(0, -100), (0, -115), (60, -120), (-60, -50), (-40, 60), (100, -20), (-100, 110)])
+def test_results_of_any_magnitude(bits, g, x_exp, s_exp):
+    """Activations and weights at the ends of what bf16 holds: results that are normal numbers have the bits of the same product nearer
+    to 1, scaled by the power of two.  (The sums are kept times a power of two, which must not take them below fp32's range.)"""
+    M, N, K = 3, 70, 2304
+    G = torch.Generator(device="cuda").manual_seed(bits)
+    x = torch.randn(M, K, generator=G, device="cuda").bfloat16()
+    wq, s, b = mb.quantize(torch.randn(N, K, generator=G, device="cuda").bfloat16(), g, bits)
+    ref = mb.quantized_matmul(x, wq, s, b, group_size=g, bits=bits)
+    f = lambda t, e: torch.ldexp(t.double(), torch.tensor(e, device="cuda")).bfloat16()
+    got = mb.quantized_matmul(f(x, x_exp), wq, f(s, s_exp), f(b, s_exp), group_size=g, bits=bits)
+    want = f(ref, x_exp + s_exp)
+    # (half a unit in the last place of either, where a tie or the order of sums computed again decides)
+    assert float((got.double() - want.double()).norm() / want.double().norm()) < 2.0 ** -8
+
+
 @pytest.mark.parametrize("bits,g", [(4, 64), (6, 128), (2, 32)])
 @pytest.mark.parametrize("dtype", ("bf16", "f16"))
 def test_nan_costs_no_time(dtype, bits, g):
