@@ -208,10 +208,12 @@ bool fast_supported(int dtype, int64_t n_idx, int64_t x_batch, int64_t E, int64_
 //   3 bits, groups of 128   64 [2048, 2048] 52, 57, 68 / 62; 8 [14336, 4096] 68, 68, 89 / 100
 //   6 bits  64 [2048, 2048] 71, 77, 92 / 70 (4 rows: 69); 8 [14336, 4096] 123, 123, 147 / 118 (4 rows: 109)
 //   6 bits, groups of 32   64 [2048, 2048] 105, 125, 152 / 75; 16 [4096, 2048] gated, 2 rows 105 / 140
-// All rows on one expert, which the host cannot see: 64 [2048, 2048] at 4 bits, 256 rows 28.
+//   3 bits, groups of 64    64 [2048, 2048] 63, 68, tensor cores / 67; 8 [14336, 4096] 107, 107 / 109; 5 bits at 4 rows 108 / 126
+// How the rows fall, which the host cannot see: all on one expert, 64 [2048, 2048] at 4 bits, 256 rows 28.  Half of them on one of 8
+// [14336, 4096]: 4 to 6 rows per expert of 3 bits in groups of 64 133 to 147 against 110, 4 of 5 bits 133 / 126, 2 of 6 bits in groups
+// of 32 105 / 84; 6 of 3 bits in groups of 128 87 / 109.  The lines stay with even routing, and with the kernel that does not round.
 bool few_rows(int64_t n_rows, int64_t E, int bits, int group) {
-  const bool runs = bits == 3 || bits == 5 || bits == 6 || (bits == 2 && group == 32);
-  const int64_t most = runs && group == 32 ? 2 : (bits == 2 ? 8 : (bits == 5 || bits == 6 ? 4 : 6));
+  const int64_t most = runs_form(bits, group) && group == 32 ? 2 : (bits == 2 ? 8 : (bits == 5 || bits == 6 ? 4 : 6));
   return n_rows <= most * E;
 }
 

@@ -108,6 +108,8 @@ struct GroupedArgs {
 // The row-owning decode kernel over the experts that have rows, for tiles of up to 8 expert-sorted rows (rows_tile: 4 where
 // groups of 32 take columns of their own).  With a second matrix the result is silu(x W0^T) * (x W1^T).
 int rows_tile(int bits, int group);
+// 3, 5 and 6 bits (fields straddle words), and 2 bits in groups of 32 (half a 16-byte unit): that kernel's "runs" form.
+constexpr bool runs_form(int bits, int group) { return bits == 3 || bits == 5 || bits == 6 || (bits == 2 && group == 32); }
 struct RowsGroup {
   const void* x;            // bf16 rows of K
   const uint32_t* wq[2];    // [E, N, K*bits/32]; the second may be null

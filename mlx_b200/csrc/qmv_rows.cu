@@ -40,8 +40,6 @@ int units_groups(int bits, int group, int mt) {
 #undef B200Q_UNITS_CASE
   return 0;
 }
-// 3, 5 and 6 bits, and 2 bits in groups of 32 (half a 16-byte unit): the runs form.
-bool runs_form(int bits, int group) { return bits == 3 || bits == 5 || bits == 6 || (bits == 2 && group == 32); }
 
 // Everything that does not depend on pointers.  `tokens`: rows of x per tile; max_rg: row groups of a matrix that a block may
 // have (times two when gated); stages: row groups that it has in all, at most.
@@ -73,7 +71,7 @@ bool lay_out(RowsPlan& pl, int tokens, int64_t K, int group, int bits, int64_t m
   }
   // As many items per warp as leave room for three stages, or two large ones; with long rows fewer, in more phases.
   for (; most >= 1; --most) {
-    // phases of equal length, a warp's share in each of them the same
+    // phases as equal as whole shares of the warps allow, a share in each of them the same
     p.nph = (p.items + kConsumers * most - 1) / (kConsumers * most);
     p.phase_items = (p.items + p.nph - 1) / p.nph;
     p.cnt = (p.phase_items + kConsumers - 1) / kConsumers;
@@ -236,7 +234,7 @@ bool qmv_rows_supported(const QmmArgs& a) {
   if (a.M > 16 && a.K % (kConsumers * a.group) != 0) return false;
   const int n = passes(a);
   if (n == 1) return make_plan(a).ok;
-  if (a.peers.n > 0 || (a.K * 2) % 16 != 0) return false;
+  if (a.peers.n > 0) return false;
   return make_plan(pass_args(a, 0)).ok && make_plan(pass_args(a, n - 1)).ok;
 }
 
@@ -254,7 +252,7 @@ int qmv_rows(const QmmArgs& a, cudaStream_t st) {
   return B200Q_OK;
 }
 
-int rows_tile(int bits, int group) { return rows::runs_form(bits, group) ? rows::cmin(8, rows::run_rows(group)) : 8; }
+int rows_tile(int bits, int group) { return runs_form(bits, group) ? rows::cmin(8, rows::run_rows(group)) : 8; }
 
 bool qmv_rows_grouped_supported(const RowsGroup& a) { return rows::make_group_plan(a).ok; }
 

@@ -195,7 +195,7 @@ __host__ __device__ constexpr int field_shift(int i) {
 }
 
 // ---- runs: pair j (0..15) of a lane's 32 fields.  Fields a and b sit at bits oa and 16 + ob of the 32 bits from bit `at` on
-// (both within the 8 bits of a bf16 subnormal); near < 0: the pair is joined from two shifts instead (a at 0, b at 16).
+// (both within the 8 bits of a bf16 subnormal); joined: the pair comes from two shifts instead (a at 0, b at 16).
 struct RunPair { int a, b, at, oa, ob; bool joined; };
 template <int BITS>
 __host__ __device__ constexpr RunPair run_pair(int j) {
@@ -1033,8 +1033,9 @@ int launch_shape(const RowsPlan& pl, cudaStream_t st) {
     if (pl.work == Work::Grouped) return launch<T, BITS, RUNS, SHAPE, 1, Work::Grouped>(pl, st);
     if (pl.work == Work::Gated) return launch<T, BITS, RUNS, SHAPE, 1, Work::Gated>(pl, st);
   }
-  // runs: two tiles of tokens where the tokens themselves are more than 8
-  return pl.mt == 2 ? launch<T, BITS, RUNS, SHAPE, 2, Work::Plain>(pl, st) : launch<T, BITS, RUNS, SHAPE, 1, Work::Plain>(pl, st);
+  if constexpr (!RUNS || (SHAPE == 2 && BITS != 2))   // (runs: more than 8 tokens only in groups of 128 and two column tiles)
+    if (pl.mt == 2) return launch<T, BITS, RUNS, SHAPE, 2, Work::Plain>(pl, st);
+  return launch<T, BITS, RUNS, SHAPE, 1, Work::Plain>(pl, st);
 }
 template <typename T, int BITS>
 int launch_width(const RowsPlan& pl, cudaStream_t st) {

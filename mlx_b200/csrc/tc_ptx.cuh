@@ -74,17 +74,6 @@ __device__ __forceinline__ bool mbar_wait_hot(uint32_t bar, uint32_t parity, vol
   *abort_flag = 1;
   return false;
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  for (uint32_t i = 0; i < kSpinLimit; ++i) {
-    if (mbar_try(bar, parity)) return true;
-    if (i > 8) {
-      __nanosleep(32);
-      if ((i & 63) == 0 && *abort_flag) return false;
-    }
-  }
-  *abort_flag = 1;
-  return false;
-}
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t done;
   asm volatile(
