@@ -31,7 +31,8 @@ int sm_count() {
 }
 
 // Groups (units form) that a warp's registers hold.
-int units_groups(int bits, int group, int mt) {
+int units_groups(int bits, int group, int mt, bool wide) {
+  if (wide) return group == 64 ? UnitsCfg<2, 64, 1, true>::NGW : UnitsCfg<2, 128, 1, true>::NGW;
 #define B200Q_UNITS_CASE(BITS_, G_) \
   if (bits == BITS_ && group == G_) return mt == 2 ? UnitsCfg<BITS_, G_, 2>::NGW : UnitsCfg<BITS_, G_, 1>::NGW;
   B200Q_UNITS_CASE(2, 64) B200Q_UNITS_CASE(2, 128)
@@ -43,7 +44,8 @@ int units_groups(int bits, int group, int mt) {
 
 // Everything that does not depend on pointers.  `tokens`: rows of x per tile; max_rg: row groups of a matrix that a block may
 // have (times two when gated); stages: row groups that it has in all, at most.
-bool lay_out(RowsPlan& pl, int tokens, int64_t K, int group, int bits, int64_t max_rg, int64_t stages) {
+constexpr int64_t kWideRows = 16384;
+bool lay_out(RowsPlan& pl, int64_t rows, int tokens, int64_t K, int group, int bits, int64_t max_rg, int64_t stages) {
   RowsParams& p = pl.prm;
   if (K < 128 || K % 128 != 0 || K > (1 << 24)) return false;   // (rows of whole 16 bytes, whole groups)
   p.K = (int)K;
@@ -62,7 +64,13 @@ bool lay_out(RowsPlan& pl, int tokens, int64_t K, int group, int bits, int64_t m
     item_groups = p.ng;
   } else {
     pl.shape = group;
-    most = units_groups(bits, group, pl.mt);
+    // Us with two phases and with one (1, 4, 8 rows): groups of 128, [28672, 8192] 27.2, 27.3, 27.6 / 23.1, 24.1, 24.8; [4096, 8192] 7.4,
+    // 7.6, 8.1 / 6.8, 7.4, 8.0.  Groups of 64, [28672, 8192] 28.3, 28.4, 28.9 / 24.4, 25.8, 26.4; [4096, 8192] 7.4, 7.5, 8.2 / 7.3, 8.1,
+    // 8.8, and with rows of scales off 16-byte boundaries [14336, 8064] 23.1 to 23.8 / 25.5 to 27.4: only many aligned rows pay for the
+    // longer start.
+    pl.wide = bits == 2 && pl.mt == 1 && pl.work == Work::Plain && K > 4096 && K <= 8192 &&
+              (group == 128 || (rows >= kWideRows && K % 512 == 0));
+    most = units_groups(bits, group, pl.mt, pl.wide);
     if (most == 0) return false;
     p.ng = 1;
     p.items = p.groups;
@@ -130,7 +138,7 @@ RowsPlan make_plan(const QmmArgs& a) {
   const int nblk8 = (int)((a.N + 7) / 8);
   pl.grid = cmin(nblk8, sm_count());
   const int max_rg = ((nblk8 + pl.grid - 1) / pl.grid + 1) / 2;
-  if (!lay_out(pl, (int)a.M, a.K, a.group, a.bits, max_rg, max_rg)) return pl;
+  if (!lay_out(pl, a.N, (int)a.M, a.K, a.group, a.bits, max_rg, max_rg)) return pl;
   RowsParams& p = pl.prm;
   p.blk_each = nblk8 / pl.grid;
   p.blk_more = nblk8 % pl.grid;
@@ -166,7 +174,7 @@ RowsPlan make_group_plan(const RowsGroup& a) {
   pl.grid = (int)(units < sm_count() ? units : sm_count());
   const int64_t most = (units + pl.grid - 1) / pl.grid;
   const int tile = rows_tile(a.bits, a.group);
-  if (!lay_out(pl, tile, a.K, a.group, a.bits, (most < rgs ? most : rgs) * nw, most * nw)) return pl;
+  if (!lay_out(pl, a.N, tile, a.K, a.group, a.bits, (most < rgs ? most : rgs) * nw, most * nw)) return pl;
   RowsParams& p = pl.prm;
   p.x = (const uint16_t*)a.x;
   for (int i = 0; i < nw; ++i) {

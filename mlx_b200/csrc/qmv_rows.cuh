@@ -59,11 +59,14 @@ using tc::smem_u32;
 
 // Registers are handed out per group of four warps; the two kinds of warps re-balance their register budgets at entry.
 constexpr int kThreads = (kConsumers + 4) * 32;
-constexpr int kRegsConsumer = 104, kRegsService = 64;
+// (WIDE in groups of 64, with eight groups' sums beside 64 registers of x, wants 112 and leaves the others 32: one row through
+// [28672, 8192] 24.4 us, 27.9 with 104; in groups of 128 23.1 with 104, 24.2 with 112.)
+__host__ __device__ constexpr int regs_consumer(bool more) { return more ? 112 : 104; }
+__host__ __device__ constexpr int regs_service(bool more) { return more ? 32 : 64; }
 // setmaxnreg only moves registers inside what the block was launched with (96 per thread at this
 // block size): a request beyond that pool would wait forever.
-static_assert(kRegsConsumer * kConsumers * 32 + kRegsService * 4 * 32 <= 96 * kThreads,
-              "register budgets exceed the launch allocation");
+constexpr bool in_pool(bool more) { return regs_consumer(more) * kConsumers * 32 + regs_service(more) * 4 * 32 <= 96 * kThreads; }
+static_assert(in_pool(false) && in_pool(true), "register budgets exceed the launch allocation");
 
 template <typename T>
 constexpr bool is_bf16 = std::is_same<T, __nv_bfloat16>::value;
@@ -305,11 +308,12 @@ __device__ __forceinline__ bool has_nan(const uint16_t* x, int K, int lane) {
 }
 
 // SHAPE: units: the group size; runs: tiles of 8 columns.  MT: units: tiles of 8 tokens.
-template <typename T, int BITS, bool RUNS, int SHAPE, int MT, Work W>
+template <typename T, int BITS, bool RUNS, int SHAPE, int MT, Work W, bool WIDE>
 __global__ void __launch_bounds__(kThreads, 1)
 qmv_rows_kernel(const __grid_constant__ RowsParams p) {
   constexpr bool kGrouped = W != Work::Plain;
   constexpr int NW = W == Work::Gated ? 2 : 1;
+  constexpr bool kMoreRegs = WIDE && SHAPE == 64;
   static_assert(!kGrouped || MT == 1, "grouped tiles have up to 8 rows");
   extern __shared__ __align__(1024) unsigned char smem[];
   // header: [0, 128) "stage landed" barriers | [128, 256) "stage consumed" barriers |
@@ -359,7 +363,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
   // other warps meet it at a named barrier (id 1) only when they first need the barriers - the
   // consumers after their x values are in registers.
   if (warp >= kConsumers) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsService));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(regs_service(kMoreRegs)));
     if (warp == kConsumers) {
       if (lane < nst) {
         mbar_init(full0 + 8 * lane, 33);           // the loader's announcement and the scales warp's lanes
@@ -476,6 +480,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
       asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
       abort_flag[1] = 1;   // all go: every role that waits for something outside the block has done so (a store in the consumers: 10 %)
       if constexpr (kGrouped) find_range();
+      constexpr int kLoads = kMoreRegs ? 2 : 8;   // partial sums under way at a time
       const int r4 = 4 * (lane & 3), tok = mt * 8 + g;
       int red = 0, uses = 0, at = b0;
       bool more = !kGrouped || next_segment(at), odd = false;   // odd: a sum of this lane's was not finite
@@ -493,13 +498,13 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
             if (tok < seg.rows) {
               const unsigned char* pb = smem + p.off_pbuf + (size_t)pbi * p.pbuf_bytes + (tok * tok_pitch(W) + r4) * 4;
 #pragma unroll
-              for (int w = 0; w < kConsumers; w += 8) {   // eight independent loads, then the additions in warp order
-                float4 v[8];
+              for (int w = 0; w < kConsumers; w += kLoads) {   // independent loads, then the additions in warp order
+                float4 v[kLoads];
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
+                for (int i = 0; i < kLoads; ++i)
                   v[i] = w + i < p.n_active ? *reinterpret_cast<const float4*>(pb + (size_t)(w + i) * p.pwarp_bytes) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) { sum.x += v[i].x; sum.y += v[i].y; sum.z += v[i].z; sum.w += v[i].w; }
+                for (int i = 0; i < kLoads; ++i) { sum.x += v[i].x; sum.y += v[i].y; sum.z += v[i].z; sum.w += v[i].w; }
               }
             }
             __syncwarp();   // every lane holds its sums: the partial buffer may be written again
@@ -599,7 +604,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
   }
 
   // ================================= consumer warps ===========================================
-  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsConsumer));
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(regs_consumer(kMoreRegs)));
   auto meet = [&]() {   // before the first stage: the barriers exist from here on
     asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
   };
@@ -668,7 +673,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
       const int lim = min(p.cnt, min(p.phase_items, p.items - ph * p.phase_items) - i0);   // items that it has (may be negative)
       if constexpr (!RUNS) {
         // ---------------------------------------------------------------------- units
-        using C = UnitsCfg<BITS, SHAPE, MT>;
+        using C = UnitsCfg<BITS, SHAPE, MT, WIDE>;
         constexpr int NGW = C::NGW, NP = C::NP, UG = C::UG, UW = C::UW, KW = C::KW;
         uint32_t X[UW][MT][NP];         // B fragments of this warp's K slice, pre-scaled
         uint32_t sx_hi[MT], sx_lo[MT];  // scaled group sums of x for groups 2t, 2t+1 of the slice (hi / lo parts)
@@ -1008,9 +1013,9 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
 // B200Q_PDL=0 turns programmatic dependent launch off (plain stream order).
 bool pdl_on();
 
-template <typename T, int BITS, bool RUNS, int SHAPE, int MT, Work W>
+template <typename T, int BITS, bool RUNS, int SHAPE, int MT, Work W, bool WIDE = false>
 int launch(const RowsPlan& pl, cudaStream_t st) {
-  auto kern = qmv_rows_kernel<T, BITS, RUNS, SHAPE, MT, W>;
+  auto kern = qmv_rows_kernel<T, BITS, RUNS, SHAPE, MT, W, WIDE>;
   if (pl.smem > 48 * 1024)
     B200Q_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
   cudaLaunchConfig_t cfg = {};
@@ -1035,6 +1040,8 @@ int launch_shape(const RowsPlan& pl, cudaStream_t st) {
   }
   if constexpr (!RUNS || (SHAPE == 2 && BITS != 2))   // (runs: more than 8 tokens only in groups of 128 and two column tiles)
     if (pl.mt == 2) return launch<T, BITS, RUNS, SHAPE, 2, Work::Plain>(pl, st);
+  if constexpr (BITS == 2 && !RUNS)
+    if (pl.wide) return launch<T, BITS, RUNS, SHAPE, 1, Work::Plain, true>(pl, st);
   return launch<T, BITS, RUNS, SHAPE, 1, Work::Plain>(pl, st);
 }
 template <typename T, int BITS>

@@ -22,7 +22,9 @@ __host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 
 // Compile-time shape of one (bits, group size, token tiles) instantiation of the units form.  A "unit" is 16 packed
 // bytes of one row (what one ldmatrix row holds); lane t of a quad owns word t of every unit.
-template <int BITS, int G, int MT>
+// WIDE (2 bits, up to 8 tokens, K from 4224 to 8192): 64 registers of x, so that a phase is all of K and a row 2 KB: in phases of 4096
+// the 16 copies of 1 KB that a stage takes cost the loader more than HBM takes for them (rule and figures: lay_out).
+template <int BITS, int G, int MT, bool WIDE = false>
 struct UnitsCfg {
   static_assert(BITS == 2 || BITS == 4 || BITS == 8, "field widths of this form");
   static constexpr int GB = G * BITS / 8;                  // packed bytes of one group of one row
@@ -30,7 +32,7 @@ struct UnitsCfg {
   static constexpr int UG = GB / 16;                       // units per group
   static constexpr int KW = 32 / BITS;                     // k values per 32-bit word
   static constexpr int NP = KW / 2;                        // registers of pairs that a word unpacks to
-  static constexpr int UW = cmax(2 * UG, cmin(cmin((MT == 1 ? 32 : 64) / (MT * NP), 8 * UG), 16));   // units per warp and phase
+  static constexpr int UW = cmax(2 * UG, cmin(cmin((MT == 1 && !WIDE ? 32 : 64) / (MT * NP), 8 * UG), 16));   // units per warp and phase
   static constexpr int NGW = UW / UG;                      // groups per warp and phase
   static_assert(NGW >= 2 && NGW <= 8 && NGW % 2 == 0, "groups are processed in pairs, eight at most feed one bias MMA");
 };
@@ -79,7 +81,7 @@ struct RowsParams {
 };
 
 struct RowsPlan {
-  bool ok, runs, f16;
+  bool ok, runs, f16, wide;
   int shape;           // units: group size; runs: column tiles (1 or 2)
   int mt, grid;
   Work work;

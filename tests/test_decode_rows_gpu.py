@@ -51,6 +51,13 @@ def test_runs(dtype, bits, g, M, N, K):
 
 
 @pytest.mark.parametrize("dtype", ("bf16", "f16"))
+@pytest.mark.parametrize("M,K", [(1, 4608), (8, 8192), (3, 8192)])
+def test_two_bits_with_all_of_a_long_row_in_one_phase(dtype, M, K):
+    """Groups of 64 from 16384 output columns on; shares that end early, a last row group of one row."""
+    check(dtype, M, 16385, K, 64, 2)
+
+
+@pytest.mark.parametrize("dtype", ("bf16", "f16"))
 @pytest.mark.parametrize("M,g,bits", [(8, 64, 5), (5, 64, 3), (16, 128, 6), (9, 128, 3)])
 def test_runs_in_two_column_tiles(dtype, M, g, bits):
     check(dtype, M, 300, 2304, g, bits)
@@ -58,7 +65,7 @@ def test_runs_in_two_column_tiles(dtype, M, g, bits):
 
 @pytest.mark.parametrize("dtype", ("bf16", "f16"))
 @pytest.mark.parametrize("bits,g,K", [(4, 32, 128), (4, 64, 384), (4, 128, 1792), (4, 64, 6912), (8, 32, 256), (8, 128, 4480), (8, 64, 5248),
-                                      (2, 64, 3328), (2, 128, 384), (2, 64, 17408), (4, 128, 16768), (8, 64, 11136)])
+                                      (2, 64, 3328), (2, 128, 384), (2, 64, 17408), (2, 128, 4224), (2, 128, 8192), (4, 128, 16768), (8, 64, 11136)])
 @pytest.mark.parametrize("M,N", [(1, 9), (8, 1201), (11, 100)])
 def test_units_with_k_of_any_length(dtype, bits, g, K, M, N):
     """Fewer groups than warps, shares that end early, odd numbers of groups (scales at 2-byte addresses), several phases."""
