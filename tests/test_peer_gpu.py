@@ -182,3 +182,25 @@ def test_weights_requested_before_the_previous_kernel_has_ended(bits, g, M):
         _lib.load().b200q_set_weights_constant(0)
     ops.check_status()
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("bits,g,M,K", [(3, 64, 8, 1152), (5, 128, 16, 2304), (6, 32, 4, 640), (6, 64, 1, 4352), (2, 32, 3, 384), (4, 64, 5, 1152)])
+def test_output_and_signal_of_every_form_of_the_decode_kernel(bits, g, M, K):
+    """Columns of a wider output in three buffers at once, twice in a row with the wait for the step before inside the second launch (whose
+    flag is there): every buffer, nothing beside the columns, one signal per launch and buffer."""
+    import mlx_b200 as mb
+
+    N, N_total, col0 = 200, 328, 96
+    assert mb.qmm_kernel_name(torch.bfloat16, M, N, K, g, bits) == "qmv_rows"
+    w = quantized(N, K, g, bits, bits)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    r = OneRank(M, N_total, copies=3)
+    r.y.fill_(7)
+    ref = mb.quantized_matmul(x, *w, group_size=g, bits=bits)
+    r.product(x, w, g, bits, col0=col0)
+    r.product(x, w, g, bits, col0=col0, wait=True, wait_before_x=1)
+    r.check_status()
+    for y in r.y:
+        assert torch.equal(y[:, col0:col0 + N], ref)
+        assert (y[:, :col0] == 7).all() and (y[:, col0 + N:] == 7).all()
+    assert int(r.sync[0]) == 6 and int(r.sync[32]) == 6 and int(r.sync[64]) == 0
