@@ -781,7 +781,7 @@ qmv_rows_kernel(const __grid_constant__ RowsParams p) {
               // (a group past the row's end multiplies what is there with x registers that are zero, and with a zero scale)
               uint32_t sl2, sh2;
               auto read_scales = [&]() { sl2 = lds_u32(sa + 2 * gq); sh2 = lds_u32(sa + s8 + 2 * gq); };
-              if constexpr (BITS == 8) read_scales();   // (8 rows through [14336, 4096]: 15.2 us before the words, 16.4 after; 4 bits the other way)
+              if constexpr (BITS == 8) read_scales();   // (4 bits: after the words)
               // units iu, iu + 1 of both groups (of one unit each: both at once); a few words at a time, for registers
               constexpr int UB = UG == 1 ? 1 : 2;
 #pragma unroll
