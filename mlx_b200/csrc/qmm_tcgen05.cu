@@ -896,18 +896,19 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcPar
           // One vote and one straight line for the slot's four units: every shared-memory read is under way before it is
           // needed.  With a vote per unit, after which its words and scales were read: 512 tokens through [28672, 8192] at 3 bits 216
           // us, now 209; 57 rows through [4096, 11008] 26.6, now 24.6 (with the shorter set-up and the helpers' sums below).
-          uint32_t sv[4], bv[4], w[2][BITS], vals[16];
+          // The biases wait for their unit: four registers less (2 bits in groups of 32, 64 rows through [14336, 4096]: 27.4 -> 26.8 us,
+          // 57 rows of 4 bits 23.2 -> 23.0).
+          uint32_t sv[4], w[2][BITS], vals[16];
 #pragma unroll
           for (int un = 0; un < 4; ++un) {
             sv[un] = lds_u16(at + 2 * (un >> gsh));
-            bv[un] = lds_u16(at + 2 * (un >> gsh) + half_chunk);
           }
           load_fields<BITS>(tile, row, 0, w[0]);
           if (__all_sync(0xFFFFFFFFu, scale_has_room(sv[0]) && scale_has_room(sv[1]) && scale_has_room(sv[2]) && scale_has_room(sv[3]))) {
 #pragma unroll
             for (int un = 0; un < 4; ++un) {
               if (un < 3) load_fields<BITS>(tile, row, un + 1, w[(un + 1) & 1]);
-              dequant32_fast<BITS>(w[un & 1], sv[un], bv[un], vals);
+              dequant32_fast<BITS>(w[un & 1], sv[un], lds_u16(at + 2 * (un >> gsh) + half_chunk), vals);
               if (un == 0) {
                 if (!slot_free()) { ok = false; break; }
                 tcgen05_fence_after();
@@ -919,7 +920,7 @@ qmm_tc_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcPar
 #pragma unroll
             for (int un = 0; un < 4; ++un) {
               load_fields<BITS>(tile, row, un, w[0]);
-              dequant32_any<BITS>(w[0], sv[un], bv[un], vals);
+              dequant32_any<BITS>(w[0], sv[un], lds_u16(at + 2 * (un >> gsh) + half_chunk), vals);
               tcgen05_st_x16(t_slot + un * 16, vals);
             }
           } else {
